@@ -108,7 +108,7 @@ struct gelios_ctx {
     DBuf fA, fB, ftype, fmaster, fsosed, fcopy, fsdown;
     DBuf rtype, rM, rpstart, rpts, rkstart, rkeys, rs;
     DBuf lc, li, lo, sp_point, sp_line, sp_inc, sp_ainc, sp_fix, sp_of_point;
-    DBuf u_slot, u_cell, u_twin, u_A, u_B, u_info, u_nb, u_sd, u_sd2, flux, aux, rec, pstar, src_lo;
+    DBuf u_slot, u_cell, u_twin, u_A, u_B, u_info, u_nb, u_sd, u_sd2, s_unit, flux, aux, rec, pstar, src_lo;
     DBuf Hn, Hu, Hv, HT, ku, kv, kT, r_istoch, cback, cnext;
     // state par[2] x 5 fields, centroids [2], scratch
     DBuf state[2];
@@ -141,10 +141,10 @@ struct gelios_ctx {
     // holds only the CF_RP cells, which the other forms do not accept
     bool cen_valid = false;
     bool cen_rp_partial = false;
-    // |face centre|^(2 gamma) per face unit for the plain form; stale once
-    // the points move, the topology or gamma changes
-    DBuf upf;
-    bool upf_valid = false;
+    // the face units' geometry of the plain form (UnitGeo rows); stale once
+    // the points move, the topology or the parameters change
+    DBuf ugeo;
+    bool ugeo_valid = false;
     // Instantiated graphs of one moving-grid step, keyed by the buffers the
     // step reads (state parity and centroid buffer); dropped whenever the
     // topology or the parameters change.
@@ -304,7 +304,7 @@ extern "C" int gelios_set_params(gelios_ctx* ctx, const gelios_params* prm) {
     ctx->prm = *prm;
     ctx->d.r11_sq = sqrt_threshold(prm->R11);
     ctx->cen_valid = false;  // the cached |centroid|^(2 gamma) depends on gamma
-    ctx->upf_valid = false;
+    ctx->ugeo_valid = false;
     ctx->drop_graphs();      // the parameters are kernel arguments
     return GELIOS_OK;
 }
@@ -839,7 +839,18 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     rc |= upload(ctx->t_fstart, tb.fstart.data(), tb.fstart.size(), s);
     rc |= upload(ctx->t_faces, tb.faces.data(), tb.faces.size(), s);
     rc |= upload<double>(ctx->flux, nullptr, 5 * static_cast<size_t>(ng), s);
-    rc |= upload<double>(ctx->upf, nullptr, static_cast<size_t>(kUnitGeoRows) * u_slot.size(), s);
+    rc |= upload<double>(ctx->ugeo, nullptr, static_cast<size_t>(kUnitGeoRows + 1) * u_slot.size(), s);
+    int max_faces = 0;
+    for (int c = 0; c < nc; c++)
+        if (v->cell_type[c] != C_CENTR) max_faces = std::max(max_faces, v->gran_start[c + 1] - v->gran_start[c]);
+    {
+        std::vector<int32_t> su(ng, -1);
+        for (size_t u = 0; u < u_slot.size(); u++) {
+            su[u_slot[u]] = static_cast<int32_t>(u << 1);
+            if (u_twin[u] >= 0) su[u_twin[u]] = static_cast<int32_t>(u << 1 | 1);
+        }
+        rc |= upload(ctx->s_unit, su.data(), su.size(), s);
+    }
     rc |= upload<double>(ctx->aux, nullptr, 3 * static_cast<size_t>(nc), s);
     rc |= upload<double>(ctx->rec, nullptr, static_cast<size_t>(kRecRows) * (u_tr1 - u_tr0 + 1), s);
     rc |= upload<double>(ctx->pstar, nullptr, static_cast<size_t>(u_tr1 - u_tr0) + 1, s);
@@ -916,6 +927,8 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     d.u_sd2 = ctx->u_sd2.as<int32_t>();
     d.u_cell = ctx->u_cell.as<int32_t>();
     d.u_twin = ctx->u_twin.as<int32_t>();
+    d.s_unit = ctx->s_unit.as<int32_t>();
+    d.max_faces = max_faces;
     d.u_c1 = u_c1;
     d.u_tr0 = u_tr0;
     d.u_tr1 = u_tr1;
@@ -973,7 +986,7 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     ctx->have_mesh = true;
     ctx->n_inner = 0;
     ctx->cen_valid = false;
-    ctx->upf_valid = false;
+    ctx->ugeo_valid = false;
     ctx->drop_graphs();
     return GELIOS_OK;
 }
@@ -1405,6 +1418,16 @@ int enqueue_pipe_step(gelios_ctx* ctx, int st, const StepBuffers& b, const StepB
     return n;
 }
 
+// the cached unit geometry in the layout the context's flux precision reads
+void set_unit_geometry(const gelios_ctx* ctx, StepBuffers& b) {
+    if (ctx->prm.precision == GELIOS_PREC_FP32_FLUX) {
+        b.upf = ctx->ugeo.as<double>();
+        b.fgeo = b.upf + ctx->d.n_units;
+    } else {
+        b.ugeo = ctx->ugeo.as<double>();
+    }
+}
+
 bool pipe_ok(const gelios_ctx* ctx) {
     const int v = ctx->mk2_variant;
     return ctx->pipelined && !ctx->timing && !(v >= 4 && v < 8);
@@ -1497,10 +1520,10 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         launches++;
         ctx->cen_rp_partial = false;
     }
-    if (form == GELIOS_FORM_STATIONARY && !ctx->upf_valid && nsteps > 0) {
-        launch_unit_geometry(d, P.gamma, cen0, cen0 + ncz, ctx->upf.as<double>(), s);
+    if (form == GELIOS_FORM_STATIONARY && !ctx->ugeo_valid && nsteps > 0) {
+        launch_unit_geometry(d, P, cen0, cen0 + ncz, cen0 + 2 * ncz, ctx->ugeo.as<double>(), s);
         launches++;
-        ctx->upf_valid = true;
+        ctx->ugeo_valid = true;
     }
     int first = 0;
     if (form == GELIOS_FORM_STATIONARY && nsteps > 0 && !ctx->timing && !ctx->coop_off) {
@@ -1521,8 +1544,7 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             b.cy = cen0 + ncz;
             b.rp = cen0 + 2 * ncz;
             b.vs = cen0 + 3 * ncz;
-            b.upf = ctx->upf.as<double>();
-            b.ugeo = b.upf + d.n_units;
+            set_unit_geometry(ctx, b);
         }
         if (launch_stationary_persistent(d, P, bb[0], bb[1], ctx->flux.as<double>(), nsteps, s) == cudaSuccess) {
             launches += 1;
@@ -1618,8 +1640,7 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             b.rp = cen0 + 2 * static_cast<size_t>(d.n_cells);
             if (form == GELIOS_FORM_STATIONARY) {
                 b.vs = cen0 + 3 * static_cast<size_t>(d.n_cells);
-                b.upf = ctx->upf.as<double>();
-                b.ugeo = b.upf + d.n_units;
+                set_unit_geometry(ctx, b);
                 cudaEvent_t e1 = ctx->phase_begin();
                 launch_stationary_units(d, P, b, ctx->flux.as<double>(), s);
                 ctx->phase_end(1, e1, 1);
@@ -1647,7 +1668,7 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
     ctx->cen_valid = true;
     if (cached_form && nsteps > 0) {
         ctx->cen_rp_partial = true;
-        ctx->upf_valid = false;
+        ctx->ugeo_valid = false;
     }
     if (status) {
         Words r{};
@@ -2284,7 +2305,7 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
         c->cen_valid = true;
         if (nsteps > 0) {
             c->cen_rp_partial = true;
-            c->upf_valid = false;
+            c->ugeo_valid = false;
         }
         c->launches = launches;
     }
@@ -2520,7 +2541,7 @@ extern "C" int gelios_plain_batch_create(gelios_plain_batch** out, gelios_ctx* c
     GELIOS_CUDA_TRY(cudaSetDevice(B->device));
     GELIOS_CUDA_TRY(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking));
     if (B->inst.alloc(sizeof(PlainInstance) * n) || B->active.alloc(sizeof(int) * n) ||
-        B->resid.alloc(sizeof(double) * kResidualScratch * n))
+        B->resid.alloc(sizeof(double) * (kResidualScratch + 4) * n))
         return GELIOS_E_CUDA;
     *out = B.release();
     return GELIOS_OK;
@@ -2556,10 +2577,11 @@ int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
             c->cen_valid = true;
             c->cen_rp_partial = false;
         }
-        if (!c->upf_valid) {
+        if (!c->ugeo_valid) {
             const double* cen = c->cen[0].as<double>();
-            launch_unit_geometry(c->d, c->prm.gamma, cen, cen + c->d.n_cells, c->upf.as<double>(), B->stream);
-            c->upf_valid = true;
+            const size_t n = c->d.n_cells;
+            launch_unit_geometry(c->d, c->prm, cen, cen + n, cen + 2 * n, c->ugeo.as<double>(), B->stream);
+            c->ugeo_valid = true;
         }
         PlainInstance& I = host[i];
         I.P = c->prm;
@@ -2580,8 +2602,7 @@ int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
             b.cy = cen0 + ncz;
             b.rp = cen0 + 2 * ncz;
             b.vs = cen0 + 3 * ncz;
-            b.upf = c->upf.as<double>();
-            b.ugeo = b.upf + c->d.n_units;
+            set_unit_geometry(c, b);
         }
         I.fl = c->flux.as<double>();
     }
@@ -2640,7 +2661,7 @@ extern "C" int gelios_plain_batch_run_to_residual(gelios_plain_batch* B, double 
     std::vector<double> rpt(n, 0.0), last_dt(n, 0.0);
     std::vector<int> list(n);
     for (int i = 0; i < n; i++) list[i] = i;
-    std::vector<double> scratch(static_cast<size_t>(kResidualScratch) * n);
+    std::vector<double> got(4 * static_cast<size_t>(n));
     int64_t total = 0;
     while (!list.empty() && total < max_steps) {
         const int chunk = static_cast<int>(std::min<int64_t>(check_every, max_steps - total) & ~1);
@@ -2649,25 +2670,21 @@ extern "C" int gelios_plain_batch_run_to_residual(gelios_plain_batch* B, double 
         if (rc) return rc;
         GELIOS_CUDA_TRY(launch_stationary_batch(B->ctxs[0]->d, B->inst.as<PlainInstance>(), B->active.as<int>(),
                                                 static_cast<int>(list.size()), chunk, B->prec, B->stream));
-        for (int i : list) {
-            gelios_ctx* c = B->ctxs[i];
-            double* sc = B->resid.as<double>() + static_cast<size_t>(kResidualScratch) * i;
-            launch_residual(c->field(0, 0), c->field(1, 0), c->d.n_cells, sc, B->stream);
-        }
+        double* sums = B->resid.as<double>() + static_cast<size_t>(kResidualScratch) * n;
+        launch_residual_batch(B->inst.as<PlainInstance>(), B->active.as<int>(), static_cast<int>(list.size()),
+                              B->ctxs[0]->d.n_cells, B->resid.as<double>(), sums, B->stream);
         GELIOS_CUDA_TRY(cudaGetLastError());
-        GELIOS_CUDA_TRY(cudaMemcpyAsync(scratch.data(), B->resid.p, sizeof(double) * scratch.size(),
-                                        cudaMemcpyDeviceToHost, B->stream));
+        GELIOS_CUDA_TRY(cudaMemcpyAsync(got.data(), sums, sizeof(double) * 4 * list.size(), cudaMemcpyDeviceToHost,
+                                        B->stream));
         GELIOS_CUDA_TRY(cudaStreamSynchronize(B->stream));
         total += chunk;
         std::vector<int> keep;
-        for (int i : list) {
-            gelios_ctx* c = B->ctxs[i];
-            double T0 = 0.0;
-            int flags = 0;
-            GELIOS_CUDA_TRY(cudaMemcpy(&T0, c->T(), sizeof(double), cudaMemcpyDeviceToHost));
-            GELIOS_CUDA_TRY(cudaMemcpy(&flags, c->status(), sizeof(int), cudaMemcpyDeviceToHost));
-            const double* sc = scratch.data() + static_cast<size_t>(kResidualScratch) * i;
+        for (size_t k = 0; k < list.size(); k++) {
+            const int i = list[k];
+            const double* sc = got.data() + 4 * k;
             const double r = sc[1] > 0.0 ? sc[0] / sc[1] : 0.0;
+            const double T0 = sc[2];
+            const int flags = static_cast<int>(sc[3]);
             done[i] += chunk;
             last_dt[i] = T0;
             rpt[i] = T0 > 0.0 ? r / T0 : 0.0;

@@ -259,6 +259,80 @@ __device__ __forceinline__ double hllc_flux(double gamma, double kurant, const S
     return time;
 }
 
+// FP64 operations that the compiler may not contract or split, so that every
+// kernel that inlines an expression written with them gives the same bits.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// sqrt(gp / ro) (a sound speed, gp = gamma p) as gp rsqrt(gp ro): one
+// reciprocal square root instead of a quotient and a square root in a row
+// (within 2 ulp of them); the quotient's own form where the product is not a
+// positive normal number.
+__device__ __forceinline__ double sound_speed(double gp, double ro) {
+    const double x = __dmul_rn(gp, ro);
+    if (x > 1e-290 && x < 1e290) return __dmul_rn(gp, rsqrt(x));
+    return sqrt(gp / ro);
+}
+
+// hllc_flux of a face at rest (W = 0, metod 1, no smoothing: the plain form,
+// Setka.cpp:10484-10700), written for few operations and short chains: only
+// the side the contact selects is evaluated, the contact speed and the
+// reciprocal of its distance to the selected wave come from two independent
+// quotients, and every operation is fixed (see above), so the plain form's
+// kernels agree bit for bit.  Not for FP32 fluxes (hllc_flux).  out = mass, momentum x, y, energy, Q; returns max(|SL|, |SR|).
+template <typename TF>
+__device__ __forceinline__ double plain_flux(const gelios_params& P, const St5& L, const St5& R, double n1, double n2,
+                                             double (&out)[5]) {
+    using TW = typename WaveArith<TF>::type;
+    const double u1 = fma_rn(L.u, n1, mul_rn(L.v, n2)), v1 = fma_rn(L.u, n2, -mul_rn(L.v, n1));
+    const double u2 = fma_rn(R.u, n1, mul_rn(R.v, n2)), v2 = fma_rn(R.u, n2, -mul_rn(R.v, n1));
+    TW c;
+    if constexpr (sizeof(TW) == 8)
+        c = dmax_ref(sound_speed(mul_rn(P.gamma, L.p), L.ro), sound_speed(mul_rn(P.gamma, R.p), R.ro));
+    else
+        c = tmax<TW>(tsqrt<TW>((TW)P.gamma * (TW)L.p / (TW)L.ro), tsqrt<TW>((TW)P.gamma * (TW)R.p / (TW)R.ro));
+    const double SL = (double)((TW)dmin_ref(u1, u2) - c), SR = (double)((TW)dmax_ref(u1, u2) + c);
+    const double suL = sub_rn(SL, u1), suR = sub_rn(SR, u2);
+    const double mL = mul_rn(suL, L.ro), mR = mul_rn(suR, R.ro);
+    const double num = add_rn(sub_rn(fma_rn(mR, u2, -mul_rn(mL, u1)), R.p), L.p), den = sub_rn(mR, mL);
+    // SM = num / den; its sign (den > 0 for SL < u1, u2 < SR) picks the
+    // side, so 1 / (S - SM) = den / (S den - num) need not wait for it
+    const double SM = num / den;
+    const bool sup = SL >= 0.0 || SR <= 0.0;  // the whole fan on one side
+    const bool left = SL >= 0.0 || (!(SR <= 0.0) && (den > 0.0 ? num >= 0.0 : SM >= 0.0));
+    const double ro = left ? L.ro : R.ro, p = left ? L.p : R.p, Q = left ? L.Q : R.Q;
+    const double u = left ? u1 : u2, v = left ? v1 : v2, S = left ? SL : SR, su = left ? suL : suR;
+    const double vx = left ? L.u : R.u, vy = left ? L.v : R.v;
+    const double rg1 = 1.0 / (P.gamma - 1.0);
+    const double e = fma_rn(p, rg1, mul_rn(mul_rn(0.5, ro), fma_rn(vx, vx, mul_rn(vy, vy))));
+    double F0 = mul_rn(ro, u), F1 = fma_rn(F0, u, p), F2 = mul_rn(F0, v), F3 = mul_rn(add_rn(e, p), u),
+           F4 = mul_rn(Q, u);
+    if (!sup) {
+        if (SM >= 0.0 || SM < 0.0) {
+            const double r = den / fma_rn(S, den, -num), k = mul_rn(su, r);
+            const double roS = mul_rn(ro, k), QS = mul_rn(Q, k);
+            const double ptz = mul_rn(0.5, add_rn(fma_rn(mR, sub_rn(SM, u2), R.p), fma_rn(mL, sub_rn(SM, u1), L.p)));
+            const double ee = fma_rn(e, k, mul_rn(fma_rn(ptz, SM, -mul_rn(p, u)), r));
+            const double dro = sub_rn(roS, ro);
+            F1 = fma_rn(S, fma_rn(roS, SM, -F0), F1);
+            F0 = fma_rn(S, dro, F0);
+            F2 = fma_rn(S, mul_rn(dro, v), F2);
+            F3 = fma_rn(S, sub_rn(ee, e), F3);
+            F4 = fma_rn(S, sub_rn(QS, Q), F4);
+        } else {  // a NaN speed selects no side: zero flux, as the reference's chain of tests leaves it
+            F0 = F1 = F2 = F3 = F4 = 0.0;
+        }
+    }
+    out[0] = F0;
+    out[1] = fma_rn(n1, F1, mul_rn(n2, F2));
+    out[2] = fma_rn(n2, F1, -mul_rn(n1, F2));
+    out[3] = F3;
+    out[4] = F4;
+    return dmax_ref(fabs(SL), fabs(SR));
+}
+
 // ---------------------------------------------------------------- exact Godunov
 // Solvers::lev, Solvers.cpp:1307-1321
 __device__ __forceinline__ double lev_dev(double ga, double enI, double pI, double rI, double enII, double pII,

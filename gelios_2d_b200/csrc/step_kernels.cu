@@ -654,6 +654,10 @@ __global__ void centroid_kernel(DevMesh d, const double* __restrict__ X, const d
 // CFL candidates of the sides whose cell is updated this step into the dt
 // word.  The cell kernels then sum their slots in Grans order.
 
+// ------------------------------------------------------------------ plain form, FP32 fluxes
+// A change in the order or contraction of the operations around an FP32 flux
+// moves its result by 1e-7 (an FP64 one by 1e-16), so this form keeps its
+// kernels; the FP64 and FP32-wave-speed forms have their own below.
 // Geometry of a face unit as its owner sees it: face centre (x2, y2), unit
 // normal (n1, n2) for the end points in the owner's order, |centre|^2, the
 // face length S, and the distances owner centroid - face centre and
@@ -729,7 +733,7 @@ __device__ __forceinline__ double stationary_side(const gelios_params& P, int ft
 // compilations may contract multiply-adds differently (last-bit
 // differences, a non-inlined body costs 12% per step).
 template <typename TF>
-__device__ __forceinline__ double stationary_unit_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
+__device__ __forceinline__ double stationary32_unit_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
                                                        double* __restrict__ fl, int u) {
     double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
     const size_t ng = d.n_slots;
@@ -752,16 +756,16 @@ __device__ __forceinline__ double stationary_unit_body(const DevMesh& d, const g
                 radn = sqrt(sq(x3) + sq(y3));
             }
             FaceGeo f;
-            if (b.ugeo) {
+            if (b.fgeo) {
                 const size_t nu = d.n_units;
-                f.x2 = b.ugeo[u];
-                f.y2 = b.ugeo[nu + u];
-                f.n1 = b.ugeo[2 * nu + u];
-                f.n2 = b.ugeo[3 * nu + u];
-                f.f2 = b.ugeo[4 * nu + u];
-                f.S = b.ugeo[5 * nu + u];
-                f.dist = b.ugeo[6 * nu + u];
-                f.distn = b.ugeo[7 * nu + u];
+                f.x2 = b.fgeo[u];
+                f.y2 = b.fgeo[nu + u];
+                f.n1 = b.fgeo[2 * nu + u];
+                f.n2 = b.fgeo[3 * nu + u];
+                f.f2 = b.fgeo[4 * nu + u];
+                f.S = b.fgeo[5 * nu + u];
+                f.dist = b.fgeo[6 * nu + u];
+                f.distn = b.fgeo[7 * nu + u];
             } else {
                 const int A = d.sA[g], B = d.sB[g];
                 f = face_geo(d.X[A], d.Y[A], d.X[B], d.Y[B], x, y, nb >= 0, x3, y3);
@@ -807,17 +811,17 @@ __device__ __forceinline__ double stationary_unit_body(const DevMesh& d, const g
 }
 
 template <typename TF>
-__global__ void __launch_bounds__(128) stationary_unit_kernel(DevMesh d, gelios_params P, StepBuffers b,
+__global__ void __launch_bounds__(128) stationary32_unit_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                               double* __restrict__ fl) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
-    if (u < d.n_units) tmin_u = stationary_unit_body<TF>(d, P, b, fl, u);
+    if (u < d.n_units) tmin_u = stationary32_unit_body<TF>(d, P, b, fl, u);
     block_reduce_commit(tmin_u, 0, 0, 0, b.dt_acc, b.counters, b.status);
 }
 
 // Go_stationary cell update (Setka.cpp:5309-5341) of cell c from the summed
 // slots; folds its `time` mark and clamps into tmark, nro, npc.
-__device__ __forceinline__ void stationary_update_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
+__device__ __forceinline__ void stationary32_update_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
                                                        const double* __restrict__ fl, int c, double& tmark, int& nro,
                                                        int& npc) {
     const size_t ng = d.n_slots;
@@ -870,12 +874,12 @@ __device__ __forceinline__ void stationary_update_body(const DevMesh& d, const g
     }
 }
 
-__global__ void __launch_bounds__(128) stationary_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
+__global__ void __launch_bounds__(128) stationary32_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                                 const double* __restrict__ fl) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double tmark = __longlong_as_double(0x7ff0000000000000LL);
     int nro = 0, npc = 0;
-    if (c < d.n_cells) stationary_update_body(d, P, b, fl, c, tmark, nro, npc);
+    if (c < d.n_cells) stationary32_update_body(d, P, b, fl, c, tmark, nro, npc);
     block_reduce_commit(tmark, nro, npc, 0, b.dt_acc, b.counters, b.status);
 }
 
@@ -887,7 +891,7 @@ __global__ void __launch_bounds__(128) stationary_update_kernel(DevMesh d, gelio
 // against 29 us for three launches per step on the 180 x 120 grid.
 // bs[0] / bs[1]: the buffers of even / odd steps.
 template <typename TF>
-__global__ void __launch_bounds__(128) stationary_persistent_kernel(DevMesh d, gelios_params P, StepBuffers b0,
+__global__ void __launch_bounds__(128) stationary32_persistent_kernel(DevMesh d, gelios_params P, StepBuffers b0,
                                                                     StepBuffers b1, double* __restrict__ fl,
                                                                     int nsteps) {
     cg::grid_group grid = cg::this_grid();
@@ -896,12 +900,12 @@ __global__ void __launch_bounds__(128) stationary_persistent_kernel(DevMesh d, g
     for (int st = 0; st < nsteps; st++) {
         const StepBuffers& b = (st & 1) ? b1 : b0;
         double tmin = __longlong_as_double(0x7ff0000000000000LL);
-        for (int u = tid; u < d.n_units; u += nth) tmin = dmin_ref(tmin, stationary_unit_body<TF>(d, P, b, fl, u));
+        for (int u = tid; u < d.n_units; u += nth) tmin = dmin_ref(tmin, stationary32_unit_body<TF>(d, P, b, fl, u));
         block_reduce_commit(tmin, 0, 0, 0, b.dt_acc, b.counters, b.status);
         grid.sync();
         double tmark = __longlong_as_double(0x7ff0000000000000LL);
         int nro = 0, npc = 0;
-        for (int c = tid; c < d.n_cells; c += nth) stationary_update_body(d, P, b, fl, c, tmark, nro, npc);
+        for (int c = tid; c < d.n_cells; c += nth) stationary32_update_body(d, P, b, fl, c, tmark, nro, npc);
         block_reduce_commit(tmark, nro, npc, 0, b.dt_acc, b.counters, b.status);
         grid.sync();
         if (tid == 0) {
@@ -922,7 +926,7 @@ __global__ void __launch_bounds__(128) stationary_persistent_kernel(DevMesh d, g
 // unit and cell bodies are the one-instance kernels'.  `active` lists the
 // instances advanced by this launch (the others keep their state).
 template <typename TF>
-__global__ void __launch_bounds__(128) stationary_batch_kernel(DevMesh d, const PlainInstance* __restrict__ inst,
+__global__ void __launch_bounds__(128) stationary32_batch_kernel(DevMesh d, const PlainInstance* __restrict__ inst,
                                                                const int* __restrict__ active, int n_active,
                                                                int nsteps) {
     cg::grid_group grid = cg::this_grid();
@@ -933,7 +937,7 @@ __global__ void __launch_bounds__(128) stationary_batch_kernel(DevMesh d, const 
             const PlainInstance& I = inst[active[t / ut]];
             const int u = (t % ut) * 128 + threadIdx.x;
             double tmin = __longlong_as_double(0x7ff0000000000000LL);
-            if (u < d.n_units) tmin = stationary_unit_body<TF>(d, I.P, I.b[par], I.fl, u);
+            if (u < d.n_units) tmin = stationary32_unit_body<TF>(d, I.P, I.b[par], I.fl, u);
             __syncthreads();  // the previous tile's reduction has read its shared words
             block_reduce_commit(tmin, 0, 0, 0, I.b[par].dt_acc, I.b[par].counters, I.b[par].status);
         }
@@ -943,7 +947,7 @@ __global__ void __launch_bounds__(128) stationary_batch_kernel(DevMesh d, const 
             const int c = (t % ct) * 128 + threadIdx.x;
             double tmark = __longlong_as_double(0x7ff0000000000000LL);
             int nro = 0, npc = 0;
-            if (c < d.n_cells) stationary_update_body(d, I.P, I.b[par], I.fl, c, tmark, nro, npc);
+            if (c < d.n_cells) stationary32_update_body(d, I.P, I.b[par], I.fl, c, tmark, nro, npc);
             __syncthreads();
             block_reduce_commit(tmark, nro, npc, 0, I.b[par].dt_acc, I.b[par].counters, I.b[par].status);
         }
@@ -955,6 +959,575 @@ __global__ void __launch_bounds__(128) stationary_batch_kernel(DevMesh d, const 
             *b.dt_acc = 0x7ff0000000000000ULL;
         }
         grid.sync();
+    }
+}
+
+// ------------------------------------------------------------------ plain form
+// What a face unit of the plain form reads of the (fixed) grid: unit normal
+// (n1, n2) for the end points in the owner's order, length S, the distances
+// owner centroid - face centre and neighbour centroid - face centre, and per
+// side the radial scaling of Setka.cpp:5256-5290: kro = |centroid|^2 /
+// |centre|^2, kp = (|centroid| / |centre|)^(2 gamma), and the rotation (C, S)
+// from the polar frame of the centroid to that of the face centre
+// (polar_perenos).  flags: bit 0 the owner's evaluation is scaled (centroid
+// radius below rad_stat), bit 1 the neighbour's.  Inner-sphere faces hold
+// |centre| and the centre in kroN, CN, SN.
+struct UnitGeo {
+    double n1, n2, S, dist, distn, kroO, kpO, CO, SO, kroN, kpN, CN, SN;
+    uint32_t flags;
+};
+__device__ __forceinline__ UnitGeo unit_geo(double gamma, double rad_stat, int ft, double xa, double ya, double xb,
+                                            double yb, int K, int nb, const double* cx, const double* cy,
+                                            const double* rp) {
+    UnitGeo f;
+    const double x2 = (xa + xb) / 2.0, y2 = (ya + yb) / 2.0;
+    double t1 = xb - xa, t2 = yb - ya;  // t = B - A normalised, n = (t2, -t1): Setka.cpp:5244-5306
+    f.S = sqrt(sq(t1) + sq(t2));
+    t1 = t1 / f.S;
+    t2 = t2 / f.S;
+    f.n1 = t2;
+    f.n2 = -t1;
+    const double f2 = sq(x2) + sq(y2), pf = pow2g(sqrt(f2), 2 * gamma);
+    double cf, sf;
+    polar_cs(x2, y2, cf, sf);
+    auto side = [&](int c, double& dist, double& kro, double& kp, double& C, double& Sn) {
+        const double x = cx[c], y = cy[c];
+        dist = sqrt(sq(x - x2) + sq(y - y2));
+        kro = (sq(x) + sq(y)) / f2;
+        kp = rp[c] / pf;
+        double c1, s1;
+        polar_cs(x, y, c1, s1);
+        C = c1 * cf + s1 * sf;
+        Sn = c1 * sf - s1 * cf;
+        return sqrt(sq(x) + sq(y)) < rad_stat;
+    };
+    f.flags = side(K, f.dist, f.kroO, f.kpO, f.CO, f.SO) ? 1u : 0u;
+    f.distn = f.kroN = f.kpN = f.CN = f.SN = 0.0;
+    if (nb >= 0) {
+        f.flags |= side(nb, f.distn, f.kroN, f.kpN, f.CN, f.SN) ? 2u : 0u;
+    } else if (ft == G_INNER_SPHERE) {
+        f.kroN = sqrt(f2);
+        f.CN = x2;
+        f.SN = y2;
+    }
+    return f;
+}
+
+// Radial scaling and rotation of one side's state to the face centre.
+__device__ __forceinline__ St5 plain_scale(const St5& s, double kro, double kp, double C, double Sn) {
+    St5 o = s;
+    o.ro = mul_rn(s.ro, kro);
+    o.p = mul_rn(s.p, kp);
+    o.u = fma_rn(s.u, C, -mul_rn(s.v, Sn));
+    o.v = fma_rn(s.u, Sn, mul_rn(s.v, C));
+    return o;
+}
+// Inner-sphere state from |centre| and the centre (inner_sphere_state without
+// a sum, so that its bits do not depend on where it is inlined).
+__device__ __forceinline__ St5 plain_inner_state(const gelios_params& P, double dist, double x, double y) {
+    St5 s;
+    s.ro = 1.0 / (P.chi * P.chi * dist * dist);
+    s.p = s.ro * P.chi * P.chi / (P.gamma * P.inner_mach * P.inner_mach);
+    s.u = P.chi * x / dist;
+    s.v = P.chi * y / dist;
+    s.Q = s.ro;
+    return s;
+}
+// The two states of a boundary face as its owner sees it (Setka.cpp:5244-5306).
+__device__ __forceinline__ void plain_boundary(const gelios_params& P, int ft, const St5& own, bool scaled,
+                                               const UnitGeo& f, St5& L, St5& R) {
+    L = own;
+    R = own;
+    if (ft == G_INNER_SPHERE) {
+        L.ro = mul_rn(own.ro, f.kroO);
+        L.p = mul_rn(own.p, f.kpO);
+        R = plain_inner_state(P, f.kroN, f.CN, f.SN);
+    } else if (ft == G_INPUT) {
+        R = input_state(P);
+    } else if (ft == G_EXTERN) {
+        if (R.u >= 0.0) R.u = P.extern_u_par;
+    } else if (ft == G_AXIS) {
+        if (scaled) L.u = fma_rn(own.u, f.CO, -mul_rn(own.v, f.SO));
+        L.v = 0.0;
+        R = L;
+    }
+}
+
+// One Go_stationary face unit: slot fluxes of the owner (and of the twin)
+// and the minimum of its CFL candidates (+inf if none).
+template <typename TF>
+__device__ __forceinline__ double stationary_unit_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
+                                                       double* __restrict__ fl, int u) {
+    double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
+    const size_t ng = d.n_slots;
+    const int g = d.u_slot[u], K = d.u_cell[u], gt = d.u_twin[u];
+    // the unit-major copies of the neighbour and the flags save a level of
+    // dependent loads; the allocation-free entry has only the slots'
+    int nb;
+    uint32_t info, cfK, cfN;
+    if (d.u_info) {
+        nb = d.u_nb[u];
+        info = d.u_info[u];
+        cfK = info >> UI_CF_OWN;
+        cfN = info >> UI_CF_NB;
+    } else {
+        nb = gt >= 0 ? d.snb[g] : -1;
+        info = d.sinfo[g];
+        cfK = d.cflags[K];
+        cfN = nb >= 0 ? d.cflags[nb] : 0u;
+    }
+    const bool procK = !(cfK & CF_CENTR);
+    const bool procN = nb >= 0 && !(cfN & CF_CENTR);
+    if (!(procK || procN)) return tmin_u;
+    const int ft = info & SI_TYPE_MASK;
+    const St5 own = load_state(b.cur, K);
+    St5 nbs = own;
+    if (nb >= 0) nbs = load_state(b.cur, nb);
+    UnitGeo f;
+    if (b.ugeo) {
+        const size_t nu = d.n_units;
+        const double* r = b.ugeo + u;
+        f.flags = reinterpret_cast<const uint32_t*>(b.ugeo + kUnitGeoRows * nu)[u];
+        f.n1 = r[0];
+        f.n2 = r[nu];
+        f.S = r[2 * nu];
+        f.dist = r[3 * nu];
+        f.distn = r[4 * nu];
+        if (f.flags || ft != G_USUALY) {
+            f.kroO = r[5 * nu];
+            f.kpO = r[6 * nu];
+            f.CO = r[7 * nu];
+            f.SO = r[8 * nu];
+            f.kroN = r[9 * nu];
+            f.kpN = r[10 * nu];
+            f.CN = r[11 * nu];
+            f.SN = r[12 * nu];
+        }
+    } else {
+        const int A = d.sA[g], B = d.sB[g];
+        f = unit_geo(P.gamma, P.rad_stat, ft, d.X[A], d.Y[A], d.X[B], d.Y[B], K, nb, b.cx, b.cy, b.rp);
+    }
+    double F[5];
+    if (ft != G_USUALY) {
+        St5 L, R;
+        plain_boundary(P, ft, own, f.flags & 1u, f, L, R);
+        const double UU = plain_flux<TF>(P, L, R, f.n1, f.n2, F);
+#pragma unroll
+        for (int k = 0; k < 5; k++) fl[k * ng + g] = mul_rn(F[k], f.S);
+        return procK ? dmin_ref(tmin_u, mul_rn(P.kurant, f.dist) / UU) : tmin_u;
+    }
+    St5 L = own, R = nbs;
+    if (f.flags & 1u) {
+        L = plain_scale(own, f.kroO, f.kpO, f.CO, f.SO);
+        R = plain_scale(nbs, f.kroN, f.kpN, f.CN, f.SN);
+    }
+    double UU = plain_flux<TF>(P, L, R, f.n1, f.n2, F);
+#pragma unroll
+    for (int k = 0; k < 5; k++) fl[k * ng + g] = mul_rn(F[k], f.S);
+    // CFL candidates; a NaN one is none, as the reference's std::min leaves it
+    if (procK) tmin_u = dmin_ref(tmin_u, mul_rn(P.kurant, f.dist) / UU);
+    if (gt < 0) return tmin_u;
+    double sg = -f.S;
+    // the twin's evaluation mirrors this one unless the radial scaling
+    // switches at rad_stat between the two cells
+    if (f.flags == 1u || f.flags == 2u) {
+        L = nbs;
+        R = own;
+        if (f.flags & 2u) {
+            L = plain_scale(nbs, f.kroN, f.kpN, f.CN, f.SN);
+            R = plain_scale(own, f.kroO, f.kpO, f.CO, f.SO);
+        }
+        UU = plain_flux<TF>(P, L, R, -f.n1, -f.n2, F);
+        sg = f.S;
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++) fl[k * ng + gt] = mul_rn(F[k], sg);
+    if (procN) tmin_u = dmin_ref(tmin_u, mul_rn(P.kurant, f.distn) / UU);
+    return tmin_u;
+}
+
+template <typename TF>
+__global__ void __launch_bounds__(128) stationary_unit_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                              double* __restrict__ fl) {
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
+    if (u < d.n_units) tmin_u = stationary_unit_body<TF>(d, P, b, fl, u);
+    block_reduce_commit(tmin_u, 0, 0, 0, b.dt_acc, b.counters, b.status);
+}
+
+// Go_stationary update (Setka.cpp:5309-5341) of a cell from its summed
+// fluxes; rV, ry: reciprocals of its area and of its centroid's y.
+__device__ __forceinline__ St5 plain_update(const gelios_params& P, const St5& s, const double (&Pt)[5], double dt,
+                                            double rV, double ry, int& nro, int& npc) {
+    const double gm1 = P.gamma - 1, rg1 = 1.0 / gm1, ndt = -dt;
+    const double roy = mul_rn(mul_rn(s.ro, s.v), ry);
+    St5 o;
+    o.ro = fma_rn(ndt, fma_rn(Pt[0], rV, roy), s.ro);
+    o.Q = fma_rn(ndt, fma_rn(Pt[4], rV, mul_rn(mul_rn(s.Q, s.v), ry)), s.Q);
+    if (o.ro <= 0) {
+        o.ro = P.ro_floor;
+        nro++;
+    }
+    const double rro = 1.0 / o.ro;
+    o.u = mul_rn(fma_rn(ndt, fma_rn(Pt[1], rV, mul_rn(roy, s.u)), mul_rn(s.ro, s.u)), rro);
+    o.v = mul_rn(fma_rn(ndt, fma_rn(Pt[2], rV, mul_rn(roy, s.v)), mul_rn(s.ro, s.v)), rro);
+    const double ek = mul_rn(mul_rn(0.5, s.ro), fma_rn(s.u, s.u, mul_rn(s.v, s.v)));
+    const double E = fma_rn(s.p, rg1, ek), H = fma_rn(mul_rn(P.gamma, s.p), rg1, ek);
+    const double E3 = fma_rn(ndt, fma_rn(Pt[3], rV, mul_rn(mul_rn(s.v, H), ry)), E);
+    o.p = mul_rn(sub_rn(E3, mul_rn(mul_rn(0.5, o.ro), fma_rn(o.u, o.u, mul_rn(o.v, o.v)))), gm1);
+    if (o.p <= 0) {
+        o.p = P.p_floor;
+        npc++;
+    }
+    return o;
+}
+
+// The update of cell c from its slots; folds its `time` mark and clamps into
+// tmark, nro, npc.
+__device__ __forceinline__ void stationary_update_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
+                                                       const double* __restrict__ fl, int c, double dt, double& tmark,
+                                                       int& nro, int& npc) {
+    const size_t ng = d.n_slots;
+    if (!(d.cflags[c] & CF_CENTR)) {
+        tmark = dmin_ref(tmark, 10000000.0);  // `time` starts at 1e7 in every step (Setka.cpp:5222)
+        const St5 par1 = load_state(b.cur, c);
+        const double y = b.cy[c];
+        const int g0 = d.gstart[c], g1 = d.gstart[c + 1];
+        double Pt[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (g1 - g0 == 4) {  // quadrilaterals: all slot loads in flight together
+            double a[5][4];
+#pragma unroll
+            for (int k = 0; k < 5; k++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) a[k][j] = fl[k * ng + g0 + j];
+#pragma unroll
+            for (int k = 0; k < 5; k++) Pt[k] = (((Pt[k] + a[k][0]) + a[k][1]) + a[k][2]) + a[k][3];
+        } else {
+            for (int g = g0; g < g1; g++)
+#pragma unroll
+                for (int k = 0; k < 5; k++) Pt[k] = Pt[k] + fl[k * ng + g];
+        }
+        // the cell's area: cached with the centroids (the plain grid does not
+        // move), or computed here when no cache is given
+        double Volume;
+        if (b.vs) {
+            Volume = b.vs[c];
+        } else {
+            const int s0 = d.cstart[c], n = d.cstart[c + 1] - s0;
+            Volume = area(d.contour + s0, n, d.sA, d.sB, g0, g1, d.X, d.Y, false);
+        }
+        const St5 o = plain_update(P, par1, Pt, dt, 1.0 / Volume, 1.0 / y, nro, npc);
+        b.nxt[0][c] = o.ro;
+        b.nxt[1][c] = o.p;
+        b.nxt[2][c] = o.u;
+        b.nxt[3][c] = o.v;
+        b.nxt[4][c] = o.Q;
+    }
+}
+
+__global__ void __launch_bounds__(128) stationary_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                                const double* __restrict__ fl) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    double tmark = __longlong_as_double(0x7ff0000000000000LL);
+    int nro = 0, npc = 0;
+    if (c < d.n_cells) stationary_update_body(d, P, b, fl, c, *b.dt_cur, tmark, nro, npc);
+    block_reduce_commit(tmark, nro, npc, 0, b.dt_acc, b.counters, b.status);
+}
+
+// Minimum over a warp / block of doubles that are not NaN and not negative.
+// Such doubles order as their bit patterns: two 32-bit warp reductions.
+// The block's minimum is valid in every lane of warp 0; sm: a word per warp.
+__device__ __forceinline__ double warp_min_nonneg(double t) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(t)), lo = static_cast<unsigned>(__double2loint(t));
+    const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? lo : 0xffffffffu);
+    return __hiloint2double(static_cast<int>(mh), static_cast<int>(ml));
+}
+__device__ __forceinline__ double block_min_nonneg(double t, double* sm) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    t = warp_min_nonneg(t);
+    if (lane == 0) sm[wid] = t;
+    __syncthreads();
+    if (wid == 0) t = warp_min_nonneg(lane < nw ? sm[lane] : __longlong_as_double(0x7ff0000000000000LL));
+    return t;
+}
+// CFL candidates in [0, inf): a NaN or negative one (a failed state) is none,
+// as block_reduce_commit has it for a block's minimum.
+__device__ __forceinline__ double dt_candidate(double t) {
+    return t >= 0.0 ? t : __longlong_as_double(0x7ff0000000000000LL);
+}
+// The CFL accumulator of step st of a one-launch call: three in turn, each
+// read after the step's grid barrier and re-armed a step later, when no block
+// can still be reading it (words_init_kernel arms them at the start).
+__device__ __forceinline__ unsigned long long* plain_acc(unsigned long long* acc, int st) {
+    const int k = st % 3;
+    return acc + (k ? 3 + k : 0);
+}
+// T[now2]: the accumulated minimum, 1e8 where no cell took part
+__device__ __forceinline__ double plain_dt(unsigned long long a) {
+    return (a == 0x7ff0000000000000ULL) ? 100000000.0 : __longlong_as_double(static_cast<long long>(a));
+}
+
+// `nsteps` Go_stationary steps in one cooperative launch: every block
+// strides over the face units, then (grid barrier) over the cells (barrier).
+// The CFL minimum of a step is complete at its first barrier, where every
+// block reads the next dt.  Taken by grids that stationary_lanes_kernel does
+// not hold.  b0 / b1: the buffers of even / odd steps.
+template <typename TF>
+__global__ void __launch_bounds__(128) stationary_persistent_kernel(DevMesh d, gelios_params P, StepBuffers b0,
+                                                                    StepBuffers b1, double* __restrict__ fl,
+                                                                    int nsteps) {
+    __shared__ double sm[32];
+    cg::grid_group grid = cg::this_grid();
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nth = gridDim.x * blockDim.x;
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    double dt = *b0.dt_cur, dt_prev = dt, tmark = inf;
+    int nro = 0, npc = 0;
+    // `time` starts at 1e7 in every step (Setka.cpp:5222) with a cell to update
+    bool any = false;
+    for (int c = tid; c < d.n_cells; c += nth) any |= !(d.cflags[c] & CF_CENTR);
+    for (int st = 0; st < nsteps; st++) {
+        const StepBuffers& b = (st & 1) ? b1 : b0;
+        double t = any ? 10000000.0 : inf;
+        for (int u = tid; u < d.n_units; u += nth)
+            t = dmin_ref(t, dt_candidate(stationary_unit_body<TF>(d, P, b, fl, u)));
+        unsigned long long* acc = plain_acc(b0.dt_acc, st);
+        t = block_min_nonneg(t, sm);
+        if (threadIdx.x == 0 && t < inf) atomicMin(acc, static_cast<unsigned long long>(__double_as_longlong(t)));
+        grid.sync();
+        const unsigned long long a = __ldcg(acc);
+        if (tid == 0) *plain_acc(b0.dt_acc, st + 2) = 0x7ff0000000000000ULL;
+        for (int c = tid; c < d.n_cells; c += nth) stationary_update_body(d, P, b, fl, c, dt, tmark, nro, npc);
+        dt_prev = dt;
+        dt = plain_dt(a);
+        grid.sync();
+    }
+    if (nro) atomicAdd(&b0.counters[0], static_cast<unsigned long long>(nro));
+    if (npc) atomicAdd(&b0.counters[1], static_cast<unsigned long long>(npc));
+    if (tid == 0) {
+        const StepBuffers& b = ((nsteps - 1) & 1) ? b1 : b0;
+        *b.dt_next = dt;
+        *const_cast<double*>(b.dt_cur) = dt_prev;
+    }
+}
+
+// The same with four lanes per cell, one per face, for grids whose 4 n_cells
+// lanes are resident at once and whose updated cells have at most four faces
+// (plain_lane_threads).  What a face needs of the fixed grid is read once per
+// call and stays in the lane's registers, as does the cell's own state; a
+// step loads the neighbour's five values, evaluates the face, adds the four
+// fluxes in Grans order by shuffles and updates the cell: no flux slots and
+// ONE grid barrier per step.  An interior face is evaluated by both its
+// cells with the same operands (in the main face's orientation), so the
+// results are those of the two-phase kernel.
+// Bound by latency (the gather from L2, the chain of the HLLC flux, the
+// barrier).  180 x 120 cells: 18.2 us per step in two phases with three grid
+// barriers, 5.0 us here; 77 x 45 cells: 17.3 and 3.9 us.
+constexpr int kLaneThreads = 640;
+template <typename TF>
+__global__ void __launch_bounds__(kLaneThreads, 1) stationary_lanes_kernel(DevMesh d, gelios_params P, StepBuffers b0,
+                                                                           StepBuffers b1, int nsteps) {
+    __shared__ double sm[32];
+    cg::grid_group grid = cg::this_grid();
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = tid >> 2, j = tid & 3, q0 = threadIdx.x & 28;
+    const unsigned full = 0xffffffffu;
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    const bool act = c < d.n_cells && !(d.cflags[c] & CF_CENTR);
+    double ry = 0.0, rV = 0.0, kd = 0.0;
+    UnitGeo f{};
+    St5 own{1.0, 1.0, 0.0, 0.0, 1.0}, bnd{};
+    int nbc = -1, ft = -1;
+    bool scaled = false, swap = false;
+    if (act) {
+        ry = 1.0 / b0.cy[c];
+        rV = 1.0 / b0.vs[c];
+        own = load_state(b0.cur, c);
+        const int g = d.gstart[c] + j;
+        if (g < d.gstart[c + 1]) {
+            const int su = d.s_unit[g], u = su >> 1;
+            const bool twin = su & 1;
+            const size_t nu = d.n_units;
+            const double* r = b0.ugeo + u;
+            ft = d.sinfo[g] & SI_TYPE_MASK;
+            nbc = twin ? d.u_cell[u] : d.u_nb[u];
+            f.flags = reinterpret_cast<const uint32_t*>(b0.ugeo + kUnitGeoRows * nu)[u];
+            f.n1 = r[0];
+            f.n2 = r[nu];
+            f.S = r[2 * nu];
+            kd = mul_rn(P.kurant, r[(twin ? 4 : 3) * nu]);
+            f.kroO = r[5 * nu];
+            f.kpO = r[6 * nu];
+            f.CO = r[7 * nu];
+            f.SO = r[8 * nu];
+            f.kroN = r[9 * nu];
+            f.kpN = r[10 * nu];
+            f.CN = r[11 * nu];
+            f.SN = r[12 * nu];
+            scaled = f.flags & (twin ? 2u : 1u);
+            // the twin evaluates the face as the main face's owner does,
+            // unless the radial scaling switches between the two cells
+            const bool same = f.flags == 0u || f.flags == 3u;
+            swap = twin && same;
+            if (twin && !same) {
+                f.n1 = -f.n1;
+                f.n2 = -f.n2;
+            }
+            if (ft == G_USUALY) {
+                if (twin) {  // own side first
+                    double w = f.kroO; f.kroO = f.kroN; f.kroN = w;
+                    w = f.kpO; f.kpO = f.kpN; f.kpN = w;
+                    w = f.CO; f.CO = f.CN; f.CN = w;
+                    w = f.SO; f.SO = f.SN; f.SN = w;
+                }
+            } else {
+                St5 L;
+                plain_boundary(P, ft, own, scaled, f, L, bnd);  // the constant state of Inner_sphere / Input
+                f.kroN = bnd.ro;
+                f.kpN = bnd.p;
+                f.CN = bnd.u;
+                f.SN = bnd.v;
+                f.distn = bnd.Q;
+            }
+        }
+    }
+    const double sg = swap ? -f.S : f.S;
+    double dt = *b0.dt_cur, dt_prev = dt;
+    int nro = 0, npc = 0;
+    for (int st = 0; st < nsteps; st++) {
+        const StepBuffers& b = (st & 1) ? b1 : b0;
+        double F[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        double t = act ? 10000000.0 : inf;  // `time` of Setka.cpp:5222
+        if (ft >= 0) {
+            St5 L = own, R;
+            if (ft == G_USUALY) {
+                R.ro = __ldcg(b.cur[0] + nbc);
+                R.p = __ldcg(b.cur[1] + nbc);
+                R.u = __ldcg(b.cur[2] + nbc);
+                R.v = __ldcg(b.cur[3] + nbc);
+                R.Q = __ldcg(b.cur[4] + nbc);
+                if (scaled) {
+                    L = plain_scale(L, f.kroO, f.kpO, f.CO, f.SO);
+                    R = plain_scale(R, f.kroN, f.kpN, f.CN, f.SN);
+                }
+                if (swap) {
+                    const St5 w = L;
+                    L = R;
+                    R = w;
+                }
+            } else if (ft == G_INNER_SPHERE || ft == G_INPUT) {
+                if (ft == G_INNER_SPHERE) {
+                    L.ro = mul_rn(L.ro, f.kroO);
+                    L.p = mul_rn(L.p, f.kpO);
+                }
+                R = St5{f.kroN, f.kpN, f.CN, f.SN, f.distn};
+            } else {
+                plain_boundary(P, ft, own, scaled, f, L, R);
+            }
+            const double UU = plain_flux<TF>(P, L, R, f.n1, f.n2, F);
+#pragma unroll
+            for (int k = 0; k < 5; k++) F[k] = mul_rn(F[k], sg);
+            t = dmin_ref(t, dt_candidate(kd / UU));
+        }
+        // the cell's slots in Grans order (a face that is not there adds 0)
+        double Pt[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int k = 0; k < 5; k++) Pt[k] = Pt[k] + __shfl_sync(full, F[k], q0 + i);
+        if (act) {
+            int ro1 = 0, p1 = 0;
+            own = plain_update(P, own, Pt, dt, rV, ry, ro1, p1);
+            if (j == 0) {
+                nro += ro1;
+                npc += p1;
+                b.nxt[0][c] = own.ro;
+                b.nxt[4][c] = own.Q;
+            } else {
+                b.nxt[j][c] = j == 1 ? own.p : j == 2 ? own.u : own.v;
+            }
+        }
+        unsigned long long* acc = plain_acc(b0.dt_acc, st);
+        t = block_min_nonneg(t, sm);
+        if (threadIdx.x == 0 && t < inf) atomicMin(acc, static_cast<unsigned long long>(__double_as_longlong(t)));
+        grid.sync();
+        dt_prev = dt;
+        dt = plain_dt(__ldcg(acc));
+        if (tid == 0) *plain_acc(b0.dt_acc, st + 2) = 0x7ff0000000000000ULL;
+    }
+    if (nro) atomicAdd(&b0.counters[0], static_cast<unsigned long long>(nro));
+    if (npc) atomicAdd(&b0.counters[1], static_cast<unsigned long long>(npc));
+    if (tid == 0) {
+        const StepBuffers& b = ((nsteps - 1) & 1) ? b1 : b0;
+        *b.dt_next = dt;
+        *const_cast<double*>(b.dt_cur) = dt_prev;
+    }
+}
+
+// `nsteps` Go_stationary steps of many instances in one launch.  The
+// instances share the mesh (topology and geometry) and have their own
+// parameters (inflow and inner-wind states), state buffers, flux slots and
+// dt words, and never exchange data: one thread-block cluster advances one
+// instance, the phases of a step separated by cluster barriers, and the CFL
+// minimum goes from block to block through distributed shared memory (no
+// atomics, no dt words inside the call).  A block owns a contiguous chunk of
+// the instance's units and cells; the cluster is the largest at which every
+// instance is resident (launch_stationary_batch).  `active` lists the
+// instances advanced by this launch (the others keep their state).
+// Bound by the latency of the unit and cell bodies at 16 warps per SM.  With
+// one grid of blocks for all instances and three grid barriers per step, 32
+// instances of 90 x 60 cells took 72.8 us per step, here 33; 60: 167 and 69;
+// 16 of 60 x 40 cells: 35.5 and 17.5; one of 90 x 60: 14.9 and 14.6.  256
+// threads at 128 registers: 512 x 1 block per SM measured 2% slower, 256
+// threads at 80 or 64 registers 26-40% (spills), 384 at 80 15%.
+constexpr int kClusterThreads = 256, kClusterMax = 16;
+template <typename TF>
+__global__ void __launch_bounds__(kClusterThreads, 2)
+    stationary_cluster_kernel(DevMesh d, const PlainInstance* __restrict__ inst, const int* __restrict__ active,
+                              int nsteps) {
+    __shared__ PlainInstance I;
+    __shared__ double sm[32];
+    __shared__ double mins[kClusterMax];  // the CFL minimum of every block of the cluster, written by that block
+    cg::cluster_group cl = cg::this_cluster();
+    const int nb = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
+    {
+        static_assert(sizeof(PlainInstance) % 8 == 0, "copied as 8-byte words");
+        const unsigned long long* s8 = reinterpret_cast<const unsigned long long*>(inst + active[blockIdx.x / nb]);
+        unsigned long long* d8 = reinterpret_cast<unsigned long long*>(&I);
+        for (int i = threadIdx.x; i < static_cast<int>(sizeof(PlainInstance) / 8); i += blockDim.x) d8[i] = s8[i];
+    }
+    cl.sync();  // the descriptor is in; every block of the cluster runs before one writes into another's memory
+    auto cut = [&](int n, int r) { return static_cast<int>(static_cast<long long>(n) * r / nb); };
+    const int u0 = cut(d.n_units, rank), u1 = cut(d.n_units, rank + 1);
+    const int c0 = cut(d.n_cells, rank), c1 = cut(d.n_cells, rank + 1);
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    bool any = false;
+    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) any |= !(d.cflags[c] & CF_CENTR);
+    double dt = *I.b[0].dt_cur, dt_prev = dt, tmark = inf;
+    int nro = 0, npc = 0;
+    for (int st = 0; st < nsteps; st++) {
+        const StepBuffers& b = I.b[st & 1];
+        double t = any ? 10000000.0 : inf;  // `time` of Setka.cpp:5222
+        for (int u = u0 + threadIdx.x; u < u1; u += blockDim.x)
+            t = dmin_ref(t, dt_candidate(stationary_unit_body<TF>(d, I.P, b, I.fl, u)));
+        t = block_min_nonneg(t, sm);
+        if (threadIdx.x < nb) *cl.map_shared_rank(&mins[rank], threadIdx.x) = t;
+        cl.sync();
+        double m = mins[0];
+        for (int k = 1; k < nb; k++) m = dmin_ref(m, mins[k]);
+        for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x)
+            stationary_update_body(d, I.P, b, I.fl, c, dt, tmark, nro, npc);
+        dt_prev = dt;
+        dt = (m == inf) ? 100000000.0 : m;
+        cl.sync();
+    }
+    if (nro) atomicAdd(&I.b[0].counters[0], static_cast<unsigned long long>(nro));
+    if (npc) atomicAdd(&I.b[0].counters[1], static_cast<unsigned long long>(npc));
+    if (rank == 0 && threadIdx.x == 0) {
+        const StepBuffers& b = I.b[(nsteps - 1) & 1];
+        *b.dt_next = dt;
+        *const_cast<double*>(b.dt_cur) = dt_prev;
     }
 }
 
@@ -3622,7 +4195,7 @@ __global__ void __launch_bounds__(128, GELIOS_BATCH_FACE_MINB) batch_mhd_persist
 
 // The dt / status words a call starts from: T[0] = T[1] = dt0, an empty CFL
 // accumulator, zero clamp counters and status (layout: T[2], acc,
-// counters[2], status).  A kernel rather than a copy from host memory: a
+// counters[2], status, two more accumulators at byte 48).  A kernel rather than a copy from host memory: a
 // copy from pageable memory would wait for the stream to drain.
 __global__ void words_init_kernel(unsigned char* w, double dt0) {
     double* T = reinterpret_cast<double*>(w);
@@ -3633,6 +4206,8 @@ __global__ void words_init_kernel(unsigned char* w, double dt0) {
     u[1] = 0;
     u[2] = 0;
     *reinterpret_cast<int*>(w + 40) = 0;
+    u[4] = 0x7ff0000000000000ULL;  // the plain form's second and third accumulators
+    u[5] = 0x7ff0000000000000ULL;
 }
 __global__ void batch_words_init_kernel(BatchTables t, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3651,9 +4226,8 @@ __global__ void batch_words_init_kernel(BatchTables t, int n) {
 // L1 change of one state row between the two buffers: per block the sums
 // of |a - b| and |a| in a fixed order, then one block adds the partials in
 // block order (deterministic, no atomics).
-__global__ void __launch_bounds__(256) residual_partial_kernel(const double* __restrict__ a,
-                                                               const double* __restrict__ b, int n,
-                                                               double* __restrict__ part) {
+__device__ __forceinline__ void residual_partial_body(const double* __restrict__ a, const double* __restrict__ b,
+                                                      int n, double* __restrict__ part) {
     __shared__ double sd[256], sa[256];
     double dsum = 0.0, asum = 0.0;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
@@ -3675,7 +4249,7 @@ __global__ void __launch_bounds__(256) residual_partial_kernel(const double* __r
         part[2 * blockIdx.x + 1] = sa[0];
     }
 }
-__global__ void residual_final_kernel(const double* __restrict__ part, int nb, double* __restrict__ out) {
+__device__ __forceinline__ void residual_final_body(const double* __restrict__ part, int nb, double* __restrict__ out) {
     double d = 0.0, s = 0.0;
     for (int k = 0; k < nb; k++) {
         d += part[2 * k];
@@ -3683,6 +4257,32 @@ __global__ void residual_final_kernel(const double* __restrict__ part, int nb, d
     }
     out[0] = d;
     out[1] = s;
+}
+__global__ void __launch_bounds__(256) residual_partial_kernel(const double* __restrict__ a,
+                                                               const double* __restrict__ b, int n,
+                                                               double* __restrict__ part) {
+    residual_partial_body(a, b, n, part);
+}
+__global__ void residual_final_kernel(const double* __restrict__ part, int nb, double* __restrict__ out) {
+    residual_final_body(part, nb, out);
+}
+// The density residual of the active instances of a plain batch after an
+// even number of steps, blockIdx.y the instance: the sums of
+// residual_partial_kernel / residual_final_kernel per instance, gathered
+// with its dt and status flags into four doubles for one read-back.
+__global__ void __launch_bounds__(256) residual_batch_partial_kernel(const PlainInstance* __restrict__ inst,
+                                                                     const int* __restrict__ active, int n,
+                                                                     double* __restrict__ part) {
+    const PlainInstance& I = inst[active[blockIdx.y]];
+    residual_partial_body(I.b[0].cur[0], I.b[1].cur[0], n, part + static_cast<size_t>(kResidualScratch) * blockIdx.y);
+}
+__global__ void residual_batch_final_kernel(const PlainInstance* __restrict__ inst, const int* __restrict__ active,
+                                            int nb, const double* __restrict__ part, double* __restrict__ out) {
+    const PlainInstance& I = inst[active[blockIdx.x]];
+    double* o = out + 4 * static_cast<size_t>(blockIdx.x);
+    residual_final_body(part + static_cast<size_t>(kResidualScratch) * blockIdx.x, nb, o);
+    o[2] = *I.b[0].dt_cur;
+    o[3] = static_cast<double>(*I.b[0].status);
 }
 
 // ------------------------------------------------------------------ launchers
@@ -3698,7 +4298,7 @@ void launch_centroid(const DevMesh& d, const double* X, const double* Y, double*
 void launch_stationary_units(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* fl,
                              cudaStream_t s) {
     if (P.precision == GELIOS_PREC_FP32_FLUX)
-        stationary_unit_kernel<float><<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, P, b, fl);
+        stationary32_unit_kernel<float><<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, P, b, fl);
     else if (P.precision == GELIOS_PREC_FP32_WAVES)
         stationary_unit_kernel<WaveF32><<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, P, b, fl);
     else
@@ -3706,32 +4306,56 @@ void launch_stationary_units(const DevMesh& d, const gelios_params& P, const Ste
 }
 void launch_stationary_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
                               cudaStream_t s) {
-    stationary_update_kernel<<<blocks_for(d.n_cells, 128), 128, 0, s>>>(d, P, b, fl);
+    if (P.precision == GELIOS_PREC_FP32_FLUX)
+        stationary32_update_kernel<<<blocks_for(d.n_cells, 128), 128, 0, s>>>(d, P, b, fl);
+    else
+        stationary_update_kernel<<<blocks_for(d.n_cells, 128), 128, 0, s>>>(d, P, b, fl);
+}
+// Lanes per block of the four-lanes-per-cell kernel, 0 where it does not take
+// the grid: more faces than lanes, or more lanes than are resident at once.
+// Where both take the grid the lanes are 3.6-4.5 times faster (see the
+// kernel); 360 x 240 cells, beyond them: 35.2 us per step with three
+// barriers, 21.9 in two phases with two.
+static int plain_lane_threads(const DevMesh& d, int sms) {
+    if (d.max_faces > 4 || !d.s_unit) return 0;
+    const int64_t per = (4 * static_cast<int64_t>(d.n_cells) + sms - 1) / sms;
+    const int64_t t = (per + 31) / 32 * 32;
+    if (t > kLaneThreads) return 0;
+    return t < 64 ? 64 : static_cast<int>(t);
 }
 cudaError_t launch_stationary_persistent(const DevMesh& d, const gelios_params& P, const StepBuffers& b0,
                                          const StepBuffers& b1, double* fl, int nsteps, cudaStream_t s) {
-    const void* fn = P.precision == GELIOS_PREC_FP32_FLUX
-                         ? reinterpret_cast<const void*>(&stationary_persistent_kernel<float>)
-                     : P.precision == GELIOS_PREC_FP32_WAVES
-                         ? reinterpret_cast<const void*>(&stationary_persistent_kernel<WaveF32>)
-                         : reinterpret_cast<const void*>(&stationary_persistent_kernel<double>);
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, 0);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
-    const int want = blocks_for(d.n_units > d.n_cells ? d.n_units : d.n_cells, 128);
-    const int grid = want < per_sm * sms ? want : per_sm * sms;
     DevMesh dd = d;
     gelios_params pp = P;
     StepBuffers c0 = b0, c1 = b1;
     double* flp = fl;
     int n = nsteps;
+    if (const int t = P.precision == GELIOS_PREC_FP32_FLUX ? 0 : plain_lane_threads(d, sms)) {
+        const void* fn = P.precision == GELIOS_PREC_FP32_WAVES
+                             ? reinterpret_cast<const void*>(&stationary_lanes_kernel<WaveF32>)
+                             : reinterpret_cast<const void*>(&stationary_lanes_kernel<double>);
+        void* args[] = {&dd, &pp, &c0, &c1, &n};
+        const int64_t lanes = 4 * static_cast<int64_t>(d.n_cells);
+        return cudaLaunchCooperativeKernel(fn, dim3(static_cast<unsigned>((lanes + t - 1) / t)), dim3(t), args, 0, s);
+    }
+    const void* fn = P.precision == GELIOS_PREC_FP32_FLUX
+                         ? reinterpret_cast<const void*>(&stationary32_persistent_kernel<float>)
+                     : P.precision == GELIOS_PREC_FP32_WAVES
+                         ? reinterpret_cast<const void*>(&stationary_persistent_kernel<WaveF32>)
+                         : reinterpret_cast<const void*>(&stationary_persistent_kernel<double>);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, 0);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
+    const int want = blocks_for(d.n_units > d.n_cells ? d.n_units : d.n_cells, 128);
+    const int grid = want < per_sm * sms ? want : per_sm * sms;
     void* args[] = {&dd, &pp, &c0, &c1, &flp, &n};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(128), args, 0, s);
 }
-__global__ void unit_geometry_kernel(DevMesh d, double g2, const double* __restrict__ cx,
+__global__ void face_geometry_kernel(DevMesh d, double g2, const double* __restrict__ cx,
                                      const double* __restrict__ cy, double* __restrict__ upf) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= d.n_units) return;
@@ -3752,17 +4376,32 @@ __global__ void unit_geometry_kernel(DevMesh d, double g2, const double* __restr
     geo[6 * nu + u] = f.dist;
     geo[7 * nu + u] = f.distn;
 }
-void launch_unit_geometry(const DevMesh& d, double gamma, const double* cx, const double* cy, double* upf,
-                          cudaStream_t s) {
-    if (d.n_units > 0) unit_geometry_kernel<<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, 2 * gamma, cx, cy, upf);
+__global__ void unit_geometry_kernel(DevMesh d, double gamma, double rad_stat, const double* __restrict__ cx,
+                                     const double* __restrict__ cy, const double* __restrict__ rp,
+                                     double* __restrict__ ugeo) {
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= d.n_units) return;
+    const int g = d.u_slot[u], A = d.sA[g], B = d.sB[g];
+    const UnitGeo f = unit_geo(gamma, rad_stat, d.u_info[u] & SI_TYPE_MASK, d.X[A], d.Y[A], d.X[B], d.Y[B], d.u_cell[u],
+                               d.u_nb[u], cx, cy, rp);
+    const size_t nu = d.n_units;
+    const double rows[kUnitGeoRows] = {f.n1, f.n2, f.S,    f.dist, f.distn, f.kroO, f.kpO,
+                                       f.CO, f.SO, f.kroN, f.kpN,  f.CN,    f.SN};
+    for (int k = 0; k < kUnitGeoRows; k++) ugeo[k * nu + u] = rows[k];
+    reinterpret_cast<uint32_t*>(ugeo + kUnitGeoRows * nu)[u] = f.flags;
 }
-cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst, const int* active, int n_active,
-                                    int nsteps, int prec, cudaStream_t s) {
-    if (n_active <= 0 || nsteps <= 0) return cudaSuccess;
-    const void* fn = prec == GELIOS_PREC_FP32_FLUX ? reinterpret_cast<const void*>(&stationary_batch_kernel<float>)
-                     : prec == GELIOS_PREC_FP32_WAVES
-                         ? reinterpret_cast<const void*>(&stationary_batch_kernel<WaveF32>)
-                         : reinterpret_cast<const void*>(&stationary_batch_kernel<double>);
+void launch_unit_geometry(const DevMesh& d, const gelios_params& P, const double* cx, const double* cy,
+                          const double* rp, double* ugeo, cudaStream_t s) {
+    if (d.n_units <= 0) return;
+    if (P.precision == GELIOS_PREC_FP32_FLUX)
+        face_geometry_kernel<<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, 2 * P.gamma, cx, cy, ugeo);
+    else
+        unit_geometry_kernel<<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, P.gamma, P.rad_stat, cx, cy, rp, ugeo);
+}
+// FP32 fluxes: one cooperative grid for all instances.
+static cudaError_t launch_stationary32_batch(const DevMesh& d, const PlainInstance* inst, const int* active,
+                                             int n_active, int nsteps, cudaStream_t s) {
+    const void* fn = reinterpret_cast<const void*>(&stationary32_batch_kernel<float>);
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -3777,6 +4416,44 @@ cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst,
     int na = n_active, n = nsteps;
     void* args[] = {&dd, &ip, &ap, &na, &n};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(128), args, 0, s);
+}
+cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst, const int* active, int n_active,
+                                    int nsteps, int prec, cudaStream_t s) {
+    if (n_active <= 0 || nsteps <= 0) return cudaSuccess;
+    if (prec == GELIOS_PREC_FP32_FLUX) return launch_stationary32_batch(d, inst, active, n_active, nsteps, s);
+    const void* fn = prec == GELIOS_PREC_FP32_WAVES
+                         ? reinterpret_cast<const void*>(&stationary_cluster_kernel<WaveF32>)
+                         : reinterpret_cast<const void*>(&stationary_cluster_kernel<double>);
+    // one cluster per instance, of the largest size at which every instance
+    // is resident; more instances than that run in waves (they are
+    // independent).  16 blocks need the non-portable size.
+    DevMesh dd = d;
+    const PlainInstance* ip = inst;
+    const int* ap = active;
+    int n = nsteps;
+    void* args[] = {&dd, &ip, &ap, &n};
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    for (int size = 16;; size /= 2) {
+        at.val.clusterDim.x = size;
+        cfg.gridDim = dim3(static_cast<unsigned>(n_active) * size);
+        int fit = 0;
+        e = cudaOccupancyMaxActiveClusters(&fit, fn, &cfg);
+        if (e != cudaSuccess) {  // a size the device does not offer
+            cudaGetLastError();
+            fit = 0;
+        }
+        if (fit >= n_active || size == 1) break;
+    }
+    return cudaLaunchKernelExC(&cfg, fn, args);
 }
 __global__ void plain_batch_words_init_kernel(const PlainInstance* inst, const int* active, int n) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -4068,6 +4745,14 @@ int launch_residual(const double* a, const double* b, int n, double* scratch, cu
     residual_partial_kernel<<<nb, 256, 0, s>>>(a, b, n, scratch + 2);
     residual_final_kernel<<<1, 1, 0, s>>>(scratch + 2, nb, scratch);
     return 2;
+}
+void launch_residual_batch(const PlainInstance* inst, const int* active, int n_active, int n_cells, double* part,
+                           double* out, cudaStream_t s) {
+    int nb = blocks_for(n_cells, 256);
+    if (nb > 296) nb = 296;
+    if (nb < 1) nb = 1;
+    residual_batch_partial_kernel<<<dim3(nb, n_active), 256, 0, s>>>(inst, active, n_cells, part);
+    residual_batch_final_kernel<<<n_active, 1, 0, s>>>(inst, active, nb, part, out);
 }
 void launch_words_init(void* words, double dt0, cudaStream_t s) {
     words_init_kernel<<<1, 1, 0, s>>>(static_cast<unsigned char*>(words), dt0);

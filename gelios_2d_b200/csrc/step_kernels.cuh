@@ -47,6 +47,9 @@ struct DevMesh {
     const uint32_t* u_info = nullptr;
     // neighbour cell (-1: one-sided unit), Sosed_down of the face and of its twin
     const int32_t *u_nb = nullptr, *u_sd = nullptr, *u_sd2 = nullptr;
+    // the unit of every slot << 1 | 1 where the slot is its twin side
+    const int32_t* s_unit = nullptr;
+    int max_faces = 0;  // most faces of a cell that is not C_centr
     const int32_t *fA = nullptr, *fB = nullptr, *ftype = nullptr, *fmaster = nullptr, *fsosed = nullptr,
                   *fcopy = nullptr, *fsdown = nullptr;
     const int32_t *rtype = nullptr, *rM = nullptr, *rpstart = nullptr, *rpts = nullptr, *rkstart = nullptr,
@@ -104,11 +107,14 @@ struct StepBuffers {
     double* rp_next = nullptr;
     double* vs_next = nullptr;
     double* vol_next = nullptr;
-    // plain form (fixed grid): |face centre|^(2 gamma) of every face unit and
-    // the units' face geometry (kUnitGeoRows - 1 unit-major rows, see
-    // FaceGeo in step_kernels.cu), or nullptr (then computed per unit)
-    const double* upf = nullptr;
+    // plain form (fixed grid): what its face units read of the grid
+    // (kUnitGeoRows unit-major rows, then one flag word per unit: UnitGeo in
+    // step_kernels.cu), or nullptr (then computed per unit)
     const double* ugeo = nullptr;
+    // with FP32 fluxes: |face centre|^(2 gamma) of every face unit and the
+    // units' face geometry (FaceGeo rows), or nullptr
+    const double* upf = nullptr;
+    const double* fgeo = nullptr;
     const double* dt_cur = nullptr;
     double* dt_next = nullptr;
     unsigned long long* dt_acc = nullptr;
@@ -120,19 +126,19 @@ struct StepBuffers {
 // area (Get_Volume) and the rotated volume (rows of the moving-grid cache).
 void launch_centroid(const DevMesh& d, const double* X, const double* Y, double* cx, double* cy, double* rp,
                      double gamma, cudaStream_t s, double* vs = nullptr, double* vol = nullptr);
-// Per face unit of the plain form (its grid does not move): row 0
-// |face centre|^(2 gamma), rows 1-8 the face geometry as the owner sees it
-// (centre x, y, normal, |centre|^2, length, owner and neighbour centroid
-// distances); needs the centroids cx, cy.
-constexpr int kUnitGeoRows = 9;
-void launch_unit_geometry(const DevMesh& d, double gamma, const double* cx, const double* cy, double* upf,
-                          cudaStream_t s);
+// Per face unit of the plain form (its grid does not move): the UnitGeo rows
+// and flag words; needs the centroids cx, cy and rp = |centroid|^(2 gamma).
+constexpr int kUnitGeoRows = 13;
+// With FP32 fluxes instead the FaceGeo rows and |face centre|^(2 gamma).
+void launch_unit_geometry(const DevMesh& d, const gelios_params& P, const double* cx, const double* cy,
+                          const double* rp, double* ugeo, cudaStream_t s);
 void launch_stationary_units(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* fl,
                              cudaStream_t s);
 void launch_stationary_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
                               cudaStream_t s);
 // `nsteps` Go_stationary steps in one cooperative launch (b0: even steps,
-// b1: odd steps); returns the launch's error code.
+// b1: odd steps); returns the launch's error code.  b0.dt_acc[0], [4] and
+// [5] are three CFL accumulators (words_init_kernel arms them).
 cudaError_t launch_stationary_persistent(const DevMesh& d, const gelios_params& P, const StepBuffers& b0,
                                          const StepBuffers& b1, double* fl, int nsteps, cudaStream_t s);
 // Instances of the plain form that share one mesh: parameters, the buffers
@@ -269,6 +275,11 @@ constexpr int kResidualScratch = 2 + 2 * 296;
 int launch_op_residual(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
                        double* scratch, cudaStream_t s);
 int launch_residual(const double* a, const double* b, int n, double* scratch, cudaStream_t s);
+// The same for the listed instances of a plain batch in two launches; out
+// gets, per listed instance, the two sums, its dt and its status flags.
+// part: kResidualScratch doubles per listed instance.
+void launch_residual_batch(const PlainInstance* inst, const int* active, int n_active, int n_cells, double* part,
+                           double* out, cudaStream_t s);
 // Words a call starts from (dt0, empty accumulator, zero counters/status),
 // on the stream: for one context / for every instance of a batch.
 void launch_words_init(void* words, double dt0, cudaStream_t s);
