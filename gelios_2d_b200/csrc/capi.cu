@@ -135,6 +135,7 @@ struct gelios_ctx {
     DBuf surface;  // Move_surface per-face speeds
     DBuf inner;
     int n_inner = 0;
+    DBuf inner_tab;  // constants of an inner call (launch_inner_lanes); empty: one thread per cell
     int n_sp = 0;
     // cen[0] holds the centroids of the current points (rows cx, cy,
     // |c|^(2 gamma), area, rotated volume); after a moving-grid call row 2
@@ -1114,6 +1115,12 @@ extern "C" int gelios_set_inner_cells(gelios_ctx* ctx, const int32_t* cells, int
     if (upload(ctx->inner, cells, n, ctx->stream)) return GELIOS_E_CUDA;
     GELIOS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     ctx->n_inner = n;
+    const size_t tb = inner_lanes_ok(ctx->d, ctx->prm, n) ? inner_table_bytes(n) : 0;
+    if (ctx->inner_tab.bytes != tb && ctx->inner_tab.alloc(tb)) {
+        // no room for the table: the steps run without it
+        cudaGetLastError();
+        ctx->inner_tab.bytes = 0;
+    }
     return GELIOS_OK;
 }
 
@@ -1548,6 +1555,34 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         }
         if (launch_stationary_persistent(d, P, bb[0], bb[1], ctx->flux.as<double>(), nsteps, s) == cudaSuccess) {
             launches += 1;
+            first = nsteps;
+        } else {
+            cudaGetLastError();
+            ctx->coop_off = true;
+        }
+    }
+    if (form == GELIOS_FORM_INNER_MK2 && nsteps > 0 && !ctx->timing && !ctx->coop_off && ctx->n_inner > 0 &&
+        inner_lanes_ok(d, P, ctx->n_inner) && ctx->inner_tab.bytes >= inner_table_bytes(ctx->n_inner)) {
+        // all steps of the inner form in one cooperative launch
+        StepBuffers bb[2];
+        for (int par = 0; par < 2; par++) {
+            StepBuffers& b = bb[par];
+            for (int k = 0; k < 5; k++) {
+                b.cur[k] = ctx->field(par, k);
+                b.nxt[k] = ctx->field(par ^ 1, k);
+            }
+            b.dt_cur = ctx->T() + par;
+            b.dt_next = ctx->T() + (par ^ 1);
+            b.dt_acc = ctx->acc();
+            b.counters = ctx->counters();
+            b.status = ctx->status();
+            b.cx = cen0;
+            b.cy = cen0 + ncz;
+            b.rp = cen0 + 2 * ncz;
+        }
+        if (launch_inner_lanes(d, P, bb[0], bb[1], ctx->inner.as<int32_t>(), ctx->n_inner,
+                               ctx->inner_tab.as<double>(), nsteps, s) == cudaSuccess) {
+            launches += 2;
             first = nsteps;
         } else {
             cudaGetLastError();

@@ -2283,7 +2283,8 @@ __global__ void __launch_bounds__(128, 8) mk2_update_kernel(DevMesh d, gelios_pa
     block_reduce_commit(tmark, nro, npc, 0, b.dt_acc, b.counters, b.status);
 }
 
-// Go_stationary_5_komponent_inner_MK2 cell update (Setka.cpp:7021-7210).
+// Go_stationary_5_komponent_inner_MK2 cell update (Setka.cpp:7021-7210), one
+// thread per cell: FP32 fluxes, and what inner_lanes_kernel does not take.
 template <typename TF>
 __global__ void __launch_bounds__(128) inner_cell_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                          const int32_t* __restrict__ list, int n_list) {
@@ -2391,6 +2392,319 @@ __global__ void __launch_bounds__(128) inner_cell_kernel(DevMesh d, gelios_param
         b.nxt[4][c] = Q33;
     }
     block_reduce_commit(tmin_c, nro, npc, status, b.dt_acc, b.counters, b.status);
+}
+
+// ------------------------------------------------------------------ inner form, four lanes per cell
+// Go_stationary_5_komponent_inner_MK2 on a fixed grid with fixed Monte-Carlo
+// moments: all a step needs beside the states is constant over a call, so one
+// launch (inner_table_kernel) computes it per (cell, face) lane and the steps
+// read it back: per lane i = 4 * (list position) + face, kInnerRows rows of
+// 4 n_list doubles and kInnerIntRows rows of ints (type | flags, other cell,
+// Sosed_down of either side).
+//   0 n1, 1 n2, 2 S, 3 kurant * dist
+//   4 kroO, 5 kpO, 6 CO, 7 SO   the cell's side: |centroid|^2 / |centre|^2,
+//                               (|centroid| / |centre|)^(2 gamma), rotation
+//                               to the face centre's polar frame
+//   8 kroN, 9 kpN, 10 CN, 11 SN the other side's; Inner_sphere: wind ro, p, u, v
+//   12 w1, 13 k1, 14 r12        radial TVD, the cell's side: factors of the
+//                               Sosed_down cell's ro and p, 1 / (dist2 - dist1)
+//   15 r23, 16 dist2            -1 / (dist2 + dist3) of both sides, distance
+//   17 w1, 18 k1, 19 r12, 20 dist2  the same seen from the other side
+//   21 uH, 22 vH, 23 roH, 24 th Monte-Carlo moments of species `face` at the
+//                               cell, th = 2 pH / roH
+//   25 k_u, k_v, k_T            of the cell, on its lanes 0, 1, 2
+//   26 1 / Volume, 27 (vs1 + vs2) / 2   on lane 0
+enum : int { IL_TYPE = 7, IL_TVD = 8, IL_RAW_O = 16, IL_RAW_N = 32, IL_SRC = 64, IL_ACT = 128 };
+
+// Get_Sourse_MK1 rates of one species from the temperature-like th = 2 pH / roH
+// (Cell.cpp:590-660): one reciprocal square root serves |U_M|, U_H / U_M, and
+// log U_M = log(U_M^2) / 2 waits for neither.
+__device__ __forceinline__ void source_rates_th(const gelios_params& P, double uH, double vH, double roH, double th,
+                                                double u, double v, double ro, double pro, double kin, double& nuu,
+                                                double& nuv, double& nue) {
+    const double du2 = sq(u - uH) + sq(v - vH), a = pro + th;
+    const double UM2 = du2 + (64.0 / (9.0 * kPi)) * a, UH2 = du2 + (4.0 / kPi) * a;
+    const double r = rsqrt(UM2);
+    const double sig = sq(1.0 - P.a_2 * (0.5 * log(UM2)));
+    const double nu = ro * roH * (UM2 * r) * sig;
+    nuu = nu * (uH - u);
+    nuv = nu * (vH - v);
+    nue = nu * ((sq(uH) + sq(vH) - kin) / 2.0 + (sqrt(UH2) * r) * (th - pro));
+}
+
+__global__ void __launch_bounds__(128) inner_table_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                          const int32_t* __restrict__ list, int n_list,
+                                                          double* __restrict__ tab, int* __restrict__ itab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t N = 4 * static_cast<size_t>(n_list);
+    if (static_cast<size_t>(i) >= N) return;
+    const int c = list[i >> 2], j = i & 3;
+    double r[kInnerRows];
+#pragma unroll
+    for (int k = 0; k < kInnerRows; k++) r[k] = 0.0;
+    int ft = IL_TYPE, flags = 0, nb = -1, sdO = c, sdN = c, status = 0;
+    if (!(d.cflags[c] & CF_CENTR)) {
+        flags = IL_ACT;
+        const uint32_t cf = d.cflags[c];
+        const int s0 = d.cstart[c], n = d.cstart[c + 1] - s0, g0 = d.gstart[c], g1 = d.gstart[c + 1];
+        const int32_t* con = d.contour + s0;
+        const double x = b.cx[c], y = b.cy[c], radius = sqrt(sq(x) + sq(y));
+        if (j == 0) {
+            r[26] = 1.0 / volume_rotate(con, n, d.X, d.Y);
+            r[27] = 0.5 * (area(con, n, d.sA, d.sB, g0, g1, d.X, d.Y, false) +
+                           area(con, n, d.sA, d.sB, g0, g1, d.X2, d.Y2, true));
+        }
+        const int g = g0 + j;
+        if (g < g1) {
+            const int A = d.sA[g], B = d.sB[g];
+            ft = d.sinfo[g] & SI_TYPE_MASK;
+            const double xa = d.X[A], ya = d.Y[A], xb = d.X[B], yb = d.Y[B];
+            const double nn = sqrt(sq(xb - xa) + sq(yb - ya));
+            const double x2 = (xa + xb) / 2.0, y2 = (ya + yb) / 2.0, dis2 = sq(x2) + sq(y2);
+            const double dist = sqrt(sq(x - x2) + sq(y - y2));
+            r[0] = (yb - ya) / nn;
+            r[1] = -((xb - xa) / nn);
+            r[2] = nn * (ya + yb) * 0.5;
+            r[3] = P.kurant * dist;
+            const double pdis = pow2g(sqrt(dis2), 2.0 * P.gamma);
+            double cf2, sf2;
+            polar_cs(x2, y2, cf2, sf2);
+            auto side = [&](int k, double xc, double yc, double* o) {
+                double c1, s1;
+                polar_cs(xc, yc, c1, s1);
+                o[0] = (sq(xc) + sq(yc)) / dis2;
+                o[1] = b.rp[k] / pdis;
+                o[2] = c1 * cf2 + s1 * sf2;
+                o[3] = c1 * sf2 - s1 * cf2;
+            };
+            side(c, x, y, r + 4);
+            if (ft == G_USUALY) {
+                nb = d.snb[g];
+                const double x3 = b.cx[nb], y3 = b.cy[nb], distn = sqrt(sq(x3 - x2) + sq(y3 - y2));
+                side(nb, x3, y3, r + 8);
+                const uint32_t nbf = d.cflags[nb];
+                if ((cf & CF_C1) && (nbf & CF_C1)) {
+                    flags |= IL_TVD;
+                    r[15] = 1.0 / (-dist - distn);
+                    // Get_par_TVD_radial of master M (centre xm, ym, distance dm)
+                    auto tvd = [&](int M, double xm, double ym, double dm, int Sd, bool axis, const double* own,
+                                   double* o, int& sd, int raw) {
+                        sd = M;
+                        if (Sd >= 0) {
+                            const double xs = b.cx[Sd], ys = b.cy[Sd];
+                            sd = Sd;
+                            o[0] = (sq(xs) + sq(ys)) / dis2;
+                            o[1] = b.rp[Sd] / pdis;
+                            o[2] = 1.0 / (dm - sqrt(sq(x2 - xs) + sq(y2 - ys)));
+                        } else if (axis) {  // the mirrored centre has the radius and state of M itself
+                            o[0] = own[0];
+                            o[1] = own[1];
+                            o[2] = 1.0 / (dm - sqrt(sq(x2 - xm) + sq(y2 + ym)));
+                        } else {
+                            flags |= raw;
+                        }
+                    };
+                    tvd(c, x, y, dist, d.ssd[g], (cf & CF_AXIS) != 0, r + 4, r + 12, sdO, IL_RAW_O);
+                    r[16] = dist;
+                    tvd(nb, x3, y3, distn, d.ssd2[g], (nbf & CF_AXIS) != 0, r + 8, r + 17, sdN, IL_RAW_N);
+                    r[20] = distn;
+                }
+            } else if (ft == G_INNER_SPHERE) {
+                const St5 w = inner_sphere_state(P, x2, y2);
+                r[8] = w.ro;
+                r[9] = w.p;
+                r[10] = w.u;
+                r[11] = w.v;
+            }
+        }
+        const bool interp = radius > P.src_rmin && radius < P.src_rmax && x >= 0.0;
+        int K_do = -1, K_posle = -1;
+        if (!interp || source_bracket(d, c, radius, K_do, K_posle, &status)) {
+            flags |= IL_SRC;
+            SrcMoments m = source_moments(d, c, j, interp, K_do, K_posle, radius);
+            if (m.roH <= 0.0) {
+                m.roH = 0.0000001;
+                m.pH = 0.0;
+            }
+            r[21] = m.uH;
+            r[22] = m.vH;
+            r[23] = m.roH;
+            r[24] = 2.0 * m.pH / m.roH;
+            r[25] = j == 0 ? m.ku : j == 1 ? m.kv : m.kT;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kInnerRows; k++) tab[k * N + i] = r[k];
+    itab[i] = ft | flags;
+    itab[N + i] = nb;
+    itab[2 * N + i] = sdO;
+    itab[3 * N + i] = sdN;
+    if (status) atomicOr(b.status, status);
+}
+
+// The steps of a call in one cooperative launch: a lane evaluates one face of
+// its cell and one species' charge exchange, the cell's four lanes add both
+// in the reference's order by shuffles, and one grid barrier ends the step
+// (the CFL accumulators as in the plain form's kernels).  One thread per
+// cell walking its faces (a pow and the radial reconstructions per face and
+// side, 233 blocks) took 41.5 us per step on the 29.7k inner cells of the
+// 200k grid, 12.1 us here.
+template <typename TF>
+__global__ void __launch_bounds__(256, 2) inner_lanes_kernel(DevMesh d, gelios_params P, StepBuffers b0, StepBuffers b1,
+                                                             const int32_t* __restrict__ list, int n_list,
+                                                             const double* __restrict__ tab,
+                                                             const int* __restrict__ itab, int nsteps) {
+    __shared__ double sm[32];
+    cg::grid_group grid = cg::this_grid();
+    const size_t N = 4 * static_cast<size_t>(n_list);
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    const int j = tid & 3, q0 = threadIdx.x & 28;
+    const unsigned full = 0xffffffffu;
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    const double gm1 = P.gamma - 1, rg1 = 1.0 / gm1;
+    const int rounds = static_cast<int>((N + nth - 1) / nth);
+    double dt = *b0.dt_cur, dt_prev = dt;
+    int nro = 0, npc = 0;
+    for (int st = 0; st < nsteps; st++) {
+        const StepBuffers& b = (st & 1) ? b1 : b0;
+        double t = inf;
+        for (int rd = 0; rd < rounds; rd++) {
+            const size_t i = static_cast<size_t>(rd) * nth + tid;
+            const bool in = i < N;
+            const int c = in ? list[i >> 2] : 0;
+            const int info = in ? itab[i] : IL_TYPE;
+            const bool act = (info & IL_ACT) != 0;
+            const int ft = info & IL_TYPE;
+            const double* r = tab + i;
+            St5 own{1.0, 1.0, 0.0, 0.0, 1.0};
+            double F[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+            double nuu = 0.0, nuv = 0.0, nue = 0.0, kk = 0.0;
+            if (act) {
+                own = St5{__ldcg(b.cur[0] + c), __ldcg(b.cur[1] + c), __ldcg(b.cur[2] + c), __ldcg(b.cur[3] + c),
+                          __ldcg(b.cur[4] + c)};
+                t = dmin_ref(t, 10000000.0);
+                if (info & IL_SRC) {
+                    kk = r[25 * N];
+                    source_rates_th(P, r[21 * N], r[22 * N], r[23 * N], r[24 * N], own.u, own.v, own.ro,
+                                    own.p / own.ro, sq(own.u) + sq(own.v), nuu, nuv, nue);
+                }
+            }
+            if (act && ft != IL_TYPE) {
+                St5 L = own, R = own;
+                const double n1 = r[0], n2 = r[N], S = r[2 * N];
+                if (ft == G_USUALY) {
+                    const int nb = itab[N + i];
+                    R = St5{__ldcg(b.cur[0] + nb), __ldcg(b.cur[1] + nb), __ldcg(b.cur[2] + nb), __ldcg(b.cur[3] + nb),
+                            __ldcg(b.cur[4] + nb)};
+                    const double kO = r[4 * N], pO = r[5 * N], kN = r[8 * N], pN = r[9 * N];
+                    const double roO = L.ro * kO, prO = L.p * pO, roN = R.ro * kN, prN = R.p * pN;
+                    const double rawRo = R.ro, rawP = R.p;
+                    L = plain_scale(L, kO, pO, r[6 * N], r[7 * N]);
+                    R = plain_scale(R, kN, pN, r[10 * N], r[11 * N]);
+                    L.Q *= kO;
+                    R.Q *= kN;
+                    if (info & IL_TVD) {
+                        const int sO = itab[2 * N + i], sN = itab[3 * N + i];
+                        const double r23 = r[15 * N];
+                        const double o1 = __ldcg(b.cur[0] + sO), o2 = __ldcg(b.cur[1] + sO);
+                        const double m1 = __ldcg(b.cur[0] + sN), m2 = __ldcg(b.cur[1] + sN);
+                        const double rO = r[14 * N], dO = -r[16 * N], rN = r[19 * N], dN = -r[20 * N];
+                        L.ro = linear3r(o1 * r[12 * N], roO, roN, rO, r23, dO);
+                        L.p = linear3r(o2 * r[13 * N], prO, prN, rO, r23, dO);
+                        R.ro = linear3r(m1 * r[17 * N], roN, roO, rN, r23, dN);
+                        R.p = linear3r(m2 * r[18 * N], prN, prO, rN, r23, dN);
+                        if (info & IL_RAW_O) {
+                            L.ro = own.ro;
+                            L.p = own.p;
+                        }
+                        if (info & IL_RAW_N) {
+                            R.ro = rawRo;
+                            R.p = rawP;
+                        }
+                    }
+                } else if (ft == G_INNER_SPHERE) {
+                    R = St5{r[8 * N], r[9 * N], r[10 * N], r[11 * N], r[8 * N]};
+                    L = R;
+                } else if (ft == G_AXIS) {
+                    const double kO = r[4 * N];
+                    L = plain_scale(L, kO, r[5 * N], r[6 * N], r[7 * N]);
+                    L.Q *= kO;
+                    R = L;
+                    R.v = -R.v;
+                } else if (ft == G_EXTERN) {
+                    if (R.u >= 0.0) R.u = P.extern_u_par;
+                } else if (ft == G_INPUT) {
+                    R = input_state(P);
+                }
+                double UU;
+                if (ft == G_AXIS) {  // HLL
+                    FluxOut<double> G;
+                    UU = hllc_flux<TF>(P.gamma, P.kurant, L, R, 0.0, n1, n2, 1.0, 0, false, G);
+                    F[0] = G.P0;
+                    F[1] = G.P1;
+                    F[2] = G.P2;
+                    F[3] = G.P3;
+                    F[4] = G.PQ;
+                } else {
+                    UU = plain_flux<TF>(P, L, R, n1, n2, F);
+                }
+#pragma unroll
+                for (int k = 0; k < 5; k++) F[k] *= S;
+                t = dmin_ref(t, dt_candidate(r[3 * N] / UU));
+            }
+            double Pt[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, Mu = 0.0, Mv = 0.0, MT = 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+#pragma unroll
+                for (int f = 0; f < 5; f++) Pt[f] = Pt[f] + __shfl_sync(full, F[f], q0 + k);
+                Mu = Mu + __shfl_sync(full, nuu, q0 + k);
+                Mv = Mv + __shfl_sync(full, nuv, q0 + k);
+                MT = MT + __shfl_sync(full, nue, q0 + k);
+            }
+            const double ku = __shfl_sync(full, kk, q0), kv = __shfl_sync(full, kk, q0 + 1),
+                         kT = __shfl_sync(full, kk, q0 + 2);
+            if (act && j == 0) {  // Setka.cpp:7167-7207
+                const double q1 = P.src_coef * Mu * ku, q2 = P.src_coef * Mv * kv, q3 = P.src_coef * MT * kT;
+                const double rV = r[26 * N], As = r[27 * N];
+                const double ro = own.ro, u = own.u, v = own.v, p = own.p;
+                double ro3 = ro - dt * (Pt[0] * rV);
+                const double Q3 = own.Q - (dt * rV) * Pt[4] - dt;
+                if (ro3 <= 0) {
+                    ro3 = P.ro_floor;
+                    nro++;
+                }
+                const double rro3 = 1.0 / ro3;
+                const double u3 = (ro * u - dt * (Pt[1] * rV - q1)) * rro3;
+                const double v3 = (ro * v - dt * ((Pt[2] - p * As) * rV - q2)) * rro3;
+                double p3 = (((p * rg1 + ro * (u * u + v * v) * 0.5) - dt * (Pt[3] * rV - q3)) -
+                             0.5 * ro3 * (u3 * u3 + v3 * v3)) *
+                            gm1;
+                if (p3 <= 0) {
+                    p3 = P.p_floor;
+                    npc++;
+                }
+                b.nxt[0][c] = ro3;
+                b.nxt[1][c] = p3;
+                b.nxt[2][c] = u3;
+                b.nxt[3][c] = v3;
+                b.nxt[4][c] = Q3;
+            }
+        }
+        unsigned long long* acc = plain_acc(b0.dt_acc, st);
+        t = block_min_nonneg(t, sm);
+        if (threadIdx.x == 0 && t < inf) atomicMin(acc, static_cast<unsigned long long>(__double_as_longlong(t)));
+        grid.sync();
+        dt_prev = dt;
+        dt = plain_dt(__ldcg(acc));
+        if (tid == 0) *plain_acc(b0.dt_acc, st + 2) = 0x7ff0000000000000ULL;
+    }
+    if (nro) atomicAdd(&b0.counters[0], static_cast<unsigned long long>(nro));
+    if (npc) atomicAdd(&b0.counters[1], static_cast<unsigned long long>(npc));
+    if (tid == 0) {
+        const StepBuffers& b = ((nsteps - 1) & 1) ? b1 : b0;
+        *b.dt_next = dt;
+        *const_cast<double*>(b.dt_cur) = dt_prev;
+    }
 }
 
 // T[now2] of the reference: min(1e7, all face candidates) if any cell took
@@ -4600,6 +4914,30 @@ void launch_inner(const DevMesh& d, const gelios_params& P, const StepBuffers& b
         inner_cell_kernel<float><<<nb, 128, 0, s>>>(d, P, b, list, n);
     else
         inner_cell_kernel<double><<<nb, 128, 0, s>>>(d, P, b, list, n);
+}
+bool inner_lanes_ok(const DevMesh& d, const gelios_params& P, int n) {
+    return P.precision != GELIOS_PREC_FP32_FLUX && d.max_faces <= 4 && n > 0 && n <= kInnerLaneCells;
+}
+cudaError_t launch_inner_lanes(const DevMesh& d, const gelios_params& P, const StepBuffers& b0, const StepBuffers& b1,
+                               const int32_t* list, int n, double* tab, int nsteps, cudaStream_t s) {
+    const void* fn = reinterpret_cast<const void*>(&inner_lanes_kernel<double>);
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
+    const int lanes = 4 * n;
+    int* itab = reinterpret_cast<int*>(tab + static_cast<size_t>(kInnerRows) * lanes);
+    inner_table_kernel<<<blocks_for(lanes, 128), 128, 0, s>>>(d, P, b0, list, n, tab, itab);
+    const int want = blocks_for(lanes, 256), most = per_sm * sms;
+    const int rounds = blocks_for(want, most), grid = blocks_for(want, rounds);  // equal rounds
+    DevMesh dd = d;
+    gelios_params pp = P;
+    StepBuffers c0 = b0, c1 = b1;
+    int nn = n, ns = nsteps;
+    void* args[] = {&dd, &pp, &c0, &c1, &list, &nn, &tab, &itab, &ns};
+    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s);
 }
 void launch_dt_finalize(const StepBuffers& b, cudaStream_t s) { dt_finalize_kernel<<<1, 1, 0, s>>>(b); }
 void launch_commit(const DevMesh& d, const StepBuffers& b, cudaStream_t s, bool cap) {

@@ -209,6 +209,17 @@ int launch_mk2_flux_tracked(const DevMesh& d, const gelios_params& P, const Step
 void launch_mk2_source(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* aux, cudaStream_t s);
 void launch_inner(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const int32_t* list, int n,
                   cudaStream_t s);
+// `nsteps` inner steps in two launches (the call's constants, then every
+// step), four lanes per listed cell: FP64 fluxes, cells of at most four
+// faces, lists of at most kInnerLaneCells cells (whose constants take 256 MB).
+// tab: inner_table_bytes(n).
+constexpr int kInnerRows = 28, kInnerIntRows = 4, kInnerLaneCells = 262144;
+inline size_t inner_table_bytes(int n) {
+    return 4 * static_cast<size_t>(n) * (kInnerRows * sizeof(double) + kInnerIntRows * sizeof(int));
+}
+bool inner_lanes_ok(const DevMesh& d, const gelios_params& P, int n);
+cudaError_t launch_inner_lanes(const DevMesh& d, const gelios_params& P, const StepBuffers& b0, const StepBuffers& b1,
+                               const int32_t* list, int n, double* tab, int nsteps, cudaStream_t s);
 void launch_dt_finalize(const StepBuffers& b, cudaStream_t s);
 void launch_commit(const DevMesh& d, const StepBuffers& b, cudaStream_t s, bool cap = false);
 // dt of the next step from the CFL accumulator when the update did not fold
