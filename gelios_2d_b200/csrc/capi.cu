@@ -1207,7 +1207,39 @@ int enqueue_mhd(gelios_ctx* ctx, const StepBuffers& b) {
     return nm + nfc + 2;
 }
 
+// Enqueues one Go_5_komponent step: Move_surface + Move_Setka_Calculate, the
+// face units (their groups beside one another on three streams), the
+// five-fluid cell update (which refills the geometry cache for the next
+// step, like the moving-grid form's), x = x2.
+int enqueue_k5(gelios_ctx* ctx, const StepBuffers& b) {
+    const DevMesh& d = ctx->d;
+    const gelios_params& P = ctx->prm;
+    cudaStream_t s = ctx->stream;
+    const int cur = b.cur[0] == ctx->field(0, 0) ? 0 : 1, nxt = cur ^ 1;
+    const double* hcur = ctx->hstate[cur].as<double>();
+    cudaEvent_t e1 = ctx->phase_begin();
+    const int nm = launch_motion(d, P, b, ctx->surface.as<double>(), s, false);
+    ctx->phase_end(2, e1, nm);
+    cudaEvent_t e3 = ctx->phase_begin();
+    GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
+    GELIOS_CUDA_TRY(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+    GELIOS_CUDA_TRY(cudaStreamWaitEvent(ctx->groups, ctx->ev_fork, 0));
+    const int nf = launch_k5_faces(d, P, b, hcur, ctx->flux_mhd.as<double>(), s, ctx->groups, ctx->side);
+    GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_tracked, ctx->side));
+    GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_groups, ctx->groups));
+    GELIOS_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_tracked, 0));
+    GELIOS_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_groups, 0));
+    launch_k5_update(d, P, b, ctx->flux_mhd.as<double>(), hcur, ctx->hstate[nxt].as<double>(), s);
+    ctx->phase_end(3, e3, nf + 1);
+    cudaEvent_t e4 = ctx->phase_begin();
+    launch_commit(d, b, s);
+    ctx->phase_end(4, e4, 1);
+    GELIOS_CUDA_TRY(cudaGetLastError());
+    return nm + nf + 2;
+}
+
 int enqueue_form(gelios_ctx* ctx, const StepBuffers& b, int form) {
+    if (form == GELIOS_FORM_5_KOMPONENT) return enqueue_k5(ctx, b);
     return form == GELIOS_FORM_MHD_PUI ? enqueue_mhd(ctx, b) : enqueue_mk2(ctx, b);
 }
 
@@ -1493,9 +1525,9 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         int pad[5];
     };
     static_assert(sizeof(Words) == 64, "device word layout");
-    // the moving-grid and MHD forms initialise the words in their first
-    // step (inside its graph); the others here
-    const bool graph_form = form == GELIOS_FORM_MK2 || mhd;
+    // the moving-grid forms initialise the words in their first step (inside
+    // its graph); the others here
+    const bool graph_form = moving;
     int64_t launches = 0;
     if (!graph_form || nsteps == 0) {
         launch_words_init(ctx->words.p, P.dt0, s);
@@ -1510,9 +1542,9 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         return GELIOS_E_STATE;
     }
     if (mhd || form == GELIOS_FORM_5_KOMPONENT) {
-        // wide flux slots of the multi-fluid forms (13 or 21 rows)
-        const int rows = mhd ? kMhdFluxRows : kK5FluxRows;
-        const size_t fb = static_cast<size_t>(rows) * d.n_slots * sizeof(double);
+        // wide flux rows of the multi-fluid forms: 13 per face slot or 21 per face unit
+        const size_t fb = (mhd ? kMhdFluxRows * static_cast<size_t>(d.n_slots)
+                               : kK5FluxRows * static_cast<size_t>(d.n_units)) * sizeof(double);
         if (ctx->flux_mhd.bytes != fb) {
             ctx->drop_graphs();
             if (ctx->flux_mhd.alloc(fb)) return GELIOS_E_CUDA;
@@ -1643,9 +1675,6 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             if (n < 0) return n;
             launches += n;
         } else if (form == GELIOS_FORM_5_KOMPONENT) {
-            // Move_surface + Move_Setka_Calculate, the face units and the
-            // five-fluid cell update (which refills the geometry cache for
-            // the next step, like the moving-grid form), x = x2
             double* cc = (st & 1) ? cen1 : cen0;
             double* cn = (st & 1) ? cen0 : cen1;
             b.cx = cc;
@@ -1658,17 +1687,9 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             b.rp_next = cn + 2 * ncz;
             b.vs_next = cn + 3 * ncz;
             b.vol_next = cn + 4 * ncz;
-            cudaEvent_t e1 = ctx->phase_begin();
-            const int nm = launch_motion(d, P, b, ctx->surface.as<double>(), s, false);
-            ctx->phase_end(2, e1, nm);
-            cudaEvent_t e3 = ctx->phase_begin();
-            launch_k5(d, P, b, ctx->hstate[cur].as<double>(), ctx->hstate[nxt].as<double>(), ctx->flux_mhd.as<double>(),
-                      s);
-            ctx->phase_end(3, e3, 2);
-            cudaEvent_t e4 = ctx->phase_begin();
-            launch_commit(d, b, s);
-            ctx->phase_end(4, e4, 1);
-            launches += nm + 3;
+            const int n = step_graph(ctx, b, GELIOS_FORM_5_KOMPONENT, st == 0);
+            if (n < 0) return n;
+            launches += n;
         } else {
             b.cx = cen0;
             b.cy = cen0 + d.n_cells;

@@ -276,54 +276,76 @@ __device__ __forceinline__ double sound_speed(double gp, double ro) {
     return sqrt(gp / ro);
 }
 
-// hllc_flux of a face at rest (W = 0, metod 1, no smoothing: the plain form,
-// Setka.cpp:10484-10700), written for few operations and short chains: only
-// the side the contact selects is evaluated, the contact speed and the
-// reciprocal of its distance to the selected wave come from two independent
-// quotients, and every operation is fixed (see above), so the plain form's
-// kernels agree bit for bit.  Not for FP32 fluxes (hllc_flux).  out = mass, momentum x, y, energy, Q; returns max(|SL|, |SR|).
-template <typename TF>
-__device__ __forceinline__ double plain_flux(const gelios_params& P, const St5& L, const St5& R, double n1, double n2,
-                                             double (&out)[5]) {
+// HLLC flux through a face moving with normal speed W (MOVING; else at rest),
+// hllc_flux with metod 1 in FP64 written for few operations and short chains:
+// only the side that the contact speed selects against W is evaluated, the
+// contact speed and the reciprocal of its distance to the selected wave come
+// from two independent quotients, and every operation is fixed (see above),
+// so kernels that inline it agree bit for bit.  SMOOTH: the tangential
+// smoothing `nul_potok` where np is set.  TF: double or WaveF32.  out = mass,
+// momentum x, y, energy, Q; returns max(|SL|, |SR|).
+template <typename TF, bool MOVING, bool SMOOTH>
+__device__ __forceinline__ double hllc_lean(double ga, const St5& L, const St5& R, double W, double n1, double n2,
+                                            bool np, double (&out)[5]) {
     using TW = typename WaveArith<TF>::type;
     const double u1 = fma_rn(L.u, n1, mul_rn(L.v, n2)), v1 = fma_rn(L.u, n2, -mul_rn(L.v, n1));
     const double u2 = fma_rn(R.u, n1, mul_rn(R.v, n2)), v2 = fma_rn(R.u, n2, -mul_rn(R.v, n1));
     TW c;
     if constexpr (sizeof(TW) == 8)
-        c = dmax_ref(sound_speed(mul_rn(P.gamma, L.p), L.ro), sound_speed(mul_rn(P.gamma, R.p), R.ro));
+        c = dmax_ref(sound_speed(mul_rn(ga, L.p), L.ro), sound_speed(mul_rn(ga, R.p), R.ro));
     else
-        c = tmax<TW>(tsqrt<TW>((TW)P.gamma * (TW)L.p / (TW)L.ro), tsqrt<TW>((TW)P.gamma * (TW)R.p / (TW)R.ro));
+        c = tmax<TW>(tsqrt<TW>((TW)ga * (TW)L.p / (TW)L.ro), tsqrt<TW>((TW)ga * (TW)R.p / (TW)R.ro));
     const double SL = (double)((TW)dmin_ref(u1, u2) - c), SR = (double)((TW)dmax_ref(u1, u2) + c);
     const double suL = sub_rn(SL, u1), suR = sub_rn(SR, u2);
     const double mL = mul_rn(suL, L.ro), mR = mul_rn(suR, R.ro);
     const double num = add_rn(sub_rn(fma_rn(mR, u2, -mul_rn(mL, u1)), R.p), L.p), den = sub_rn(mR, mL);
-    // SM = num / den; its sign (den > 0 for SL < u1, u2 < SR) picks the
-    // side, so 1 / (S - SM) = den / (S den - num) need not wait for it
+    // SM = num / den; at rest its sign (den > 0 for SL < u1, u2 < SR) picks
+    // the side without it, and 1 / (S - SM) = den / (S den - num) never waits
     const double SM = num / den;
-    const bool sup = SL >= 0.0 || SR <= 0.0;  // the whole fan on one side
-    const bool left = SL >= 0.0 || (!(SR <= 0.0) && (den > 0.0 ? num >= 0.0 : SM >= 0.0));
+    const double Ws = MOVING ? W : 0.0;
+    const bool sup = SL >= Ws || SR <= Ws;  // the whole fan on one side
+    const bool right_of = MOVING ? SM >= Ws : (den > 0.0 ? num >= 0.0 : SM >= 0.0);
+    const bool left = SL >= Ws || (!(SR <= Ws) && right_of);
     const double ro = left ? L.ro : R.ro, p = left ? L.p : R.p, Q = left ? L.Q : R.Q;
     const double u = left ? u1 : u2, v = left ? v1 : v2, S = left ? SL : SR, su = left ? suL : suR;
     const double vx = left ? L.u : R.u, vy = left ? L.v : R.v;
-    const double rg1 = 1.0 / (P.gamma - 1.0);
+    const double rg1 = 1.0 / (ga - 1.0);
     const double e = fma_rn(p, rg1, mul_rn(mul_rn(0.5, ro), fma_rn(vx, vx, mul_rn(vy, vy))));
     double F0 = mul_rn(ro, u), F1 = fma_rn(F0, u, p), F2 = mul_rn(F0, v), F3 = mul_rn(add_rn(e, p), u),
            F4 = mul_rn(Q, u);
-    if (!sup) {
-        if (SM >= 0.0 || SM < 0.0) {
-            const double r = den / fma_rn(S, den, -num), k = mul_rn(su, r);
-            const double roS = mul_rn(ro, k), QS = mul_rn(Q, k);
-            const double ptz = mul_rn(0.5, add_rn(fma_rn(mR, sub_rn(SM, u2), R.p), fma_rn(mL, sub_rn(SM, u1), L.p)));
-            const double ee = fma_rn(e, k, mul_rn(fma_rn(ptz, SM, -mul_rn(p, u)), r));
-            const double dro = sub_rn(roS, ro);
-            F1 = fma_rn(S, fma_rn(roS, SM, -F0), F1);
-            F0 = fma_rn(S, dro, F0);
-            F2 = fma_rn(S, mul_rn(dro, v), F2);
-            F3 = fma_rn(S, sub_rn(ee, e), F3);
-            F4 = fma_rn(S, sub_rn(QS, Q), F4);
-        } else {  // a NaN speed selects no side: zero flux, as the reference's chain of tests leaves it
-            F0 = F1 = F2 = F3 = F4 = 0.0;
+    if (sup) {
+        if (MOVING) {
+            F1 = fma_rn(-W, F0, F1);  // U = (ro, ro u, ro v, e, Q)
+            F2 = fma_rn(-W, mul_rn(ro, v), F2);
+            F0 = fma_rn(-W, ro, F0);
+            F3 = fma_rn(-W, e, F3);
+            F4 = fma_rn(-W, Q, F4);
         }
+    } else if (SM >= Ws || SM < Ws) {
+        const double r = den / fma_rn(S, den, -num), k = mul_rn(su, r);
+        const double roS = mul_rn(ro, k), QS = mul_rn(Q, k);
+        const double ptz = mul_rn(0.5, add_rn(fma_rn(mR, sub_rn(SM, u2), R.p), fma_rn(mL, sub_rn(SM, u1), L.p)));
+        const double ee = fma_rn(e, k, mul_rn(fma_rn(ptz, SM, -mul_rn(p, u)), r));
+        double vS = v;
+        if (SMOOTH && np) {  // tangential velocity of the HLL state, Setka.cpp:10644-10653
+            const double f1 = mul_rn(L.ro, sub_rn(SL, u1)), f2 = mul_rn(R.ro, sub_rn(SR, u2));
+            vS = fma_rn(f2, v2, -mul_rn(f1, v1)) / sub_rn(f2, f1);
+        }
+        const double roSM = mul_rn(roS, SM);
+        F1 = fma_rn(S, fma_rn(roS, SM, -F0), F1);
+        F2 = fma_rn(S, SMOOTH ? fma_rn(roS, vS, -mul_rn(ro, v)) : mul_rn(sub_rn(roS, ro), v), F2);
+        F0 = fma_rn(S, sub_rn(roS, ro), F0);
+        F3 = fma_rn(S, sub_rn(ee, e), F3);
+        F4 = fma_rn(S, sub_rn(QS, Q), F4);
+        if (MOVING) {
+            F0 = fma_rn(-W, roS, F0);
+            F1 = fma_rn(-W, roSM, F1);
+            F2 = fma_rn(-W, mul_rn(roS, vS), F2);
+            F3 = fma_rn(-W, ee, F3);
+            F4 = fma_rn(-W, QS, F4);
+        }
+    } else {  // a NaN speed selects no side: zero flux, as the reference's chain of tests leaves it
+        F0 = F1 = F2 = F3 = F4 = 0.0;
     }
     out[0] = F0;
     out[1] = fma_rn(n1, F1, mul_rn(n2, F2));
@@ -331,6 +353,12 @@ __device__ __forceinline__ double plain_flux(const gelios_params& P, const St5& 
     out[3] = F3;
     out[4] = F4;
     return dmax_ref(fabs(SL), fabs(SR));
+}
+// The plain form's flux: a face at rest, no smoothing (Setka.cpp:10484-10700).
+template <typename TF>
+__device__ __forceinline__ double plain_flux(const gelios_params& P, const St5& L, const St5& R, double n1, double n2,
+                                             double (&out)[5]) {
+    return hllc_lean<TF, false, false>(P.gamma, L, R, 0.0, n1, n2, false, out);
 }
 
 // ---------------------------------------------------------------- exact Godunov

@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -3341,218 +3342,333 @@ __global__ void hlld_batch_kernel(gelios_params P, int n, const double* __restri
 // fluids H1..H4, each with its own HLLC flux, on the grid moved by
 // Move_surface + Move_Setka_Calculate.  The 21-field state follows the
 // member order of Parametr's aggregate initialisers (Gran.cpp:262-265):
-// ro, p, u, v, Q, then ro, p, u, v of H1..H4.  One thread per cell, faces in
-// Grans order, every face evaluated from each side as the reference does.
-struct St21 {
-    double f[21];
-};
+// ro, p, u, v, Q, then ro, p, u, v of H1..H4.
 constexpr int kRo = 0, kP = 1, kU = 2, kV = 3, kQ = 4;
-__device__ __forceinline__ int fh(int k, int j) { return 5 + 4 * k + j; }  // hydrogen fluid k: ro, p, u, v
 constexpr double kHPow = 0.5;              // H_pow, Help.h:90
 constexpr double kNHOverKn = 1.0 / 6.0;   // n_H_LISM_ / Kn_, Help.h:60, 65
 
-__device__ __forceinline__ St21 load21(const double* const* st, const double* __restrict__ hs, size_t nc, int c) {
-    St21 s;
-#pragma unroll
-    for (int q = 0; q < 5; q++) s.f[q] = st[q][c];
-#pragma unroll
-    for (int q = 0; q < 16; q++) s.f[5 + q] = hs[q * nc + c];
-    return s;
-}
-__device__ __forceinline__ void mirror21(St21& s) {
-    s.f[kV] = -s.f[kV];
-#pragma unroll
-    for (int k = 0; k < 4; k++) s.f[fh(k, 3)] = -s.f[fh(k, 3)];
-}
-
-// Inner_sphere with the hydrogen fluids (Gran.cpp:236-265, 520-534): plasma
-// and H1 of the solar wind, H2..H4 of the master cell.
-__device__ __forceinline__ St21 inner_sphere21(const gelios_params& P, double x, double y, const St21& master) {
-    St21 s = master;
-    const St5 w = inner_sphere_state(P, x, y);
-    s.f[kRo] = w.ro;
-    s.f[kP] = w.p;
-    s.f[kU] = w.u;
-    s.f[kV] = w.v;
-    s.f[kQ] = w.Q;
-    const double dist = sqrt(x * x + y * y);
-    s.f[fh(0, 0)] = 0.0000001;
-    s.f[fh(0, 1)] = (0.0000001 * P.chi * P.chi / (P.gamma * 14.1344 * 14.1344));
-    s.f[fh(0, 2)] = P.chi * x / dist;
-    s.f[fh(0, 3)] = P.chi * y / dist;
-    return s;
-}
-// Input (Gran.cpp:267-276, 536-545): plasma and H4 of the LISM, H1..H3 of the master cell.
-__device__ __forceinline__ St21 input21(const gelios_params& P, const St21& master) {
-    St21 s = master;
-    s.f[kRo] = P.in_ro;
-    s.f[kP] = P.in_p;
-    s.f[kU] = P.in_u;
-    s.f[kV] = P.in_v;
-    s.f[kQ] = P.in_Q;
-    s.f[fh(3, 0)] = 1.0;
-    s.f[fh(3, 1)] = 0.5;
-    s.f[fh(3, 2)] = P.in_u;  // Velosity_inf
-    s.f[fh(3, 3)] = 0.0;
-    return s;
-}
-
-// Gran::Get_par with the hydrogen fluids (Gran.cpp:205-289); own = the face
-// master's state.
-__device__ St21 get_par21(const gelios_params& P, int ft, const St21& own, const double* const* st,
-                          const double* __restrict__ hs, size_t nc, int nb, double fx, double fy) {
-    switch (ft) {
-        case G_USUALY: return load21(st, hs, nc, nb);
-        case G_EXTERN: {
-            St21 s = own;
-            if (s.f[kU] >= 0.0) s.f[kU] = P.extern_u_par;
-            return s;
-        }
-        case G_AXIS: {
-            St21 s = own;
-            mirror21(s);
-            return s;
-        }
-        case G_INNER_SPHERE: return inner_sphere21(P, fx, fy, own);
-        case G_INPUT: return input21(P, own);
-        default: return own;  // Upper_wall
+// The state rows of the five fluids: fluid 0 the plasma (with Q), 1..4 the
+// hydrogen fluids H1..H4 (Q = the plasma's, which their flux ignores).
+struct K5Rows {
+    const double* const* st;
+    const double* hs;
+    size_t nc;
+    __device__ __forceinline__ St5 load(int f, int c) const {
+        if (f == 0) return load_state(st, c);
+        const double* h = hs + static_cast<size_t>(4 * (f - 1)) * nc + c;
+        return St5{h[0], h[nc], h[2 * nc], h[3 * nc], 0.0};
     }
+};
+
+// What the reconstruction of one side of a face needs of the grid, the same
+// for the five fluids.  M the side's cell, So the other one, Sd Sosed_down.
+struct K5Side {
+    int M, Sd;
+    bool axis, c1;
+    double dM, dS, r12;        // face centre to M and So, 1 / (dM - d(Sd))
+    double dm;                 // to the mirror image of M (axis cells without Sd)
+    // C_1 cells: |M|^2 / |f|^2, (|M| / |f|)^(2 gamma), sqrt(|M| / |f|), the
+    // same of So (S) and Sd (D), and the rotation to the face centre's frame
+    double kro, kp, kh, kroS, kpS, khS, kroD, kpD, khD, C, Sn;
+};
+template <int GROUP>
+__device__ __forceinline__ K5Side k5_side(const StepBuffers& b, int M, double xm, double ym, int So, double xs,
+                                          double ys, int Sd, uint32_t mf, double x2, double y2, double dM, double dS,
+                                          double dis2, double pdis, double cf, double sf) {
+    K5Side s;
+    s.M = M;
+    s.Sd = Sd;
+    s.axis = (mf & CF_AXIS) != 0;
+    s.c1 = GROUP != kPlainGroup && (mf & CF_C1);
+    s.dM = dM;
+    s.dS = dS;
+    s.r12 = s.dm = 0.0;
+    double xd = 0.0, yd = 0.0;
+    if (Sd >= 0) {
+        xd = b.cx[Sd];
+        yd = b.cy[Sd];
+        s.r12 = 1.0 / (dM - sqrt(sq(x2 - xd) + sq(y2 - yd)));
+    } else if (s.axis) {
+        s.dm = sqrt(sq(x2 - xm) + sq(y2 + ym));
+        s.r12 = 1.0 / (dM - s.dm);
+    }
+    if (s.c1) {
+        auto fac = [&](double x, double y, double rp, double& ro, double& p, double& h) {
+            ro = (sq(x) + sq(y)) / dis2;
+            p = rp / pdis;
+            h = sqrt(sqrt(ro));  // (|c| / |f|)^H_pow
+        };
+        fac(xm, ym, b.rp[M], s.kro, s.kp, s.kh);
+        fac(xs, ys, b.rp[So], s.kroS, s.kpS, s.khS);
+        if (Sd >= 0) {
+            fac(xd, yd, b.rp[Sd], s.kroD, s.kpD, s.khD);
+        } else {  // the mirrored centre has the radius of M itself
+            s.kroD = s.kro;
+            s.kpD = s.kp;
+            s.khD = s.kh;
+        }
+        double c1, s1;
+        polar_cs(xm, ym, c1, s1);
+        s.C = c1 * cf + s1 * sf;
+        s.Sn = c1 * sf - s1 * cf;
+    }
+    return s;
 }
 
-// Gran::Get_par_TVD of an Usualy face with the hydrogen fluids
-// (Gran.cpp:296-472): master M (state Ms, centroid Mx, My), Sosed So,
-// Sosed_down Sd, face centre (fx, fy).
-__device__ St21 tvd21_usualy(const double* const* st, const double* __restrict__ hs, size_t nc, const double* cx,
-                             const double* cy, double fx, double fy, const St21& Ms, double Mx, double My, int So,
-                             int Sd, bool m_has_axis, bool tracked, int* status) {
-    if (Sd < 0) {
-        St21 par = Ms;
-        if (m_has_axis) {  // Gran.cpp:308-338: mirrored master below the axis
-            const St21 par3 = load21(st, hs, nc, So);
-            const double dist2 = sqrt(sq(fx - Mx) + sq(fy - My));
-            const double dist3 = sqrt(sq(fx - cx[So]) + sq(fy - cy[So]));
-            const double dist1 = sqrt(sq(fx - Mx) + sq(fy - (-My)));
-            const int vi[5] = {kV, fh(0, 3), fh(1, 3), fh(2, 3), fh(3, 3)};
-#pragma unroll
-            for (int q = 0; q < 5; q++)
-                par.f[vi[q]] = linear3(-dist1, -Ms.f[vi[q]], -dist2, Ms.f[vi[q]], dist3, par3.f[vi[q]], 0.0);
-        }
-        return par;
-    }
-    const St21 par1 = load21(st, hs, nc, Sd);
-    const double dist2 = sqrt(sq(fx - Mx) + sq(fy - My));
-    St21 o;
-    if (tracked) {  // Gran.cpp:345-426
-        const double dist1 = sqrt(sq(fx - cx[Sd]) + sq(fy - cy[Sd]));
-        const double r = 1.0 / (-dist1 - (-dist2)), x2 = -dist2;
-#pragma unroll
-        for (int q = 0; q < 21; q++) o.f[q] = (par1.f[q] - Ms.f[q]) * r * (0.0 - x2) + Ms.f[q];
-        if (o.f[kRo] <= 0.0) o.f[kRo] = Ms.f[kRo];
-        if (o.f[kP] <= 0.0) o.f[kP] = Ms.f[kP];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (o.f[fh(k, 0)] <= 0.0) o.f[fh(k, 0)] = Ms.f[fh(k, 0)];
-            if (o.f[fh(k, 1)] <= 0.0) o.f[fh(k, 1)] = Ms.f[fh(k, 1)];
+// Fluid f at a Usualy face seen from s.M (state Ms; So's state Ss): Get_par_TVD
+// (Gran.cpp:296-472), or in C_1 cells the radial scaling of Setka.cpp:8337-8349
+// with Get_par_TVD_radial (Gran.cpp:562-675) for ro and p of the plasma and H1.
+template <int GROUP>
+__device__ __forceinline__ St5 k5_recon(const K5Rows& rows, const K5Side& s, double r23, bool tracked, int f,
+                                        const St5& Ms, const St5& Ss, int* status) {
+    St5 o = Ms;
+    const double x2 = -s.dM;
+    if (s.c1) {
+        if (f > 1) return o;
+        o.u = Ms.u * s.C - Ms.v * s.Sn;
+        o.v = Ms.u * s.Sn + Ms.v * s.C;
+        if (f == 0) o.Q = Ms.Q * s.kro;
+        if (s.Sd < 0 && !s.axis) return o;
+        const St5 p1 = s.Sd >= 0 ? rows.load(f, s.Sd) : Ms;
+        if (f == 0) {
+            o.ro = linear3r(p1.ro * s.kroD, Ms.ro * s.kro, Ss.ro * s.kroS, s.r12, r23, x2);
+            o.p = linear3r(p1.p * s.kpD, Ms.p * s.kp, Ss.p * s.kpS, s.r12, r23, x2);
+        } else {
+            o.ro = linear3r(p1.ro * s.khD, Ms.ro * s.kh, Ss.ro * s.khS, s.r12, r23, x2);
+            o.p = linear3r(p1.p, Ms.p, Ss.p, s.r12, r23, x2);
         }
         return o;
     }
-    const St21 par3 = load21(st, hs, nc, So);
-    const double dist3 = sqrt(sq(fx - cx[So]) + sq(fy - cy[So]));
-    const double dist1 = sqrt(sq(fx - cx[Sd]) + sq(fy - cy[Sd]));
-    const double r12 = 1.0 / (-dist1 - (-dist2)), r23 = 1.0 / (-dist2 - dist3), x2 = -dist2;
-#pragma unroll
-    for (int q = 0; q < 21; q++) o.f[q] = linear3r(par1.f[q], Ms.f[q], par3.f[q], r12, r23, x2);
-    if (o.f[kRo] <= 0.0 || o.f[kP] <= 0.0) *status |= ST_TVD_BAD;  // the reference exits (Gran.cpp:444-455)
-    return o;
-}
-
-// Gran::Get_par_TVD of an Axis face with the hydrogen fluids (Gran.cpp:486-519).
-__device__ St21 tvd21_axis(const double* const* st, const double* __restrict__ hs, size_t nc, const double* cx,
-                           const double* cy, double fx, double fy, const St21& Ms, double Mx, double My, int Sd) {
-    St21 o = Ms;
-    if (Sd < 0) return o;
-    const St21 par1 = load21(st, hs, nc, Sd);
-    const double dist2 = sqrt(sq(fx - Mx) + sq(fy - My));
-    const double dist1 = sqrt(sq(fx - cx[Sd]) + sq(fy - cy[Sd]));
-    const int vi[5] = {kV, fh(0, 3), fh(1, 3), fh(2, 3), fh(3, 3)};
-#pragma unroll
-    for (int q = 0; q < 5; q++)
-        o.f[vi[q]] = linear3(-dist1, par1.f[vi[q]], -dist2, Ms.f[vi[q]], dist2, -Ms.f[vi[q]], 0.0);
-    return o;
-}
-
-// Gran::Get_par_TVD_radial with the H1 fields (Gran.cpp:562-675): o = ro,
-// p, p_H1, ro_H1 (the fields Go_5_komponent takes from it,
-// Setka.cpp:8342-8349).
-__device__ void tvd21_radial(const double* const* st, const double* __restrict__ hs, size_t nc, const double* cx,
-                             const double* cy, double fx, double fy, const St21& Ms, double Mx, double My, int So,
-                             int Sd, bool m_has_axis, double g2, double* o) {
-    const double r = sqrt(sq(fx) + sq(fy));
-    St21 par1, par3;
-    double r1, r2, r3, dist1, dist2, dist3;
-    if (Sd < 0) {
-        if (!m_has_axis) {
-            o[0] = Ms.f[kRo];
-            o[1] = Ms.f[kP];
-            o[2] = Ms.f[fh(0, 1)];
-            o[3] = Ms.f[fh(0, 0)];
-            return;
-        }
-        par1 = Ms;
-        mirror21(par1);
-        par3 = load21(st, hs, nc, So);
-        r2 = sqrt(sq(Mx) + sq(My));
-        dist2 = sqrt(sq(fx - Mx) + sq(fy - My));
-        r3 = sqrt(sq(cx[So]) + sq(cy[So]));
-        dist3 = sqrt(sq(fx - cx[So]) + sq(fy - cy[So]));
-        r1 = sqrt(sq(Mx) + sq(-My));
-        dist1 = sqrt(sq(fx - Mx) + sq(fy - (-My)));
-    } else {
-        par1 = load21(st, hs, nc, Sd);
-        par3 = load21(st, hs, nc, So);
-        r2 = sqrt(sq(Mx) + sq(My));
-        dist2 = sqrt(sq(fx - Mx) + sq(fy - My));
-        r3 = sqrt(sq(cx[So]) + sq(cy[So]));
-        dist3 = sqrt(sq(fx - cx[So]) + sq(fy - cy[So]));
-        r1 = sqrt(sq(cx[Sd]) + sq(cy[Sd]));
-        dist1 = sqrt(sq(fx - cx[Sd]) + sq(fy - cy[Sd]));
+    if (s.Sd < 0) {
+        if (s.axis) o.v = linear3r(-Ms.v, Ms.v, Ss.v, s.r12, r23, x2);  // Gran.cpp:308-338
+        return o;
     }
-    const double r12 = 1.0 / (-dist1 - (-dist2)), r23 = 1.0 / (-dist2 - dist3), x2 = -dist2;
-    o[0] = linear3r(par1.f[kRo] * sq(r1), Ms.f[kRo] * sq(r2), par3.f[kRo] * sq(r3), r12, r23, x2) / sq(r);
-    o[1] = linear3r(par1.f[kP] * pow(r1, g2), Ms.f[kP] * pow(r2, g2), par3.f[kP] * pow(r3, g2), r12, r23, x2) /
-           pow(r, g2);
-    o[2] = linear3r(par1.f[fh(0, 1)], Ms.f[fh(0, 1)], par3.f[fh(0, 1)], r12, r23, x2);
-    o[3] = linear3r(par1.f[fh(0, 0)] * pow(r1, kHPow), Ms.f[fh(0, 0)] * pow(r2, kHPow),
-                    par3.f[fh(0, 0)] * pow(r3, kHPow), r12, r23, x2) /
-           pow(r, kHPow);
+    const St5 p1 = rows.load(f, s.Sd);
+    if (GROUP == kAnyGroup && tracked) {  // Gran.cpp:345-426
+        const double r = s.r12;
+        o.ro = (p1.ro - Ms.ro) * r * (0.0 - x2) + Ms.ro;
+        o.p = (p1.p - Ms.p) * r * (0.0 - x2) + Ms.p;
+        o.u = (p1.u - Ms.u) * r * (0.0 - x2) + Ms.u;
+        o.v = (p1.v - Ms.v) * r * (0.0 - x2) + Ms.v;
+        o.Q = (p1.Q - Ms.Q) * r * (0.0 - x2) + Ms.Q;
+        if (o.ro <= 0.0) o.ro = Ms.ro;
+        if (o.p <= 0.0) o.p = Ms.p;
+        return o;
+    }
+    o.ro = linear3r(p1.ro, Ms.ro, Ss.ro, s.r12, r23, x2);
+    o.p = linear3r(p1.p, Ms.p, Ss.p, s.r12, r23, x2);
+    o.u = linear3r(p1.u, Ms.u, Ss.u, s.r12, r23, x2);
+    o.v = linear3r(p1.v, Ms.v, Ss.v, s.r12, r23, x2);
+    if (f == 0) {
+        o.Q = linear3r(p1.Q, Ms.Q, Ss.Q, s.r12, r23, x2);
+        if (o.ro <= 0.0 || o.p <= 0.0) *status |= ST_TVD_BAD;  // the reference exits (Gran.cpp:444-455)
+    }
+    return o;
 }
 
-// radial scaling of a side's state to the face centre (Setka.cpp:8337-8341)
-__device__ __forceinline__ void radial_scale21(St21& s, double rc, double dis, double g2) {
-    s.f[kRo] = s.f[kRo] * sq(rc) / sq(dis);
-    s.f[fh(0, 0)] = s.f[fh(0, 0)] * pow(rc / dis, kHPow);
-    s.f[kQ] = s.f[kQ] * sq(rc) / sq(dis);
-    s.f[kP] = s.f[kP] * pow(rc / dis, g2);
+// The two states of fluid f at a boundary face of cell `own` (Gran.cpp:205-289
+// and 486-545, Setka.cpp:8392-8440).
+__device__ __forceinline__ void k5_boundary(const gelios_params& P, const K5Rows& rows, const K5Side& s, int ft,
+                                            double x2, double y2, int f, const St5& own, St5& L, St5& R) {
+    L = own;
+    R = own;
+    if (ft == G_EXTERN) {
+        if (f == 0 && R.u >= 0.0) R.u = P.extern_u_par;
+    } else if (ft == G_INNER_SPHERE) {
+        // plasma and H1 of the solar wind, H2..H4 of the cell
+        if (f == 0) {
+            L.ro = own.ro * s.kro;
+            L.Q = own.Q * s.kro;
+            L.p = own.p * s.kp;
+            R = inner_sphere_state(P, x2, y2);
+        } else if (f == 1) {
+            L.ro = own.ro * s.kh;
+            const double dist = sqrt(x2 * x2 + y2 * y2);
+            R.ro = 0.0000001;
+            R.p = (0.0000001 * P.chi * P.chi / (P.gamma * 14.1344 * 14.1344));
+            R.u = P.chi * x2 / dist;
+            R.v = P.chi * y2 / dist;
+        }
+    } else if (ft == G_INPUT) {
+        // plasma and H4 of the LISM, H1..H3 of the cell
+        if (f == 0) {
+            R = input_state(P);
+        } else if (f == 4) {
+            R.ro = 1.0;
+            R.p = 0.5;
+            R.u = P.in_u;  // Velosity_inf
+            R.v = 0.0;
+        }
+    } else if (ft == G_AXIS) {
+        if (s.c1) {
+            if (f == 0) {
+                L.ro = own.ro * s.kro;
+                L.Q = own.Q * s.kro;
+                L.p = own.p * s.kp;
+            } else if (f == 1) {
+                L.ro = own.ro * s.kh;
+            }
+            if (f <= 1) {
+                L.u = own.u * s.C - own.v * s.Sn;
+                L.v = own.u * s.Sn + own.v * s.C;
+            }
+        } else if (s.Sd >= 0) {  // Gran.cpp:486-519
+            const St5 p1 = rows.load(f, s.Sd);
+            L.v = linear3r(p1.v, own.v, -own.v, s.r12, -0.5 / s.dM, -s.dM);
+        }
+        R = L;
+        R.v = -R.v;
+    }
+}
+
+// Go_5_komponent face units (the face loop of Setka.cpp:8300-8570): each face
+// once, after the motion.  The geometry of both sides' reconstructions once,
+// then fluid by fluid: both sides' states, the HLLC flux through the moving
+// face (on tracked faces the plasma takes the exact Godunov flux and HLLC's
+// tracer flux), F*S into the unit's row (the reference evaluates the face
+// from each side; the two results are negatives of each other up to
+// rounding).  Flux rows: plasma mass, mom x, mom y, energy, Q (0-4), then
+// mass, mom x, mom y, energy of H1..H4 (5-20).  Returns the minimum of the
+// CFL candidates of each updated side, H1's only where that side is not
+// C_centr (Setka.cpp:8500): kurant * distance / the largest wave speed.
+// Holding all 21 fields of four cells at once took 255 registers and spilled,
+// in one launch of every kind of unit: 223 us on the 200k grid (401k units,
+// ncu).  One fluid at a time in a launch per group: 73 us for the plain units
+// at 96 registers (21, 31, 20 us for the C_1, tracked and one-sided ones
+// beside them); 80 or 128 registers, or the fluids unrolled: 1-5% slower per
+// step.  Bound by the latency of its loads and FP64 chains.
+// COOP: all lanes of a warp evaluate one tracked unit; lane 0 stores.
+template <int GROUP, bool COOP>
+__device__ __forceinline__ double k5_face_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
+                                               const double* __restrict__ hcur, double* __restrict__ fl, int u,
+                                               int& status) {
+    constexpr bool USUALY = GROUP != kAnyGroup || COOP;
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    const size_t nu = d.n_units;
+    const int K = d.u_cell[u], nb = d.u_nb[u];
+    const uint32_t info = d.u_info[u];
+    const uint32_t cf = (info >> UI_CF_OWN) & 15u, nbf = (info >> UI_CF_NB) & 15u;
+    const double x = b.cx[K], y = b.cy[K];
+    const bool procK = !(sq(x) + sq(y) < d.r11_sq);
+    double x3 = 0.0, y3 = 0.0;
+    bool procN = false;
+    if (nb >= 0) {
+        x3 = b.cx[nb];
+        y3 = b.cy[nb];
+        procN = !(sq(x3) + sq(y3) < d.r11_sq);
+    }
+    if (!(procK || procN)) return inf;
+    const int ft = USUALY ? static_cast<int>(G_USUALY) : static_cast<int>(info & SI_TYPE_MASK);
+    const bool tracked = COOP;
+    const int A = d.u_A[u], B = d.u_B[u];
+    const double xa = d.X[A], ya = d.Y[A], xb = d.X[B], yb = d.Y[B];
+    const double x2 = (xa + xb) / 2.0, y2 = (ya + yb) / 2.0;
+    const double x4 = (d.X2[A] + d.X2[B]) / 2.0, y4 = (d.Y2[A] + d.Y2[B]) / 2.0;
+    const double S = sqrt(sq(xb - xa) + sq(yb - ya)), rS = 1.0 / S;
+    const double n1 = (yb - ya) * rS, n2 = -((xb - xa) * rS);
+    const double W = ((x4 - x2) * n1 + (y4 - y2) * n2) / *b.dt_cur;
+    const double dK = sqrt(sq(x - x2) + sq(y - y2)), dN = sqrt(sq(x3 - x2) + sq(y3 - y2));
+    const double dis2 = sq(x2) + sq(y2);
+    const bool radial = GROUP != kPlainGroup && ((cf & CF_C1) || ft == G_INNER_SPHERE || (nb >= 0 && (nbf & CF_C1)));
+    double pdis = 1.0, cfc = 1.0, sfc = 0.0;
+    if (radial) {
+        pdis = pow2g(sqrt(dis2), 2.0 * P.gamma);
+        polar_cs(x2, y2, cfc, sfc);
+    }
+    // an inner-sphere face scales its cell as a C_1 side does
+    const K5Side sK = k5_side<GROUP>(b, K, x, y, nb >= 0 ? nb : K, nb >= 0 ? x3 : x, nb >= 0 ? y3 : y, d.u_sd[u],
+                                     ft == G_INNER_SPHERE ? (cf | CF_C1) : cf, x2, y2, dK, dN, dis2, pdis, cfc, sfc);
+    K5Side sN{};
+    double r23 = 0.0;
+    if (USUALY || ft == G_USUALY) {
+        sN = k5_side<GROUP>(b, nb, x3, y3, K, x, y, d.u_sd2[u], nbf, x2, y2, dN, dK, dis2, pdis, cfc, sfc);
+        r23 = 1.0 / (-dK - dN);
+    }
+    const K5Rows rows{b.cur, hcur, static_cast<size_t>(d.n_cells)};
+    double um = 0.0, um1 = 0.0;  // largest wave speed without H1, of H1
+#pragma unroll 1
+    for (int f = 0; f < 5; f++) {
+        const St5 own = rows.load(f, K);
+        St5 L, R;
+        if (USUALY || ft == G_USUALY) {
+            const St5 oth = rows.load(f, nb);
+            constexpr int G = COOP ? kAnyGroup : GROUP;
+            L = k5_recon<G>(rows, sK, r23, tracked, f, own, oth, &status);
+            R = k5_recon<G>(rows, sN, r23, tracked, f, oth, own, &status);
+        } else {
+            k5_boundary(P, rows, sK, ft, x2, y2, f, own, L, R);
+        }
+        double F[5];
+        double UU = hllc_lean<double, true, true>(P.gamma, L, R, W, n1, n2, f == 0 && (info & SI_NP), F);
+        if (COOP && f == 0) {
+            double q1[5] = {L.ro, L.p, L.u, L.v, 0.0}, q2[5] = {R.ro, R.p, R.u, R.v, 0.0};
+            double nv[3] = {n1, n2, 0.0}, qq[5], ds[3];
+            const double UG = godunov_dev<true>(P.gamma, P.kurant, q1, q2, nv, qq, ds, W, 1.0, P.godunov_max_iter,
+                                                &status);
+            F[0] = qq[0];
+            F[1] = qq[1];
+            F[2] = qq[2];
+            F[3] = qq[4];
+            um = UG > um ? UG : um;
+        }
+        if (!COOP || (threadIdx.x & 31) == 0) {
+            double* o = fl + (f == 0 ? 0 : 1 + 4 * f) * nu + u;
+#pragma unroll
+            for (int k = 0; k < 4; k++) o[k * nu] = F[k] * S;
+            if (f == 0) o[4 * nu] = F[4] * S;
+        }
+        if (f == 1) um1 = UU > um1 ? UU : um1;
+        else um = UU > um ? UU : um;
+    }
+    const double ua = um1 > um ? um1 : um;
+    double t = inf;
+    if (procK) t = dmin_ref(t, P.kurant * dK / ((cf & CF_CENTR) ? um : ua));
+    if (nb >= 0 && procN) t = dmin_ref(t, P.kurant * dN / ((nbf & CF_CENTR) ? um : ua));
+    return t;
+}
+template <int GROUP, int MINB>
+__global__ void __launch_bounds__(128, MINB) k5_face_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                            const double* __restrict__ hcur, double* __restrict__ fl,
+                                                            int n_launch) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double t = __longlong_as_double(0x7ff0000000000000LL);
+    int status = 0;
+    if (i < n_launch) {
+        const int u = GROUP == kPlainGroup ? i : GROUP == kC1Group ? d.u_c1 + i : d.u_tr1 + i;
+        t = k5_face_body<GROUP, false>(d, P, b, hcur, fl, u, status);
+    }
+    block_reduce_commit(t, 0, 0, status, b.dt_acc, b.counters, b.status);
+}
+// The tracked units, one warp each: the exact solver's bisection runs
+// warp-cooperatively (one thread per unit holds up its block for 30
+// iterations in a row).
+__global__ void __launch_bounds__(64) k5_tracked_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                        const double* __restrict__ hcur, double* __restrict__ fl) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    double t = __longlong_as_double(0x7ff0000000000000LL);
+    int status = 0;
+    if (i < d.u_tr1 - d.u_tr0) t = k5_face_body<kAnyGroup, true>(d, P, b, hcur, fl, d.u_tr0 + i, status);
+    block_reduce_commit(t, 0, 0, status, b.dt_acc, b.counters, b.status);
 }
 
 // conservative update of one hydrogen fluid with its sources and the
 // cylindrical terms (Setka.cpp:8808-8940)
 __device__ __forceinline__ void k5_update_h(double ga, const double* pot, double ro_H, double p_H, double u_H,
                                             double v_H, double q1, double q21, double q22, double q3, double VV,
-                                            double rV2, double y, double dt, double ro_floor, double p_floor,
+                                            double rV2, double ry, double dt, double ro_floor, double p_floor,
                                             double* out, int& nro, int& npc) {
-    double ro3 = ro_H * VV - dt * (pot[0] * rV2 + ro_H * v_H / y - q1);
+    const double gm1 = ga - 1, rg1 = 1.0 / gm1, vy = v_H * ry, ek = ro_H * (u_H * u_H + v_H * v_H) * 0.5;
+    double ro3 = ro_H * VV - dt * (pot[0] * rV2 + ro_H * vy - q1);
     if (ro3 <= 0) {
         ro3 = ro_floor;
         nro++;
     }
     const double rro3 = 1.0 / ro3;
-    const double u3 = (ro_H * u_H * VV - dt * (pot[1] * rV2 + ro_H * v_H * u_H / y - q21)) * rro3;
-    const double v3 = (ro_H * v_H * VV - dt * (pot[2] * rV2 + ro_H * v_H * v_H / y - q22)) * rro3;
-    double p3 = (((p_H / (ga - 1) + ro_H * (u_H * u_H + v_H * v_H) * 0.5) * VV -
-                  dt * (pot[3] * rV2 + v_H * (ga * p_H / (ga - 1) + ro_H * (u_H * u_H + v_H * v_H) * 0.5) / y - q3)) -
+    const double u3 = (ro_H * u_H * VV - dt * (pot[1] * rV2 + ro_H * vy * u_H - q21)) * rro3;
+    const double v3 = (ro_H * v_H * VV - dt * (pot[2] * rV2 + ro_H * vy * v_H - q22)) * rro3;
+    double p3 = (((p_H * rg1 + ek) * VV - dt * (pot[3] * rV2 + vy * (ga * p_H * rg1 + ek) - q3)) -
                  0.5 * ro3 * (u3 * u3 + v3 * v3)) *
-                (ga - 1);
+                gm1;
     if (p3 <= 0) {
         p3 = p_floor;
         npc++;
@@ -3563,327 +3679,219 @@ __device__ __forceinline__ void k5_update_h(double ga, const double* pot, double
     out[3] = v3;
 }
 
-// Go_5_komponent face units (the face loop of Setka.cpp:8300-8570): each
-// face once, after the motion.  Both sides' 21-field reconstructions (the
-// plasma and H1..H4; radial in C_1 cells), four hydrogen HLLC problems and
-// the plasma's HLLC (exact Godunov plus HLLC's tracer flux on tracked
-// faces); F*S to the owner slot, -F*S to the twin (the reference evaluates
-// the face from each side; the two results are negatives of each other up to
-// rounding).  Flux rows: plasma mass, mom x, mom y, energy, Q (0-4), then
-// mass, mom x, mom y, energy of H1..H4 (5-20).  CFL candidates of each
-// updated side, H1's only where that side is not C_centr (Setka.cpp:8500).
-__global__ void __launch_bounds__(128) k5_face_kernel(DevMesh d, gelios_params P, StepBuffers b,
-                                                      const double* __restrict__ hcur, double* __restrict__ fl) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    double tmin = __longlong_as_double(0x7ff0000000000000LL);
-    int status = 0;
-    if (u < d.n_units) {
-        const size_t nc = d.n_cells, ng = d.n_slots;
-        const int c = d.u_cell[u], nb = d.u_nb[u];
-        const uint32_t info = d.u_info[u];
-        const uint32_t cf = (info >> UI_CF_OWN) & 15u, nbf = (info >> UI_CF_NB) & 15u;
-        const double x = b.cx[c], y = b.cy[c];
-        const double radius = sqrt(sq(x) + sq(y));
-        const bool procK = !(radius < P.R11);
-        double x3 = 0.0, y3 = 0.0;
-        bool procN = false;
-        if (nb >= 0) {
-            x3 = b.cx[nb];
-            y3 = b.cy[nb];
-            procN = !(sqrt(sq(x3) + sq(y3)) < P.R11);
-        }
-        if (procK || procN) {
-            const double ga = P.gamma, g2 = 2.0 * P.gamma;
-            const double dt = *b.dt_cur;
-            const bool kC1 = (cf & CF_C1) != 0;
-            const St21 par1 = load21(b.cur, hcur, nc, c);
-            const int ft = info & SI_TYPE_MASK;
-            const int A = d.u_A[u], B = d.u_B[u];
-            const double xa = d.X[A], ya = d.Y[A], xb = d.X[B], yb = d.Y[B];
-            const double S = sqrt(sq(xb - xa) + sq(yb - ya));
-            const double x2 = (xa + xb) / 2.0, y2 = (ya + yb) / 2.0;
-            const double x4 = (d.X2[A] + d.X2[B]) / 2.0, y4 = (d.Y2[A] + d.Y2[B]) / 2.0;
-            const double dist = sqrt(sq(x - x2) + sq(y - y2));
-            St21 par11 = par1;
-            St21 par2 = get_par21(P, ft, par1, b.cur, hcur, nc, nb, x2, y2);
-            double t1 = xb - xa, t2 = yb - ya;
-            const double nn = sqrt(sq(t1) + sq(t2));
-            t1 = t1 / nn;
-            t2 = t2 / nn;
-            const double n1 = t2, n2 = -t1;
-            const double W = ((x4 - x2) * n1 + (y4 - y2) * n2) / dt;
-            const double dis = sqrt(sq(x2) + sq(y2));
-            const bool tracked = (info & SI_GOD) != 0;
-            if (ft == G_USUALY) {
-                const double dd = sqrt(sq(x3) + sq(y3));
-                if (kC1) {
-                    radial_scale21(par11, radius, dis, g2);
-                    polar_perenos(x, y, x2, y2, par11.f[kU], par11.f[kV]);
-                    polar_perenos(x, y, x2, y2, par11.f[fh(0, 2)], par11.f[fh(0, 3)]);
-                    double o[4];
-                    tvd21_radial(b.cur, hcur, nc, b.cx, b.cy, x2, y2, par1, x, y, nb, d.u_sd[u], (cf & CF_AXIS) != 0,
-                                 g2, o);
-                    par11.f[kRo] = o[0];
-                    par11.f[kP] = o[1];
-                    par11.f[fh(0, 1)] = o[2];
-                    par11.f[fh(0, 0)] = o[3];
-                } else {
-                    par11 = tvd21_usualy(b.cur, hcur, nc, b.cx, b.cy, x2, y2, par1, x, y, nb, d.u_sd[u],
-                                         (cf & CF_AXIS) != 0, tracked, &status);
-                }
-                if (nbf & CF_C1) {
-                    const St21 parN = par2;  // the neighbour's stored state
-                    radial_scale21(par2, dd, dis, g2);
-                    polar_perenos(x3, y3, x2, y2, par2.f[kU], par2.f[kV]);
-                    polar_perenos(x3, y3, x2, y2, par2.f[fh(0, 2)], par2.f[fh(0, 3)]);
-                    double o[4];
-                    tvd21_radial(b.cur, hcur, nc, b.cx, b.cy, x2, y2, parN, x3, y3, c, d.u_sd2[u],
-                                 (nbf & CF_AXIS) != 0, g2, o);
-                    par2.f[kRo] = o[0];
-                    par2.f[kP] = o[1];
-                    par2.f[fh(0, 1)] = o[2];
-                    par2.f[fh(0, 0)] = o[3];
-                } else {
-                    par2 = tvd21_usualy(b.cur, hcur, nc, b.cx, b.cy, x2, y2, par2, x3, y3, c, d.u_sd2[u],
-                                        (nbf & CF_AXIS) != 0, tracked, &status);
-                }
-            } else if (ft == G_INNER_SPHERE) {
-                radial_scale21(par11, radius, dis, g2);
-            } else if (kC1 && ft == G_AXIS) {
-                radial_scale21(par11, radius, dis, g2);
-                polar_perenos(x, y, x2, y2, par11.f[kU], par11.f[kV]);
-                polar_perenos(x, y, x2, y2, par11.f[fh(0, 2)], par11.f[fh(0, 3)]);
-                par2 = par11;
-                mirror21(par2);
-            } else if (!kC1 && ft == G_AXIS) {
-                par11 = tvd21_axis(b.cur, hcur, nc, b.cx, b.cy, x2, y2, par1, x, y, d.u_sd[u]);
-                par2 = par11;
-                mirror21(par2);
-            }
-            const bool np = (info & SI_NP) != 0;
-            const int g = d.u_slot[u], gt = d.u_twin[u];
-            FluxOut<double> F;
-            double UUh[4];
-            for (int hk = 0; hk < 4; hk++) {
-                St5 L, R;
-                L.ro = par11.f[fh(hk, 0)];
-                L.p = par11.f[fh(hk, 1)];
-                L.u = par11.f[fh(hk, 2)];
-                L.v = par11.f[fh(hk, 3)];
-                L.Q = par11.f[kQ];
-                R.ro = par2.f[fh(hk, 0)];
-                R.p = par2.f[fh(hk, 1)];
-                R.u = par2.f[fh(hk, 2)];
-                R.v = par2.f[fh(hk, 3)];
-                R.Q = par2.f[kQ];
-                UUh[hk] = hllc_flux<double>(ga, P.kurant, L, R, W, n1, n2, 1.0, 1, false, F);
-                const double h[4] = {F.P0 * S, F.P1 * S, F.P2 * S, F.P3 * S};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    fl[(5 + 4 * hk + j) * ng + g] = h[j];
-                    if (gt >= 0) fl[(5 + 4 * hk + j) * ng + gt] = -h[j];
-                }
-            }
-            St5 L, R;
-            L.ro = par11.f[kRo];
-            L.p = par11.f[kP];
-            L.u = par11.f[kU];
-            L.v = par11.f[kV];
-            L.Q = par11.f[kQ];
-            R.ro = par2.f[kRo];
-            R.p = par2.f[kP];
-            R.u = par2.f[kU];
-            R.v = par2.f[kV];
-            R.Q = par2.f[kQ];
-            double pl[5];
-            double UG = 0.0;
-            if (tracked) {
-                double q1[5] = {L.ro, L.p, L.u, L.v, 0.0};
-                double q2[5] = {R.ro, R.p, R.u, R.v, 0.0};
-                double nvv[3] = {n1, n2, 0.0};
-                double qq[5], ds[3];
-                UG = godunov_dev<false>(ga, P.kurant, q1, q2, nvv, qq, ds, W, dist, P.godunov_max_iter, &status);
-                pl[0] = qq[0] * S;
-                pl[1] = qq[1] * S;
-                pl[2] = qq[2] * S;
-                pl[3] = qq[4] * S;
-            }
-            const double UU = hllc_flux<double>(ga, P.kurant, L, R, W, n1, n2, 1.0, 1, np, F);
-            if (!tracked) {
-                pl[0] = F.P0 * S;
-                pl[1] = F.P1 * S;
-                pl[2] = F.P2 * S;
-                pl[3] = F.P3 * S;
-            }
-            pl[4] = F.PQ * S;
-#pragma unroll
-            for (int j = 0; j < 5; j++) {
-                fl[j * ng + g] = pl[j];
-                if (gt >= 0) fl[j * ng + gt] = -pl[j];
-            }
-            // CFL candidates in the reference's order per side (Setka.cpp:8500-8560)
-            auto side = [&](double dd, bool centr) {
-                for (int hk = 0; hk < 4; hk++)
-                    if (!(hk == 0 && centr)) tmin = dmin_ref(tmin, P.kurant * dd / UUh[hk]);
-                if (tracked) tmin = dmin_ref(tmin, P.kurant * dd / UG);
-                tmin = dmin_ref(tmin, P.kurant * dd / UU);
-            };
-            if (procK) side(dist, (cf & CF_CENTR) != 0);
-            if (gt >= 0 && procN) side(sqrt(sq(x3 - x2) + sq(y3 - y2)), (nbf & CF_CENTR) != 0);
-        }
-    }
-    block_reduce_commit(tmin, 0, 0, status, b.dt_acc, b.counters, b.status);
-}
-
-// Go_5_komponent cell update (Setka.cpp:8570-8950) from the summed face
-// slots: multi-fluid charge exchange, cylindrical 1/y terms, clamps; it also
-// refills the geometry cache for the next step.
-__global__ void __launch_bounds__(128) k5_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
-                                                        const double* __restrict__ fl,
-                                                        const double* __restrict__ hcur, double* __restrict__ hnxt) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double tmin = __longlong_as_double(0x7ff0000000000000LL);
-    int nro = 0, npc = 0, status = 0;
-    const size_t nc = d.n_cells;
+// Go_5_komponent cell update (Setka.cpp:8570-8950) from the face units' fluxes
+// summed in Grans order: multi-fluid charge exchange, cylindrical 1/y terms,
+// clamps; it also refills the geometry cache for the next step.  The area
+// before the motion comes from that cache; a quadrilateral's corners come in
+// one load.
+// 32 cells per warp in three phases, every lane busy in each: one lane per
+// cell (geometry, the plasma's state, into shared memory), four rounds of
+// eight cells x four hydrogen fluids (a fluid's exchange rate, its update;
+// the rates summed over the cell's four lanes in fluid order), one lane per
+// cell again (the plasma's update).  With one thread per cell throughout, 21
+// fields and 21 flux sums took 128 registers: 89 us against 78 on the 200k
+// grid (97 before the flux rows were the units'; ncu).
+__global__ void __launch_bounds__(128, 6) k5_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                           const double* __restrict__ fl,
+                                                           const double* __restrict__ hcur, double* __restrict__ hnxt) {
+    // per-cell values of the block's 128 cells: u, v, ro, p/ro, V/V2, 1/V2, 1/y, then the summed exchange terms
+    __shared__ double sd[10][128];
+    __shared__ int si[128];    // kind of the cell (Cell_type), -1: not updated
+    __shared__ int4 ssu[128];  // the units of a quadrilateral's four slots (s_unit), x < 0: another cell
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31, th_ = threadIdx.x;
+    const int c0 = blockIdx.x * blockDim.x + wbase, c = c0 + lane;
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    double tmin = inf;
+    int nro = 0, npc = 0;
+    const size_t nc = d.n_cells, nu = d.n_units;
+    const K5Rows rows{b.cur, hcur, nc};
+    const double ga = P.gamma, gm1 = ga - 1, rg1 = 1.0 / gm1, dt = *b.dt_cur;
+    St5 pl{};
+    int kind = -1;
     if (c < d.n_cells) {
+        const uint32_t cfl = d.cflags[c];
+        const double x = b.cx[c], y = b.cy[c];
+        const bool proc = !(sq(x) + sq(y) < d.r11_sq);
+        {
+            const int g0 = d.gstart[c];
+            int4 su = make_int4(-1, -1, -1, -1);
+            if (d.gstart[c + 1] - g0 == 4)
+                su = make_int4(d.s_unit[g0], d.s_unit[g0 + 1], d.s_unit[g0 + 2], d.s_unit[g0 + 3]);
+            ssu[th_] = su;
+        }
+        double Volume2 = 0.0;
         {  // the next step's geometry cache from the moved points (see mk2_update_cell)
-            const int s0 = d.cstart[c], n = d.cstart[c + 1] - s0;
-            const int32_t* con = d.contour + s0;
-            double xn, yn;
-            centroid(con, n, d.X2, d.Y2, xn, yn);
+            double xn, yn, vs, vol;
+            const int4 qc = d.qcorner[c];
+            if (qc.x >= 0) {
+                const double qx[4] = {d.X2[qc.x], d.X2[qc.y], d.X2[qc.z], d.X2[qc.w]};
+                const double qy[4] = {d.Y2[qc.x], d.Y2[qc.y], d.Y2[qc.z], d.Y2[qc.w]};
+                quad_geometry(qx, qy, xn, yn, vs, vol);
+                Volume2 = vs;
+            } else {
+                const int s0 = d.cstart[c], n = d.cstart[c + 1] - s0, g0 = d.gstart[c], g1 = d.gstart[c + 1];
+                const int32_t* con = d.contour + s0;
+                centroid(con, n, d.X2, d.Y2, xn, yn);
+                vs = area(con, n, d.sA, d.sB, g0, g1, d.X2, d.Y2, false);
+                vol = volume_rotate(con, n, d.X2, d.Y2);
+                if (proc) Volume2 = area(con, n, d.sA, d.sB, g0, g1, d.X2, d.Y2, true);
+            }
             b.cx_next[c] = xn;
             b.cy_next[c] = yn;
-            const uint32_t cfl = d.cflags[c];
             if (cfl & CF_RP) b.rp_next[c] = pow2g(sqrt(sq(xn) + sq(yn)), 2 * P.gamma);
             if (!(cfl & CF_CENTR)) {
-                b.vs_next[c] = area(con, n, d.sA, d.sB, d.gstart[c], d.gstart[c + 1], d.X2, d.Y2, false);
-                b.vol_next[c] = volume_rotate(con, n, d.X2, d.Y2);
+                b.vs_next[c] = vs;
+                b.vol_next[c] = vol;
             }
         }
-        const double x = b.cx[c], y = b.cy[c];
-        const double radius = sqrt(sq(x) + sq(y));
-        if (!(radius < P.R11)) {
+        if (proc) {
             tmin = 10000000.0;  // `time` starts at 1e7 in every step (Setka.cpp:8286)
-            const double ga = P.gamma;
-            const double dt = *b.dt_cur;
-            const int kt = d.ctype[c];
-            const St21 par1 = load21(b.cur, hcur, nc, c);
-            const int s0 = d.cstart[c], nv = d.cstart[c + 1] - s0;
-            const int32_t* con = d.contour + s0;
-            const int g0 = d.gstart[c], g1 = d.gstart[c + 1];
-            const double Volume = area(con, nv, d.sA, d.sB, g0, g1, d.X, d.Y, false);
-            const double Volume2 = area(con, nv, d.sA, d.sB, g0, g1, d.X2, d.Y2, true);
-            // face fluxes summed in Grans order: plasma rows 0-4, hydrogen
-            // fluid k rows 5 + 4k .. 8 + 4k
-            const size_t ng = d.n_slots;
-            double Potok[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-            double PH[4][4];
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) PH[k][j] = 0.0;
-            for (int g = g0; g < g1; g++) {
-#pragma unroll
-                for (int j = 0; j < 5; j++) Potok[j] = Potok[j] + fl[j * ng + g];
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) PH[k][j] = PH[k][j] + fl[(5 + 4 * k + j) * ng + g];
+            kind = d.ctype[c];
+            double Volume;
+            if (!(cfl & CF_CENTR)) {
+                Volume = b.vs[c];
+            } else {  // the cache holds no area of the C_centr cells
+                const int s0 = d.cstart[c];
+                Volume = area(d.contour + s0, d.cstart[c + 1] - s0, d.sA, d.sB, d.gstart[c], d.gstart[c + 1], d.X, d.Y,
+                              false);
             }
-            // multi-fluid charge exchange (Setka.cpp:8575-8660)
-            const double u = par1.f[kU], v = par1.f[kV], ro = par1.f[kRo], p = par1.f[kP], Q = par1.f[kQ];
-            double UM[4], UH[4], nu[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const double roH = par1.f[fh(k, 0)], pH = par1.f[fh(k, 1)];
-                const double uH = par1.f[fh(k, 2)], vH = par1.f[fh(k, 3)];
-                UM[k] = sqrt(sq(u - uH) + sq(v - vH) + (64.0 / (9.0 * kPi)) * (p / ro + 2.0 * pH / roH));
-                UH[k] = sqrt(sq(u - uH) + sq(v - vH) + (4.0 / kPi) * (p / ro + 2.0 * pH / roH));
-                nu[k] = ro * roH * UM[k] * sq(1.0 - P.a_2 * log(UM[k]));
-            }
-            const double cp = P.src_coef;  // n_p_LISM_ / Kn_
-            const double q2_1 = cp * (nu[0] * (par1.f[fh(0, 2)] - u) + nu[1] * (par1.f[fh(1, 2)] - u) +
-                                      nu[2] * (par1.f[fh(2, 2)] - u) + nu[3] * (par1.f[fh(3, 2)] - u));
-            const double q2_2 = cp * (nu[0] * (par1.f[fh(0, 3)] - v) + nu[1] * (par1.f[fh(1, 3)] - v) +
-                                      nu[2] * (par1.f[fh(2, 3)] - v) + nu[3] * (par1.f[fh(3, 3)] - v));
-            double e[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const double roH = par1.f[fh(k, 0)], pH = par1.f[fh(k, 1)];
-                const double uH = par1.f[fh(k, 2)], vH = par1.f[fh(k, 3)];
-                e[k] = nu[k] * ((sq(uH) + sq(vH) - sq(u) - sq(v)) / 2.0 + (UH[k] / UM[k]) * (2.0 * pH / roH - p / ro));
-            }
-            const double q3 = cp * (e[0] + e[1] + e[2] + e[3]);
-            const double rV2 = 1.0 / Volume2, VV = Volume * rV2;
-            if (kt != C_CENTR) {
-                double ro3 = ro * VV - dt * (Potok[0] * rV2 + ro * v / y);
-                const double Q33 = Q * VV - (dt * rV2) * Potok[4] - dt * Q * v / y;
-                if (ro3 <= 0.0) {
-                    ro3 = P.ro_floor;
-                    nro++;
-                }
-                const double rro3 = 1.0 / ro3;
-                const double u3 = (ro * u * VV - dt * (Potok[1] * rV2 + ro * v * u / y - q2_1)) * rro3;
-                const double v3 = (ro * v * VV - dt * (Potok[2] * rV2 + ro * v * v / y - q2_2)) * rro3;
-                double p3 = (((p / (ga - 1) + ro * (u * u + v * v) * 0.5) * VV -
-                              dt * (Potok[3] * rV2 + v * (ga * p / (ga - 1) + ro * (u * u + v * v) * 0.5) / y - q3)) -
-                             0.5 * ro3 * (u3 * u3 + v3 * v3)) *
-                            (ga - 1);
-                if (p3 <= 0) {
-                    p3 = P.p_floor;
-                    npc++;
-                }
-                b.nxt[0][c] = ro3;
-                b.nxt[1][c] = p3;
-                b.nxt[2][c] = u3;
-                b.nxt[3][c] = v3;
-                b.nxt[4][c] = Q33;
-            } else {
-#pragma unroll
-                for (int q = 0; q < 5; q++) b.nxt[q][c] = par1.f[q];
-            }
-            // hydrogen sources by cell kind (Setka.cpp:8734-8806)
-            int kk[4] = {0, 0, 0, 0};
-            if (kt == C_CENTR || kt == C_1 || kt == C_2 || kt == C_3) {
-                if (kt == C_1 || kt == C_CENTR) kk[0] = 1;
-                else kk[1] = 1;
-            } else {
-                if (kt == C_4) kk[2] = 1;
-                else kk[3] = 1;
-            }
-            const double S1 = nu[0] + nu[1] + nu[2] + nu[3];
-            double s2[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) s2[k] = nu[k] * ((sq(u) + sq(v)) / 2.0 + (UH[k] / UM[k]) * (p / ro));
-            const double S2 = s2[0] + s2[1] + s2[2] + s2[3];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const double roH = par1.f[fh(k, 0)], pH = par1.f[fh(k, 1)];
-                const double uH = par1.f[fh(k, 2)], vH = par1.f[fh(k, 3)];
-                double out[4];
-                if (k == 0 && kt == C_CENTR) {
-                    out[0] = roH;
-                    out[1] = pH;
-                    out[2] = uH;
-                    out[3] = vH;
-                } else {
-                    const double q1h = kNHOverKn * (kk[k] * S1 - nu[k]);
-                    const double q21h = kNHOverKn * (kk[k] * S1 * u - nu[k] * uH);
-                    const double q22h = kNHOverKn * (kk[k] * S1 * v - nu[k] * vH);
-                    const double q3h = kNHOverKn * (kk[k] * S2 - nu[k] * ((sq(uH) + sq(vH)) / 2.0 +
-                                                                         (UH[k] / UM[k]) * 2.0 * (pH / roH)));
-                    // floors: Setka.cpp:8817, 8829, 8859, 8871, 8893, 8905, 8927, 8939
-                    const double rf = k == 0 ? 0.0000001 : 0.000001;
-                    const double pf = k == 3 ? 0.0000001 : 0.000001;
-                    k5_update_h(ga, PH[k], roH, pH, uH, vH, q1h, q21h, q22h, q3h, VV, rV2, y, dt, rf, pf, out, nro,
-                                npc);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) hnxt[(4 * k + j) * nc + c] = out[j];
-            }
+            pl = rows.load(0, c);
+            const double rV2 = 1.0 / Volume2;
+            sd[0][th_] = pl.u;
+            sd[1][th_] = pl.v;
+            sd[2][th_] = pl.ro;
+            sd[3][th_] = pl.p / pl.ro;
+            sd[4][th_] = Volume * rV2;
+            sd[5][th_] = rV2;
+            sd[6][th_] = 1.0 / y;
         }
     }
-    block_reduce_commit(tmin, nro, npc, status, b.dt_acc, b.counters, b.status);
+    si[th_] = kind;
+    __syncwarp();
+    // the flux rows first .. first + N - 1 of cell k's faces, summed in Grans order
+    auto sums = [&](int k, int t, int first, double* out, auto n_const) {
+        constexpr int N = decltype(n_const)::value;
+#pragma unroll
+        for (int q = 0; q < N; q++) out[q] = 0.0;
+        const double* r = fl + first * nu;
+        const int4 s4 = ssu[t];
+        if (s4.x >= 0) {  // quadrilaterals: all loads in flight together
+            const int su[4] = {s4.x, s4.y, s4.z, s4.w};
+            double a[N][4];
+#pragma unroll
+            for (int q = 0; q < N; q++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) a[q][j] = r[q * nu + (su[j] >> 1)];
+#pragma unroll
+            for (int q = 0; q < N; q++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) out[q] = out[q] + ((su[j] & 1) ? -a[q][j] : a[q][j]);
+        } else {
+            const int g0 = d.gstart[k], nf = d.gstart[k + 1] - g0;
+            for (int j = 0; j < nf; j++) {
+                const int w = d.s_unit[g0 + j];
+#pragma unroll
+                for (int q = 0; q < N; q++) {
+                    const double v = r[q * nu + (w >> 1)];
+                    out[q] = out[q] + ((w & 1) ? -v : v);
+                }
+            }
+        }
+    };
+    const int f = lane & 3, q0 = lane & ~3;
+#pragma unroll 1
+    for (int rd = 0; rd < 4; rd++) {
+        const int t = wbase + 8 * rd + (lane >> 2), k = c0 + 8 * rd + (lane >> 2);
+        const int kt = si[t];
+        St5 h{1.0, 1.0, 0.0, 0.0, 0.0};
+        double u = 0.0, v = 0.0, nu4 = 0.0, uhm = 0.0, th = 0.0, mu = 0.0, mv = 0.0, mt = 0.0, s2 = 0.0;
+        double PH[4];
+        if (kt >= 0) {  // charge exchange with the plasma (Setka.cpp:8575-8660)
+            u = sd[0][t];
+            v = sd[1][t];
+            const double ro = sd[2][t], pro = sd[3][t];
+            h = rows.load(f + 1, k);
+            sums(k, t, 5 + 4 * f, PH, std::integral_constant<int, 4>{});
+            th = 2.0 * h.p / h.ro;
+            const double du2 = sq(u - h.u) + sq(v - h.v), a = pro + th;
+            const double UM2 = du2 + (64.0 / (9.0 * kPi)) * a, UH2 = du2 + (4.0 / kPi) * a;
+            const double r = rsqrt(UM2);
+            uhm = sqrt(UH2) * r;
+            nu4 = ro * h.ro * (UM2 * r) * sq(1.0 - P.a_2 * (0.5 * log(UM2)));
+            mu = nu4 * (h.u - u);
+            mv = nu4 * (h.v - v);
+            mt = nu4 * ((sq(h.u) + sq(h.v) - sq(u) - sq(v)) / 2.0 + uhm * (th - pro));
+            s2 = nu4 * ((sq(u) + sq(v)) / 2.0 + uhm * pro);
+        }
+        double S1 = 0.0, S2 = 0.0, Mu = 0.0, Mv = 0.0, MT = 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            S1 += __shfl_sync(full, nu4, q0 + j);
+            S2 += __shfl_sync(full, s2, q0 + j);
+            Mu += __shfl_sync(full, mu, q0 + j);
+            Mv += __shfl_sync(full, mv, q0 + j);
+            MT += __shfl_sync(full, mt, q0 + j);
+        }
+        if (kt >= 0) {
+            if (f == 0) {
+                sd[7][t] = Mu;
+                sd[8][t] = Mv;
+                sd[9][t] = MT;
+            }
+            // hydrogen sources by cell kind (Setka.cpp:8734-8806)
+            const int born = (kt == C_1 || kt == C_CENTR) ? 0 : (kt == C_2 || kt == C_3) ? 1 : kt == C_4 ? 2 : 3;
+            double out[4] = {h.ro, h.p, h.u, h.v};
+            if (!(f == 0 && kt == C_CENTR)) {
+                const double kk = f == born ? 1.0 : 0.0;
+                const double q1h = kNHOverKn * (kk * S1 - nu4);
+                const double q21h = kNHOverKn * (kk * S1 * u - nu4 * h.u);
+                const double q22h = kNHOverKn * (kk * S1 * v - nu4 * h.v);
+                const double q3h = kNHOverKn * (kk * S2 - nu4 * ((sq(h.u) + sq(h.v)) / 2.0 + uhm * th));
+                // floors: Setka.cpp:8817, 8829, 8859, 8871, 8893, 8905, 8927, 8939
+                const double rf = f == 0 ? 0.0000001 : 0.000001;
+                const double pf = f == 3 ? 0.0000001 : 0.000001;
+                k5_update_h(ga, PH, h.ro, h.p, h.u, h.v, q1h, q21h, q22h, q3h, sd[4][t], sd[5][t], sd[6][t], dt, rf, pf,
+                            out, nro, npc);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) hnxt[(4 * f + j) * nc + k] = out[j];
+        }
+    }
+    __syncwarp();
+    if (kind >= 0) {
+        const double ro = pl.ro, u = pl.u, v = pl.v, p = pl.p, Q = pl.Q;
+        St5 o = pl;
+        if (kind != C_CENTR) {
+            const double cp = P.src_coef;  // n_p_LISM_ / Kn_
+            const double q2_1 = cp * sd[7][th_], q2_2 = cp * sd[8][th_], q3 = cp * sd[9][th_];
+            const double VV = sd[4][th_], rV2 = sd[5][th_], vy = v * sd[6][th_];
+            double Pt[5];
+            sums(c, th_, 0, Pt, std::integral_constant<int, 5>{});
+            o.ro = ro * VV - dt * (Pt[0] * rV2 + ro * vy);
+            o.Q = Q * VV - (dt * rV2) * Pt[4] - dt * Q * vy;
+            if (o.ro <= 0.0) {
+                o.ro = P.ro_floor;
+                nro++;
+            }
+            const double rro3 = 1.0 / o.ro, ek = ro * (u * u + v * v) * 0.5;
+            o.u = (ro * u * VV - dt * (Pt[1] * rV2 + ro * vy * u - q2_1)) * rro3;
+            o.v = (ro * v * VV - dt * (Pt[2] * rV2 + ro * vy * v - q2_2)) * rro3;
+            o.p = (((p * rg1 + ek) * VV - dt * (Pt[3] * rV2 + vy * (ga * p * rg1 + ek) - q3)) -
+                   0.5 * o.ro * (o.u * o.u + o.v * o.v)) *
+                  gm1;
+            if (o.p <= 0) {
+                o.p = P.p_floor;
+                npc++;
+            }
+        }
+        b.nxt[0][c] = o.ro;
+        b.nxt[1][c] = o.p;
+        b.nxt[2][c] = o.u;
+        b.nxt[3][c] = o.v;
+        b.nxt[4][c] = o.Q;
+    }
+    block_reduce_commit(tmin, nro, npc, 0, b.dt_acc, b.counters, b.status);
 }
 
 // ------------------------------------------------------------------ MHD + pickup protons
@@ -4980,9 +4988,30 @@ int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b
 void launch_hllc_batch(const gelios_params& P, int n, const double* in, double* out, cudaStream_t s) {
     hllc_batch_kernel<<<blocks_for(n, 128), 128, 0, s>>>(P, n, in, out);
 }
-void launch_k5(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* hcur, double* hnxt,
-               double* fl, cudaStream_t s) {
-    if (d.n_units > 0) k5_face_kernel<<<blocks_for(d.n_units, 128), 128, 0, s>>>(d, P, b, hcur, fl);
+int launch_k5_faces(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* hcur, double* fl,
+                    cudaStream_t s, cudaStream_t s_c1, cudaStream_t s_rest) {
+    const int nc1 = d.u_tr0 - d.u_c1, nt = d.u_tr1 - d.u_tr0, no = d.n_units - d.u_tr1;
+    int n = 0;
+    if (nt > 0) {  // first: the longest chain
+        k5_tracked_kernel<<<blocks_for(nt, 2), 64, 0, s_rest>>>(d, P, b, hcur, fl);
+        n++;
+    }
+    if (no > 0) {
+        k5_face_kernel<kAnyGroup, 3><<<blocks_for(no, 128), 128, 0, s_rest>>>(d, P, b, hcur, fl, no);
+        n++;
+    }
+    if (nc1 > 0) {
+        k5_face_kernel<kC1Group, 4><<<blocks_for(nc1, 128), 128, 0, s_c1>>>(d, P, b, hcur, fl, nc1);
+        n++;
+    }
+    if (d.u_c1 > 0) {
+        k5_face_kernel<kPlainGroup, 5><<<blocks_for(d.u_c1, 128), 128, 0, s>>>(d, P, b, hcur, fl, d.u_c1);
+        n++;
+    }
+    return n;
+}
+void launch_k5_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
+                      const double* hcur, double* hnxt, cudaStream_t s) {
     k5_update_kernel<<<blocks_for(d.n_cells, 128), 128, 0, s>>>(d, P, b, fl, hcur, hnxt);
 }
 void launch_hlldq_batch(const gelios_params& P, int n, const double* in, double* out, cudaStream_t s) {

@@ -232,12 +232,17 @@ void launch_mk2_update(const DevMesh& d, const gelios_params& P, const StepBuffe
                        const double* aux, cudaStream_t s, int mode, const int32_t* list, int n_list);
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
                   bool copy_outer_shock = true);
-// Go_5_komponent: face units then the cell update.  Hydrogen state rows
+// Go_5_komponent: face units, then the cell update.  Hydrogen state rows
 // (ro, p, u, v of H1..H4), 16 rows of n_cells each, of the current and the
-// next buffer; fl: kK5FluxRows flux rows per face slot.
+// next buffer; fl: kK5FluxRows flux rows of n_units, F.S once per face unit
+// as its owner sees it (the update subtracts it on the other side).  The
+// plain interior units run on s, the C_1 interior ones on s_c1, the tracked
+// and one-sided ones on s_rest; returns the launch count.
 constexpr int kK5FluxRows = 21;
-void launch_k5(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* hcur, double* hnxt,
-               double* fl, cudaStream_t s);
+int launch_k5_faces(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* hcur, double* fl,
+                    cudaStream_t s, cudaStream_t s_c1, cudaStream_t s_rest);
+void launch_k5_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
+                      const double* hcur, double* hnxt, cudaStream_t s);
 // MHD + pickup-proton form: extra rows (8 x n_cells: w, Bx, By, Bz, pickup
 // ro, p, u, v), 13 flux rows per slot, fixed sources (3 x n_cells).
 constexpr int kMhdFluxRows = 13;
