@@ -1542,9 +1542,8 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         return GELIOS_E_STATE;
     }
     if (mhd || form == GELIOS_FORM_5_KOMPONENT) {
-        // wide flux rows of the multi-fluid forms: 13 per face slot or 21 per face unit
-        const size_t fb = (mhd ? kMhdFluxRows * static_cast<size_t>(d.n_slots)
-                               : kK5FluxRows * static_cast<size_t>(d.n_units)) * sizeof(double);
+        // wide flux rows of the multi-fluid forms: 13 or 21 per face unit
+        const size_t fb = static_cast<size_t>(mhd ? kMhdFluxRows : kK5FluxRows) * d.n_units * sizeof(double);
         if (ctx->flux_mhd.bytes != fb) {
             ctx->drop_graphs();
             if (ctx->flux_mhd.alloc(fb)) return GELIOS_E_CUDA;
@@ -1776,7 +1775,7 @@ extern "C" int gelios_operator_residual(gelios_ctx* ctx, int form, int buf, doub
     const size_t need = (kResidualScratch + 8) * sizeof(double);
     if (ctx->resid.bytes < need && ctx->resid.alloc(need)) return GELIOS_E_CUDA;
     if (mhd) {
-        const size_t fb = static_cast<size_t>(kMhdFluxRows) * d.n_slots * sizeof(double);
+        const size_t fb = static_cast<size_t>(kMhdFluxRows) * d.n_units * sizeof(double);
         if (ctx->flux_mhd.bytes != fb) {
             ctx->drop_graphs();  // they hold the buffer about to be replaced
             if (ctx->flux_mhd.alloc(fb)) return GELIOS_E_CUDA;
@@ -2027,7 +2026,7 @@ extern "C" int gelios_autotune(gelios_ctx* ctx, int form, int reps, int32_t* var
     GELIOS_CUDA_TRY(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
     if (mhd) {
-        const size_t fb = static_cast<size_t>(kMhdFluxRows) * d.n_slots * sizeof(double);
+        const size_t fb = static_cast<size_t>(kMhdFluxRows) * d.n_units * sizeof(double);
         if (ctx->flux_mhd.bytes != fb) {
             ctx->drop_graphs();
             if (ctx->flux_mhd.alloc(fb)) return GELIOS_E_CUDA;
@@ -2189,7 +2188,7 @@ extern "C" int gelios_batch_create(gelios_batch** out, gelios_ctx* const* ctxs, 
             return GELIOS_E_STATE;
         }
         GELIOS_CUDA_TRY(cudaSetDevice(c->device));
-        const size_t fb = static_cast<size_t>(kMhdFluxRows) * d.n_slots * sizeof(double);
+        const size_t fb = static_cast<size_t>(kMhdFluxRows) * d.n_units * sizeof(double);
         if (c->flux_mhd.bytes != fb) {
             c->drop_graphs();
             if (c->flux_mhd.alloc(fb)) return GELIOS_E_CUDA;

@@ -582,6 +582,14 @@ __device__ void source_mk1(const DevMesh& d, const gelios_params& P, int k, doub
     q3 = MT * m.kT;
 }
 
+// The flux rows of the moving-grid forms hold each face unit's F.S once, as
+// its owner sees it; the other side of an interior face takes its negative.
+// w: the s_unit word of a cell's slot (unit << 1 | 1 on the other side).
+__device__ __forceinline__ double unit_flux(const double* __restrict__ row, int w) {
+    const double v = row[w >> 1];
+    return (w & 1) ? -v : v;
+}
+
 // Block-level minimum of `t` (non-negative doubles; NaN ignored) folded into
 // the device word acc with one atomicMin per block; clamp counters likewise.
 __device__ __forceinline__ void block_reduce_commit(double t, int nro, int np_, int status, unsigned long long* acc,
@@ -1706,19 +1714,18 @@ __device__ __forceinline__ void mk2_recon_unit(const DevMesh& d, const gelios_pa
 // The flux of one MK2 face unit once the grid has moved (Setka.cpp:10198-10209,
 // 10335-10393): face speed W from the moved points, HLL (`metod 0`), exact
 // Godunov sampled at W on tracked faces (star pressure pstar solved before the
-// motion), F.S to the owner slot and -F.S to the twin slot, CFL candidates.
+// motion), F.S into the unit's flux rows, CFL candidates.
 template <typename TF, bool TRACKED>
 __device__ __forceinline__ void mk2_flux_unit(const DevMesh& d, const gelios_params& P, const StepBuffers& b, int u,
                                               const RecUnit& r, double* __restrict__ fl, const double* pstar,
                                               double& tmin_u, int* status) {
     const bool procK = !(r.dist < 0.0), procN = !(r.distn < 0.0);
     if (!(procK || procN)) return;
-    const size_t ng = d.n_slots;
+    const size_t nu = d.n_units;
     const double dt = *b.dt_cur;
     const int A = d.u_A[u], B = d.u_B[u];
     const double x4 = (d.X2[A] + d.X2[B]) / 2.0, y4 = (d.Y2[A] + d.Y2[B]) / 2.0;
     const double W = ((x4 - r.x2) * r.n1 + (y4 - r.y2) * r.n2) / dt;
-    const int g = d.u_slot[u], gt = d.u_twin[u];
     const bool np = (d.u_info[u] & SI_NP) != 0;
     FluxOut<double> F;
     const double UU = hllc_flux<TF>(P.gamma, P.kurant, r.a, r.o, W, r.n1, r.n2, 1.0, 0, np, F);
@@ -1737,28 +1744,19 @@ __device__ __forceinline__ void mk2_flux_unit(const DevMesh& d, const gelios_par
         fm3 = qq[4] * S;
     }
     const double fq = F.PQ * S;
-    // the slots are read once, by the update: streaming stores keep the
-    // gathered cell data in L2
-    __stcs(fl + 0 * ng + g, fm0);
-    __stcs(fl + 1 * ng + g, fm1);
-    __stcs(fl + 2 * ng + g, fm2);
-    __stcs(fl + 3 * ng + g, fm3);
-    __stcs(fl + 4 * ng + g, fq);
+    fl[0 * nu + u] = fm0;
+    fl[1 * nu + u] = fm1;
+    fl[2 * nu + u] = fm2;
+    fl[3 * nu + u] = fm3;
+    fl[4 * nu + u] = fq;
     if (procK) {
         // reference order: Godunov candidate first, then HLL (Setka.cpp:10359, 10366)
         if (TRACKED) tmin_u = dmin_ref(tmin_u, P.kurant * r.dist / UG);
         tmin_u = dmin_ref(tmin_u, P.kurant * r.dist / UU);
     }
-    if (gt >= 0) {
-        __stcs(fl + 0 * ng + gt, -fm0);
-        __stcs(fl + 1 * ng + gt, -fm1);
-        __stcs(fl + 2 * ng + gt, -fm2);
-        __stcs(fl + 3 * ng + gt, -fm3);
-        __stcs(fl + 4 * ng + gt, -fq);
-        if (procN) {
-            if (TRACKED) tmin_u = dmin_ref(tmin_u, P.kurant * r.distn / UG);
-            tmin_u = dmin_ref(tmin_u, P.kurant * r.distn / UU);
-        }
+    if (procN) {
+        if (TRACKED) tmin_u = dmin_ref(tmin_u, P.kurant * r.distn / UG);
+        tmin_u = dmin_ref(tmin_u, P.kurant * r.distn / UU);
     }
 }
 
@@ -2065,18 +2063,18 @@ __global__ void __launch_bounds__(128, GELIOS_SOURCE_MINB) mk2_source_kernel(Dev
 #endif
 
 // Go_5_komponent__MK2 cell update (Setka.cpp:10386-10468) of cell c from its
-// face slots' fluxes (fetch(k, j): row k of the cell's j-th slot, Grans
-// order).  The area and rotated volume before the motion come from the cache
+// nf face slots' fluxes (fetch4 / fetch(k, j): row k of the cell's j-th slot,
+// Grans order; fetch4 where there are four).  The area and rotated volume before the motion come from the cache
 // (b.vs, b.vol); the cache is refilled for the next step from the moved
 // points: centroid, and area and rotated volume of every cell but the C_centr
 // ones (the points after the commit are these moved points, bit for bit),
 // |centroid|^(2 gamma) of the cells flagged CF_RP.  For a quadrilateral
 // Get_Volume and Get_Volume_posle are the same formula; other cells get the
 // Get_Volume form for the cache.
-template <typename Fetch>
+template <typename Fetch4, typename Fetch>
 __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_params& P, const StepBuffers& b, int c,
-                                                Fetch fetch, const double* __restrict__ aux, double& tmark, int& nro,
-                                                int& npc) {
+                                                int nf, Fetch4 fetch4, Fetch fetch, const double* __restrict__ aux,
+                                                double& tmark, int& nro, int& npc) {
     const uint32_t cfl = d.cflags[c];
     const double x = b.cx[c], y = b.cy[c];
     double xn, yn, vs2 = 0.0, Volume2 = 0.0;
@@ -2120,14 +2118,13 @@ __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_p
     if (sqrt(sq(x) + sq(y)) < P.R11) return;
     tmark = dmin_ref(tmark, 10000000.0);  // `time` starts at 1e7 in every step (Setka.cpp:10141)
     const double dt = *b.dt_cur;
-    const int nf = d.gstart[c + 1] - d.gstart[c];
     double Pt0 = 0.0, Pt1 = 0.0, Pt2 = 0.0, Pt3 = 0.0, Pt4 = 0.0;
     if (nf == 4) {  // quadrilaterals: all slot loads in flight together
         double a[5][4];
 #pragma unroll
         for (int k = 0; k < 5; k++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) a[k][j] = fetch(k, j);
+            for (int j = 0; j < 4; j++) a[k][j] = fetch4(k, j);
         Pt0 = (((Pt0 + a[0][0]) + a[0][1]) + a[0][2]) + a[0][3];
         Pt1 = (((Pt1 + a[1][0]) + a[1][1]) + a[1][2]) + a[1][3];
         Pt2 = (((Pt2 + a[2][0]) + a[2][1]) + a[2][2]) + a[2][3];
@@ -2198,7 +2195,7 @@ __global__ void __launch_bounds__(NT, MINB) mk2_tile_kernel(DevMesh d, gelios_pa
     extern __shared__ double sfl[];  // 5 rows of t.max_slots
     const int tile = blockIdx.x;
     const int ms = t.max_slots;
-    const size_t ng = d.n_slots;
+    const size_t nu = d.n_units;
     double tmin = __longlong_as_double(0x7ff0000000000000LL);
     int nro = 0, npc = 0, status = 0;
     const int f0 = t.fstart[tile], f1 = t.fstart[tile + 1];
@@ -2207,11 +2204,11 @@ __global__ void __launch_bounds__(NT, MINB) mk2_tile_kernel(DevMesh d, gelios_pa
         const int u = rec.x;
         const int own = rec.y & 0xffff, tw = (rec.y >> 16) & 0xffff;
         if (u >= d.u_tr0 && u < d.u_tr1) {
-            const int g = d.u_slot[u], gt = d.u_twin[u];
 #pragma unroll
             for (int k = 0; k < 5; k++) {
-                if (own != kTileNone) sfl[k * ms + own] = fl[k * ng + g];
-                if (tw != kTileNone) sfl[k * ms + tw] = fl[k * ng + gt];
+                const double v = fl[k * nu + u];
+                if (own != kTileNone) sfl[k * ms + own] = v;
+                if (tw != kTileNone) sfl[k * ms + tw] = -v;
             }
             continue;
         }
@@ -2246,7 +2243,8 @@ __global__ void __launch_bounds__(NT, MINB) mk2_tile_kernel(DevMesh d, gelios_pa
     for (int i = c0 + threadIdx.x; i < c1; i += NT) {
         const int c = t.cells[i];
         const int base = t.lbase[i];
-        mk2_update_cell(d, P, b, c, [&](int k, int jj) { return sfl[k * ms + base + jj]; }, aux, tmin, nro, npc);
+        auto fetch = [&](int k, int jj) { return sfl[k * ms + base + jj]; };
+        mk2_update_cell(d, P, b, c, d.gstart[c + 1] - d.gstart[c], fetch, fetch, aux, tmin, nro, npc);
     }
     block_reduce_commit(tmin, nro, npc, status, b.dt_acc, b.counters, b.status);
 }
@@ -2268,7 +2266,7 @@ __global__ void __launch_bounds__(128, 8) mk2_update_kernel(DevMesh d, gelios_pa
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double tmark = __longlong_as_double(0x7ff0000000000000LL);
     int nro = 0, npc = 0;
-    const size_t ng = d.n_slots;
+    const size_t nu = d.n_units;
     int c = -1;
     if (MODE == kUpdEarly) {
         if (i < n_list) c = list[i];
@@ -2277,8 +2275,15 @@ __global__ void __launch_bounds__(128, 8) mk2_update_kernel(DevMesh d, gelios_pa
         if (MODE == kUpdRest && (d.cflags[c] & CF_EARLY)) c = -1;
     }
     if (c >= 0) {
-        const int g0 = d.gstart[c];
-        mk2_update_cell(d, P, b, c, [&](int k, int j) { return __ldcs(fl + k * ng + g0 + j); }, aux, tmark, nro, npc);
+        const int g0 = d.gstart[c], nf = d.gstart[c + 1] - g0;
+        int su[4] = {0, 0, 0, 0};
+        if (nf == 4) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) su[j] = d.s_unit[g0 + j];
+        }
+        mk2_update_cell(
+            d, P, b, c, nf, [&](int k, int j) { return unit_flux(fl + k * nu, su[j]); },
+            [&](int k, int j) { return unit_flux(fl + k * nu, d.s_unit[g0 + j]); }, aux, tmark, nro, npc);
     }
     if (MODE != kUpdAll) tmark = __longlong_as_double(0x7ff0000000000000LL);
     block_reduce_commit(tmark, nro, npc, 0, b.dt_acc, b.counters, b.status);
@@ -4064,7 +4069,7 @@ __device__ __forceinline__ double mhd_face_flux(double ga, const St5& iL, const 
 // sides (ion rows: the moving-grid rules of Setka.cpp:10204-10276, extra
 // rows: mhd_usualy_side / get_par_ext) on the pre-motion points, face speed
 // from the moved points, HLLD for the ions and HLLC for the pickup protons,
-// 13 flux rows times S to the owner slot and their negatives to the twin,
+// 13 flux rows times S into the unit's rows,
 // CFL candidates of both fluids.  BLOCK x MINB: the launch shape (threads
 // per block, minimum resident blocks per SM, which caps the registers).
 // PLAIN: a unit of the plain interior group [0, u_c1) (see mk2_recon_unit).
@@ -4074,7 +4079,7 @@ __device__ __forceinline__ double mhd_face_body(const DevMesh& d, const gelios_p
                                                 double* __restrict__ fl, int u, int& status) {
     double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
     {
-        const size_t nc = d.n_cells, ng = d.n_slots;
+        const size_t nc = d.n_cells, nu = d.n_units;
         const int K = d.u_cell[u], nb = d.u_nb[u];
         const uint32_t info = d.u_info[u];
         const double x = b.cx[K], y = b.cy[K];
@@ -4163,20 +4168,14 @@ __device__ __forceinline__ double mhd_face_body(const DevMesh& d, const gelios_p
             F[10] = G.P1;
             F[11] = G.P2;
             F[12] = G.P3;
-            const int g = d.u_slot[u], gt = d.u_twin[u];
-            // slots are read once, by the update: streaming stores
 #pragma unroll
-            for (int k = 0; k < kMhdFlux; k++) __stcs(fl + k * ng + g, F[k] * S);
-            if (gt >= 0) {
-#pragma unroll
-                for (int k = 0; k < kMhdFlux; k++) __stcs(fl + k * ng + gt, -(F[k] * S));
-            }
+            for (int k = 0; k < kMhdFlux; k++) fl[k * nu + u] = F[k] * S;
             if (procK) {
                 const double dist = dK;
                 tmin_u = dmin_ref(tmin_u, P.kurant * dist * tI);
                 tmin_u = dmin_ref(tmin_u, P.kurant * dist / UUp);
             }
-            if (gt >= 0 && procN) {
+            if (procN) {
                 const double distn = dN;
                 tmin_u = dmin_ref(tmin_u, P.kurant * distn * tI);
                 tmin_u = dmin_ref(tmin_u, P.kurant * distn / UUp);
@@ -4208,7 +4207,7 @@ __device__ __forceinline__ void mhd_update_body(const DevMesh& d, const gelios_p
                                                 const double* __restrict__ fl, const double* __restrict__ src,
                                                 const double* __restrict__ hcur, double* __restrict__ hnxt, int c,
                                                 double& tmark, int& nro, int& npc) {
-    const size_t ng = d.n_slots, nc = d.n_cells;
+    const size_t nu = d.n_units, nc = d.n_cells;
     {
         const uint32_t cfl = d.cflags[c];
         double xn, yn;
@@ -4253,17 +4252,22 @@ __device__ __forceinline__ void mhd_update_body(const DevMesh& d, const gelios_p
                 double Pt[kMhdFlux];
 #pragma unroll
                 for (int k = 0; k < kMhdFlux; k++) Pt[k] = 0.0;
-                if (g1 - g0 == 4) {  // quadrilaterals: all slot loads in flight together
+                if (g1 - g0 == 4) {  // quadrilaterals: all flux loads in flight together
+                    int su[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) su[j] = d.s_unit[g0 + j];
 #pragma unroll
                     for (int k = 0; k < kMhdFlux; k++) {
-                        const double* f = fl + k * ng + g0;
-                        const double a0 = __ldcs(f), a1 = __ldcs(f + 1), a2 = __ldcs(f + 2), a3 = __ldcs(f + 3);
+                        const double* f = fl + k * nu;
+                        const double a0 = unit_flux(f, su[0]), a1 = unit_flux(f, su[1]), a2 = unit_flux(f, su[2]),
+                                     a3 = unit_flux(f, su[3]);
                         Pt[k] = (((Pt[k] + a0) + a1) + a2) + a3;
                     }
                 } else {
                     for (int g = g0; g < g1; g++) {
+                        const int w = d.s_unit[g];
 #pragma unroll
-                        for (int k = 0; k < kMhdFlux; k++) Pt[k] = Pt[k] + fl[k * ng + g];
+                        for (int k = 0; k < kMhdFlux; k++) Pt[k] = Pt[k] + unit_flux(fl + k * nu, w);
                     }
                 }
                 const double q1 = src[c], q2 = src[nc + c], q3 = src[2 * nc + c];
@@ -5081,7 +5085,7 @@ __global__ void __launch_bounds__(256) op_residual_partial_kernel(DevMesh d, gel
         const double x = b.cx[c], y = b.cy[c];
         if (sqrt(sq(x) + sq(y)) < P.R11 || (d.cflags[c] & CF_CENTR)) continue;
         double pt = 0.0;
-        for (int g = d.gstart[c]; g < d.gstart[c + 1]; g++) pt = pt + fl[g];
+        for (int g = d.gstart[c]; g < d.gstart[c + 1]; g++) pt = pt + unit_flux(fl, d.s_unit[g]);
         dsum += fabs(pt) / b.vol[c];
     }
     sd[threadIdx.x] = dsum;
