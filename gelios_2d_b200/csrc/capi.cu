@@ -2142,7 +2142,7 @@ extern "C" int gelios_autotune(gelios_ctx* ctx, int form, int reps, int32_t* var
 struct gelios_batch {
     int device = 0;
     std::vector<gelios_ctx*> ctxs;
-    DBuf inst, surf, rails, units, cells, points;
+    DBuf inst, surf, rails, plain, units, cells, points;
     BatchTables tab;
     std::vector<BatchInstance> host_inst;  // one descriptor per instance, rebuilt per call
     BatchInstance* pinned = nullptr;       // staging of the descriptors' upload (pinned: the copy is asynchronous)
@@ -2167,7 +2167,7 @@ extern "C" int gelios_batch_create(gelios_batch** out, gelios_ctx* const* ctxs, 
     *out = nullptr;
     auto B = std::make_unique<gelios_batch>();
     B->device = ctxs[0] ? ctxs[0]->device : 0;
-    std::vector<int2> surf, rails, units, cells, points;
+    std::vector<int2> surf, rails, plain, units, cells, points;
     for (int i = 0; i < n; i++) {
         gelios_ctx* c = ctxs[i];
         if (!c || !c->have_mesh) {
@@ -2197,7 +2197,8 @@ extern "C" int gelios_batch_create(gelios_batch** out, gelios_ctx* const* ctxs, 
         for (int j = 0; j < nt; j += 2) surf.push_back(make_int2(i, j));
         const int nr = d.n_rail_a + d.n_rail_b + d.n_rail_c + d.n_rail_d;
         for (int q = 0; q < nr; q++) rails.push_back(make_int2(i, q));
-        for (int u = 0; u < d.n_units; u += 128) units.push_back(make_int2(i, u));
+        for (int u = 0; u < d.u_c1; u += 128) plain.push_back(make_int2(i, u));
+        for (int u = d.u_c1; u < d.n_units; u += 128) units.push_back(make_int2(i, u));
         for (int k = 0; k < d.n_cells; k += 128) cells.push_back(make_int2(i, k));
         for (int k = 0; k < d.n_points; k += 256) points.push_back(make_int2(i, k));
         B->ctxs.push_back(c);
@@ -2207,6 +2208,7 @@ extern "C" int gelios_batch_create(gelios_batch** out, gelios_ctx* const* ctxs, 
     int rc = 0;
     rc |= upload(B->surf, surf.data(), surf.size(), s);
     rc |= upload(B->rails, rails.data(), rails.size(), s);
+    rc |= upload(B->plain, plain.data(), plain.size(), s);
     rc |= upload(B->units, units.data(), units.size(), s);
     rc |= upload(B->cells, cells.data(), cells.size(), s);
     rc |= upload(B->points, points.data(), points.size(), s);
@@ -2219,11 +2221,13 @@ extern "C" int gelios_batch_create(gelios_batch** out, gelios_ctx* const* ctxs, 
     BatchTables& t = B->tab;
     t.surf = B->surf.as<int2>();
     t.rails = B->rails.as<int2>();
+    t.plain = B->plain.as<int2>();
     t.units = B->units.as<int2>();
     t.cells = B->cells.as<int2>();
     t.points = B->points.as<int2>();
     t.n_surf = static_cast<int>(surf.size());
     t.n_rails = static_cast<int>(rails.size());
+    t.n_plain = static_cast<int>(plain.size());
     t.n_units = static_cast<int>(units.size());
     t.n_cells = static_cast<int>(cells.size());
     t.n_points = static_cast<int>(points.size());
@@ -2248,7 +2252,8 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
     }
     GELIOS_CUDA_TRY(cudaSetDevice(B->device));
     const int n = static_cast<int>(B->ctxs.size());
-    cudaStream_t s = B->ctxs[0]->stream;
+    gelios_ctx* c0 = B->ctxs[0];
+    cudaStream_t s = c0->stream;
     // order after each context's own pending work
     for (int i = 1; i < n; i++) {
         GELIOS_CUDA_TRY(cudaEventRecord(B->ev, B->ctxs[i]->stream));
@@ -2320,7 +2325,8 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
     B->tab.inst = B->inst.as<BatchInstance>();
     launch_batch_words_init(B->tab, n, s);  // dt0, empty accumulators: every instance starts a call
     int64_t launches = 1;
-    const int per_step = (B->tab.n_surf > 0) + (B->tab.n_rails > 0) + (B->tab.n_units > 0) + (B->tab.n_cells > 0) +
+    const int per_step = (B->tab.n_surf > 0) + (B->tab.n_rails > 0) + (B->tab.n_plain > 0) +
+                         (B->tab.n_units > 0) + (B->tab.n_cells > 0) +
                          (B->tab.n_points > 0);
     if (B->schedule > 0 && nsteps > 0) {
         GELIOS_CUDA_TRY(launch_batch_mhd_persistent(B->tab, nsteps, B->schedule, s));
@@ -2331,8 +2337,8 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
         if (!B->graphs_off && !B->graph[par]) {
             cudaGraph_t g = nullptr;
             if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-                launch_batch_mhd_step(B->tab, par, s);
-                if (cudaStreamEndCapture(s, &g) != cudaSuccess || !g ||
+                const cudaError_t le = launch_batch_mhd_step(B->tab, par, s, c0->side, c0->ev_fork, c0->ev_tracked);
+                if (le != cudaSuccess || cudaStreamEndCapture(s, &g) != cudaSuccess || !g ||
                     cudaGraphInstantiate(&B->graph[par], g, 0) != cudaSuccess) {
                     B->graph[par] = nullptr;
                     B->graphs_off = true;
@@ -2346,7 +2352,7 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
         if (B->graph[par]) {
             GELIOS_CUDA_TRY(cudaGraphLaunch(B->graph[par], s));
         } else {
-            launch_batch_mhd_step(B->tab, par, s);
+            GELIOS_CUDA_TRY(launch_batch_mhd_step(B->tab, par, s, c0->side, c0->ev_fork, c0->ev_tracked));
         }
         launches += per_step;
     }

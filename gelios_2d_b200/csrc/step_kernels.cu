@@ -4372,6 +4372,9 @@ __global__ void __launch_bounds__(128) mhd_update_kernel(DevMesh d, gelios_param
 #ifndef GELIOS_BATCH_FACE_MINB
 #define GELIOS_BATCH_FACE_MINB 4
 #endif
+#ifndef GELIOS_BATCH_PLAIN_MINB
+#define GELIOS_BATCH_PLAIN_MINB 4
+#endif
 #if GELIOS_BATCH_SMEM_DESC
 #define BATCH_INSTANCE(I, e)          \
     __shared__ BatchInstance I;       \
@@ -4401,15 +4404,21 @@ __global__ void __launch_bounds__(128) batch_rails_kernel(BatchTables t, int par
     rails_body(I.d, I.P, I.b[parity].dt_cur, I.surface, true, e.y);
 }
 
-template <typename TF>
-__global__ void __launch_bounds__(128, GELIOS_BATCH_FACE_MINB) batch_mhd_face_kernel(BatchTables t, int parity) {
-    const int2 e = t.units[blockIdx.x];
+// PLAIN: the plain interior group's tiles in the lean instance of the body,
+// otherwise the other units'.  One generic launch for both took 628 us per
+// step of 8 instances (1.32M cells, FP32 fluxes, ncu), these 334 and 100.
+// Register caps of 160 or 96 instead of 128: 6% and 2% slower per step.
+template <typename TF, bool PLAIN>
+__global__ void __launch_bounds__(128, PLAIN ? GELIOS_BATCH_PLAIN_MINB : GELIOS_BATCH_FACE_MINB)
+    batch_mhd_face_kernel(BatchTables t, int parity) {
+    const int2 e = PLAIN ? t.plain[blockIdx.x] : t.units[blockIdx.x];
     BATCH_INSTANCE(I, e)
     const int u = e.y + threadIdx.x;
     const StepBuffers& b = I.b[parity];
     double tmin = __longlong_as_double(0x7ff0000000000000LL);
     int status = 0;
-    if (u < I.d.n_units) tmin = mhd_face_body<TF>(I.d, I.P, I.M, b, I.hs[parity], I.fl, u, status);
+    if (u < (PLAIN ? I.d.u_c1 : I.d.n_units))
+        tmin = mhd_face_body<TF, PLAIN>(I.d, I.P, I.M, b, I.hs[parity], I.fl, u, status);
     block_reduce_commit(tmin, 0, 0, status, b.dt_acc, b.counters, b.status);
 }
 
@@ -4471,14 +4480,15 @@ __global__ void __launch_bounds__(128, GELIOS_BATCH_FACE_MINB) batch_mhd_persist
             __syncthreads();  // the next rail reuses the block's shared words
         }
         grid.sync();
-        for (int i = blockIdx.x; i < t.n_units; i += gridDim.x) {
-            const int2 e = t.units[i];
+        for (int i = blockIdx.x; i < t.n_plain + t.n_units; i += gridDim.x) {
+            const bool plain = i < t.n_plain;
+            const int2 e = plain ? t.plain[i] : t.units[i - t.n_plain];
             const BatchInstance& I = t.inst[e.x];
             const int u = e.y + threadIdx.x;
             const StepBuffers& b = I.b[parity];
             double tmin = __longlong_as_double(0x7ff0000000000000LL);
             int status = 0;
-            if (u < I.d.n_units) tmin = mhd_face_body<TF>(I.d, I.P, I.M, b, I.hs[parity], I.fl, u, status);
+            if (u < (plain ? I.d.u_c1 : I.d.n_units)) tmin = mhd_face_body<TF>(I.d, I.P, I.M, b, I.hs[parity], I.fl, u, status);
             block_reduce_commit(tmin, 0, 0, status, b.dt_acc, b.counters, b.status);
             __syncthreads();  // the next tile reuses the reduction's shared words
         }
@@ -5131,17 +5141,31 @@ void launch_words_init(void* words, double dt0, cudaStream_t s) {
 void launch_batch_words_init(const BatchTables& t, int n, cudaStream_t s) {
     if (n > 0) batch_words_init_kernel<<<blocks_for(n, 128), 128, 0, s>>>(t, n);
 }
-void launch_batch_mhd_step(const BatchTables& t, int parity, cudaStream_t s) {
+cudaError_t launch_batch_mhd_step(const BatchTables& t, int parity, cudaStream_t s, cudaStream_t s_rest,
+                                  cudaEvent_t fork, cudaEvent_t join) {
     if (t.n_surf > 0) batch_surface_kernel<<<t.n_surf, 64, 0, s>>>(t, parity);
     if (t.n_rails > 0) batch_rails_kernel<<<t.n_rails, 128, 0, s>>>(t, parity);
+    cudaError_t e = cudaEventRecord(fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s_rest, fork, 0);
+    if (e != cudaSuccess) return e;
     if (t.n_units > 0) {
         if (t.fp32)
-            batch_mhd_face_kernel<float><<<t.n_units, 128, 0, s>>>(t, parity);
+            batch_mhd_face_kernel<float, false><<<t.n_units, 128, 0, s_rest>>>(t, parity);
         else
-            batch_mhd_face_kernel<double><<<t.n_units, 128, 0, s>>>(t, parity);
+            batch_mhd_face_kernel<double, false><<<t.n_units, 128, 0, s_rest>>>(t, parity);
     }
+    if (t.n_plain > 0) {
+        if (t.fp32)
+            batch_mhd_face_kernel<float, true><<<t.n_plain, 128, 0, s>>>(t, parity);
+        else
+            batch_mhd_face_kernel<double, true><<<t.n_plain, 128, 0, s>>>(t, parity);
+    }
+    e = cudaEventRecord(join, s_rest);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join, 0);
+    if (e != cudaSuccess) return e;
     if (t.n_cells > 0) batch_mhd_update_kernel<<<t.n_cells, 128, 0, s>>>(t, parity);
     if (t.n_points > 0) batch_commit_kernel<<<t.n_points, 256, 0, s>>>(t, parity);
+    return cudaSuccess;
 }
 cudaError_t launch_batch_mhd_persistent(const BatchTables& t, int nsteps, int blocks_per_sm, cudaStream_t s,
                                         int* max_per_sm) {

@@ -276,10 +276,11 @@ struct BatchTables {
     const BatchInstance* inst = nullptr;
     const int2* surf = nullptr;    // 64-thread blocks, two tracked faces each
     const int2* rails = nullptr;   // one block per rail
-    const int2* units = nullptr;   // 128 face units per block
+    const int2* plain = nullptr;   // 128 units of the plain interior group [0, u_c1) per block
+    const int2* units = nullptr;   // 128 of the other face units [u_c1, n_units) per block
     const int2* cells = nullptr;   // 128 cells per block
     const int2* points = nullptr;  // 256 points per block (y == 0: the block that also finalises the dt)
-    int n_surf = 0, n_rails = 0, n_units = 0, n_cells = 0, n_points = 0;
+    int n_surf = 0, n_rails = 0, n_plain = 0, n_units = 0, n_cells = 0, n_points = 0;
     int fp32 = 0;                  // the instances' flux precision (all equal)
 };
 // sum |a - b| and sum |a| over n doubles into scratch[0], scratch[1]
@@ -300,8 +301,10 @@ void launch_residual_batch(const PlainInstance* inst, const int* active, int n_a
 // on the stream: for one context / for every instance of a batch.
 void launch_words_init(void* words, double dt0, cudaStream_t s);
 void launch_batch_words_init(const BatchTables& t, int n, cudaStream_t s);
-// The five launches of one batched MHD step (parity: even / odd step of the call).
-void launch_batch_mhd_step(const BatchTables& t, int parity, cudaStream_t s);
+// The six launches of one batched MHD step (parity: even / odd step of the
+// call); the units outside the plain group run on s_rest between the events.
+cudaError_t launch_batch_mhd_step(const BatchTables& t, int parity, cudaStream_t s, cudaStream_t s_rest,
+                                  cudaEvent_t fork, cudaEvent_t join);
 // All phases of `nsteps` batched MHD steps in one cooperative launch of
 // blocks_per_sm 128-thread blocks per SM (0: as many as fit); *max_per_sm
 // (optional) receives how many fit.  Errors: cudaErrorCooperativeLaunchTooLarge
