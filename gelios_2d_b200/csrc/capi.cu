@@ -107,7 +107,8 @@ struct gelios_ctx {
     DBuf X, Y, X2, Y2, ptype, cstart, contour, gstart, cflags, ctype, sA, sB, snb, ssd, ssd2, sinfo, qcorner;
     DBuf fA, fB, ftype, fmaster, fsosed, fcopy, fsdown;
     DBuf rtype, rM, rpstart, rpts, rkstart, rkeys, rs;
-    DBuf lc, li, lo, sp_point, sp_line, sp_inc, sp_ainc, sp_fix, sp_of_point;
+    DBuf lc, li, lo, sp_point, sp_line, sp_inc, sp_ainc, sp_fix, sp_of_point, rk_point, rk_node, sf_rec, rail_tab;
+    bool rail_tab_valid = false;  // launch_rail_table; stale once the topology or the parameters change
     DBuf u_slot, u_cell, u_twin, u_A, u_B, u_info, u_nb, u_sd, u_sd2, s_unit, flux, aux, rec, pstar, src_lo;
     DBuf Hn, Hu, Hv, HT, ku, kv, kT, r_istoch, cback, cnext;
     // state par[2] x 5 fields, centroids [2], scratch
@@ -118,7 +119,7 @@ struct gelios_ctx {
     gelios_mhd_params mprm{};
     DBuf src_fixed;  // MHD form: fixed charge-exchange sources (3 rows)
     DBuf flux_mhd;   // multi-fluid forms: 13 (MHD) or 21 (Go_5_komponent) flux rows per face slot, on first use
-    int mhd_face_variant = 0;  // launch shape of the MHD face kernel (gelios_autotune)
+    int mhd_face_variant = kMhdFaceDefault;  // launch shape of the MHD face kernel (gelios_autotune)
     int mk2_variant = 0;  // arrangement / launch shape of the moving-grid face units + update (gelios_autotune)
     // tiles of the moving-grid step (see TileView)
     DBuf t_cstart, t_cells, t_lbase, t_fstart, t_faces;
@@ -306,6 +307,7 @@ extern "C" int gelios_set_params(gelios_ctx* ctx, const gelios_params* prm) {
     ctx->d.r11_sq = sqrt_threshold(prm->R11);
     ctx->cen_valid = false;  // the cached |centroid|^(2 gamma) depends on gamma
     ctx->ugeo_valid = false;
+    ctx->rail_tab_valid = false;
     ctx->drop_graphs();      // the parameters are kernel arguments
     return GELIOS_OK;
 }
@@ -861,6 +863,52 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     rc |= upload(ctx->sp_ainc, sp_ainc.data(), sp_ainc.size(), s);
     rc |= upload(ctx->sp_fix, sp_fix.data(), sp_fix.size(), s);
     rc |= upload(ctx->sp_of_point, local.data(), local.size(), s);
+    if (nr > 0) {
+        const int first_c = na + nb;
+        std::vector<int4> rkp(nr), rkn(nr);
+        for (int q = 0; q < nr; q++) {
+            int k[3] = {-1, -1, -1};
+            const int k0 = v->rail_kstart[q], t = v->rail_type[q];
+            if (t <= 1)
+                for (int i = 0; i < 3; i++) k[i] = v->rail_keys[k0 + i];
+            else if (t == 2)
+                k[0] = v->rail_keys[k0];
+            else {
+                if (ncr > 0) k[0] = v->rail_keys[v->rail_kstart[first_c]];
+                k[1] = v->rail_keys[k0 + 1];
+                k[2] = v->rail_keys[k0 + 2];
+            }
+            auto node = [&](int p) { return p >= 0 ? local[p] : -1; };
+            rkp[q] = make_int4(k[0], k[1], k[2], -1);
+            rkn[q] = make_int4(node(k[0]), node(k[1]), node(k[2]), -1);
+        }
+        rc |= upload(ctx->rk_point, rkp.data(), rkp.size(), s);
+        rc |= upload(ctx->rk_node, rkn.data(), rkn.size(), s);
+    }
+    {
+        const int32_t* lines[3] = {v->line_contact, v->line_inner, v->line_outer};
+        const int nl[3] = {v->n_contact, v->n_inner_line, v->n_outer_line};
+        std::vector<int4> rec;
+        for (int l = 0; l < 3; l++)
+            for (int j = 0; j < nl[l]; j++) {
+                const int f = lines[l][j], g = v->face_copy[f];
+                const int a = v->face_A[f], b = v->face_B[f], m1 = v->face_master[f];
+                const int m2 = g >= 0 ? v->face_master[g] : -1;
+                const int ta = v->point_type[a], tb = v->point_type[b];
+                int fl = v->face_type[f] & 7;
+                if (g >= 0) fl |= (v->face_type[g] & 7) << SF_TYPE2;
+                if (m1 >= 0 && (cflags[m1] & CF_AXIS)) fl |= SF_AXIS1;
+                if (m2 >= 0 && (cflags[m2] & CF_AXIS)) fl |= SF_AXIS2;
+                if (ta == tb && (ta == P_CONTACT || ta == P_INNER_SHOCK || ta == P_OUTER_SHOCK)) fl |= SF_TRACKED;
+                rec.push_back(make_int4(a, b, m1, v->face_sosed[f]));
+                rec.push_back(make_int4(fsdown[f], m2, g >= 0 ? v->face_sosed[g] : -1, g >= 0 ? fsdown[g] : -1));
+                rec.push_back(make_int4(fl, 0, 0, 0));
+            }
+        rc |= upload(ctx->sf_rec, rec.data(), rec.size(), s);
+    }
+    rc |= upload<double>(ctx->rail_tab, nullptr,
+                         2 * static_cast<size_t>(nr) + (nr > 0 ? v->rail_pstart[nr] : 0) + 1, s);
+    ctx->rail_tab_valid = false;
     rc |= upload<double>(ctx->Hn, nullptr, 4 * static_cast<size_t>(nc), s);
     rc |= upload<double>(ctx->Hu, nullptr, 4 * static_cast<size_t>(nc), s);
     rc |= upload<double>(ctx->Hv, nullptr, 4 * static_cast<size_t>(nc), s);
@@ -964,6 +1012,12 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     d.sp_ainc = ctx->sp_ainc.as<int32_t>();
     d.sp_fix = ctx->sp_fix.as<int32_t>();
     d.sp_of_point = ctx->sp_of_point.as<int32_t>();
+    d.rk_point = ctx->rk_point.as<int4>();
+    d.rk_node = ctx->rk_node.as<int4>();
+    d.sf_rec = ctx->sf_rec.as<int4>();
+    d.rcs = ctx->rail_tab.as<double>();
+    d.rsn = d.rcs + nr;
+    d.rfrac = d.rsn + nr;
     d.Hn = ctx->Hn.as<double>();
     d.Hu = ctx->Hu.as<double>();
     d.Hv = ctx->Hv.as<double>();
@@ -1467,6 +1521,15 @@ void set_unit_geometry(const gelios_ctx* ctx, StepBuffers& b) {
     }
 }
 
+// the rails' constant tables, before the motion kernels read them
+void ensure_rail_table(gelios_ctx* ctx, cudaStream_t s) {
+    if (ctx->rail_tab_valid) return;
+    const DevMesh& d = ctx->d;
+    launch_rail_table(d, ctx->prm.n_inner, const_cast<double*>(d.rcs), const_cast<double*>(d.rsn),
+                      const_cast<double*>(d.rfrac), s);
+    ctx->rail_tab_valid = true;
+}
+
 bool pipe_ok(const gelios_ctx* ctx) {
     const int v = ctx->mk2_variant;
     return ctx->pipelined && !ctx->timing && !(v >= 4 && v < 8);
@@ -1620,6 +1683,7 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             ctx->coop_off = true;
         }
     }
+    if (moving) ensure_rail_table(ctx, s);
     // a one-step call has no next step to overlap: one graph per step
     if (form == GELIOS_FORM_MK2 && nsteps > 1 && pipe_ok(ctx)) {
         const int n = mk2_pipelined(ctx, nsteps, cen0, cen1);
@@ -2277,6 +2341,7 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
             launch_centroid(d, d.X, d.Y, cen0, cen0 + nc, cen0 + 2 * nc, c->prm.gamma, s, cen0 + 3 * nc, cen0 + 4 * nc);
             c->cen_rp_partial = false;
         }
+        ensure_rail_table(c, s);
         {
             BatchInstance& I = B->host_inst[i];
             I.d = d;

@@ -377,14 +377,20 @@ __device__ __forceinline__ double lev_dev(double ga, double enI, double pI, doub
 // between pI and pII, stopping where |lev| <= 1e-9 (cap max_iter).
 //
 // COOP = true: the 32 lanes of a warp call it with identical arguments and
-// walk the same bisection together.  Each round, lanes 0..30 evaluate lev at
-// the 31 midpoints of the next five bisection levels (lane j = node j+1 of a
-// heap-ordered binary tree, its interval derived from the round's interval by
-// the same halvings the sequential loop performs), then every lane replays
-// the five sequential decisions on the broadcast values.  The midpoints, the
-// function values and the decisions are the ones of the sequential loop, so
-// the result and the iteration count are the same; the latency is one lev
-// evaluation per five iterations instead of five.
+// walk the same bisection together, many levels per round.  A round covers the
+// next D levels: the bracket's dyadic points at depth D, of which the lanes
+// evaluate a window of 32 consecutive ones (each lane derives its point by the
+// halvings the sequential loop performs).  lev increases with the pressure, so
+// a window whose ends straddle the root decides every level: a midpoint in
+// the window by its value, one outside it by its side (and |lev| there is
+// above the window end's, so above epsil).  The first round has D = 5 and
+// evaluates every point; later rounds centre the window on the root of the
+// cubic through the four values around the bracket (inverse interpolation, in
+// FP32: it only picks where to look), down to the level where |lev| <= epsil
+// must hold.  A window that misses is followed by a plain D = 5 round.  The
+// midpoints, the values that decide and the order of the decisions are the
+// sequential loop's, so the result and the iteration count are too.  About 30
+// levels take three rounds instead of six (one lev costs ~2400 cycles).
 template <bool COOP>
 __device__ __forceinline__ double godunov_devtwo(double ga, double enI, double pI, double rI, double enII, double pII,
                                                  double rII, int max_iter, int* status) {
@@ -413,36 +419,90 @@ __device__ __forceinline__ double godunov_devtwo(double ga, double enI, double p
             }
         }
     }
-    const int node = (threadIdx.x & 31) + 1;  // 1..32; node 32 (level 5) evaluates nothing
-    const int L = 31 - __clz(node);
-    const int idx = node - (1 << L);
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int D = 5, k0 = 0;
+    double kr = ksir0;  // lev at kp
     for (;;) {
-        double a = kl, b = kp;
-        for (int l = 0; l < L; l++) {
-            const double c = (a + b) / 2.0;
-            if ((idx >> (L - 1 - l)) & 1) a = c;
-            else b = c;
+        // the lane's dyadic point k0 + lane of 2^D: the odd part of its index
+        // gives the level, the bits above it the path
+        const int idx = k0 + lane;
+        const int z = idx ? __ffs(idx) - 1 : 0, L = idx ? D - z : 0;
+        const int path = idx >> (z + 1);
+        double a = kl, b = kp, x = kl;
+        for (int l = 1; l <= L; l++) {
+            x = (a + b) / 2.0;
+            if (l < L) {
+                if ((path >> (L - 1 - l)) & 1) a = x;
+                else b = x;
+            }
         }
-        double f = 0.0;
-        if (L < 5) f = lev_dev(ga, enI, pI, rI, enII, pII, rII, (a + b) / 2.0);
-        int nd = 1;
-        for (int l = 0; l < 5; l++) {
+        const double f = lev_dev(ga, enI, pI, rI, enII, pII, rII, x);
+        if (D > 5) {
+            const double f0 = __shfl_sync(full, f, 0), f31 = __shfl_sync(full, f, 31);
+            const bool lo = k0 == 0 || (ksi * f0 > 0.0 && fabs(f0) > epsil);
+            const bool hi = k0 + 32 == (1 << D) || (ksi * f31 <= 0.0 && fabs(f31) > epsil);
+            if (!(lo && hi)) {  // the root is elsewhere
+                D = 5;
+                k0 = 0;
+                continue;
+            }
+        }
+        int I = 0;  // index of kl at depth D
+        for (int l = 0; l < D; l++) {
             k = k + 1;
             if (k >= max_iter) {
                 *status |= ST_ITER_CAP;
                 return (kl + kp) / 2.0;
             }
             const double kc = (kl + kp) / 2.0;
-            const double ksit = __shfl_sync(0xffffffffu, f, nd - 1);
-            if (fabs(ksit) <= epsil) return kc;
-            if ((ksi * ksit) <= 0.0) {
-                kp = kc;
-                nd = 2 * nd;
-            } else {
+            const int half = 1 << (D - 1 - l), m = I + half - k0;
+            const double ksit = __shfl_sync(full, f, m & 31);
+            if (m >= 0 && m < 32) {
+                if (fabs(ksit) <= epsil) return kc;
+                if ((ksi * ksit) <= 0.0) {
+                    kp = kc;
+                    kr = ksit;
+                } else {
+                    kl = kc;
+                    ksi = ksit;
+                    I += half;
+                }
+            } else if (m < 0) {  // left of the window, left of the root
                 kl = kc;
-                ksi = ksit;
-                nd = 2 * nd + 1;
+                I += half;
+            } else {
+                kp = kc;
             }
+        }
+        // where in [kl, kp] the root lies: inverse interpolation through the
+        // window's values at I - 1, I, I + 1, I + 2 (two values at its ends)
+        const int w = I - k0;
+        const double fm = __shfl_sync(full, f, (w - 1) & 31), fn = __shfl_sync(full, f, (w + 2) & 31);
+        if (w >= 0 && w < 32) ksi = __shfl_sync(full, f, w);  // the value at kl itself (a level outside kept its sign only)
+        if (w >= 0 && w < 31) kr = __shfl_sync(full, f, w + 1);
+        const float y1 = static_cast<float>(ksi), y2 = static_cast<float>(kr);
+        float th = y1 / (y1 - y2);
+        if (w >= 1 && w <= 29) {
+            const float y0 = static_cast<float>(fm), y3 = static_cast<float>(fn);
+            // Neville at f = 0 through (y, position) = (y0, -1), (y1, 0), (y2, 1), (y3, 2)
+            const float p01 = -y1 / (y1 - y0), p12 = th, p23 = 1.f - y2 / (y3 - y2);
+            const float p02 = (y2 * p01 - y0 * p12) / (y2 - y0), p13 = (y3 * p12 - y1 * p23) / (y3 - y1);
+            th = (y3 * p02 - y0 * p13) / (y3 - y0);
+        }
+        // depth at which a midpoint must satisfy |lev| <= epsil, at most 8
+        // levels after the first round (its estimate holds to about 1e-3)
+        const float span = fabsf(y2 - y1);
+        int need = span > 1e-9f ? static_cast<int>(ceilf(log2f(span * 1e9f))) + 1 : 1;
+        if (D == 5 && need > 8) need = 8;
+        if (need > 22) need = 22;
+        D = 5;
+        k0 = 0;
+        if (need > 5 && th > 0.f && th < 1.f) {
+            D = need;
+            k0 = static_cast<int>(th * static_cast<float>(1 << D)) - 15;
+            if (k0 < 0) k0 = 0;
+            if (k0 > (1 << D) - 32) k0 = (1 << D) - 32;
         }
     }
 }
@@ -495,13 +555,15 @@ __device__ __forceinline__ double godunov_newton(double ga, double enI, double p
 // The star pressure of the two iterative branches does not depend on the
 // face speed w: p_out (if given) receives the pressure after the branch
 // selection, and p_in (if given) replaces the iteration by that value, so a
-// caller can solve before the grid moves and sample after it.  COOP selects
-// the warp-cooperative bisection (all 32 lanes, identical arguments).
+// caller can solve before the grid moves and sample after it.  With p_out the
+// call ends there; with only_speeds it ends once ds is known (neither then
+// samples a flux).  COOP selects the warp-cooperative bisection (all 32
+// lanes, identical arguments).
 template <bool COOP>
 static __device__ __noinline__ double godunov_dev(double ga, double kurant, const double* qqq1, const double* qqq2,
                                            const double* n, double* qqq, double* ds, double w, double DIST,
                                            int max_iter, int* status, const double* p_in = nullptr,
-                                           double* p_out = nullptr) {
+                                           double* p_out = nullptr, bool only_speeds = false) {
     const double g1 = ga - 1.0, g2 = ga + 1.0, gm = (g1 / ga) / 2.0;
     const double eps = 10e-10, eps8 = 10e-8;
     const double al = n[0], be = n[1], ge = n[2];
@@ -547,7 +609,10 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
         p = p_in ? *p_in : godunov_newton(ga, enI, pI, rI, enII, pII, rII, max_iter, status);
         il = 1; ip = 1;
     }
-    if (p_out) *p_out = p;
+    if (p_out) {
+        *p_out = p;
+        return time;
+    }
     if ((il == 1) && (ip == 1)) {  // two shocks
         const double aI = sqrt(rI * (g2 / 2.0 * p + g1 / 2.0 * pI));
         const double aII = sqrt(rII * (g2 / 2.0 * p + g1 / 2.0 * pII));
@@ -557,7 +622,8 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
         dsl = dI; dsp = dII; dsc = u;
         const double UU = dmax_ref(fabs(dsl), fabs(dsp));
         time = (UU > eps8) ? UU : eps8;
-        if (w <= dI) {
+        if (only_speeds) {
+        } else if (w <= dI) {
             en = enI; p = pI; r = rI; te2 = teI2; te3 = teI3;
         } else if ((w > dI) && (w <= u)) {
             en = u; r = rI * aI / (aI - rI * (enI - u)); te2 = teI2; te3 = teI3;
@@ -580,6 +646,7 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
         double UU = dmax_ref(fabs(dsl), fabs(dsp));
         UU = dmax_ref(UU, fabs(ddII));
         time = (UU > eps8) ? UU : eps8;
+        if (only_speeds) goto speeds;
         if (w <= dI) {
             en = enI; p = pI; r = rI; te2 = teI2; te3 = teI3;
         }
@@ -614,6 +681,7 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
         UU = dmax_ref(UU, fabs(ddII));
         UU = dmax_ref(UU, fabs(ddI));
         time = (UU > eps8) ? UU : eps8;
+        if (only_speeds) goto speeds;
         if (w <= dI) {
             en = enI; p = pI; r = rI; te2 = teI2; te3 = teI3;
         }
@@ -647,6 +715,7 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
         UU = dmax_ref(UU, fabs(ddII));
         UU = dmax_ref(UU, fabs(ddI));
         time = (UU > eps8) ? UU : eps8;
+        if (only_speeds) goto speeds;
         if (w <= dI) {
             en = enI; p = pI; r = rI; te2 = teI2; te3 = teI3;
         }
@@ -665,6 +734,7 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
             en = enII; p = pII; r = rII; te2 = teII2; te3 = teII3;
         }
     }
+speeds:
     if (ipiz == 1) {
         en = -en;
         const double dsl1 = dsl, dsp1 = dsp;
@@ -672,6 +742,12 @@ static __device__ __noinline__ double godunov_dev(double ga, double kurant, cons
         dsp = -dsl1;
         dsc = -dsc;
         w = -w;
+    }
+    if (only_speeds) {
+        ds[0] = dsl;
+        ds[1] = dsp;
+        ds[2] = dsc;
+        return time;
     }
     const double uo = al * en + al2 * te2 + al3 * te3;
     const double vo = be * en + be2 * te2 + be3 * te3;

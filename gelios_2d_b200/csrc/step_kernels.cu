@@ -2770,18 +2770,28 @@ __global__ void commit_kernel(DevMesh d, StepBuffers b) {
 // end nodes of its line.  point_velocity replays exactly those operations for
 // one point, so the rails can evaluate their key points directly from the
 // per-face speeds (bit-identical to the serial passes).
-__device__ __forceinline__ void node_pass1(const DevMesh& d, const double* __restrict__ scratch, int i, double& v,
-                                           double& w, int& c) {
-    const int line = d.sp_line[i];
+__device__ __forceinline__ void node_pass1(const DevMesh& d, const double* __restrict__ scratch, int i, int line,
+                                           double& v, double& w, int& c) {
+    // the node's faces and their rows, each in one level of loads
+    const int4 inc = reinterpret_cast<const int4*>(d.sp_inc)[i];
+    const int e[4] = {inc.x, inc.y, inc.z, inc.w};
+    const int4 ai = reinterpret_cast<const int4*>(d.sp_ainc)[i];
+    const int an[4] = {ai.x, ai.y, ai.z, ai.w};
+    double2 f01[4], f23[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double2* r = reinterpret_cast<const double2*>(scratch + 4 * (e[k] < 0 ? 0 : e[k] >> 1));
+        f01[k] = r[0];
+        f23[k] = r[1];
+    }
     v = 0.0;
     w = 0.0;
     c = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int e = d.sp_inc[4 * i + k];
-        if (e < 0) break;
-        const int j = e >> 1, role = e & 1;  // role 0: A end, 1: B end
-        const double* f = scratch + 4 * j;
+        if (e[k] < 0) break;
+        const int role = e[k] & 1;  // role 0: A end, 1: B end
+        const double f[4] = {f01[k].x, f01[k].y, f23[k].x, f23[k].y};
         const double br = f[3];
         bool add;
         if (line == 0) add = role == 1;
@@ -2796,8 +2806,7 @@ __device__ __forceinline__ void node_pass1(const DevMesh& d, const double* __res
     if (line == 0) {  // first averaging pass: every contact face (Setka.cpp:3522-3530)
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const int j = d.sp_ainc[4 * i + k];
-            if (j < 0) break;
+            if (an[k] < 0) break;
             if (c > 0) {
                 v /= (1.0 * c);
                 w /= (1.0 * c);
@@ -2806,60 +2815,74 @@ __device__ __forceinline__ void node_pass1(const DevMesh& d, const double* __res
     }
 }
 
-// Vx, Vy of point p after Move_surface (0 for points off the tracked lines:
-// every step starts from zero velocities, Setka.cpp:10473-10480).
-__device__ void point_velocity(const DevMesh& d, const double* __restrict__ scratch, double dt, int p, double& vx,
-                               double& vy) {
-    const int i = d.sp_of_point[p];
-    vx = 0.0;
-    vy = 0.0;
+// Vx, Vy after Move_surface of the node i of each group of eight lanes (0 for
+// i < 0, a point off the tracked lines: every step starts from zero
+// velocities, Setka.cpp:10473-10480), called by a whole warp.  Lane 4 of the
+// group takes the node's own first pass, lanes 0-3 those of the four end
+// nodes of its line when the node is one of them; every lane gets the result.
+__device__ __forceinline__ void point_velocity(const DevMesh& d, const double* __restrict__ scratch, double dt, int i,
+                                               double& vx, double& vy) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, m = lane & 7, g0 = lane & 24;
+    const int line = i >= 0 ? d.sp_line[i] : 0;
+    const int4 fx = reinterpret_cast<const int4*>(d.sp_fix)[line];  // a0, b0 (first face), a_last, b_last
+    const bool end = i >= 0 && (i == fx.x || i == fx.w);
+    const int own = m == 0 ? fx.x : m == 1 ? fx.y : m == 2 ? fx.z : fx.w;
+    const int node = m == 4 ? i : (end && m < 4) ? own : -1;
+    double v = 0.0, w = 0.0, px = 0.0, py = 0.0;
+    int c = 0;
+    if (node >= 0) {
+        if (end) {
+            const int p = d.sp_point[node];
+            px = d.X[p];
+            py = d.Y[p];
+        }
+        node_pass1(d, scratch, node, line, v, w, c);
+    }
+    double lx[4], ly[4], ex[4], ey[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        lx[q] = __shfl_sync(full, v, g0 + q);
+        ly[q] = __shfl_sync(full, w, g0 + q);
+        ex[q] = __shfl_sync(full, px, g0 + q);
+        ey[q] = __shfl_sync(full, py, g0 + q);
+    }
+    vx = __shfl_sync(full, v, g0 + 4);
+    vy = __shfl_sync(full, w, g0 + 4);
+    c = __shfl_sync(full, c, g0 + 4);
     if (i < 0) return;
-    int c;
-    node_pass1(d, scratch, i, vx, vy, c);
-    const int line = d.sp_line[i];
-    const int32_t* fx = d.sp_fix + 4 * line;  // a0, b0 (first face), a_last, b_last
-    if (i == fx[0] || i == fx[3]) {
+    if (end) {
         // replay the end-node fix-ups of this line in the reference's order
         // on local copies of the four end nodes (aliases kept in sync)
-        int id[4];
-        double lx[4], ly[4];
+        const int id[4] = {fx.x, fx.y, fx.z, fx.w};
+        auto setx = [&](int nd, double val) {
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-            id[m] = fx[m];
-            int cm;
-            node_pass1(d, scratch, id[m], lx[m], ly[m], cm);
-        }
-        auto setx = [&](int node, double val) {
-#pragma unroll
-            for (int m = 0; m < 4; m++)
-                if (id[m] == node) lx[m] = val;
+            for (int q = 0; q < 4; q++)
+                if (id[q] == nd) lx[q] = val;
         };
-        auto sety = [&](int node, double val) {
+        auto sety = [&](int nd, double val) {
 #pragma unroll
-            for (int m = 0; m < 4; m++)
-                if (id[m] == node) ly[m] = val;
+            for (int q = 0; q < 4; q++)
+                if (id[q] == nd) ly[q] = val;
         };
-        const double* X = d.X;
-        const double* Y = d.Y;
-        const int pa0 = d.sp_point[id[0]], pb0 = d.sp_point[id[1]], pa1 = d.sp_point[id[2]], pb1 = d.sp_point[id[3]];
         // fx[0]: vx[a0] = vx[b0] + (X[b0] - X[a0]) / dt on every line
-        setx(id[0], lx[1] + (X[pb0] - X[pa0]) / dt);
+        setx(id[0], lx[1] + (ex[1] - ex[0]) / dt);
         if (line == 1) {
             // inner shock: vx[b1] = vx[a1] + (X[a1] - X[b1]) / dt (Setka.cpp:3733-3736)
             double a1x = lx[2];
 #pragma unroll
-            for (int m = 0; m < 4; m++)
-                if (id[m] == id[2]) a1x = lx[m];
-            setx(id[3], a1x + (X[pa1] - X[pb1]) / dt);
+            for (int q = 0; q < 4; q++)
+                if (id[q] == id[2]) a1x = lx[q];
+            setx(id[3], a1x + (ex[2] - ex[3]) / dt);
         } else {
             // contact / outer shock: vy[b1] = vy[a1] + (Y[a1] - Y[b1]) / dt
-            sety(id[3], ly[2] + (Y[pa1] - Y[pb1]) / dt);
+            sety(id[3], ly[2] + (ey[2] - ey[3]) / dt);
         }
 #pragma unroll
-        for (int m = 0; m < 4; m++)
-            if (id[m] == i) {
-                vx = lx[m];
-                vy = ly[m];
+        for (int q = 0; q < 4; q++)
+            if (id[q] == i) {
+                vx = lx[q];
+                vy = ly[q];
             }
     }
     if (line == 0) {
@@ -2868,11 +2891,13 @@ __device__ void point_velocity(const DevMesh& d, const double* __restrict__ scra
         const int nC = d.n_lc, nI = d.n_li, nO = d.n_lo;
         const int lim2 = nI > 0 ? (nI < nC ? nI : nC) : 0;
         const int lim3 = nO > 0 ? (nO < nC ? nO : nC) : 0;
+        const int4 ai = reinterpret_cast<const int4*>(d.sp_ainc)[i];
+        const int an[4] = {ai.x, ai.y, ai.z, ai.w};
         for (int pass = 0; pass < 2; pass++) {
             const int lim = pass == 0 ? lim2 : lim3;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const int j = d.sp_ainc[4 * i + k];
+                const int j = an[k];
                 if (j < 0) break;
                 if (j < lim && c > 0) {
                     vx /= (1.0 * c);
@@ -2894,13 +2919,37 @@ __device__ void point_velocity(const DevMesh& d, const double* __restrict__ scra
 //  * the first point of every D rail is a point of C_Rails[0]; the D block
 //    recomputes that point's new position from C_Rails[0]'s key point with
 //    the same operations (bit-identical to reading it back).
-__device__ __forceinline__ void c0_key(const DevMesh& d, int q, double dt, double vx, double vy, double& x2,
-                                       double& y2) {
-    const int K0 = d.rkeys[d.rkstart[q]];
-    const double s = d.rs[q], cs = cos(s), sn = sin(s);
-    const double V = vx * cs + vy * sn;
-    x2 = d.X[K0] + dt * V * cs;
-    y2 = d.Y[K0] + dt * V * sn;
+// The rails' constants: cos and sin of their angle, and of every point the
+// power law its radius or height follows between two key points (inner layer,
+// Setka.cpp:4390-4406; the A rails' outer layer, 4443-4456).
+__global__ void rail_table_kernel(DevMesh d, int ni, double* __restrict__ rcs, double* __restrict__ rsn,
+                                  double* __restrict__ rfrac) {
+    const int q = blockIdx.x;
+    const double s = d.rs[q];
+    if (threadIdx.x == 0) {
+        rcs[q] = cos(s);
+        rsn[q] = sin(s);
+    }
+    const int t = d.rtype[q], p0 = d.rpstart[q], np = d.rpstart[q + 1] - p0;
+    const int M1 = d.rM[4 * q], M2 = d.rM[4 * q + 1], M3 = d.rM[4 * q + 2], M4 = d.rM[4 * q + 3];
+    const double dd = 1.5708 / sqrt(1.0 - 1.0 / 1.76);
+    const double e = 1.76 * (1.0 - sq(s / dd));
+    for (int j = threadIdx.x; j < np; j += blockDim.x) {
+        double f = 0.0;
+        if (t <= 2 && j < M1 - 1) {
+            if (j < ni) {
+                const double x = j * 1.0 / (ni);
+                f = pow(x, 1.3);
+            } else {
+                const double x = (j - ni) * 1.0 / (M1 - 1 - ni);
+                f = pow(x, 1.05);
+            }
+        } else if (t == 0 && j >= M1 + M2 + M3) {
+            const double x = (j - (M1 + M2 + M3) + 1) * 1.0 / (M4);
+            f = pow(x, e);
+        }
+        rfrac[p0 + j] = f;
+    }
 }
 
 // copy_outer_shock: Move_Setka_Calculate_2 gives the D rails beyond
@@ -2925,59 +2974,71 @@ __device__ __forceinline__ void rails_body(const DevMesh& d, const gelios_params
     const double* Y = d.Y;
     __shared__ double sh[6];
     const int ni = P.n_inner;
-    // velocities of the key points this rail reads, one thread each
-    __shared__ double kvx[4], kvy[4];
-    if (threadIdx.x < 4) {
-        int pt = -1;
-        const int k = threadIdx.x;
-        if (t == 0 || t == 1) {
-            if (k < 3) pt = kp[k];
-        } else if (t == 2) {
-            if (k == 0) pt = kp[0];
-        } else {
-            if (k == 0) pt = d.rkeys[d.rkstart[first_c]];  // key point 0 of C_Rails[0]
-            else if (k < 3) pt = kp[k];
-            else if (copy_outer_shock && q - first_d >= P.n_outer_shock && P.n_outer_shock >= 1)
-                pt = d.rkeys[d.rkstart[first_d + P.n_outer_shock - 1] + 2];
+    // velocities and positions of the key points this rail reads, by the
+    // first warp, eight lanes a point
+    __shared__ double kvx[4], kvy[4], kx[4], ky[4];
+    const double* frac = d.rfrac + d.rpstart[q];
+    const int K3 = t == 2 ? -1 : kp[3];
+    double x3 = 0.0, y3 = 0.0;
+    if (threadIdx.x == 0 && K3 >= 0) {
+        x3 = X[K3];
+        y3 = Y[K3];
+    }
+    if (threadIdx.x < 32) {
+        const int k = threadIdx.x >> 3;
+        const int4 pp = d.rk_point[q], nn = d.rk_node[q];
+        int pt = k == 0 ? pp.x : k == 1 ? pp.y : k == 2 ? pp.z : -1;
+        int node = k == 0 ? nn.x : k == 1 ? nn.y : k == 2 ? nn.z : -1;
+        if (k == 3 && t == 3 && copy_outer_shock && q - first_d >= P.n_outer_shock && P.n_outer_shock >= 1) {
+            pt = d.rkeys[d.rkstart[first_d + P.n_outer_shock - 1] + 2];
+            node = d.sp_of_point[pt];
         }
-        double vx = 0.0, vy = 0.0;
-        if (pt >= 0) point_velocity(d, scratch, dt, pt, vx, vy);
-        kvx[k] = vx;
-        kvy[k] = vy;
+        double xp = 0.0, yp = 0.0;
+        if (pt >= 0) {
+            xp = X[pt];
+            yp = Y[pt];
+        }
+        double vx, vy;
+        point_velocity(d, scratch, dt, node, vx, vy);
+        if ((threadIdx.x & 7) == 0) {
+            kvx[k] = vx;
+            kvy[k] = vy;
+            kx[k] = xp;
+            ky[k] = yp;
+        }
     }
     __syncthreads();
     if (t == 0 || t == 1 || t == 2) {
-        const double s = d.rs[q];
-        const double cs = cos(s), sn = sin(s);
+        const double cs = d.rcs[q], sn = d.rsn[q];
         if (threadIdx.x == 0) {
             if (t == 0) {  // A rail, Setka.cpp:4331-4356
                 for (int kk = 0; kk < 3; kk++) {
                     const int K = kp[kk];
                     const double V = kvx[kk] * cs + kvy[kk] * sn;
-                    X2[K] = X[K] + dt * V * cs;
-                    Y2[K] = Y[K] + dt * V * sn;
+                    X2[K] = kx[kk] + dt * V * cs;
+                    Y2[K] = ky[kk] + dt * V * sn;
                 }
-                X2[kp[3]] = X[kp[3]];
-                Y2[kp[3]] = Y[kp[3]];
+                X2[K3] = x3;
+                Y2[K3] = y3;
                 sh[0] = sqrt(sq(X2[kp[0]]) + sq(Y2[kp[0]]));
                 sh[1] = sqrt(sq(X2[kp[1]]) + sq(Y2[kp[1]]));
                 sh[2] = sqrt(sq(X2[kp[2]]) + sq(Y2[kp[2]]));
             } else if (t == 1) {  // B rail, Setka.cpp:4469-4502
-                const int K0 = kp[0], K1 = kp[1], K2 = kp[2], K3 = kp[3];
+                const int K0 = kp[0], K1 = kp[1], K2 = kp[2];
                 double V = kvx[0] * cs + kvy[0] * sn;
-                const double x0 = X[K0] + dt * V * cs, y0 = Y[K0] + dt * V * sn;
+                const double x0 = kx[0] + dt * V * cs, y0 = ky[0] + dt * V * sn;
                 if (!handoff) {
                     X2[K0] = x0;
                     Y2[K0] = y0;
                 }
                 V = kvx[1] * 0.0 + kvy[1] * 1.0;
                 X2[K1] = x0;
-                Y2[K1] = Y[K1] + dt * V;
+                Y2[K1] = ky[1] + dt * V;
                 V = kvx[2] * 0.0 + kvy[2] * 1.0;
                 X2[K2] = x0;
-                Y2[K2] = Y[K2] + dt * V;
+                Y2[K2] = ky[2] + dt * V;
                 X2[K3] = x0;
-                Y2[K3] = Y[K3];
+                Y2[K3] = y3;
                 sh[0] = sqrt(sq(x0) + sq(y0));
                 sh[1] = Y2[K1];
                 sh[2] = Y2[K2];
@@ -2986,8 +3047,8 @@ __device__ __forceinline__ void rails_body(const DevMesh& d, const gelios_params
             } else {  // C rail, Setka.cpp:4603-4614
                 const int K0 = kp[0], K1 = kp[1];
                 const double V = kvx[0] * cs + kvy[0] * sn;
-                X2[K0] = X[K0] + dt * V * cs;
-                Y2[K0] = Y[K0] + dt * V * sn;
+                X2[K0] = kx[0] + dt * V * cs;
+                Y2[K0] = ky[0] + dt * V * sn;
                 X2[K1] = P.Left;
                 Y2[K1] = Y[K1];
                 sh[0] = sqrt(sq(X2[K0]) + sq(Y2[K0]));
@@ -3000,13 +3061,8 @@ __device__ __forceinline__ void rails_body(const DevMesh& d, const gelios_params
         if (!handoff) {  // inner layer, Setka.cpp:4390-4406 (and 4532-4548, 4644-4660)
             for (int j = threadIdx.x; j < M1 - 1; j += blockDim.x) {
                 double r;
-                if (j < ni) {
-                    const double x = j * 1.0 / (ni);
-                    r = P.R1 + pow(x, 1.3) * (P.R111 - P.R1);
-                } else {
-                    const double x = (j - ni) * 1.0 / (M1 - 1 - ni);
-                    r = P.R111 + pow(x, 1.05) * (R2 - P.R111);
-                }
+                if (j < ni) r = P.R1 + frac[j] * (P.R111 - P.R1);
+                else r = P.R111 + frac[j] * (R2 - P.R111);
                 X2[ap[j]] = r * cs;
                 Y2[ap[j]] = r * sn;
             }
@@ -3023,11 +3079,8 @@ __device__ __forceinline__ void rails_body(const DevMesh& d, const gelios_params
                 X2[ap[M1 + M2 + j]] = r * cs;
                 Y2[ap[M1 + M2 + j]] = r * sn;
             }
-            const double dd = 1.5708 / sqrt(1.0 - 1.0 / 1.76);
-            const double e = 1.76 * (1.0 - sq(s / dd));
             for (int j = threadIdx.x; j < M4; j += blockDim.x) {
-                const double x = (j + 1) * 1.0 / (M4);
-                const double r = R4 + pow(x, e) * (P.R5 - R4);
+                const double r = R4 + frac[M1 + M2 + M3 + j] * (P.R5 - R4);
                 X2[ap[M1 + M2 + M3 + j]] = r * cs;
                 Y2[ap[M1 + M2 + M3 + j]] = r * sn;
             }
@@ -3059,10 +3112,11 @@ __device__ __forceinline__ void rails_body(const DevMesh& d, const gelios_params
     const int jj = q - first_d;
     const int sM2 = d.dims[5], sM3 = d.dims[6], sM4 = d.dims[7];
     if (threadIdx.x == 0) {
-        const int K1 = kp[1], K2 = kp[2], K3 = kp[3];
+        const int K1 = kp[1], K2 = kp[2];
         // key point 0 = point M1 + jj of C_Rails[0], as the C pass moves it
-        double c0x, c0y;
-        c0_key(d, first_c, dt, kvx[0], kvy[0], c0x, c0y);
+        const double cs = d.rcs[first_c], sn = d.rsn[first_c];
+        const double V0 = kvx[0] * cs + kvy[0] * sn;
+        const double c0x = kx[0] + dt * V0 * cs, c0y = ky[0] + dt * V0 * sn;
         const int Mc1 = d.rM[4 * first_c], Mc2 = d.rM[4 * first_c + 1];
         const int j = Mc1 + jj;
         const double xr = pow(P.Left / (c0x), 1.0 / (Mc2));
@@ -3070,18 +3124,16 @@ __device__ __forceinline__ void rails_body(const DevMesh& d, const gelios_params
         const double y0 = c0y;
         double V = kvy[1];
         X2[K1] = x0;
-        Y2[K1] = Y[K1] + dt * V;
+        Y2[K1] = ky[1] + dt * V;
         V = kvy[2];
         X2[K2] = x0;
         if (copy_outer_shock && jj >= P.n_outer_shock && P.n_outer_shock >= 1) {
-            const int qs = first_d + P.n_outer_shock - 1;
-            const int Ks = d.rkeys[d.rkstart[qs] + 2];
-            Y2[K2] = Y[Ks] + dt * kvy[3];
+            Y2[K2] = ky[3] + dt * kvy[3];
         } else {
-            Y2[K2] = Y[K2] + dt * V;
+            Y2[K2] = ky[2] + dt * V;
         }
         X2[K3] = x0;
-        Y2[K3] = Y[K3];
+        Y2[K3] = y3;
         sh[0] = y0;
         sh[1] = Y2[K1];
         sh[2] = Y2[K2];
@@ -3109,22 +3161,13 @@ __global__ void __launch_bounds__(128) rails_kernel(DevMesh d, gelios_params P, 
 }
 
 // ------------------------------------------------------------------ surface tracking
-// Get_par_TVD of a main/copy face f read through the face table.
-__device__ St5 face_tvd(const DevMesh& d, const double* const* st, const double* cx, const double* cy, int f,
-                        int* status) {
-    const int ft = d.ftype[f];
-    const int M = d.fmaster[f];
-    const int a = d.fA[f], bb = d.fB[f];
+// Get_par_TVD of a tracked face with end points a, bb seen from master M.
+__device__ St5 face_tvd(const DevMesh& d, const double* const* st, const double* cx, const double* cy, int a, int bb,
+                        int ft, int M, int So, int Sd, bool axis, bool tracked, int* status) {
     const double fx = (d.X[a] + d.X[bb]) / 2.0, fy = (d.Y[a] + d.Y[bb]) / 2.0;
     const St5 Ms = load_state(st, M);
-    if (ft == G_USUALY) {
-        const int ta = d.ptype[a], tb = d.ptype[bb];
-        const bool tracked = (ta == P_CONTACT && tb == P_CONTACT) || (ta == P_INNER_SHOCK && tb == P_INNER_SHOCK) ||
-                             (ta == P_OUTER_SHOCK && tb == P_OUTER_SHOCK);
-        return tvd_usualy(st, cx, cy, fx, fy, Ms, cx[M], cy[M], d.fsosed[f], d.fsdown[f],
-                          (d.cflags[M] & CF_AXIS) != 0, tracked, status);
-    }
-    if (ft == G_AXIS) return tvd_axis(st, cx, cy, fx, fy, Ms, cx[M], cy[M], d.fsdown[f]);
+    if (ft == G_USUALY) return tvd_usualy(st, cx, cy, fx, fy, Ms, cx[M], cy[M], So, Sd, axis, tracked, status);
+    if (ft == G_AXIS) return tvd_axis(st, cx, cy, fx, fy, Ms, cx[M], cy[M], Sd);
     St5 o = Ms;
     return o;  // Extern/Upper_wall/Input/Inner faces do not occur on tracked lines
 }
@@ -3147,11 +3190,15 @@ __device__ __forceinline__ void surface_face_body(const DevMesh& d, const gelios
     int status = 0;
     const double ga = P.gamma, g2 = 2.0 * P.gamma;
     double nv[3], q1[5], q2[5], qq[5], ds[3];
-    int f;
-    if (j < nC) f = d.lc[j];
-    else if (j < nC + nI) f = d.li[j - nC];
-    else f = d.lo[j - nC - nI];
-    const int a = d.fA[f], bb = d.fB[f];
+    const int4 r0 = d.sf_rec[3 * j], r1 = d.sf_rec[3 * j + 1];
+    const int fl = d.sf_rec[3 * j + 2].x;
+    const int a = r0.x, bb = r0.y;
+    const bool trk = (fl & SF_TRACKED) != 0;
+    // the face as its copy's master sees it
+    auto tvd_copy = [&]() {
+        return face_tvd(d, st, b.cx, b.cy, a, bb, (fl >> SF_TYPE2) & 7, r1.y, r1.z, r1.w, (fl & SF_AXIS2) != 0, trk,
+                        &status);
+    };
     double t1 = d.X[bb] - d.X[a], t2 = d.Y[bb] - d.Y[a];
     const double nn = sqrt(sq(t1) + sq(t2));
     t1 /= nn;
@@ -3162,7 +3209,10 @@ __device__ __forceinline__ void surface_face_body(const DevMesh& d, const gelios
     // TVD states of the face (even lanes) and of its twin (odd lanes),
     // exchanged between lane pairs
     auto tvd_pair = [&](St5& pf, St5& pc) {
-        const St5 mine = face_tvd(d, st, b.cx, b.cy, (lane & 1) ? d.fcopy[f] : f, &status);
+        const bool cp = lane & 1;
+        const St5 mine = face_tvd(d, st, b.cx, b.cy, a, bb, (cp ? fl >> SF_TYPE2 : fl) & 7, cp ? r1.y : r0.z,
+                                  cp ? r1.z : r0.w, cp ? r1.w : r1.x, (fl & (cp ? SF_AXIS2 : SF_AXIS1)) != 0, trk,
+                                  &status);
         St5 other;
         other.ro = __shfl_xor_sync(0xffffffffu, mine.ro, 1);
         other.p = __shfl_xor_sync(0xffffffffu, mine.p, 1);
@@ -3177,23 +3227,25 @@ __device__ __forceinline__ void surface_face_body(const DevMesh& d, const gelios
         tvd_pair(p1, p2);
         q1[0] = p1.ro; q1[1] = p1.p; q1[2] = p1.u; q1[3] = p1.v; q1[4] = 0.0;
         q2[0] = p2.ro; q2[1] = p2.p; q2[2] = p2.u; q2[3] = p2.v; q2[4] = 0.0;
-        godunov_dev<true>(ga, P.kurant, q1, q2, nv, qq, ds, 0.0, 0.0, P.godunov_max_iter, &status);
+        godunov_dev<true>(ga, P.kurant, q1, q2, nv, qq, ds, 0.0, 0.0, P.godunov_max_iter, &status, nullptr,
+                          nullptr, true);
         o0 = ds[2] * P.koef * 0.3;
         o3 = 0.0;
     } else if (j < nC + nI) {
-        const int M = d.fmaster[f];
+        const int M = r0.z;
         St5 p1 = load_state(st, M);
         const double x = b.cx[M], y = b.cy[M];
         const double radius = sqrt(sq(x) + sq(y));
         const double x2 = (d.X[a] + d.X[bb]) / 2.0, y2 = (d.Y[a] + d.Y[bb]) / 2.0;
         const double dis = sqrt(sq(x2) + sq(y2));
-        const St5 p2 = face_tvd(d, st, b.cx, b.cy, d.fcopy[f], &status);
+        const St5 p2 = tvd_copy();
         p1.ro = p1.ro * sq(radius) / sq(dis);
         p1.p = p1.p * (b.rp[M] / pow2g(dis, g2));
         polar_perenos(x, y, x2, y2, p1.u, p1.v);
         q1[0] = p1.ro; q1[1] = p1.p; q1[2] = p1.u; q1[3] = p1.v; q1[4] = 0.0;
         q2[0] = p2.ro; q2[1] = p2.p; q2[2] = p2.u; q2[3] = p2.v; q2[4] = 0.0;
-        godunov_dev<true>(ga, P.kurant, q1, q2, nv, qq, ds, 0.0, 0.0, P.godunov_max_iter, &status);
+        godunov_dev<true>(ga, P.kurant, q1, q2, nv, qq, ds, 0.0, 0.0, P.godunov_max_iter, &status, nullptr,
+                          nullptr, true);
         o0 = ds[0] * P.koef * 0.1;
         const double tt1 = -n2, tt2 = n1;
         o3 = (fabs(p2.u * tt1 + p2.v * tt2) < 0.1) ? 1.0 : 0.0;
@@ -3208,7 +3260,8 @@ __device__ __forceinline__ void surface_face_body(const DevMesh& d, const gelios
             tvd_pair(p1, p2);
             q1[0] = p1.ro; q1[1] = p1.p; q1[2] = p1.u; q1[3] = p1.v; q1[4] = 0.0;
             q2[0] = p2.ro; q2[1] = p2.p; q2[2] = p2.u; q2[3] = p2.v; q2[4] = 0.0;
-            godunov_dev<true>(ga, P.kurant, q1, q2, nv, qq, ds, 0.0, 0.0, P.godunov_max_iter, &status);
+            godunov_dev<true>(ga, P.kurant, q1, q2, nv, qq, ds, 0.0, 0.0, P.godunov_max_iter, &status, nullptr,
+                          nullptr, true);
             o0 = ds[1] * P.koef;
             const double tt1 = -n2, tt2 = n1;
             double br;
@@ -4347,7 +4400,7 @@ __device__ __forceinline__ void mhd_update_body(const DevMesh& d, const gelios_p
     }
 }
 
-__global__ void __launch_bounds__(128) mhd_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
+__global__ void __launch_bounds__(128, 6) mhd_update_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                          const double* __restrict__ fl,
                                                          const double* __restrict__ src,
                                                          const double* __restrict__ hcur, double* __restrict__ hnxt) {
@@ -4422,7 +4475,7 @@ __global__ void __launch_bounds__(128, PLAIN ? GELIOS_BATCH_PLAIN_MINB : GELIOS_
     block_reduce_commit(tmin, 0, 0, status, b.dt_acc, b.counters, b.status);
 }
 
-__global__ void __launch_bounds__(128) batch_mhd_update_kernel(BatchTables t, int parity) {
+__global__ void __launch_bounds__(128, 6) batch_mhd_update_kernel(BatchTables t, int parity) {
     const int2 e = t.cells[blockIdx.x];
     BATCH_INSTANCE(I, e)
     const int c = e.y + threadIdx.x;
@@ -4983,6 +5036,10 @@ void launch_mk2_update(const DevMesh& d, const gelios_params& P, const StepBuffe
         mk2_update_kernel<kUpdAllNoMark><<<nb, 128, 0, s>>>(d, P, b, fl, aux, list, n_list);
     else
         mk2_update_kernel<kUpdAll><<<nb, 128, 0, s>>>(d, P, b, fl, aux, list, n_list);
+}
+void launch_rail_table(const DevMesh& d, int n_inner, double* rcs, double* rsn, double* rfrac, cudaStream_t s) {
+    const int nr = d.n_rail_a + d.n_rail_b + d.n_rail_c + d.n_rail_d;
+    if (nr > 0) rail_table_kernel<<<nr, 128, 0, s>>>(d, n_inner, rcs, rsn, rfrac);
 }
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
                   bool copy_outer_shock) {

@@ -67,6 +67,15 @@ struct DevMesh {
     const int32_t *sp_point = nullptr, *sp_line = nullptr, *sp_inc = nullptr, *sp_ainc = nullptr,
                   *sp_fix = nullptr;
     const int32_t* sp_of_point = nullptr;  // tracked-surface node of each point, -1 if none
+    // what the motion kernels read of the topology, one level of loads deep:
+    // per rail its key points 0-2 (a D rail: key 0 of C_Rails[0] first) and
+    // their surface nodes (-1: none); per tracked face (concatenated lines)
+    // three int4: {A, B, master, Sosed}, {Sosed_down, the copy's master,
+    // Sosed, Sosed_down}, {SF_* flags}
+    const int4 *rk_point = nullptr, *rk_node = nullptr, *sf_rec = nullptr;
+    // per rail cos s, sin s; per rail point the fraction its fixed power law
+    // gives (launch_rail_table): constants of the topology and of n_inner
+    const double *rcs = nullptr, *rsn = nullptr, *rfrac = nullptr;
     const double *Hn = nullptr, *Hu = nullptr, *Hv = nullptr, *HT = nullptr, *ku = nullptr, *kv = nullptr,
                  *kT = nullptr, *r_istoch = nullptr;
     const int32_t *cback = nullptr, *cnext = nullptr;
@@ -230,6 +239,11 @@ void launch_dt_finalize_cap(const StepBuffers& b, cudaStream_t s);
 // 3 every cell (modes 1-3 fold nothing into the CFL accumulator)
 void launch_mk2_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
                        const double* aux, cudaStream_t s, int mode, const int32_t* list, int n_list);
+// flags of a tracked face record: types of the face and of its copy, whether
+// their masters have an Axis face, both end points on one tracked surface
+enum : int { SF_TYPE2 = 3, SF_AXIS1 = 1 << 6, SF_AXIS2 = 1 << 7, SF_TRACKED = 1 << 8 };
+// rcs, rsn (n_rails each) and rfrac (one per rail point) of d
+void launch_rail_table(const DevMesh& d, int n_inner, double* rcs, double* rsn, double* rfrac, cudaStream_t s);
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
                   bool copy_outer_shock = true);
 // Go_5_komponent: face units, then the cell update.  Hydrogen state rows
@@ -247,9 +261,12 @@ void launch_k5_update(const DevMesh& d, const gelios_params& P, const StepBuffer
 // ro, p, u, v), 13 flux rows per slot, fixed sources (3 x n_cells).
 constexpr int kMhdFluxRows = 13;
 // The face kernel has kMhdFaceVariants launch shapes (threads per block x
-// minimum blocks per SM); variant 0 is the default, gelios_autotune picks
+// minimum blocks per SM); kMhdFaceDefault is the default, gelios_autotune picks
 // the fastest for a grid.  All shapes give the same bits.
 constexpr int kMhdFaceVariants = 6;
+// 128 threads x 4 blocks: 20 steps of 200k cells (FP64) 3702 us against 3728
+// for 128 x 3, of 938k cells (FP32 fluxes) 11616 against 12418
+constexpr int kMhdFaceDefault = 2;
 const char* mhd_face_variant_name(int v);
 // Returns the number of launches (the plain interior group, then the rest).
 // s_rest: stream of the groups other than the plain interior one (null: s)
