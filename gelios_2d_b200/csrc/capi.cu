@@ -159,7 +159,7 @@ struct gelios_ctx {
         cudaGraphExec_t exec = nullptr;
         int launches = 0;
     };
-    StepGraph graphs[16];
+    StepGraph graphs[48];
     bool graphs_off = false;  // capture failed once: launch directly
     bool coop_off = false;    // the cooperative plain step could not launch once: three kernels per step
     void drop_graphs() {
@@ -1465,10 +1465,21 @@ int enqueue_pipe_step(gelios_ctx* ctx, int st, const StepBuffers& b, const StepB
     // units on the main stream.  The next step's tracked reconstructions
     // (side stream) overwrite the rows the tracked fluxes read: they wait
     // for the early update, which waits for the motion stream.
+    // On a small grid (kMk2SmallCells) every one of these kernels is a few
+    // blocks bound by latency: the source terms and the one-sided group then
+    // run on the side and extra streams, beside instead of behind the others.
+    const bool small = d.n_cells <= kMk2SmallCells;
     GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
     GELIOS_CUDA_TRY(cudaStreamWaitEvent(sm, ctx->ev_fork, 0));
     n += launch_mk2_flux_tracked(d, P, b, ctx->rec.as<double>(), ctx->pstar.as<double>(), fl, sm);
-    launch_mk2_source(d, P, b, aux, sm);
+    if (small) {
+        GELIOS_CUDA_TRY(cudaStreamWaitEvent(sd, ctx->ev_fork, 0));
+        launch_mk2_source(d, P, b, aux, sd);
+        GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_side2, sd));
+        GELIOS_CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_side2, 0));
+    } else {
+        launch_mk2_source(d, P, b, aux, sm);
+    }
     GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_motion, sm));
     n++;
     GELIOS_CUDA_TRY(cudaStreamWaitEvent(ctx->groups, ctx->ev_fork, 0));
@@ -1490,11 +1501,9 @@ int enqueue_pipe_step(gelios_ctx* ctx, int st, const StepBuffers& b, const StepB
     launch_mk2_update(d, P, b, fl, aux, s, 1, early, ctx->n_early);
     n += ctx->n_early > 0 ? 1 : 0;
     GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_early, s));
-    // step st + 1: dt, then surface tracking + rails
+    // step st + 1: surface tracking (which finalises its dt) + rails
     GELIOS_CUDA_TRY(cudaStreamWaitEvent(sm, ctx->ev_early, 0));
-    launch_dt_finalize_cap(b, sm);
-    n++;
-    n += launch_motion(dn, P, *bn, ctx->surface.as<double>(), sm);
+    n += launch_motion(dn, P, *bn, ctx->surface.as<double>(), sm, true, &b);
     GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_motion, sm));
     // step st + 1: tracked-face reconstructions and star pressures
     GELIOS_CUDA_TRY(cudaStreamWaitEvent(sd, ctx->ev_early, 0));

@@ -49,11 +49,6 @@ namespace cg = cooperative_groups;
 #ifndef GELIOS_SOURCE_MINB
 #define GELIOS_SOURCE_MINB 10
 #endif
-// Source kernel arrangement: 32 cells per warp in a cell phase and a
-// species phase (1), or four lanes per cell throughout (0).
-#ifndef GELIOS_SOURCE_WARP
-#define GELIOS_SOURCE_WARP 1
-#endif
 
 namespace gelios {
 
@@ -197,6 +192,28 @@ __device__ __forceinline__ void quad_geometry(const double (&X)[4], const double
     const double cc = a1 * b1 + a2 * b2;
     const double sn = sqrt(1 - sq(cc));
     vs = 0.5 * a * bb * sn;
+}
+
+// The same for the moving-grid update: the area as half the cross product of
+// the diagonals (the reference's |d1| |d2| sin(angle) / 2 without its three
+// square roots and four quotients; it rounds less, its sine loses digits
+// where the diagonals are nearly parallel) and one reciprocal.
+__device__ __forceinline__ void quad_geometry_lean(const double (&X)[4], const double (&Y)[4], double& ox, double& oy,
+                                                   double& vs, double& vol) {
+    double A = 0.0, Gx = 0.0, Gy = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const double xa = X[i], ya = Y[i], xb = X[(i + 1) & 3], yb = Y[(i + 1) & 3];
+        const double cr = xa * yb - ya * xb;
+        A = A + cr;
+        Gx = Gx + (xa + xb) * cr;
+        Gy = Gy + (ya + yb) * cr;
+    }
+    const double r = 1.0 / (3.0 * A);  // 1 / (6 area)
+    ox = Gx * r;
+    oy = Gy * r;
+    vol = fabs(0.5 * A) * r * Gy * kPi * 360.0 / 180.0 / (2.0 * kPi);
+    vs = 0.5 * fabs((X[0] - X[2]) * (Y[1] - Y[3]) - (Y[0] - Y[2]) * (X[1] - X[3]));
 }
 
 // Inner_sphere BC state (Gran.cpp:234-265, 520-534) at face centre (x, y).
@@ -550,6 +567,22 @@ __device__ __forceinline__ void source_rates(const gelios_params& P, SrcMoments 
     nuu = nu * (m.uH - u);
     nuv = nu * (m.vH - v);
     nue = nu * ((sq(m.uH) + sq(m.vH) - kin) / 2.0 + (UH / UM) * (th - pro));
+}
+
+// Get_Sourse_MK1 rates of one species from the temperature-like th = 2 pH / roH
+// (Cell.cpp:590-660): one reciprocal square root serves |U_M|, U_H / U_M, and
+// log U_M = log(U_M^2) / 2 waits for neither.
+__device__ __forceinline__ void source_rates_th(const gelios_params& P, double uH, double vH, double roH, double th,
+                                                double u, double v, double ro, double pro, double kin, double& nuu,
+                                                double& nuv, double& nue) {
+    const double du2 = sq(u - uH) + sq(v - vH), a = pro + th;
+    const double UM2 = du2 + (64.0 / (9.0 * kPi)) * a, UH2 = du2 + (4.0 / kPi) * a;
+    const double r = rsqrt(UM2);
+    const double sig = sq(1.0 - P.a_2 * (0.5 * log(UM2)));
+    const double nu = ro * roH * (UM2 * r) * sig;
+    nuu = nu * (uH - u);
+    nuv = nu * (vH - v);
+    nue = nu * ((sq(uH) + sq(vH) - kin) / 2.0 + (sqrt(UH2) * r) * (th - pro));
 }
 
 // Cell::Get_Sourse_MK1 (Cell.cpp:498-665), one thread per cell.
@@ -1728,7 +1761,9 @@ __device__ __forceinline__ void mk2_flux_unit(const DevMesh& d, const gelios_par
     const double W = ((x4 - r.x2) * r.n1 + (y4 - r.y2) * r.n2) / dt;
     const bool np = (d.u_info[u] & SI_NP) != 0;
     FluxOut<double> F;
-    const double UU = hllc_flux<TF>(P.gamma, P.kurant, r.a, r.o, W, r.n1, r.n2, 1.0, 0, np, F);
+    double UU;
+    if constexpr (sizeof(TF) == 8) UU = hll_lean(P.gamma, r.a, r.o, W, r.n1, r.n2, F);
+    else UU = hllc_flux<TF>(P.gamma, P.kurant, r.a, r.o, W, r.n1, r.n2, 1.0, 0, np, F);
     const double S = r.S;
     double fm0 = F.P0 * S, fm1 = F.P1 * S, fm2 = F.P2 * S, fm3 = F.P3 * S;
     double UG = 1.0;
@@ -1749,15 +1784,13 @@ __device__ __forceinline__ void mk2_flux_unit(const DevMesh& d, const gelios_par
     fl[2 * nu + u] = fm2;
     fl[3 * nu + u] = fm3;
     fl[4 * nu + u] = fq;
-    if (procK) {
-        // reference order: Godunov candidate first, then HLL (Setka.cpp:10359, 10366)
-        if (TRACKED) tmin_u = dmin_ref(tmin_u, P.kurant * r.dist / UG);
-        tmin_u = dmin_ref(tmin_u, P.kurant * r.dist / UU);
-    }
-    if (procN) {
-        if (TRACKED) tmin_u = dmin_ref(tmin_u, P.kurant * r.distn / UG);
-        tmin_u = dmin_ref(tmin_u, P.kurant * r.distn / UU);
-    }
+    // the CFL candidates kurant * distance / speed of the updated sides and of
+    // both solvers (Setka.cpp:10359, 10366): the least is that of the smaller
+    // distance and the larger speed (a NaN speed gives none)
+    const double dm = procK ? (procN ? dmin_ref(r.dist, r.distn) : r.dist) : r.distn;
+    const double us = TRACKED && UG > UU ? UG : UU;
+    tmin_u = dmin_ref(tmin_u, P.kurant * dm / us);
+    if (TRACKED && !(us == us)) tmin_u = dmin_ref(tmin_u, P.kurant * dm / UG);
 }
 
 // Rows of the tracked units' reconstruction (kRecRows rows of n_tracked
@@ -1853,6 +1886,34 @@ __global__ void __launch_bounds__(128, MINB) mk2_face_kernel(DevMesh d, gelios_p
     block_reduce_commit(tmin_u, 0, 0, status, b.dt_acc, b.counters, b.status);
 }
 
+// The C_1 interior and the one-sided units in one launch (each block one
+// kind), so that a small grid has one kernel less in its chain; 38 us on the
+// 938k grid (41 + 12 in two launches with the flux of hllc_flux; ncu).
+template <typename TF, int MINB, bool PF>
+__global__ void __launch_bounds__(128, MINB) mk2_face_rest_kernel(DevMesh d, gelios_params P, StepBuffers b,
+                                                                  double* __restrict__ fl, int n_one_blocks) {
+    double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
+    int status = 0;
+    RecUnit r;
+    r.a = St5{};
+    r.o = St5{};
+    if (static_cast<int>(blockIdx.x) < n_one_blocks) {
+        const int u = d.u_tr1 + blockIdx.x * blockDim.x + threadIdx.x;
+        if (u < d.n_units) {
+            mk2_recon_unit<kAnyGroup>(d, P, b, u, r, &status);
+            mk2_flux_unit<TF, false>(d, P, b, u, r, fl, nullptr, tmin_u, &status);
+        }
+    } else {
+        const int u = d.u_c1 + (blockIdx.x - n_one_blocks) * blockDim.x + threadIdx.x;
+        if (u < d.u_tr0) {
+            if (PF) mk2_prefetch_unit<true>(d, b, u);
+            mk2_recon_unit<kC1Group>(d, P, b, u, r, &status);
+            mk2_flux_unit<TF, false>(d, P, b, u, r, fl, nullptr, tmin_u, &status);
+        }
+    }
+    block_reduce_commit(tmin_u, 0, 0, status, b.dt_acc, b.counters, b.status);
+}
+
 // Star pressure of the exact Godunov problem of every tracked-face unit
 // (Solvers.cpp:1174-1305).  It depends on the reconstructed states and on
 // the face normal before the motion, not on the face speed, so it runs on a
@@ -1884,7 +1945,6 @@ __global__ void __launch_bounds__(64) mk2_tracked_solve_kernel(DevMesh d, gelios
 // the motion: the charge-exchange source Get_Sourse_MK1 (Cell.cpp:498-665).
 // Runs on a side stream while surface tracking and the rails move the grid.
 // aux rows: q1, q2, q3
-#if GELIOS_SOURCE_WARP
 // 32 cells per warp in two phases, every lane busy in both.  Cell phase: one
 // lane per cell decides whether the cell takes part, finds the bracket of
 // the radial interpolation, loads the cell's state and interpolates the
@@ -1956,24 +2016,27 @@ __global__ void __launch_bounds__(128, GELIOS_SOURCE_MINB) mk2_source_kernel(Dev
         const int flags = c < d.n_cells ? si[2][t] : 0;
         double nuu = 0.0, nuv = 0.0, nue = 0.0;
         if ((flags & 3) == 3) {
-            SrcMoments m;
+            double uH, vH, roH, TH;
             if (flags & 4) {
                 const int K_do = si[0][t], K_posle = si[1][t];
                 const double ir = sd[5][t], dr = sd[6][t];
                 auto lin = [&](double t1, double t2) { return (t1 - t2) * ir * dr + t2; };
-                m.uH = lin(d.Hu[4 * K_do + sp], d.Hu[4 * K_posle + sp]);
-                m.vH = lin(d.Hv[4 * K_do + sp], d.Hv[4 * K_posle + sp]);
-                m.roH = lin(d.Hn[4 * K_do + sp], d.Hn[4 * K_posle + sp]);
-                const double TH = lin(d.HT[4 * K_do + sp], d.HT[4 * K_posle + sp]);
-                m.pH = 0.5 * TH * m.roH;
+                uH = lin(d.Hu[4 * K_do + sp], d.Hu[4 * K_posle + sp]);
+                vH = lin(d.Hv[4 * K_do + sp], d.Hv[4 * K_posle + sp]);
+                roH = lin(d.Hn[4 * K_do + sp], d.Hn[4 * K_posle + sp]);
+                TH = lin(d.HT[4 * K_do + sp], d.HT[4 * K_posle + sp]);
             } else {
-                m.uH = d.Hu[4 * c + sp];
-                m.vH = d.Hv[4 * c + sp];
-                m.roH = d.Hn[4 * c + sp];
-                m.pH = 0.5 * d.HT[4 * c + sp] * d.Hn[4 * c + sp];
+                uH = d.Hu[4 * c + sp];
+                vH = d.Hv[4 * c + sp];
+                roH = d.Hn[4 * c + sp];
+                TH = d.HT[4 * c + sp];
             }
-            m.ku = m.kv = m.kT = 0.0;
-            source_rates(P, m, sd[0][t], sd[1][t], sd[2][t], sd[3][t], sd[4][t], nuu, nuv, nue);
+            // th = 2 pH / roH with pH = TH roH / 2, or pH = 0 where there is no hydrogen (Cell.cpp:590-594)
+            if (roH <= 0.0) {
+                roH = 0.0000001;
+                TH = 0.0;
+            }
+            source_rates_th(P, uH, vH, roH, TH, sd[0][t], sd[1][t], sd[2][t], sd[3][t], sd[4][t], nuu, nuv, nue);
         }
         double su[3], sv[3], se[3];
 #pragma unroll
@@ -2000,67 +2063,6 @@ __global__ void __launch_bounds__(128, GELIOS_SOURCE_MINB) mk2_source_kernel(Dev
     }
     if (status) atomicOr(b.status, status);
 }
-#else
-__global__ void __launch_bounds__(128, GELIOS_SOURCE_MINB) mk2_source_kernel(DevMesh d, gelios_params P, StepBuffers b,
-                                                         double* __restrict__ aux) {
-    // four lanes per cell, one hydrogen species per lane; the cell's first
-    // lane finds the bracket of the radial interpolation and hands it to the
-    // others; the four rates are summed on it in the reference's order
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = t >> 2, sp = t & 3;
-    const unsigned full = 0xffffffffu;
-    const int q0 = (threadIdx.x & 31) & ~3;
-    int status = 0;
-    bool proc = false, interp = false;
-    double x = 0.0, y = 0.0, rr = 0.0;
-    if (c < d.n_cells) {
-        x = b.cx[c];
-        y = b.cy[c];
-        rr = sqrt(sq(x) + sq(y));
-        proc = !(rr < P.R11);
-        interp = proc && rr > P.src_rmin && rr < P.src_rmax && x >= 0.0;
-    }
-    int K_do = -1, K_posle = -1, ok = 1;
-    if (interp && sp == 0) {
-        int2 cached;
-        ok = source_bracket(d, c, rr, K_do, K_posle, &status, &cached) ? 1 : 0;
-        if (ok && d.src_lo_out && cached.x != K_do) d.src_lo_out[c] = make_int2(K_do, K_posle);
-    }
-    K_do = __shfl_sync(full, K_do, q0);
-    K_posle = __shfl_sync(full, K_posle, q0);
-    ok = __shfl_sync(full, ok, q0);
-    double nuu = 0.0, nuv = 0.0, nue = 0.0;
-    SrcMoments m{};
-    if (proc && ok) {
-        const St5 par1 = load_state(b.cur, c);
-        m = source_moments(d, c, sp, interp, K_do, K_posle, rr, sp == 0);
-        source_rates(P, m, par1.u, par1.v, par1.ro, par1.p / par1.ro, sq(par1.u) + sq(par1.v), nuu, nuv, nue);
-    }
-    double su[3], sv[3], se[3];
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-        su[j] = __shfl_sync(full, nuu, q0 + 1 + j);
-        sv[j] = __shfl_sync(full, nuv, q0 + 1 + j);
-        se[j] = __shfl_sync(full, nue, q0 + 1 + j);
-    }
-    if (proc && sp == 0) {
-        const size_t n = d.n_cells;
-        double q1 = 0.0, q2 = 0.0, q3 = 0.0;
-        if (ok) {
-            const double Mu = P.src_coef * (nuu + su[0] + su[1] + su[2]);
-            const double Mv = P.src_coef * (nuv + sv[0] + sv[1] + sv[2]);
-            const double MT = P.src_coef * (nue + se[0] + se[1] + se[2]);
-            q1 = Mu * m.ku;
-            q2 = Mv * m.kv;
-            q3 = MT * m.kT;
-        }
-        aux[0 * n + c] = q1;
-        aux[1 * n + c] = q2;
-        aux[2 * n + c] = q3;
-    }
-    if (status) atomicOr(b.status, status);
-}
-#endif
 
 // Go_5_komponent__MK2 cell update (Setka.cpp:10386-10468) of cell c from its
 // nf face slots' fluxes (fetch4 / fetch(k, j): row k of the cell's j-th slot,
@@ -2086,7 +2088,7 @@ __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_p
         // centroid / area / volume_rotate)
         const double qx[4] = {d.X2[qc.x], d.X2[qc.y], d.X2[qc.z], d.X2[qc.w]};
         const double qy[4] = {d.Y2[qc.x], d.Y2[qc.y], d.Y2[qc.z], d.Y2[qc.w]};
-        quad_geometry(qx, qy, xn, yn, vs2, Volume2);
+        quad_geometry_lean(qx, qy, xn, yn, vs2, Volume2);
         if (!(cfl & CF_CENTR)) {
             b.vs_next[c] = vs2;
             b.vol_next[c] = Volume2;
@@ -2096,7 +2098,7 @@ __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_p
         const int p0 = con[0], p1 = con[1], p2 = con[2], p3 = con[3];
         const double qx[4] = {d.X2[p0], d.X2[p1], d.X2[p2], d.X2[p3]};
         const double qy[4] = {d.Y2[p0], d.Y2[p1], d.Y2[p2], d.Y2[p3]};
-        quad_geometry(qx, qy, xn, yn, vs2, Volume2);
+        quad_geometry_lean(qx, qy, xn, yn, vs2, Volume2);
         if (!(cfl & CF_CENTR)) {
             b.vs_next[c] = vs2;
             b.vol_next[c] = Volume2;
@@ -2115,7 +2117,7 @@ __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_p
     b.cx_next[c] = xn;
     b.cy_next[c] = yn;
     if (cfl & CF_RP) b.rp_next[c] = pow2g(sqrt(sq(xn) + sq(yn)), 2 * P.gamma);
-    if (sqrt(sq(x) + sq(y)) < P.R11) return;
+    if (sq(x) + sq(y) < d.r11_sq) return;
     tmark = dmin_ref(tmark, 10000000.0);  // `time` starts at 1e7 in every step (Setka.cpp:10141)
     const double dt = *b.dt_cur;
     double Pt0 = 0.0, Pt1 = 0.0, Pt2 = 0.0, Pt3 = 0.0, Pt4 = 0.0;
@@ -2146,7 +2148,7 @@ __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_p
         const double vs1 = b.vs[c];
         const double Volume = b.vol[c];
         const double ro = par1.ro, u = par1.u, v = par1.v, p = par1.p, Q = par1.Q;
-        const double gm1 = P.gamma - 1;
+        const double gm1 = P.gamma - 1, rg1 = 1.0 / gm1;
         const double rV2 = 1.0 / Volume2, VV = Volume * rV2;
         double ro3 = ro * VV - dt * (Pt0 * rV2);
         const double Q33 = Q * VV - (dt * rV2) * Pt4;
@@ -2158,7 +2160,7 @@ __device__ __forceinline__ void mk2_update_cell(const DevMesh& d, const gelios_p
         const double u3 = (ro * u * VV - dt * (Pt1 * rV2 - q2_1)) * rro3;
         const double v3 = (ro * v * VV - dt * ((Pt2 - p * 0.5 * (vs1 + vs2)) * rV2 - q2_2)) * rro3;
         double p3 =
-            (((p / gm1 + ro * (u * u + v * v) * 0.5) * VV - dt * (Pt3 * rV2 - q3)) - 0.5 * ro3 * (u3 * u3 + v3 * v3)) *
+            (((p * rg1 + ro * (u * u + v * v) * 0.5) * VV - dt * (Pt3 * rV2 - q3)) - 0.5 * ro3 * (u3 * u3 + v3 * v3)) *
             gm1;
         if (p3 <= 0) {
             p3 = P.p_floor;
@@ -2224,7 +2226,9 @@ __global__ void __launch_bounds__(NT, MINB) mk2_tile_kernel(DevMesh d, gelios_pa
         const double W = ((x4 - r.x2) * r.n1 + (y4 - r.y2) * r.n2) / dt;
         const bool np = (d.u_info[u] & SI_NP) != 0;
         FluxOut<double> F;
-        const double UU = hllc_flux<TF>(P.gamma, P.kurant, r.a, r.o, W, r.n1, r.n2, 1.0, 0, np, F);
+        double UU;
+        if constexpr (sizeof(TF) == 8) UU = hll_lean(P.gamma, r.a, r.o, W, r.n1, r.n2, F);
+        else UU = hllc_flux<TF>(P.gamma, P.kurant, r.a, r.o, W, r.n1, r.n2, 1.0, 0, np, F);
         const double S = r.S;
         const double fm[5] = {F.P0 * S, F.P1 * S, F.P2 * S, F.P3 * S, F.PQ * S};
         if (own != kTileNone) {
@@ -2421,22 +2425,6 @@ __global__ void __launch_bounds__(128) inner_cell_kernel(DevMesh d, gelios_param
 //   25 k_u, k_v, k_T            of the cell, on its lanes 0, 1, 2
 //   26 1 / Volume, 27 (vs1 + vs2) / 2   on lane 0
 enum : int { IL_TYPE = 7, IL_TVD = 8, IL_RAW_O = 16, IL_RAW_N = 32, IL_SRC = 64, IL_ACT = 128 };
-
-// Get_Sourse_MK1 rates of one species from the temperature-like th = 2 pH / roH
-// (Cell.cpp:590-660): one reciprocal square root serves |U_M|, U_H / U_M, and
-// log U_M = log(U_M^2) / 2 waits for neither.
-__device__ __forceinline__ void source_rates_th(const gelios_params& P, double uH, double vH, double roH, double th,
-                                                double u, double v, double ro, double pro, double kin, double& nuu,
-                                                double& nuv, double& nue) {
-    const double du2 = sq(u - uH) + sq(v - vH), a = pro + th;
-    const double UM2 = du2 + (64.0 / (9.0 * kPi)) * a, UH2 = du2 + (4.0 / kPi) * a;
-    const double r = rsqrt(UM2);
-    const double sig = sq(1.0 - P.a_2 * (0.5 * log(UM2)));
-    const double nu = ro * roH * (UM2 * r) * sig;
-    nuu = nu * (uH - u);
-    nuv = nu * (vH - v);
-    nue = nu * ((sq(uH) + sq(vH) - kin) / 2.0 + (sqrt(UH2) * r) * (th - pro));
-}
 
 __global__ void __launch_bounds__(128) inner_table_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                           const int32_t* __restrict__ list, int n_list,
@@ -3283,8 +3271,12 @@ __device__ __forceinline__ void surface_face_body(const DevMesh& d, const gelios
     }
 }
 
+// fin: finalise the step's dt first (fb: the buffers of the step before), for
+// a call whose steps follow one another without a commit; nothing here reads
+// it, the rails do.
 __global__ void __launch_bounds__(64) surface_faces_kernel(DevMesh d, gelios_params P, StepBuffers b,
-                                                           double* __restrict__ scratch) {
+                                                           double* __restrict__ scratch, StepBuffers fb, bool fin) {
+    if (fin && blockIdx.x == 0 && threadIdx.x == 0) dt_finalize_cap(fb);
     const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (j >= d.n_lc + d.n_li + d.n_lo) return;
     surface_face_body(d, P, b, scratch, j, threadIdx.x & 31);
@@ -4899,9 +4891,8 @@ static void launch_faces_pf(const DevMesh& d, const gelios_params& P, const Step
 template <typename TF, bool PF>
 static void launch_faces_rest(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* fl,
                               cudaStream_t s) {
-    const int n1 = d.u_tr0 - d.u_c1, n3 = d.n_units - d.u_tr1;
-    if (n1 > 0) mk2_face_kernel<TF, 6, kC1Group, PF><<<blocks_for(n1, 128), 128, 0, s>>>(d, P, b, fl, n1);
-    if (n3 > 0) mk2_face_kernel<TF, 4, kAnyGroup, PF><<<blocks_for(n3, 128), 128, 0, s>>>(d, P, b, fl, n3);
+    const int n1 = blocks_for(d.n_units - d.u_tr1, 128), nc = blocks_for(d.u_tr0 - d.u_c1, 128);
+    if (n1 + nc > 0) mk2_face_rest_kernel<TF, 6, PF><<<n1 + nc, 128, 0, s>>>(d, P, b, fl, n1);
 }
 template <typename TF>
 static cudaError_t launch_cells_p(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const TileView& t,
@@ -4951,7 +4942,7 @@ int mk2_variant_launches(const DevMesh& d, int v, int part) {
     if (part == 2) return 1;
     if (tiles) return 0;
     if (part == 1) return d.u_c1 > 0 ? 1 : 0;
-    return (d.u_tr0 > d.u_c1 ? 1 : 0) + (d.n_units > d.u_tr1 ? 1 : 0);
+    return d.u_tr0 > d.u_c1 || d.n_units > d.u_tr1 ? 1 : 0;
 }
 cudaError_t launch_mk2_cells(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const TileView& t,
                              double* fl, const double* aux, cudaStream_t s, int variant, int part) {
@@ -4976,11 +4967,7 @@ int launch_mk2_flux_tracked(const DevMesh& d, const gelios_params& P, const Step
     return 1;
 }
 void launch_mk2_source(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* aux, cudaStream_t s) {
-#if GELIOS_SOURCE_WARP
-    mk2_source_kernel<<<blocks_for(d.n_cells, 128), 128, 0, s>>>(d, P, b, aux);
-#else
-    mk2_source_kernel<<<blocks_for(4 * d.n_cells, 128), 128, 0, s>>>(d, P, b, aux);
-#endif
+    if (d.n_cells > 0) mk2_source_kernel<<<blocks_for(d.n_cells, 128), 128, 0, s>>>(d, P, b, aux);
 }
 void launch_inner(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const int32_t* list, int n,
                   cudaStream_t s) {
@@ -5042,11 +5029,12 @@ void launch_rail_table(const DevMesh& d, int n_inner, double* rcs, double* rsn, 
     if (nr > 0) rail_table_kernel<<<nr, 128, 0, s>>>(d, n_inner, rcs, rsn, rfrac);
 }
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
-                  bool copy_outer_shock) {
+                  bool copy_outer_shock, const StepBuffers* fin) {
     int launches = 0;
     const int nf = d.n_lc + d.n_li + d.n_lo;
-    if (nf > 0) {
-        surface_faces_kernel<<<blocks_for(nf, 2), 64, 0, s>>>(d, P, b, scratch);
+    if (nf > 0 || fin) {
+        surface_faces_kernel<<<blocks_for(nf > 0 ? nf : 1, 2), 64, 0, s>>>(d, P, b, scratch, fin ? *fin : b,
+                                                                            fin != nullptr);
         launches += 1;
     }
     const int nr = d.n_rail_a + d.n_rail_b + d.n_rail_c + d.n_rail_d;

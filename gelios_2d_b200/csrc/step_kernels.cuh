@@ -213,6 +213,11 @@ int launch_mk2_tracked_solve(const DevMesh& d, const gelios_params& P, const Ste
                              double* pstar, cudaStream_t s);
 int launch_mk2_flux_tracked(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* rec,
                             const double* pstar, double* fl, cudaStream_t s);
+// Grids of at most this many cells run the source terms of a pipelined step on
+// a stream of their own.  us per 10-step call behind the tracked fluxes /
+// beside them: 8k cells 664 / 620, 50k 766 / 714, 392k 1916 / 1862; 938k, 20
+// steps: 6901 / 6956 (there the priority of the motion stream counts more).
+constexpr int kMk2SmallCells = 524288;
 // Charge-exchange source terms of the moving-grid step (aux rows q1, q2, q3),
 // 128 cells per block (a cell phase, then a species phase).
 void launch_mk2_source(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* aux, cudaStream_t s);
@@ -245,7 +250,7 @@ enum : int { SF_TYPE2 = 3, SF_AXIS1 = 1 << 6, SF_AXIS2 = 1 << 7, SF_TRACKED = 1 
 // rcs, rsn (n_rails each) and rfrac (one per rail point) of d
 void launch_rail_table(const DevMesh& d, int n_inner, double* rcs, double* rsn, double* rfrac, cudaStream_t s);
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
-                  bool copy_outer_shock = true);
+                  bool copy_outer_shock = true, const StepBuffers* fin = nullptr);
 // Go_5_komponent: face units, then the cell update.  Hydrogen state rows
 // (ro, p, u, v of H1..H4), 16 rows of n_cells each, of the current and the
 // next buffer; fl: kK5FluxRows flux rows of n_units, F.S once per face unit
