@@ -18,6 +18,18 @@
 //                         staged in shared memory and stored by the TMA;
 //                         used whenever both operands' rows are 16-byte
 //                         aligned
+//                         In a training step the same epilogue also stores
+//                         H^T, and the backward data GEMMs (EPI 2) apply
+//                         GELU' to the accumulator and store dZ, dZ^T and the
+//                         tile's column sums: no fp32 dH or dZ in memory, no
+//                         transpose, activation or column-sum launch
+//   grad_adam_kernel      a training step's end: every gradient from its
+//                         split partial sums in a fixed order, Adam, and the
+//                         bf16 copies of the weights (W and W^T)
+//   mse_grad_kernel       dY = 2 (Y - T) / (M N) as the last layer's dZ, dZ^T
+//                         and column sums, squared error per row
+// The kernels below serve networks the fused training step does not take
+// (see train_fused):
 //   transpose_bf16_kernel the transposed operands of the backward GEMMs
 //   features_kernel       network inputs: the raw inputs, then sin / cos of
 //                         2^f pi s of the last two (the cell position), bf16
@@ -35,6 +47,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -302,7 +315,7 @@ __device__ __forceinline__ float gelu_grad(float x) {
 // mbarrier before refilling it.  Out-of-range rows and k are zero-filled by
 // the TMA unit.  EPI 0: C (fp32) as gemm_tc_kernel writes it;
 // EPI 1: z = C + bias per column, then Z = z, H = bf16(act(z)), Hf = act(z)
-// (each output optional, rows of N).
+// (each output optional, rows of N); EPI 2: see GemmEpilogue.
 // tile: TM_BN = 64 columns per CTA (256 CTAs for a 8192 x 256 layer, two
 // resident per SM: one's epilogue overlaps the other's loads); k-chunk
 // stride of the A stage 128 rows x 16 bytes, of the B stage 64 x 16 bytes
@@ -348,7 +361,17 @@ struct GemmEpilogue {
     __nv_bfloat16* H = nullptr;
     float* Hf = nullptr;
     int act = 0;
+    // training: the transpose of H (EPI 1, with tstore) or of dZ (EPI 2), N
+    // rows of ldt (a multiple of 8, >= M; 16-byte aligned)
+    __nv_bfloat16* HT = nullptr;
+    int64_t ldt = 0;
+    // EPI 2: dZ = acc * GELU'(Zin) -> H (rows of N, N % 8 == 0), HT, and the
+    // column sums of every 128-row tile, row by row, -> colpart[tile][N]
+    const float* Zin = nullptr;
+    float* colpart = nullptr;
 };
+// transposed tile in shared memory: 64 columns of 128 rows, pitch 136
+constexpr int TM_TPITCH = 136;
 
 // 16 warps: warp w reads TMEM lanes 32 (w % 4) .. (its rows) and the
 // columns 16 (w / 4) .. +16 of the tile.
@@ -363,6 +386,9 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     __shared__ uint64_t full[TC_STAGES], empty[TC_STAGES];
     __shared__ uint32_t tmem_slot;
+    static_assert(3 * (TC_BM * 128) + TM_BN * TM_TPITCH * 2 <= TC_STAGES * (TC_TILE + TM_TILE_B) &&
+                      TC_BM * (TM_BN + 1) * 4 <= 3 * (TC_BM * 128),
+                  "the epilogue's tiles fit into the stage buffers");
     // 1024-byte aligned stage buffers (the swizzle pattern repeats every
     // 1024 bytes and the descriptors assume it starts at the buffer)
     uint8_t* base = tc_smem + ((1024u - (smem_u32(tc_smem) & 1023u)) & 1023u);
@@ -499,6 +525,44 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
             }
             // the generic-proxy writes, visible to the bulk copies
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            if (ep.HT) {
+                __nv_bfloat16* tt = reinterpret_cast<__nv_bfloat16*>(base + 3 * (TC_BM * 128));
+#pragma unroll
+                for (int j = 0; j < 16; j++) tt[(c0 + j) * TM_TPITCH + r] = __float2bfloat16(h[j]);
+            }
+        } else if (EPI == 2) {
+            const int r = wl * 32 + lane;
+            float* sd = reinterpret_cast<float*>(base);
+            __nv_bfloat16* tt = reinterpret_cast<__nv_bfloat16*>(base + 3 * (TC_BM * 128));
+            float z[16];
+            const float* zp = ep.Zin + row * N + col0;
+            if (row < M && col0 + 16 <= N) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    const float4 q = __ldg(reinterpret_cast<const float4*>(zp + j));
+                    z[j] = q.x;
+                    z[j + 1] = q.y;
+                    z[j + 2] = q.z;
+                    z[j + 3] = q.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; j++) z[j] = row < M && col0 + j < N ? zp[j] : 0.f;
+            }
+            __align__(16) __nv_bfloat16 hb[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const float dz = __uint_as_float(v[j]) * gelu_grad(z[j]);
+                sd[r * (TM_BN + 1) + c0 + j] = dz;
+                hb[j] = __float2bfloat16(dz);
+                tt[(c0 + j) * TM_TPITCH + r] = hb[j];
+            }
+            if (row < M) {
+                __nv_bfloat16* hp = ep.H + row * N + col0;
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    if (col0 + 8 * q + 8 <= N) *reinterpret_cast<uint4*>(hp + 8 * q) = *reinterpret_cast<uint4*>(hb + 8 * q);
+            }
         } else if (row >= M) {
         } else if (EPI == 0) {
             float* dst = C + blockIdx.z * c_split + row * ldc + col0;
@@ -555,6 +619,24 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TM_BN) : "memory");
     }
+    if ((EPI == 1 && tstore && ep.HT) || EPI == 2) {
+        // the transposed tile, 16 bytes (8 rows) a thread and pass
+        const __nv_bfloat16* tt = reinterpret_cast<const __nv_bfloat16*>(base + 3 * (TC_BM * 128));
+        for (int i = threadIdx.x; i < TM_BN * (TC_BM / 8); i += TM_THREADS) {
+            const int c = i >> 4, r = (i & 15) * 8;
+            if (n0 + c < N && m0 + r < ep.ldt)
+                *reinterpret_cast<uint4*>(ep.HT + static_cast<int64_t>(n0 + c) * ep.ldt + m0 + r) =
+                    *reinterpret_cast<const uint4*>(tt + c * TM_TPITCH + r);
+        }
+    }
+    if (EPI == 2 && threadIdx.x < TM_BN && n0 + static_cast<int>(threadIdx.x) < N) {
+        const float* sd = reinterpret_cast<const float*>(base) + threadIdx.x;
+        const int nr = min(TC_BM, M - m0);
+        float sum = 0.f;
+#pragma unroll 8
+        for (int r = 0; r < nr; r++) sum += sd[r * (TM_BN + 1)];
+        ep.colpart[static_cast<int64_t>(blockIdx.y) * N + n0 + threadIdx.x] = sum;
+    }
     if (EPI == 1 && tstore && threadIdx.x == 0) {
         // x = n0 and n0 + 32: multiples of 32 columns, 128-byte aligned
         tma_store_2d(&tmZ, smem_u32(base), n0, m0);
@@ -593,21 +675,30 @@ __device__ __forceinline__ void write_features(const float* __restrict__ x, int 
     }
 }
 
-__global__ void features_kernel(int64_t M, int n_in, int nf, int width, const float* __restrict__ x,
+// rows of ld (in_w inputs, then zeros)
+__global__ void features_kernel(int64_t M, int n_in, int nf, int in_w, int ld, const float* __restrict__ x,
                                 __nv_bfloat16* __restrict__ h) {
     const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= M) return;
-    write_features(x + r * n_in, n_in, nf, h + r * width);
+    __nv_bfloat16* o = h + r * ld;
+    write_features(x + r * n_in, n_in, nf, o);
+    for (int j = in_w; j < ld; j++) o[j] = __float2bfloat16(0.f);
 }
 
-__global__ void gather_kernel(int M, int64_t n_rows, int n_in, int nf, int width, int n_out,
+// ht (may be null): the transposed inputs, in_w rows of ldt
+__global__ void gather_kernel(int M, int64_t n_rows, int n_in, int nf, int in_w, int ld, int n_out,
                               const float* __restrict__ X, const float* __restrict__ T, uint64_t key,
-                              __nv_bfloat16* __restrict__ h, float* __restrict__ tb) {
+                              __nv_bfloat16* __restrict__ h, float* __restrict__ tb, __nv_bfloat16* __restrict__ ht,
+                              int64_t ldt) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= M) return;
     const int64_t src = static_cast<int64_t>(mix64(key + static_cast<uint64_t>(r) * 0x9E3779B97F4A7C15ULL) %
                                              static_cast<uint64_t>(n_rows));
-    write_features(X + src * n_in, n_in, nf, h + static_cast<int64_t>(r) * width);
+    __nv_bfloat16* o = h + static_cast<int64_t>(r) * ld;
+    write_features(X + src * n_in, n_in, nf, o);
+    for (int j = in_w; j < ld; j++) o[j] = __float2bfloat16(0.f);
+    if (ht)
+        for (int j = 0; j < in_w; j++) ht[j * ldt + r] = o[j];
     for (int j = 0; j < n_out; j++) tb[static_cast<int64_t>(r) * n_out + j] = T[src * n_out + j];
 }
 
@@ -691,6 +782,98 @@ __global__ void adam_kernel(int64_t n, float* __restrict__ w, const float* __res
     const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
     wb[i] = __float2bfloat16(wi);
+}
+
+// The last layer's dZ = dY of kColRows rows per block: bf16 rows of ld (zeros
+// beyond N) and their transpose, column sums of the block row by row, squared
+// error per row.  N <= kMseCols.
+constexpr int kMseCols = 32;
+__global__ void __launch_bounds__(kColRows) mse_grad_kernel(int M, int N, int ld, const float* __restrict__ Y,
+                                                            const float* __restrict__ T,
+                                                            __nv_bfloat16* __restrict__ dz,
+                                                            __nv_bfloat16* __restrict__ dzt, int64_t ldt,
+                                                            float* __restrict__ colpart, float* __restrict__ row_err) {
+    __shared__ float sd[kColRows][kMseCols + 1];
+    const int r = blockIdx.x * kColRows + threadIdx.x;
+    const float scale = 2.f / (static_cast<float>(M) * N);
+    if (r < M) {
+        float e = 0.f;
+        for (int c = 0; c < N; c++) {
+            const float d = Y[static_cast<int64_t>(r) * N + c] - T[static_cast<int64_t>(r) * N + c];
+            e += d * d;
+            const float g = scale * d;
+            sd[threadIdx.x][c] = g;
+            const __nv_bfloat16 h = __float2bfloat16(g);
+            dz[static_cast<int64_t>(r) * ld + c] = h;
+            dzt[c * ldt + r] = h;
+        }
+        for (int c = N; c < ld; c++) dz[static_cast<int64_t>(r) * ld + c] = __float2bfloat16(0.f);
+        row_err[r] = e;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        const int nr = min(kColRows, M - static_cast<int>(blockIdx.x) * kColRows);
+        float sum = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < nr; i++) sum += sd[i][threadIdx.x];
+        colpart[static_cast<int64_t>(blockIdx.x) * N + threadIdx.x] = sum;
+    }
+}
+
+// One layer as grad_adam_kernel reads it.
+struct LayerGrad {
+    int64_t w_off, b_off, part_off;  // part_off: its S x (dout * din) weight partials
+    int din, dout, ld_in, ld_t;      // row strides of the padded W (layer 0) and of W^T
+    int64_t col_off;                 // its chunks x dout column sums
+    __nv_bfloat16* wpad;             // layer 0: W with rows of ld_in (or null)
+    __nv_bfloat16* wt;               // W^T, din rows of ld_t (null for layer 0)
+};
+// The gradients of layer blockIdx.y (weights: the S split partial sums in
+// order; bias: the chunks' column sums in order) into g, then, if adam, the
+// Adam step and the bf16 copies.
+__global__ void __launch_bounds__(256) grad_adam_kernel(const LayerGrad* __restrict__ layers, int S, int chunks,
+                                                        const float* __restrict__ part,
+                                                        const float* __restrict__ colpart, float* __restrict__ g,
+                                                        bool adam, float* __restrict__ w, float* __restrict__ m,
+                                                        float* __restrict__ v, float lr, float b1, float b2, float eps,
+                                                        float c1, float c2, __nv_bfloat16* __restrict__ wb) {
+    const LayerGrad L = layers[blockIdx.y];
+    const int64_t wn = static_cast<int64_t>(L.din) * L.dout;
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= wn + L.dout) return;
+    const bool weight = i < wn;
+    const float* p = weight ? part + L.part_off + i : colpart + L.col_off + (i - wn);
+    const int64_t step = weight ? wn : L.dout;
+    const int n = weight ? S : chunks;
+    float gr = 0.f;
+#pragma unroll 8
+    for (int z = 0; z < n; z++) gr += p[z * step];
+    const int64_t k = weight ? L.w_off + i : L.b_off + (i - wn);
+    g[k] = gr;
+    if (!adam) return;
+    const float mi = b1 * m[k] + (1.f - b1) * gr;
+    const float vi = b2 * v[k] + (1.f - b2) * gr * gr;
+    m[k] = mi;
+    v[k] = vi;
+    const float wi = w[k] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[k] = wi;
+    const __nv_bfloat16 h = __float2bfloat16(wi);
+    wb[k] = h;
+    if (weight) {
+        const int o = static_cast<int>(i / L.din), q = static_cast<int>(i - static_cast<int64_t>(o) * L.din);
+        if (L.wpad) L.wpad[static_cast<int64_t>(o) * L.ld_in + q] = h;
+        if (L.wt) L.wt[static_cast<int64_t>(q) * L.ld_t + o] = h;
+    }
+}
+// the padded W of layer 0 and the W^T of the others from the bf16 weights
+__global__ void weight_copies_kernel(const LayerGrad* __restrict__ layers, const __nv_bfloat16* __restrict__ wb) {
+    const LayerGrad L = layers[blockIdx.y];
+    const int64_t wn = static_cast<int64_t>(L.din) * L.dout;
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= wn) return;
+    const int o = static_cast<int>(i / L.din), q = static_cast<int>(i - static_cast<int64_t>(o) * L.din);
+    if (L.wpad) L.wpad[static_cast<int64_t>(o) * L.ld_in + q] = wb[L.w_off + i];
+    if (L.wt) L.wt[static_cast<int64_t>(q) * L.ld_t + o] = wb[L.w_off + i];
 }
 
 __global__ void to_bf16_kernel(int64_t n, const float* __restrict__ x, __nv_bfloat16* __restrict__ y) {
@@ -861,6 +1044,11 @@ void gemm(int M, int N, int K, const __nv_bfloat16* A, int64_t lda, const __nv_b
         launch_tc<false, false>(grid, M, N, K, kc, A, lda, B, ldb, C, ldc, c_split, s);
 }
 
+// enqueues the read of the GEMM status word into pinned memory, before the
+// call's own synchronisation
+void gemm_status_fetch(int* pinned, cudaStream_t s) {
+    cudaMemcpyAsync(pinned, gemm_status_ptr(), sizeof(int), cudaMemcpyDeviceToHost, s);
+}
 // reads and clears the GEMM status word (after a synchronisation)
 bool gemm_status_ok() {
     int v = 0;
@@ -898,12 +1086,37 @@ struct gelios_mlp {
     std::vector<Buf> z;  // fp32 pre-activations of every hidden layer
     Buf c, y, dh, dz, dzb, tb, rowerr, part, colpart, loss, xin;
     Buf wt, dzt, ht;  // transposes for the backward GEMMs: W_l^T, dZ^T, H_l^T
+    int ld0 = 0;      // row stride of the first layer's input and of wpad (in_w rounded up to 8: TMA rows)
+    Buf wpad;         // bf16 W of the first layer, rows of ld0
+    // the fused training step (allocated by gelios_mlp_create where it takes
+    // the network): per layer H^T and dZ^T, W^T, gradient partials
+    bool fused = false;
+    Buf f_ht, f_dzt, f_wt, f_part, f_col, f_dzb2, f_layers;
+    std::vector<LayerGrad> layers_host;
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_dz = nullptr, ev_side = nullptr;
+    int* status_host = nullptr;  // pinned copy of the GEMM status word
     Buf X, T;  // training set (fp32 rows)
     int64_t n_rows = 0;
     ~gelios_mlp() {
+        if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
+        if (ev_dz) cudaEventDestroy(ev_dz);
+        if (ev_side) cudaEventDestroy(ev_side);
+        if (status_host) cudaFreeHost(status_host);
     }
     int layers() const { return depth + 1; }
+    // splits of a weight GEMM over the rows of the batch
+    static int split_target(int M) {
+        const int s = (M + 255) / 256;
+        return s > kMaxSplit ? kMaxSplit : s < 1 ? 1 : s;
+    }
+    static int splits_of(int M) { return split_count(M, tc_split_len(M, split_target(M))); }
+    // H_l^T (din[l] rows) and dZ_l^T (dout[l] rows), max_batch rounded up to 8 apart
+    __nv_bfloat16* ht_of(int l) const {
+        return f_ht.as<__nv_bfloat16>() + (l == 0 ? 0 : pad8(max_batch) * (in_w + static_cast<int64_t>(l - 1) * width));
+    }
+    __nv_bfloat16* dzt_of(int l) const { return f_dzt.as<__nv_bfloat16>() + pad8(max_batch) * width * l; }
 };
 
 namespace {
@@ -921,8 +1134,9 @@ int cuda_fail(cudaError_t e) {
         if (e_ != cudaSuccess) return cuda_fail(e_); \
     } while (0)
 
-// forward pass of M rows whose network inputs are in h[0]; output in y
-void forward(gelios_mlp* n, int M) {
+// forward pass of M rows whose network inputs are in h[0]; output in y.
+// train: the hidden layers' H^T as well (f_ht, rows of pad8(M)).
+void forward(gelios_mlp* n, int M, bool train = false) {
     cudaStream_t s = n->stream;
     const __nv_bfloat16* wb = n->wb.as<__nv_bfloat16>();
     for (int l = 0; l < n->layers(); l++) {
@@ -934,17 +1148,78 @@ void forward(gelios_mlp* n, int M) {
         ep.H = last ? nullptr : n->h[l + 1].as<__nv_bfloat16>();
         ep.Hf = last ? n->y.as<float>() : nullptr;
         ep.act = last ? 0 : 1;
+        if (train && !last) {
+            ep.ldt = pad8(M);
+            ep.HT = n->ht_of(l + 1);
+        }
         // bias and activation applied as the accumulator leaves tensor memory
         // (TMA path), or by bias_act_kernel after the GEMM
         const __nv_bfloat16* A = n->h[l].as<__nv_bfloat16>();
+        const __nv_bfloat16* W = l == 0 ? n->wpad.as<__nv_bfloat16>() : wb + n->w_off[l];
+        const int ld = l == 0 ? n->ld0 : di;
         dim3 grid(blocks(dO, TC_BN), blocks(M, TC_BM), 1);
-        if (M > 0 && launch_tma<1>(grid, M, dO, di, tc_split_len(di, 1), A, di, wb + n->w_off[l], di, nullptr, 0, 0,
-                                   ep, s))
+        if (M > 0 &&
+            launch_tma<1>(grid, M, dO, di, tc_split_len(di, 1), A, ld, W, ld, nullptr, 0, 0, ep, s))
             continue;
-        gemm(M, dO, di, A, di, wb + n->w_off[l], di, n->c.as<float>(), dO, s);
+        gemm(M, dO, di, A, ld, W, ld, n->c.as<float>(), dO, s);
         const int64_t e = static_cast<int64_t>(M) * dO;
         bias_act_kernel<<<blocks(e, 256), 256, 0, s>>>(M, dO, n->c.as<float>(), ep.bias, ep.Z, ep.H, ep.Hf, ep.act);
     }
+}
+
+// The backward pass of the fused training step: loss of the batch into
+// loss[0]; the gradients' partial sums into f_part and f_col, which
+// grad_adam_kernel then adds up.  The data GEMMs run down the layers on the
+// main stream, each layer's weight GEMM and the loss beside them on the side
+// stream.  Per 8192-row step of the 31 -> 5 x 256 -> 5 network, as ~45
+// launches of separate transposes, activations, sums and reductions the
+// whole step took 480 us, TRAIN_US.
+bool backward_fused(gelios_mlp* n, int M, float* loss) {
+    cudaStream_t s = n->stream, s2 = n->side;
+    const int L = n->layers();
+    const int64_t Mp = pad8(M);
+    const int S = n->splits_of(M), kc = tc_split_len(M, n->split_target(M)), chunks = (M + kColRows - 1) / kColRows;
+    const int ldo = static_cast<int>(pad8(n->n_out));
+    __nv_bfloat16* dz[2] = {n->dzb.as<__nv_bfloat16>(), n->f_dzb2.as<__nv_bfloat16>()};
+    float* col = n->f_col.as<float>();
+    mse_grad_kernel<<<chunks, kColRows, 0, s>>>(M, n->n_out, ldo, n->y.as<float>(), n->tb.as<float>(), dz[0],
+                                                n->dzt_of(L - 1), Mp, col + n->layers_host[L - 1].col_off,
+                                                n->rowerr.as<float>());
+    for (int l = L - 1; l >= 0; l--) {
+        const int di = n->din[l], dO = n->dout[l];
+        cudaEventRecord(n->ev_dz, s);
+        cudaStreamWaitEvent(s2, n->ev_dz, 0);
+        if (l == L - 1) loss_kernel<<<1, 256, 0, s2>>>(M, n->n_out, n->rowerr.as<float>(), loss);
+        // dW[dO][di] = dZ^T . H_l, split over the rows of the batch
+        bool ok = launch_tma<0>(dim3(1, blocks(dO, TC_BM), S), dO, di, M, kc, n->dzt_of(l), Mp, n->ht_of(l), Mp,
+                                n->f_part.as<float>() + n->layers_host[l].part_off, di, static_cast<int64_t>(dO) * di,
+                                GemmEpilogue{}, s2);
+        if (!ok) return false;  // an operand without a tensor map (not with the strides gelios_mlp_create chose)
+        if (l == 0) break;
+        // dZ_{l-1} = (dZ . W_l) * GELU'(Z_{l-1})
+        const int b = (L - 1 - l) & 1;
+        GemmEpilogue ep;
+        ep.Zin = n->z[l - 1].as<float>();
+        ep.H = dz[b ^ 1];
+        ep.HT = n->dzt_of(l - 1);
+        ep.ldt = Mp;
+        ep.colpart = col + n->layers_host[l - 1].col_off;
+        const int ldz = l == L - 1 ? ldo : dO;
+        ok = launch_tma<2>(dim3(1, blocks(M, TC_BM), 1), M, di, dO, tc_split_len(dO, 1), dz[b], ldz,
+                           n->layers_host[l].wt, n->layers_host[l].ld_t, nullptr, 0, 0, ep, s);
+        if (!ok) return false;
+    }
+    return cudaEventRecord(n->ev_side, s2) == cudaSuccess && cudaStreamWaitEvent(s, n->ev_side, 0) == cudaSuccess;
+}
+// the gradients into g32 and, with adam, the step (see grad_adam_kernel)
+void reduce_fused(gelios_mlp* n, int M, bool adam, float lr, float b1, float b2, float eps, float c1, float c2) {
+    int64_t most = 0;
+    for (int l = 0; l < n->layers(); l++)
+        most = std::max(most, static_cast<int64_t>(n->din[l] + 1) * n->dout[l]);
+    grad_adam_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(
+        n->f_layers.as<LayerGrad>(), n->splits_of(M), (M + kColRows - 1) / kColRows, n->f_part.as<float>(),
+        n->f_col.as<float>(), n->g32.as<float>(), adam, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(), lr, b1,
+        b2, eps, c1, c2, n->wb.as<__nv_bfloat16>());
 }
 
 // loss of the batch (targets in tb) into loss[0]; gradients into g32
@@ -959,10 +1234,7 @@ void backward(gelios_mlp* n, int M) {
                                                    n->dzb.as<__nv_bfloat16>(), 0);
     const __nv_bfloat16* wb = n->wb.as<__nv_bfloat16>();
     float* g = n->g32.as<float>();
-    int splits = (M + 255) / 256;
-    if (splits > kMaxSplit) splits = kMaxSplit;
-    if (splits < 1) splits = 1;
-    const int S = split_count(M, tc_split_len(M, splits));
+    const int splits = n->split_target(M), S = n->splits_of(M);
     const int64_t Mp = pad8(M);
     __nv_bfloat16* dzt = n->dzt.as<__nv_bfloat16>();
     __nv_bfloat16* ht = n->ht.as<__nv_bfloat16>();
@@ -972,7 +1244,7 @@ void backward(gelios_mlp* n, int M) {
         // contiguous), split over the rows of the batch
         const int64_t wn = static_cast<int64_t>(dO) * di;
         transpose(M, dO, n->dzb.as<__nv_bfloat16>(), dO, dzt, Mp, s);
-        transpose(M, di, n->h[l].as<__nv_bfloat16>(), di, ht, Mp, s);
+        transpose(M, di, n->h[l].as<__nv_bfloat16>(), l == 0 ? n->ld0 : di, ht, Mp, s);
         gemm(dO, di, M, dzt, Mp, ht, Mp, n->part.as<float>(), di, s, splits, wn);
         splitk_reduce_kernel<<<blocks(wn, 256), 256, 0, s>>>(wn, S, n->part.as<float>(), g + n->w_off[l]);
         // db = column sums of dZ
@@ -1008,6 +1280,7 @@ extern "C" int gelios_mlp_create(gelios_mlp** out, int device, int n_in, int n_f
     n->n_out = n_out;
     n->max_batch = max_batch;
     n->in_w = n_in + 4 * n_fourier;
+    n->ld0 = static_cast<int>(pad8(n->in_w));
     MLP_TRY(cudaSetDevice(device));
     MLP_TRY(cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking));
     int64_t off = 0;
@@ -1029,15 +1302,67 @@ extern "C" int gelios_mlp_create(gelios_mlp** out, int device, int n_in, int n_f
               n->wb.alloc(P * 2);
     n->h.resize(depth + 1);
     n->z.resize(depth);
-    for (int l = 0; l <= depth; l++) ok = ok && n->h[l].alloc(MB * n->din[l] * 2);
+    for (int l = 0; l <= depth; l++) ok = ok && n->h[l].alloc(MB * (l == 0 ? n->ld0 : n->din[l]) * 2);
+    ok = ok && n->wpad.alloc(static_cast<size_t>(n->dout[0]) * n->ld0 * 2);
     for (int l = 0; l < depth; l++) ok = ok && n->z[l].alloc(MB * width * 4);
     ok = ok && n->c.alloc(MB * W * 4) && n->y.alloc(MB * n_out * 4) && n->dh.alloc(MB * W * 4) &&
-         n->dz.alloc(MB * W * 4) && n->dzb.alloc(MB * W * 2) && n->tb.alloc(MB * n_out * 4) &&
+         n->dz.alloc(MB * W * 4) && n->dzb.alloc(MB * pad8(widest) * 2) && n->tb.alloc(MB * n_out * 4) &&
          n->rowerr.alloc(MB * 4) && n->part.alloc(static_cast<size_t>(kMaxSplit) * W * W * 4) &&
          n->colpart.alloc(((MB + kColRows - 1) / kColRows) * W * 4) && n->loss.alloc(16) &&
          n->xin.alloc(MB * n_in * 4) && n->wt.alloc(W * pad8(widest) * 2) &&
          n->dzt.alloc(W * pad8(max_batch) * 2) && n->ht.alloc(W * pad8(max_batch) * 2);
     if (!ok) return cuda_fail(cudaErrorMemoryAllocation);
+    MLP_TRY(cudaMallocHost(&n->status_host, sizeof(int)));
+    MLP_TRY(cudaMemsetAsync(n->wpad.p, 0, n->wpad.bytes, n->stream));
+    // W^T of the layers above the first, gradient partials and column sums,
+    // and what the fused training step needs beside them
+    int64_t part = 0, col = 0, wt = 0;
+    const int64_t chunks = (max_batch + kColRows - 1) / kColRows;
+    for (int l = 0; l <= depth; l++) {
+        LayerGrad g{};
+        g.w_off = n->w_off[l];
+        g.b_off = n->b_off[l];
+        g.din = n->din[l];
+        g.dout = n->dout[l];
+        g.ld_in = n->ld0;
+        g.ld_t = static_cast<int>(pad8(g.dout));
+        g.part_off = part;
+        g.col_off = col;
+        part += static_cast<int64_t>(gelios_mlp::splits_of(max_batch)) * g.din * g.dout;
+        col += chunks * g.dout;
+        if (l > 0) wt += static_cast<int64_t>(g.din) * g.ld_t;
+        n->layers_host.push_back(g);
+    }
+    // the fused step: 16-byte rows for the TMA (width a multiple of 8), the
+    // output columns in mse_grad_kernel's tile, partials of at most 256 MB
+    CUtensorMap tz, th;
+    n->fused = width % 8 == 0 && n_out <= kMseCols && part <= (int64_t(64) << 20) &&
+               output_map(&tz, n->z[0].p, true, max_batch, width) && output_map(&th, n->h[1].p, false, max_batch, width);
+    if (n->fused) {
+        const size_t Mp = static_cast<size_t>(pad8(max_batch));
+        ok = n->f_ht.alloc(Mp * (n->in_w + static_cast<size_t>(depth) * width) * 2) &&
+             n->f_dzt.alloc(Mp * width * (static_cast<size_t>(depth) + 1) * 2 + Mp * kMseCols * 2) &&
+             n->f_wt.alloc(static_cast<size_t>(wt) * 2) && n->f_part.alloc(static_cast<size_t>(part) * 4) &&
+             n->f_col.alloc(static_cast<size_t>(col) * 4) && n->f_dzb2.alloc(MB * pad8(widest) * 2);
+        if (!ok) return cuda_fail(cudaErrorMemoryAllocation);
+        MLP_TRY(cudaMemsetAsync(n->f_wt.p, 0, n->f_wt.bytes, n->stream));
+        MLP_TRY(cudaStreamCreateWithFlags(&n->side, cudaStreamNonBlocking));
+        MLP_TRY(cudaEventCreateWithFlags(&n->ev_dz, cudaEventDisableTiming));
+        MLP_TRY(cudaEventCreateWithFlags(&n->ev_side, cudaEventDisableTiming));
+    }
+    int64_t wo = 0;
+    for (int l = 0; l <= depth; l++) {
+        LayerGrad& g = n->layers_host[l];
+        if (l == 0) {
+            g.wpad = n->wpad.as<__nv_bfloat16>();
+        } else if (n->fused) {
+            g.wt = n->f_wt.as<__nv_bfloat16>() + wo;
+            wo += static_cast<int64_t>(g.din) * g.ld_t;
+        }
+    }
+    if (!n->f_layers.alloc(sizeof(LayerGrad) * n->layers_host.size())) return cuda_fail(cudaErrorMemoryAllocation);
+    MLP_TRY(cudaMemcpyAsync(n->f_layers.p, n->layers_host.data(), sizeof(LayerGrad) * n->layers_host.size(),
+                            cudaMemcpyHostToDevice, n->stream));
     MLP_TRY(cudaMemsetAsync(n->w32.p, 0, P * 4, n->stream));
     MLP_TRY(cudaMemsetAsync(n->wb.p, 0, P * 2, n->stream));
     MLP_TRY(cudaMemsetAsync(n->m.p, 0, P * 4, n->stream));
@@ -1063,6 +1388,10 @@ extern "C" int gelios_mlp_set_params(gelios_mlp* n, const float* host, int64_t c
     MLP_TRY(cudaMemcpyAsync(n->w32.p, host, P * 4, cudaMemcpyHostToDevice, n->stream));
     to_bf16_kernel<<<blocks(n->n_params, 256), 256, 0, n->stream>>>(n->n_params, n->w32.as<float>(),
                                                                     n->wb.as<__nv_bfloat16>());
+    int64_t most = 0;
+    for (int l = 0; l < n->layers(); l++) most = std::max(most, static_cast<int64_t>(n->din[l]) * n->dout[l]);
+    weight_copies_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(n->f_layers.as<LayerGrad>(),
+                                                                                      n->wb.as<__nv_bfloat16>());
     MLP_TRY(cudaMemsetAsync(n->m.p, 0, P * 4, n->stream));
     MLP_TRY(cudaMemsetAsync(n->v.p, 0, P * 4, n->stream));
     MLP_TRY(cudaGetLastError());
@@ -1085,17 +1414,24 @@ extern "C" int gelios_mlp_loss_grad(gelios_mlp* n, const float* x, const float* 
     cudaStream_t s = n->stream;
     MLP_TRY(cudaMemcpyAsync(n->xin.p, x, static_cast<size_t>(M) * n->n_in * 4, cudaMemcpyHostToDevice, s));
     MLP_TRY(cudaMemcpyAsync(n->tb.p, t, static_cast<size_t>(M) * n->n_out * 4, cudaMemcpyHostToDevice, s));
-    features_kernel<<<blocks(M, 128), 128, 0, s>>>(M, n->n_in, n->nf, n->in_w, n->xin.as<float>(),
+    features_kernel<<<blocks(M, 128), 128, 0, s>>>(M, n->n_in, n->nf, n->in_w, n->ld0, n->xin.as<float>(),
                                                    n->h[0].as<__nv_bfloat16>());
-    forward(n, M);
-    backward(n, M);
+    forward(n, M, n->fused);
+    if (n->fused) {
+        transpose(M, n->in_w, n->h[0].as<__nv_bfloat16>(), n->ld0, n->ht_of(0), pad8(M), s);
+        if (!backward_fused(n, M, n->loss.as<float>())) return cuda_fail(cudaErrorInvalidValue);
+        reduce_fused(n, M, false, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
+    } else {
+        backward(n, M);
+    }
     MLP_TRY(cudaGetLastError());
     float l = 0.f;
     MLP_TRY(cudaMemcpyAsync(&l, n->loss.p, 4, cudaMemcpyDeviceToHost, s));
     if (grad)
         MLP_TRY(cudaMemcpyAsync(grad, n->g32.p, static_cast<size_t>(n->n_params) * 4, cudaMemcpyDeviceToHost, s));
+    gemm_status_fetch(n->status_host, s);
     MLP_TRY(cudaStreamSynchronize(s));
-    if (!gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     if (loss) *loss = l;
     return GELIOS_OK;
 }
@@ -1125,12 +1461,16 @@ extern "C" int gelios_mlp_train(gelios_mlp* n, int iters, int batch, float lr_ma
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     for (int it = 0; it < iters; it++) {
         const uint64_t key = seed * 0xD1B54A32D192ED03ULL + static_cast<uint64_t>(n->step) * 0x8CB92BA72F3D8DD7ULL;
-        gather_kernel<<<blocks(batch, 128), 128, 0, s>>>(batch, n->n_rows, n->n_in, n->nf, n->in_w, n->n_out,
-                                                         n->X.as<float>(), n->T.as<float>(), key,
-                                                         n->h[0].as<__nv_bfloat16>(), n->tb.as<float>());
-        forward(n, batch);
-        backward(n, batch);
-        MLP_TRY(cudaMemcpyAsync(hist.as<float>() + it, n->loss.p, 4, cudaMemcpyDeviceToDevice, s));
+        gather_kernel<<<blocks(batch, 128), 128, 0, s>>>(
+            batch, n->n_rows, n->n_in, n->nf, n->in_w, n->ld0, n->n_out, n->X.as<float>(), n->T.as<float>(), key,
+            n->h[0].as<__nv_bfloat16>(), n->tb.as<float>(), n->fused ? n->ht_of(0) : nullptr, pad8(batch));
+        forward(n, batch, n->fused);
+        if (n->fused) {
+            if (!backward_fused(n, batch, hist.as<float>() + it)) return cuda_fail(cudaErrorInvalidValue);
+        } else {
+            backward(n, batch);
+            MLP_TRY(cudaMemcpyAsync(hist.as<float>() + it, n->loss.p, 4, cudaMemcpyDeviceToDevice, s));
+        }
         float lr;
         if (it < warmup) {
             lr = lr_max * static_cast<float>(it + 1) / static_cast<float>(warmup);
@@ -1141,15 +1481,22 @@ extern "C" int gelios_mlp_train(gelios_mlp* n, int iters, int batch, float lr_ma
         n->step++;
         const float c1 = static_cast<float>(1.0 - std::pow(static_cast<double>(b1), n->step));
         const float c2 = static_cast<float>(1.0 - std::pow(static_cast<double>(b2), n->step));
-        adam_kernel<<<blocks(n->n_params, 256), 256, 0, s>>>(n->n_params, n->w32.as<float>(), n->g32.as<float>(),
-                                                             n->m.as<float>(), n->v.as<float>(), lr, b1, b2, eps, c1,
-                                                             c2, n->wb.as<__nv_bfloat16>());
+        if (n->fused)
+            reduce_fused(n, batch, true, lr, b1, b2, eps, c1, c2);
+        else
+            adam_kernel<<<blocks(n->n_params, 256), 256, 0, s>>>(n->n_params, n->w32.as<float>(), n->g32.as<float>(),
+                                                                 n->m.as<float>(), n->v.as<float>(), lr, b1, b2, eps,
+                                                                 c1, c2, n->wb.as<__nv_bfloat16>());
+        if (!n->fused)
+            weight_copies_kernel<<<dim3(blocks(static_cast<int64_t>(n->din[0]) * n->dout[0], 256), 1), 256, 0, s>>>(
+                n->f_layers.as<LayerGrad>(), n->wb.as<__nv_bfloat16>());
         MLP_TRY(cudaGetLastError());
     }
     if (loss_hist && iters > 0)
         MLP_TRY(cudaMemcpyAsync(loss_hist, hist.p, static_cast<size_t>(iters) * 4, cudaMemcpyDeviceToHost, s));
+    gemm_status_fetch(n->status_host, s);
     MLP_TRY(cudaStreamSynchronize(s));
-    if (!gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     return GELIOS_OK;
 }
 
@@ -1161,15 +1508,16 @@ extern "C" int gelios_mlp_predict(gelios_mlp* n, const float* x, int64_t M, floa
         const int m = static_cast<int>(M - r0 < n->max_batch ? M - r0 : n->max_batch);
         MLP_TRY(cudaMemcpyAsync(n->xin.p, x + r0 * n->n_in, static_cast<size_t>(m) * n->n_in * 4,
                                 cudaMemcpyHostToDevice, s));
-        features_kernel<<<blocks(m, 128), 128, 0, s>>>(m, n->n_in, n->nf, n->in_w, n->xin.as<float>(),
+        features_kernel<<<blocks(m, 128), 128, 0, s>>>(m, n->n_in, n->nf, n->in_w, n->ld0, n->xin.as<float>(),
                                                        n->h[0].as<__nv_bfloat16>());
         forward(n, m);
         MLP_TRY(cudaGetLastError());
         MLP_TRY(cudaMemcpyAsync(y + r0 * n->n_out, n->y.p, static_cast<size_t>(m) * n->n_out * 4,
                                 cudaMemcpyDeviceToHost, s));
     }
+    gemm_status_fetch(n->status_host, s);
     MLP_TRY(cudaStreamSynchronize(s));
-    if (!gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     return GELIOS_OK;
 }
 
