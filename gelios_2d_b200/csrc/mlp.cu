@@ -655,51 +655,64 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-// Row of the network input from raw input row x (n_in floats): x, then per
-// frequency f < nf: sin(2^f pi s), cos(2^f pi s) for s = x[n_in-2] and for
-// s = x[n_in-1].
-__device__ __forceinline__ void write_features(const float* __restrict__ x, int n_in, int nf,
-                                               __nv_bfloat16* __restrict__ out) {
-    for (int j = 0; j < n_in; j++) out[j] = __float2bfloat16(x[j]);
-    int o = n_in;
-    for (int c = 0; c < 2; c++) {
-        const float s = x[n_in - 2 + c];
-        float w = 3.14159265358979f;
-        for (int f = 0; f < nf; f++) {
-            float sn, cs;
-            sincosf(w * s, &sn, &cs);
-            out[o++] = __float2bfloat16(sn);
-            out[o++] = __float2bfloat16(cs);
-            w *= 2.f;
-        }
+// One row of the network input from raw input row x (n_in floats) by kRowThreads
+// threads (t = 0..): x, then per frequency f < nf sin(2^f pi s), cos(2^f pi s)
+// for s = x[n_in-2] and for s = x[n_in-1], then zeros up to ld.  ht (may be
+// null): the same values down column r of rows of ldt.
+constexpr int kRowThreads = 16;
+__device__ __forceinline__ void write_features(const float* __restrict__ x, int n_in, int nf, int ld, int t,
+                                               __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ ht,
+                                               int64_t ldt) {
+    const int in_w = n_in + 4 * nf;
+    auto put = [&](int j, float v) {
+        const __nv_bfloat16 b = __float2bfloat16(v);
+        out[j] = b;
+        if (ht && j < in_w) ht[j * ldt] = b;
+    };
+    for (int j = t; j < n_in; j += kRowThreads) put(j, x[j]);
+    for (int i = t; i < 2 * nf; i += kRowThreads) {
+        const int c = i >= nf ? 1 : 0, f = i - c * nf;
+        const float w = ldexpf(3.14159265358979f, f);  // doubled f times: exact
+        float sn, cs;
+        sincosf(w * x[n_in - 2 + c], &sn, &cs);
+        put(n_in + 2 * i, sn);
+        put(n_in + 2 * i + 1, cs);
     }
+    for (int j = in_w + t; j < ld; j += kRowThreads) put(j, 0.f);
 }
 
-// rows of ld (in_w inputs, then zeros)
-__global__ void features_kernel(int64_t M, int n_in, int nf, int in_w, int ld, const float* __restrict__ x,
-                                __nv_bfloat16* __restrict__ h) {
-    const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) features_kernel(int64_t M, int n_in, int nf, int ld,
+                                                       const float* __restrict__ x, __nv_bfloat16* __restrict__ h) {
+    const int64_t r = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kRowThreads;
     if (r >= M) return;
-    __nv_bfloat16* o = h + r * ld;
-    write_features(x + r * n_in, n_in, nf, o);
-    for (int j = in_w; j < ld; j++) o[j] = __float2bfloat16(0.f);
+    write_features(x + r * n_in, n_in, nf, ld, threadIdx.x % kRowThreads, h + r * ld, nullptr, 0);
 }
 
-// ht (may be null): the transposed inputs, in_w rows of ldt
-__global__ void gather_kernel(int M, int64_t n_rows, int n_in, int nf, int in_w, int ld, int n_out,
-                              const float* __restrict__ X, const float* __restrict__ T, uint64_t key,
-                              __nv_bfloat16* __restrict__ h, float* __restrict__ tb, __nv_bfloat16* __restrict__ ht,
-                              int64_t ldt) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// What changes from one training step to the next; the steps of a call read
+// entry *at of an array, so that one captured graph serves every step.
+// loss_kernel moves *at on once the batch is drawn; grad_adam_kernel, later in
+// the step, reads the entry before it.
+struct StepArgs {
+    uint64_t key;
+    float lr, c1, c2;
+    int pad;
+};
+
+// ht (may be null): the transposed inputs, rows of ldt.  One thread per row
+// took 11.4 us for 8192 rows (64 blocks, 12 sincosf in a row), 5.7 here.
+__global__ void __launch_bounds__(128) gather_kernel(int M, int64_t n_rows, int n_in, int nf, int ld, int n_out,
+                                                     const float* __restrict__ X, const float* __restrict__ T,
+                                                     const StepArgs* __restrict__ args,
+                                                     const int* __restrict__ at, __nv_bfloat16* __restrict__ h,
+                                                     float* __restrict__ tb, __nv_bfloat16* __restrict__ ht,
+                                                     int64_t ldt) {
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) / kRowThreads, t = threadIdx.x % kRowThreads;
     if (r >= M) return;
+    const uint64_t key = args[*at].key;
     const int64_t src = static_cast<int64_t>(mix64(key + static_cast<uint64_t>(r) * 0x9E3779B97F4A7C15ULL) %
                                              static_cast<uint64_t>(n_rows));
-    __nv_bfloat16* o = h + static_cast<int64_t>(r) * ld;
-    write_features(X + src * n_in, n_in, nf, o);
-    for (int j = in_w; j < ld; j++) o[j] = __float2bfloat16(0.f);
-    if (ht)
-        for (int j = 0; j < in_w; j++) ht[j * ldt + r] = o[j];
-    for (int j = 0; j < n_out; j++) tb[static_cast<int64_t>(r) * n_out + j] = T[src * n_out + j];
+    write_features(X + src * n_in, n_in, nf, ld, t, h + static_cast<int64_t>(r) * ld, ht ? ht + r : nullptr, ldt);
+    for (int j = t; j < n_out; j += kRowThreads) tb[static_cast<int64_t>(r) * n_out + j] = T[src * n_out + j];
 }
 
 __global__ void bias_act_kernel(int M, int N, const float* __restrict__ C, const float* __restrict__ bias,
@@ -755,8 +768,10 @@ __global__ void mse_kernel(int M, int N, const float* __restrict__ Y, const floa
     row_err[r] = e;
 }
 
-// one block of 256 threads: strided partial sums, then a fixed tree
-__global__ void loss_kernel(int M, int N, const float* __restrict__ row_err, float* __restrict__ out) {
+// one block of 256 threads: strided partial sums, then a fixed tree; into
+// out[0], or with `at` (see StepArgs) into out[*at], which it moves on
+__global__ void loss_kernel(int M, int N, const float* __restrict__ row_err, float* __restrict__ out,
+                            int* __restrict__ at) {
     __shared__ double s[256];
     double a = 0.0;
     for (int r = threadIdx.x; r < M; r += 256) a += row_err[r];
@@ -766,7 +781,11 @@ __global__ void loss_kernel(int M, int N, const float* __restrict__ row_err, flo
         if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = static_cast<float>(s[0] / (static_cast<double>(M) * N));
+    if (threadIdx.x == 0) {
+        const float l = static_cast<float>(s[0] / (static_cast<double>(M) * N));
+        if (at) out[(*at)++] = l;
+        else *out = l;
+    }
 }
 
 __global__ void adam_kernel(int64_t n, float* __restrict__ w, const float* __restrict__ gr, float* __restrict__ m,
@@ -829,14 +848,15 @@ struct LayerGrad {
     __nv_bfloat16* wt;               // W^T, din rows of ld_t (null for layer 0)
 };
 // The gradients of layer blockIdx.y (weights: the S split partial sums in
-// order; bias: the chunks' column sums in order) into g, then, if adam, the
+// order; bias: the chunks' column sums in order) into g, then, given args, the
 // Adam step and the bf16 copies.
 __global__ void __launch_bounds__(256) grad_adam_kernel(const LayerGrad* __restrict__ layers, int S, int chunks,
                                                         const float* __restrict__ part,
                                                         const float* __restrict__ colpart, float* __restrict__ g,
-                                                        bool adam, float* __restrict__ w, float* __restrict__ m,
-                                                        float* __restrict__ v, float lr, float b1, float b2, float eps,
-                                                        float c1, float c2, __nv_bfloat16* __restrict__ wb) {
+                                                        const StepArgs* __restrict__ args,
+                                                        const int* __restrict__ at, float* __restrict__ w,
+                                                        float* __restrict__ m, float* __restrict__ v, float b1, float b2,
+                                                        float eps, __nv_bfloat16* __restrict__ wb) {
     const LayerGrad L = layers[blockIdx.y];
     const int64_t wn = static_cast<int64_t>(L.din) * L.dout;
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -846,11 +866,20 @@ __global__ void __launch_bounds__(256) grad_adam_kernel(const LayerGrad* __restr
     const int64_t step = weight ? wn : L.dout;
     const int n = weight ? S : chunks;
     float gr = 0.f;
-#pragma unroll 8
-    for (int z = 0; z < n; z++) gr += p[z * step];
+    int z = 0;
+    for (; z + 16 <= n; z += 16) {  // sixteen loads in flight, added in order
+        float e[16];
+#pragma unroll
+        for (int q = 0; q < 16; q++) e[q] = __ldcs(p + (z + q) * step);
+#pragma unroll
+        for (int q = 0; q < 16; q++) gr += e[q];
+    }
+    for (; z < n; z++) gr += p[z * step];
     const int64_t k = weight ? L.w_off + i : L.b_off + (i - wn);
     g[k] = gr;
-    if (!adam) return;
+    if (!args) return;
+    const StepArgs a = args[*at - 1];
+    const float lr = a.lr, c1 = a.c1, c2 = a.c2;
     const float mi = b1 * m[k] + (1.f - b1) * gr;
     const float vi = b2 * v[k] + (1.f - b2) * gr * gr;
     m[k] = mi;
@@ -892,6 +921,11 @@ struct Buf {
     Buf(Buf&& o) noexcept : p(o.p), bytes(o.bytes) { o.p = nullptr; }
     ~Buf() {
         if (p) cudaFree(p);
+    }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        bytes = 0;
     }
     bool alloc(size_t n) {
         if (p) cudaFree(p);
@@ -1088,14 +1122,30 @@ struct gelios_mlp {
     Buf wt, dzt, ht;  // transposes for the backward GEMMs: W_l^T, dZ^T, H_l^T
     int ld0 = 0;      // row stride of the first layer's input and of wpad (in_w rounded up to 8: TMA rows)
     Buf wpad;         // bf16 W of the first layer, rows of ld0
-    // the fused training step (allocated by gelios_mlp_create where it takes
-    // the network): per layer H^T and dZ^T, W^T, gradient partials
-    bool fused = false;
+    // the fused training step (ensure_fused): per layer H^T and dZ^T, W^T,
+    // gradient partials
+    bool fused = false, fused_known = false;
     Buf f_ht, f_dzt, f_wt, f_part, f_col, f_dzb2, f_layers;
     std::vector<LayerGrad> layers_host;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_dz = nullptr, ev_side = nullptr;
-    int* status_host = nullptr;  // pinned copy of the GEMM status word
+    // one pinned allocation: a copy of the GEMM status word, then the staging
+    // of gelios_mlp_predict (px, py)
+    int* status_host = nullptr;
+    // steps of a training call: their StepArgs, losses and the step counter,
+    // kept from call to call (they grow with the longest call)
+    Buf args, hist, at;
+    int64_t steps_cap = 0;
+    cudaGraphExec_t graph = nullptr;  // one fused step of graph_batch rows
+    int graph_batch = 0;
+    void drop_graph() {
+        if (graph) cudaGraphExecDestroy(graph);
+        graph = nullptr;
+    }
+    // gelios_mlp_predict: pinned staging of two chunks' inputs and outputs
+    int64_t stage_rows = 0;
+    float *px[2] = {nullptr, nullptr}, *py[2] = {nullptr, nullptr};
+    cudaEvent_t ev_chunk[2] = {nullptr, nullptr};
     Buf X, T;  // training set (fp32 rows)
     int64_t n_rows = 0;
     ~gelios_mlp() {
@@ -1104,6 +1154,9 @@ struct gelios_mlp {
         if (ev_dz) cudaEventDestroy(ev_dz);
         if (ev_side) cudaEventDestroy(ev_side);
         if (status_host) cudaFreeHost(status_host);
+        drop_graph();
+        for (int k = 0; k < 2; k++)
+            if (ev_chunk[k]) cudaEventDestroy(ev_chunk[k]);
     }
     int layers() const { return depth + 1; }
     // splits of a weight GEMM over the rows of the batch
@@ -1173,8 +1226,9 @@ void forward(gelios_mlp* n, int M, bool train = false) {
 // main stream, each layer's weight GEMM and the loss beside them on the side
 // stream.  Per 8192-row step of the 31 -> 5 x 256 -> 5 network, as ~45
 // launches of separate transposes, activations, sums and reductions the
-// whole step took 480 us, TRAIN_US.
-bool backward_fused(gelios_mlp* n, int M, float* loss) {
+// whole step took 480 us, 189 here;
+// as a captured graph (train_graph) 156 (115 of 4096 rows, 97 of 128).
+bool backward_fused(gelios_mlp* n, int M, float* loss, int* at) {
     cudaStream_t s = n->stream, s2 = n->side;
     const int L = n->layers();
     const int64_t Mp = pad8(M);
@@ -1189,7 +1243,7 @@ bool backward_fused(gelios_mlp* n, int M, float* loss) {
         const int di = n->din[l], dO = n->dout[l];
         cudaEventRecord(n->ev_dz, s);
         cudaStreamWaitEvent(s2, n->ev_dz, 0);
-        if (l == L - 1) loss_kernel<<<1, 256, 0, s2>>>(M, n->n_out, n->rowerr.as<float>(), loss);
+        if (l == L - 1) loss_kernel<<<1, 256, 0, s2>>>(M, n->n_out, n->rowerr.as<float>(), loss, at);
         // dW[dO][di] = dZ^T . H_l, split over the rows of the batch
         bool ok = launch_tma<0>(dim3(1, blocks(dO, TC_BM), S), dO, di, M, kc, n->dzt_of(l), Mp, n->ht_of(l), Mp,
                                 n->f_part.as<float>() + n->layers_host[l].part_off, di, static_cast<int64_t>(dO) * di,
@@ -1211,25 +1265,58 @@ bool backward_fused(gelios_mlp* n, int M, float* loss) {
     }
     return cudaEventRecord(n->ev_side, s2) == cudaSuccess && cudaStreamWaitEvent(s, n->ev_side, 0) == cudaSuccess;
 }
-// the gradients into g32 and, with adam, the step (see grad_adam_kernel)
-void reduce_fused(gelios_mlp* n, int M, bool adam, float lr, float b1, float b2, float eps, float c1, float c2) {
+// the gradients into g32 and, given args, the Adam step (see grad_adam_kernel)
+constexpr float kAdamB1 = 0.9f, kAdamB2 = 0.999f, kAdamEps = 1e-8f;
+void reduce_fused(gelios_mlp* n, int M, const StepArgs* args, const int* at) {
     int64_t most = 0;
     for (int l = 0; l < n->layers(); l++)
         most = std::max(most, static_cast<int64_t>(n->din[l] + 1) * n->dout[l]);
     grad_adam_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(
         n->f_layers.as<LayerGrad>(), n->splits_of(M), (M + kColRows - 1) / kColRows, n->f_part.as<float>(),
-        n->f_col.as<float>(), n->g32.as<float>(), adam, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(), lr, b1,
-        b2, eps, c1, c2, n->wb.as<__nv_bfloat16>());
+        n->f_col.as<float>(), n->g32.as<float>(), args, at, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(),
+        kAdamB1, kAdamB2, kAdamEps, n->wb.as<__nv_bfloat16>());
+}
+void draw_batch(gelios_mlp* n, int batch) {
+    gather_kernel<<<blocks(static_cast<int64_t>(batch) * kRowThreads, 128), 128, 0, n->stream>>>(
+        batch, n->n_rows, n->n_in, n->nf, n->ld0, n->n_out, n->X.as<float>(), n->T.as<float>(),
+        n->args.as<StepArgs>(), n->at.as<int>(), n->h[0].as<__nv_bfloat16>(), n->tb.as<float>(),
+        n->fused ? n->ht_of(0) : nullptr, pad8(batch));
+}
+// One fused training step on the network's streams.
+bool enqueue_train_step(gelios_mlp* n, int batch) {
+    draw_batch(n, batch);
+    forward(n, batch, true);
+    if (!backward_fused(n, batch, n->hist.as<float>(), n->at.as<int>())) return false;
+    reduce_fused(n, batch, n->args.as<StepArgs>(), n->at.as<int>());
+    return cudaGetLastError() == cudaSuccess;
+}
+// The same as a graph, captured once per batch size and training set; null
+// where it cannot be captured (the step is then enqueued directly).
+cudaGraphExec_t train_graph(gelios_mlp* n, int batch) {
+    if (n->graph && n->graph_batch == batch) return n->graph;
+    n->drop_graph();
+    if (cudaStreamBeginCapture(n->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    const bool ok = enqueue_train_step(n, batch);
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(n->stream, &g);
+    if (!ok || e != cudaSuccess || !g || cudaGraphInstantiate(&n->graph, g, 0) != cudaSuccess) n->graph = nullptr;
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    n->graph_batch = batch;
+    return n->graph;
 }
 
 // loss of the batch (targets in tb) into loss[0]; gradients into g32
-void backward(gelios_mlp* n, int M) {
+void backward(gelios_mlp* n, int M, float* loss, int* at) {
     cudaStream_t s = n->stream;
     const int L = n->layers();
     const int64_t eo = static_cast<int64_t>(M) * n->n_out;
     mse_kernel<<<blocks(M, 256), 256, 0, s>>>(M, n->n_out, n->y.as<float>(), n->tb.as<float>(), n->dh.as<float>(),
                                               n->rowerr.as<float>());
-    loss_kernel<<<1, 256, 0, s>>>(M, n->n_out, n->rowerr.as<float>(), n->loss.as<float>());
+    loss_kernel<<<1, 256, 0, s>>>(M, n->n_out, n->rowerr.as<float>(), loss, at);
     act_bwd_kernel<<<blocks(eo, 256), 256, 0, s>>>(eo, n->dh.as<float>(), nullptr, n->dz.as<float>(),
                                                    n->dzb.as<__nv_bfloat16>(), 0);
     const __nv_bfloat16* wb = n->wb.as<__nv_bfloat16>();
@@ -1261,6 +1348,69 @@ void backward(gelios_mlp* n, int M) {
         act_bwd_kernel<<<blocks(e, 256), 256, 0, s>>>(e, n->dh.as<float>(), n->z[l - 1].as<float>(),
                                                       n->dz.as<float>(), n->dzb.as<__nv_bfloat16>(), 1);
     }
+}
+
+// The W^T copies (and layer 0's padded W) of the current bf16 weights.
+void copy_weights(gelios_mlp* n) {
+    int64_t most = 0;
+    for (int l = 0; l < n->layers(); l++) most = std::max(most, static_cast<int64_t>(n->din[l]) * n->dout[l]);
+    weight_copies_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(n->f_layers.as<LayerGrad>(),
+                                                                                      n->wb.as<__nv_bfloat16>());
+}
+
+// Decides, at the first use of a gradient, whether the fused training step
+// takes the network (16-byte rows for the TMA: a width that is a multiple of
+// 8; the output columns in mse_grad_kernel's tile; partial sums of at most
+// 256 MB) and allocates what it needs: per layer H^T, dZ^T, W^T, the partial
+// and column sums.  Without room for them the separate kernels run.
+int ensure_fused(gelios_mlp* n) {
+    if (n->fused_known) return GELIOS_OK;
+    const int depth = n->depth, width = n->width;
+    const int64_t chunks = (n->max_batch + kColRows - 1) / kColRows;
+    int64_t part = 0, col = 0, wt = 0;
+    for (int l = 0; l <= depth; l++) {
+        LayerGrad& g = n->layers_host[l];
+        g.part_off = part;
+        g.col_off = col;
+        part += static_cast<int64_t>(gelios_mlp::splits_of(n->max_batch)) * g.din * g.dout;
+        col += chunks * g.dout;
+        if (l > 0) wt += static_cast<int64_t>(g.din) * g.ld_t;
+    }
+    CUtensorMap tz, th;
+    bool ok = width % 8 == 0 && n->n_out <= kMseCols && part <= (int64_t(64) << 20) &&
+              output_map(&tz, n->z[0].p, true, n->max_batch, width) &&
+              output_map(&th, n->h[1].p, false, n->max_batch, width);
+    if (ok) {
+        const size_t Mp = static_cast<size_t>(pad8(n->max_batch));
+        const int64_t widest = std::max({n->in_w, width, n->n_out});
+        ok = n->f_ht.alloc(Mp * (n->in_w + static_cast<size_t>(depth) * width) * 2) &&
+             n->f_dzt.alloc(Mp * width * (static_cast<size_t>(depth) + 1) * 2 + Mp * kMseCols * 2) &&
+             n->f_wt.alloc(static_cast<size_t>(wt) * 2) && n->f_part.alloc(static_cast<size_t>(part) * 4) &&
+             n->f_col.alloc(static_cast<size_t>(col) * 4) &&
+             n->f_dzb2.alloc(static_cast<size_t>(n->max_batch) * pad8(widest) * 2);
+        if (!ok) {
+            cudaGetLastError();
+            for (Buf* b : {&n->f_ht, &n->f_dzt, &n->f_wt, &n->f_part, &n->f_col, &n->f_dzb2}) b->release();
+        }
+    }
+    n->fused_known = true;
+    if (!ok) return GELIOS_OK;
+    int64_t wo = 0;
+    for (int l = 1; l <= depth; l++) {
+        LayerGrad& g = n->layers_host[l];
+        g.wt = n->f_wt.as<__nv_bfloat16>() + wo;
+        wo += static_cast<int64_t>(g.din) * g.ld_t;
+    }
+    MLP_TRY(cudaStreamCreateWithFlags(&n->side, cudaStreamNonBlocking));
+    MLP_TRY(cudaEventCreateWithFlags(&n->ev_dz, cudaEventDisableTiming));
+    MLP_TRY(cudaEventCreateWithFlags(&n->ev_side, cudaEventDisableTiming));
+    MLP_TRY(cudaMemsetAsync(n->f_wt.p, 0, n->f_wt.bytes, n->stream));
+    MLP_TRY(cudaMemcpyAsync(n->f_layers.p, n->layers_host.data(), sizeof(LayerGrad) * n->layers_host.size(),
+                            cudaMemcpyHostToDevice, n->stream));
+    copy_weights(n);
+    MLP_TRY(cudaGetLastError());
+    n->fused = true;
+    return GELIOS_OK;
 }
 }  // namespace
 
@@ -1312,12 +1462,18 @@ extern "C" int gelios_mlp_create(gelios_mlp** out, int device, int n_in, int n_f
          n->xin.alloc(MB * n_in * 4) && n->wt.alloc(W * pad8(widest) * 2) &&
          n->dzt.alloc(W * pad8(max_batch) * 2) && n->ht.alloc(W * pad8(max_batch) * 2);
     if (!ok) return cuda_fail(cudaErrorMemoryAllocation);
-    MLP_TRY(cudaMallocHost(&n->status_host, sizeof(int)));
+    // at most 16 MB of staging per chunk
+    n->stage_rows = std::min<int64_t>(max_batch, std::max<int64_t>(1024, (int64_t(4) << 20) / (n_in + n_out)));
+    const int64_t xf = pad8(n->stage_rows * n_in), yf = pad8(n->stage_rows * n_out);
+    float* pin = nullptr;
+    MLP_TRY(cudaMallocHost(&pin, static_cast<size_t>(16 + 2 * (xf + yf)) * 4));
+    n->status_host = reinterpret_cast<int*>(pin);
+    for (int k = 0; k < 2; k++) {
+        n->px[k] = pin + 16 + k * (xf + yf);
+        n->py[k] = n->px[k] + xf;
+        MLP_TRY(cudaEventCreateWithFlags(&n->ev_chunk[k], cudaEventDisableTiming));
+    }
     MLP_TRY(cudaMemsetAsync(n->wpad.p, 0, n->wpad.bytes, n->stream));
-    // W^T of the layers above the first, gradient partials and column sums,
-    // and what the fused training step needs beside them
-    int64_t part = 0, col = 0, wt = 0;
-    const int64_t chunks = (max_batch + kColRows - 1) / kColRows;
     for (int l = 0; l <= depth; l++) {
         LayerGrad g{};
         g.w_off = n->w_off[l];
@@ -1326,39 +1482,8 @@ extern "C" int gelios_mlp_create(gelios_mlp** out, int device, int n_in, int n_f
         g.dout = n->dout[l];
         g.ld_in = n->ld0;
         g.ld_t = static_cast<int>(pad8(g.dout));
-        g.part_off = part;
-        g.col_off = col;
-        part += static_cast<int64_t>(gelios_mlp::splits_of(max_batch)) * g.din * g.dout;
-        col += chunks * g.dout;
-        if (l > 0) wt += static_cast<int64_t>(g.din) * g.ld_t;
+        if (l == 0) g.wpad = n->wpad.as<__nv_bfloat16>();
         n->layers_host.push_back(g);
-    }
-    // the fused step: 16-byte rows for the TMA (width a multiple of 8), the
-    // output columns in mse_grad_kernel's tile, partials of at most 256 MB
-    CUtensorMap tz, th;
-    n->fused = width % 8 == 0 && n_out <= kMseCols && part <= (int64_t(64) << 20) &&
-               output_map(&tz, n->z[0].p, true, max_batch, width) && output_map(&th, n->h[1].p, false, max_batch, width);
-    if (n->fused) {
-        const size_t Mp = static_cast<size_t>(pad8(max_batch));
-        ok = n->f_ht.alloc(Mp * (n->in_w + static_cast<size_t>(depth) * width) * 2) &&
-             n->f_dzt.alloc(Mp * width * (static_cast<size_t>(depth) + 1) * 2 + Mp * kMseCols * 2) &&
-             n->f_wt.alloc(static_cast<size_t>(wt) * 2) && n->f_part.alloc(static_cast<size_t>(part) * 4) &&
-             n->f_col.alloc(static_cast<size_t>(col) * 4) && n->f_dzb2.alloc(MB * pad8(widest) * 2);
-        if (!ok) return cuda_fail(cudaErrorMemoryAllocation);
-        MLP_TRY(cudaMemsetAsync(n->f_wt.p, 0, n->f_wt.bytes, n->stream));
-        MLP_TRY(cudaStreamCreateWithFlags(&n->side, cudaStreamNonBlocking));
-        MLP_TRY(cudaEventCreateWithFlags(&n->ev_dz, cudaEventDisableTiming));
-        MLP_TRY(cudaEventCreateWithFlags(&n->ev_side, cudaEventDisableTiming));
-    }
-    int64_t wo = 0;
-    for (int l = 0; l <= depth; l++) {
-        LayerGrad& g = n->layers_host[l];
-        if (l == 0) {
-            g.wpad = n->wpad.as<__nv_bfloat16>();
-        } else if (n->fused) {
-            g.wt = n->f_wt.as<__nv_bfloat16>() + wo;
-            wo += static_cast<int64_t>(g.din) * g.ld_t;
-        }
     }
     if (!n->f_layers.alloc(sizeof(LayerGrad) * n->layers_host.size())) return cuda_fail(cudaErrorMemoryAllocation);
     MLP_TRY(cudaMemcpyAsync(n->f_layers.p, n->layers_host.data(), sizeof(LayerGrad) * n->layers_host.size(),
@@ -1388,10 +1513,7 @@ extern "C" int gelios_mlp_set_params(gelios_mlp* n, const float* host, int64_t c
     MLP_TRY(cudaMemcpyAsync(n->w32.p, host, P * 4, cudaMemcpyHostToDevice, n->stream));
     to_bf16_kernel<<<blocks(n->n_params, 256), 256, 0, n->stream>>>(n->n_params, n->w32.as<float>(),
                                                                     n->wb.as<__nv_bfloat16>());
-    int64_t most = 0;
-    for (int l = 0; l < n->layers(); l++) most = std::max(most, static_cast<int64_t>(n->din[l]) * n->dout[l]);
-    weight_copies_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(n->f_layers.as<LayerGrad>(),
-                                                                                      n->wb.as<__nv_bfloat16>());
+    copy_weights(n);
     MLP_TRY(cudaMemsetAsync(n->m.p, 0, P * 4, n->stream));
     MLP_TRY(cudaMemsetAsync(n->v.p, 0, P * 4, n->stream));
     MLP_TRY(cudaGetLastError());
@@ -1411,18 +1533,19 @@ extern "C" int gelios_mlp_get_params(const gelios_mlp* n, float* host, int64_t c
 extern "C" int gelios_mlp_loss_grad(gelios_mlp* n, const float* x, const float* t, int M, double* loss, float* grad) {
     if (!n || !x || !t || M < 1 || M > n->max_batch) return fail("gelios_mlp_loss_grad: bad arguments");
     MLP_TRY(cudaSetDevice(n->device));
+    if (const int rc = ensure_fused(n)) return rc;
     cudaStream_t s = n->stream;
     MLP_TRY(cudaMemcpyAsync(n->xin.p, x, static_cast<size_t>(M) * n->n_in * 4, cudaMemcpyHostToDevice, s));
     MLP_TRY(cudaMemcpyAsync(n->tb.p, t, static_cast<size_t>(M) * n->n_out * 4, cudaMemcpyHostToDevice, s));
-    features_kernel<<<blocks(M, 128), 128, 0, s>>>(M, n->n_in, n->nf, n->in_w, n->ld0, n->xin.as<float>(),
+    features_kernel<<<blocks(static_cast<int64_t>(M) * kRowThreads, 128), 128, 0, s>>>(M, n->n_in, n->nf, n->ld0, n->xin.as<float>(),
                                                    n->h[0].as<__nv_bfloat16>());
     forward(n, M, n->fused);
     if (n->fused) {
         transpose(M, n->in_w, n->h[0].as<__nv_bfloat16>(), n->ld0, n->ht_of(0), pad8(M), s);
-        if (!backward_fused(n, M, n->loss.as<float>())) return cuda_fail(cudaErrorInvalidValue);
-        reduce_fused(n, M, false, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
+        if (!backward_fused(n, M, n->loss.as<float>(), nullptr)) return cuda_fail(cudaErrorInvalidValue);
+        reduce_fused(n, M, nullptr, nullptr);
     } else {
-        backward(n, M);
+        backward(n, M, n->loss.as<float>(), nullptr);
     }
     MLP_TRY(cudaGetLastError());
     float l = 0.f;
@@ -1439,6 +1562,9 @@ extern "C" int gelios_mlp_loss_grad(gelios_mlp* n, const float* x, const float* 
 extern "C" int gelios_mlp_set_data(gelios_mlp* n, const float* x, const float* t, int64_t n_rows) {
     if (!n || !x || !t || n_rows < 1) return fail("gelios_mlp_set_data: bad arguments");
     MLP_TRY(cudaSetDevice(n->device));
+    n->drop_graph();  // it holds the training set's addresses and size
+    if (const int rc = ensure_fused(n)) return rc;
+    n->n_rows = 0;
     if (!n->X.alloc(static_cast<size_t>(n_rows) * n->n_in * 4) ||
         !n->T.alloc(static_cast<size_t>(n_rows) * n->n_out * 4))
         return cuda_fail(cudaErrorMemoryAllocation);
@@ -1456,44 +1582,56 @@ extern "C" int gelios_mlp_train(gelios_mlp* n, int iters, int batch, float lr_ma
     if (n->n_rows < 1) return fail("gelios_mlp_train: no training set (gelios_mlp_set_data)");
     MLP_TRY(cudaSetDevice(n->device));
     cudaStream_t s = n->stream;
-    Buf hist;
-    if (!hist.alloc(static_cast<size_t>(iters > 0 ? iters : 1) * 4)) return cuda_fail(cudaErrorMemoryAllocation);
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    if (iters > n->steps_cap) {
+        const int64_t cap = std::max<int64_t>(iters, 256);
+        n->drop_graph();
+        n->steps_cap = 0;
+        if (!n->args.alloc(static_cast<size_t>(cap) * sizeof(StepArgs)) ||
+            !n->hist.alloc(static_cast<size_t>(cap) * 4) || (!n->at.p && !n->at.alloc(sizeof(int))))
+            return cuda_fail(cudaErrorMemoryAllocation);
+        n->steps_cap = cap;
+    }
+    const float b1 = kAdamB1, b2 = kAdamB2;
+    std::vector<StepArgs> args(static_cast<size_t>(iters));
     for (int it = 0; it < iters; it++) {
-        const uint64_t key = seed * 0xD1B54A32D192ED03ULL + static_cast<uint64_t>(n->step) * 0x8CB92BA72F3D8DD7ULL;
-        gather_kernel<<<blocks(batch, 128), 128, 0, s>>>(
-            batch, n->n_rows, n->n_in, n->nf, n->in_w, n->ld0, n->n_out, n->X.as<float>(), n->T.as<float>(), key,
-            n->h[0].as<__nv_bfloat16>(), n->tb.as<float>(), n->fused ? n->ht_of(0) : nullptr, pad8(batch));
-        forward(n, batch, n->fused);
-        if (n->fused) {
-            if (!backward_fused(n, batch, hist.as<float>() + it)) return cuda_fail(cudaErrorInvalidValue);
-        } else {
-            backward(n, batch);
-            MLP_TRY(cudaMemcpyAsync(hist.as<float>() + it, n->loss.p, 4, cudaMemcpyDeviceToDevice, s));
-        }
-        float lr;
+        StepArgs& a = args[it];
+        a.key = seed * 0xD1B54A32D192ED03ULL + static_cast<uint64_t>(n->step) * 0x8CB92BA72F3D8DD7ULL;
         if (it < warmup) {
-            lr = lr_max * static_cast<float>(it + 1) / static_cast<float>(warmup);
+            a.lr = lr_max * static_cast<float>(it + 1) / static_cast<float>(warmup);
         } else {
             const double q = iters > warmup ? static_cast<double>(it - warmup) / (iters - warmup) : 1.0;
-            lr = static_cast<float>(lr_min + 0.5 * (lr_max - lr_min) * (1.0 + std::cos(3.14159265358979 * q)));
+            a.lr = static_cast<float>(lr_min + 0.5 * (lr_max - lr_min) * (1.0 + std::cos(3.14159265358979 * q)));
         }
         n->step++;
-        const float c1 = static_cast<float>(1.0 - std::pow(static_cast<double>(b1), n->step));
-        const float c2 = static_cast<float>(1.0 - std::pow(static_cast<double>(b2), n->step));
-        if (n->fused)
-            reduce_fused(n, batch, true, lr, b1, b2, eps, c1, c2);
-        else
+        a.c1 = static_cast<float>(1.0 - std::pow(static_cast<double>(b1), n->step));
+        a.c2 = static_cast<float>(1.0 - std::pow(static_cast<double>(b2), n->step));
+        a.pad = 0;
+    }
+    if (iters > 0) {
+        MLP_TRY(cudaMemcpyAsync(n->args.p, args.data(), sizeof(StepArgs) * args.size(), cudaMemcpyHostToDevice, s));
+        MLP_TRY(cudaMemsetAsync(n->at.p, 0, sizeof(int), s));
+    }
+    cudaGraphExec_t graph = n->fused && iters > 1 ? train_graph(n, batch) : nullptr;
+    for (int it = 0; it < iters; it++) {
+        if (graph) {
+            MLP_TRY(cudaGraphLaunch(graph, s));
+        } else if (n->fused) {
+            if (!enqueue_train_step(n, batch)) return cuda_fail(cudaErrorInvalidValue);
+        } else {
+            draw_batch(n, batch);
+            forward(n, batch);
+            backward(n, batch, n->hist.as<float>(), n->at.as<int>());
+            const StepArgs& a = args[it];
             adam_kernel<<<blocks(n->n_params, 256), 256, 0, s>>>(n->n_params, n->w32.as<float>(), n->g32.as<float>(),
-                                                                 n->m.as<float>(), n->v.as<float>(), lr, b1, b2, eps,
-                                                                 c1, c2, n->wb.as<__nv_bfloat16>());
-        if (!n->fused)
+                                                                 n->m.as<float>(), n->v.as<float>(), a.lr, b1, b2,
+                                                                 kAdamEps, a.c1, a.c2, n->wb.as<__nv_bfloat16>());
             weight_copies_kernel<<<dim3(blocks(static_cast<int64_t>(n->din[0]) * n->dout[0], 256), 1), 256, 0, s>>>(
                 n->f_layers.as<LayerGrad>(), n->wb.as<__nv_bfloat16>());
+        }
         MLP_TRY(cudaGetLastError());
     }
     if (loss_hist && iters > 0)
-        MLP_TRY(cudaMemcpyAsync(loss_hist, hist.p, static_cast<size_t>(iters) * 4, cudaMemcpyDeviceToHost, s));
+        MLP_TRY(cudaMemcpyAsync(loss_hist, n->hist.p, static_cast<size_t>(iters) * 4, cudaMemcpyDeviceToHost, s));
     gemm_status_fetch(n->status_host, s);
     MLP_TRY(cudaStreamSynchronize(s));
     if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
@@ -1504,20 +1642,33 @@ extern "C" int gelios_mlp_predict(gelios_mlp* n, const float* x, int64_t M, floa
     if (!n || !x || !y || M < 0) return fail("gelios_mlp_predict: bad arguments");
     MLP_TRY(cudaSetDevice(n->device));
     cudaStream_t s = n->stream;
-    for (int64_t r0 = 0; r0 < M; r0 += n->max_batch) {
-        const int m = static_cast<int>(M - r0 < n->max_batch ? M - r0 : n->max_batch);
-        MLP_TRY(cudaMemcpyAsync(n->xin.p, x + r0 * n->n_in, static_cast<size_t>(m) * n->n_in * 4,
-                                cudaMemcpyHostToDevice, s));
-        features_kernel<<<blocks(m, 128), 128, 0, s>>>(m, n->n_in, n->nf, n->in_w, n->ld0, n->xin.as<float>(),
-                                                       n->h[0].as<__nv_bfloat16>());
+    // the chunks pass through pinned staging, two at a time: a copy from or to
+    // pageable memory of this size goes through the driver's own, in turn
+    const int64_t mb = n->stage_rows;
+    auto rows = [&](int64_t k) { return std::min(mb, M - k * mb); };
+    auto collect = [&](int64_t k) {
+        const cudaError_t e = cudaEventSynchronize(n->ev_chunk[k & 1]);
+        if (e == cudaSuccess)
+            std::memcpy(y + k * mb * n->n_out, n->py[k & 1], static_cast<size_t>(rows(k)) * n->n_out * 4);
+        return e;
+    };
+    const int64_t chunks = (M + mb - 1) / mb;
+    for (int64_t k = 0; k < chunks; k++) {
+        const int b = static_cast<int>(k & 1), m = static_cast<int>(rows(k));
+        if (k >= 2) MLP_TRY(collect(k - 2));
+        const size_t xb = static_cast<size_t>(m) * n->n_in * 4;
+        std::memcpy(n->px[b], x + k * mb * n->n_in, xb);
+        MLP_TRY(cudaMemcpyAsync(n->xin.p, n->px[b], xb, cudaMemcpyHostToDevice, s));
+        features_kernel<<<blocks(static_cast<int64_t>(m) * kRowThreads, 128), 128, 0, s>>>(
+            m, n->n_in, n->nf, n->ld0, n->xin.as<float>(), n->h[0].as<__nv_bfloat16>());
         forward(n, m);
         MLP_TRY(cudaGetLastError());
-        MLP_TRY(cudaMemcpyAsync(y + r0 * n->n_out, n->y.p, static_cast<size_t>(m) * n->n_out * 4,
-                                cudaMemcpyDeviceToHost, s));
+        MLP_TRY(cudaMemcpyAsync(n->py[b], n->y.p, static_cast<size_t>(m) * n->n_out * 4, cudaMemcpyDeviceToHost, s));
+        if (k + 1 == chunks) gemm_status_fetch(n->status_host, s);
+        MLP_TRY(cudaEventRecord(n->ev_chunk[b], s));
     }
-    gemm_status_fetch(n->status_host, s);
-    MLP_TRY(cudaStreamSynchronize(s));
-    if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    for (int64_t k = std::max<int64_t>(0, chunks - 2); k < chunks; k++) MLP_TRY(collect(k));
+    if (chunks > 0 && *n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     return GELIOS_OK;
 }
 
