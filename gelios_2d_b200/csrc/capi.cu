@@ -1553,14 +1553,33 @@ int mk2_pipelined(gelios_ctx* ctx, int nsteps, double* cen0, double* cen1) {
                             [&]() { return enqueue_pipe_head(ctx, 0, b, true); });
     if (n < 0) return n;
     launches += n;
-    for (int st = 0; st < nsteps; st++) {
-        const bool last = st + 1 == nsteps;
-        const StepBuffers bn = last ? b : mk2_buffers(ctx, st + 1, cen0, cen1);
-        n = graph_or_direct(ctx, GELIOS_FORM_MK2, last ? 3 : 2, false, st & 1, b.cx,
-                            [&]() { return enqueue_pipe_step(ctx, st, b, last ? nullptr : &bn); });
+    // two bodies (an even and an odd step) are one graph: a graph launch costs
+    // the chain of a small grid about as much as a kernel of it
+    for (int st = 0; st < nsteps;) {
+        const int left = nsteps - st;
+        const StepBuffers b1 = mk2_buffers(ctx, st + 1, cen0, cen1);
+        if (left == 1) {
+            n = graph_or_direct(ctx, GELIOS_FORM_MK2, 3, false, st & 1, b.cx,
+                                [&]() { return enqueue_pipe_step(ctx, st, b, nullptr); });
+            st += 1;
+        } else if (left >= 3 && !(st & 1)) {
+            const StepBuffers b2 = mk2_buffers(ctx, st + 2, cen0, cen1);
+            n = graph_or_direct(ctx, GELIOS_FORM_MK2, 4, false, 0, b.cx, [&]() {
+                const int n0 = enqueue_pipe_step(ctx, st, b, &b1);
+                if (n0 < 0) return n0;
+                const int n1 = enqueue_pipe_step(ctx, st + 1, b1, &b2);
+                return n1 < 0 ? n1 : n0 + n1;
+            });
+            b = b2;
+            st += 2;
+        } else {
+            n = graph_or_direct(ctx, GELIOS_FORM_MK2, 2, false, st & 1, b.cx,
+                                [&]() { return enqueue_pipe_step(ctx, st, b, &b1); });
+            b = b1;
+            st += 1;
+        }
         if (n < 0) return n;
         launches += n;
-        b = bn;
     }
     return launches;
 }
