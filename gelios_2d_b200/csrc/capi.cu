@@ -152,7 +152,9 @@ struct gelios_ctx {
     // topology or the parameters change.
     struct StepGraph {
         int form = -1;
-        int kind = 0;   // 0: one whole step; 1-3: head / body / last part of a pipelined moving-grid call
+        // 0: one whole step; 1-3: head / body / last part of a pipelined
+        // moving-grid call; 4: two bodies (MK2 pipelined) or two whole steps
+        int kind = 0;
         int first = 0;  // the first step of a call: the graph starts with the words' initialisation
         int parity = -1;
         const void* cen = nullptr;
@@ -1721,6 +1723,27 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
     }
     for (int st = first; st < nsteps; st++) {
         const int cur = st & 1, nxt = cur ^ 1;
+        if (moving) {
+            // a step of a moving-grid form in one graph, two steps after the
+            // first in one (as in mk2_pipelined)
+            const StepBuffers b = mk2_buffers(ctx, st, cen0, cen1);
+            int n;
+            if (st > 0 && st + 1 < nsteps) {
+                const StepBuffers b1 = mk2_buffers(ctx, st + 1, cen0, cen1);
+                n = graph_or_direct(ctx, form, 4, false, cur, b.cx, [&]() {
+                    const int n0 = enqueue_form(ctx, b, form);
+                    if (n0 < 0) return n0;
+                    const int n1 = enqueue_form(ctx, b1, form);
+                    return n1 < 0 ? n1 : n0 + n1;
+                });
+                st++;
+            } else {
+                n = step_graph(ctx, b, form, st == 0);
+            }
+            if (n < 0) return n;
+            launches += n;
+            continue;
+        }
         StepBuffers b;
         for (int k = 0; k < 5; k++) {
             b.cur[k] = ctx->field(cur, k);
@@ -1731,57 +1754,7 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         b.dt_acc = ctx->acc();
         b.counters = ctx->counters();
         b.status = ctx->status();
-        if (mhd) {
-            // moving-grid step of the MHD form on the main stream:
-            // Move_surface + rails, face units, cell update, x = x2
-            double* cc = (st & 1) ? cen1 : cen0;
-            double* cn = (st & 1) ? cen0 : cen1;
-            b.cx = cc;
-            b.cy = cc + ncz;
-            b.rp = cc + 2 * ncz;
-            b.vs = cc + 3 * ncz;
-            b.vol = cc + 4 * ncz;
-            b.cx_next = cn;
-            b.cy_next = cn + ncz;
-            b.rp_next = cn + 2 * ncz;
-            b.vs_next = cn + 3 * ncz;
-            b.vol_next = cn + 4 * ncz;
-            const int n = step_graph(ctx, b, GELIOS_FORM_MHD_PUI, st == 0);
-            if (n < 0) return n;
-            launches += n;
-        } else if (form == GELIOS_FORM_MK2) {
-            double* cc = (st & 1) ? cen1 : cen0;
-            double* cn = (st & 1) ? cen0 : cen1;
-            b.cx = cc;
-            b.cy = cc + d.n_cells;
-            b.rp = cc + 2 * static_cast<size_t>(d.n_cells);
-            b.vs = cc + 3 * ncz;
-            b.vol = cc + 4 * ncz;
-            b.cx_next = cn;
-            b.cy_next = cn + d.n_cells;
-            b.rp_next = cn + 2 * static_cast<size_t>(d.n_cells);
-            b.vs_next = cn + 3 * ncz;
-            b.vol_next = cn + 4 * ncz;
-            const int n = step_graph(ctx, b, GELIOS_FORM_MK2, st == 0);
-            if (n < 0) return n;
-            launches += n;
-        } else if (form == GELIOS_FORM_5_KOMPONENT) {
-            double* cc = (st & 1) ? cen1 : cen0;
-            double* cn = (st & 1) ? cen0 : cen1;
-            b.cx = cc;
-            b.cy = cc + ncz;
-            b.rp = cc + 2 * ncz;
-            b.vs = cc + 3 * ncz;
-            b.vol = cc + 4 * ncz;
-            b.cx_next = cn;
-            b.cy_next = cn + ncz;
-            b.rp_next = cn + 2 * ncz;
-            b.vs_next = cn + 3 * ncz;
-            b.vol_next = cn + 4 * ncz;
-            const int n = step_graph(ctx, b, GELIOS_FORM_5_KOMPONENT, st == 0);
-            if (n < 0) return n;
-            launches += n;
-        } else {
+        {
             b.cx = cen0;
             b.cy = cen0 + d.n_cells;
             b.rp = cen0 + 2 * static_cast<size_t>(d.n_cells);
