@@ -3584,10 +3584,10 @@ __device__ __forceinline__ void k5_boundary(const gelios_params& P, const K5Rows
 // Holding all 21 fields of four cells at once took 255 registers and spilled,
 // in one launch of every kind of unit: 223 us on the 200k grid (401k units,
 // ncu).  One fluid at a time in a launch per group: 73 us for the plain units
-// at 96 registers (21, 31, 20 us for the C_1, tracked and one-sided ones
-// beside them); 80 or 128 registers, or the fluids unrolled: 1-5% slower per
+// at 96 registers (21, 30, 19 us for the C_1, tracked and one-sided ones
+// beside them, 35 for the tracked before a lane took a fluid); 80 or 128 registers, or the fluids unrolled: 1-5% slower per
 // step.  Bound by the latency of its loads and FP64 chains.
-// COOP: all lanes of a warp evaluate one tracked unit; lane 0 stores.
+// COOP: a warp evaluates one tracked unit, a lane per fluid.
 template <int GROUP, bool COOP>
 __device__ __forceinline__ double k5_face_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
                                                const double* __restrict__ hcur, double* __restrict__ fl, int u,
@@ -3636,10 +3636,9 @@ __device__ __forceinline__ double k5_face_body(const DevMesh& d, const gelios_pa
     }
     const K5Rows rows{b.cur, hcur, static_cast<size_t>(d.n_cells)};
     double um = 0.0, um1 = 0.0;  // largest wave speed without H1, of H1
-#pragma unroll 1
-    for (int f = 0; f < 5; f++) {
+    // fluid f: the two states, the HLLC flux and its wave speed; the flux row
+    auto flux = [&](int f, St5& L, St5& R, double (&F)[5]) {
         const St5 own = rows.load(f, K);
-        St5 L, R;
         if (USUALY || ft == G_USUALY) {
             const St5 oth = rows.load(f, nb);
             constexpr int G = COOP ? kAnyGroup : GROUP;
@@ -3648,27 +3647,55 @@ __device__ __forceinline__ double k5_face_body(const DevMesh& d, const gelios_pa
         } else {
             k5_boundary(P, rows, sK, ft, x2, y2, f, own, L, R);
         }
+        return hllc_lean<double, true, true>(P.gamma, L, R, W, n1, n2, f == 0 && (info & SI_NP), F);
+    };
+    auto store = [&](int f, const double* F) {
+        double* o = fl + (f == 0 ? 0 : 1 + 4 * f) * nu + u;
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k * nu] = F[k] * S;
+        if (f == 0) o[4 * nu] = F[4] * S;
+    };
+    if constexpr (COOP) {
+        // a lane per fluid (the lanes above 4 repeat H4), then the exact
+        // solution of the plasma's states by the whole warp
+        const unsigned full = 0xffffffffu;
+        const int lane = threadIdx.x & 31, f = lane < 4 ? lane : 4;
+        St5 L, R;
         double F[5];
-        double UU = hllc_lean<double, true, true>(P.gamma, L, R, W, n1, n2, f == 0 && (info & SI_NP), F);
-        if (COOP && f == 0) {
-            double q1[5] = {L.ro, L.p, L.u, L.v, 0.0}, q2[5] = {R.ro, R.p, R.u, R.v, 0.0};
-            double nv[3] = {n1, n2, 0.0}, qq[5], ds[3];
-            const double UG = godunov_dev<true>(P.gamma, P.kurant, q1, q2, nv, qq, ds, W, 1.0, P.godunov_max_iter,
-                                                &status);
+        const double UU = flux(f, L, R, F);
+        __syncwarp();
+        double q1[5] = {L.ro, L.p, L.u, L.v, 0.0}, q2[5] = {R.ro, R.p, R.u, R.v, 0.0};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            q1[k] = __shfl_sync(full, q1[k], 0);
+            q2[k] = __shfl_sync(full, q2[k], 0);
+        }
+        double nv[3] = {n1, n2, 0.0}, qq[5], ds[3];
+        um = godunov_dev<true>(P.gamma, P.kurant, q1, q2, nv, qq, ds, W, 1.0, P.godunov_max_iter, &status);
+        um = um > 0.0 ? um : 0.0;
+        if (f == 0) {
             F[0] = qq[0];
             F[1] = qq[1];
             F[2] = qq[2];
             F[3] = qq[4];
-            um = UG > um ? UG : um;
         }
-        if (!COOP || (threadIdx.x & 31) == 0) {
-            double* o = fl + (f == 0 ? 0 : 1 + 4 * f) * nu + u;
+        if (lane < 5) store(f, F);
 #pragma unroll
-            for (int k = 0; k < 4; k++) o[k * nu] = F[k] * S;
-            if (f == 0) o[4 * nu] = F[4] * S;
+        for (int j = 0; j < 5; j++) {
+            const double w = __shfl_sync(full, UU, j);
+            if (j == 1) um1 = w > um1 ? w : um1;
+            else um = w > um ? w : um;
         }
-        if (f == 1) um1 = UU > um1 ? UU : um1;
-        else um = UU > um ? UU : um;
+    } else {
+#pragma unroll 1
+        for (int f = 0; f < 5; f++) {
+            St5 L, R;
+            double F[5];
+            const double UU = flux(f, L, R, F);
+            store(f, F);
+            if (f == 1) um1 = UU > um1 ? UU : um1;
+            else um = UU > um ? UU : um;
+        }
     }
     const double ua = um1 > um ? um1 : um;
     double t = inf;
@@ -3689,9 +3716,12 @@ __global__ void __launch_bounds__(128, MINB) k5_face_kernel(DevMesh d, gelios_pa
     }
     block_reduce_commit(t, 0, 0, status, b.dt_acc, b.counters, b.status);
 }
-// The tracked units, one warp each: the exact solver's bisection runs
-// warp-cooperatively (one thread per unit holds up its block for 30
-// iterations in a row).
+// The tracked units, one warp each: the five fluids in five lanes, then the
+// exact solver's bisection warp-cooperatively (one thread per unit holds up
+// its block for 30 iterations in a row).  With the fluids one after another in
+// every lane the 1150 units of the 200k grid took as many issue slots of the
+// FP64 pipes, which the face kernels share, as a fifth of the 328k plain ones.
+// 20 steps of that grid: 5870 -> 5603 us.
 __global__ void __launch_bounds__(64) k5_tracked_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                         const double* __restrict__ hcur, double* __restrict__ fl) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
