@@ -107,7 +107,7 @@ struct gelios_ctx {
     DBuf X, Y, X2, Y2, ptype, cstart, contour, gstart, cflags, ctype, sA, sB, snb, ssd, ssd2, sinfo, qcorner;
     DBuf fA, fB, ftype, fmaster, fsosed, fcopy, fsdown;
     DBuf rtype, rM, rpstart, rpts, rkstart, rkeys, rs;
-    DBuf lc, li, lo, sp_point, sp_line, sp_inc, sp_ainc, sp_fix, sp_of_point, rk_point, rk_node, sf_rec, rail_tab;
+    DBuf sp_point, sp_line, sp_inc, sp_ainc, sp_fix, sp_of_point, rk_point, rk_node, sf_rec, rail_tab;
     bool rail_tab_valid = false;  // launch_rail_table; stale once the topology or the parameters change
     DBuf u_slot, u_cell, u_twin, u_A, u_B, u_info, u_nb, u_sd, u_sd2, s_unit, flux, aux, rec, pstar, src_lo;
     DBuf Hn, Hu, Hv, HT, ku, kv, kT, r_istoch, cback, cnext;
@@ -118,7 +118,7 @@ struct gelios_ctx {
     DBuf hstate[2];
     gelios_mhd_params mprm{};
     DBuf src_fixed;  // MHD form: fixed charge-exchange sources (3 rows)
-    DBuf flux_mhd;   // multi-fluid forms: 13 (MHD) or 21 (Go_5_komponent) flux rows per face slot, on first use
+    DBuf flux_mhd;   // multi-fluid forms: 13 (MHD) or 21 (Go_5_komponent) flux rows per face unit, on first use
     int mhd_face_variant = kMhdFaceDefault;  // launch shape of the MHD face kernel (gelios_autotune)
     int mk2_variant = 0;  // arrangement / launch shape of the moving-grid face units + update (gelios_autotune)
     // tiles of the moving-grid step (see TileView)
@@ -803,9 +803,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
         rc |= upload(ctx->rkeys, v->rail_keys, v->rail_kstart[nr], s);
         rc |= upload(ctx->rs, v->rail_s, nr, s);
     }
-    rc |= upload(ctx->lc, v->line_contact, v->n_contact, s);
-    rc |= upload(ctx->li, v->line_inner, v->n_inner_line, s);
-    rc |= upload(ctx->lo, v->line_outer, v->n_outer_line, s);
     rc |= upload(ctx->u_slot, u_slot.data(), u_slot.size(), s);
     {
         // unit-major copies of what a unit reads about its face and cells:
@@ -1001,9 +998,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     d.n_rail_b = nb;
     d.n_rail_c = ncr;
     d.n_rail_d = nd;
-    d.lc = ctx->lc.as<int32_t>();
-    d.li = ctx->li.as<int32_t>();
-    d.lo = ctx->lo.as<int32_t>();
     d.n_lc = v->n_contact;
     d.n_li = v->n_inner_line;
     d.n_lo = v->n_outer_line;
@@ -2618,15 +2612,16 @@ extern "C" int gelios_hlld_batch(const gelios_params* prm, int n, const double* 
 
 // ------------------------------------------------------------------ plain-form batch
 // Instances of the Go_stationary form that share one mesh, advanced together
-// by one cooperative launch per chunk of steps (the converged states of an
+// chunk of steps by chunk of steps (the converged states of an
 // inflow-parameter sweep).  Each instance keeps its own context: state,
-// parameters, flux slots and dt words.
+// parameters, flux rows and dt words.
 struct gelios_plain_batch {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::vector<gelios_ctx*> ctxs;
     DBuf inst, active, resid;
-    int prec = GELIOS_PREC_FP64;  // flux precision of every instance
+    std::vector<PlainInstance> host;  // what inst holds, rebuilt per call
+    int prec = GELIOS_PREC_FP64;      // flux precision of every instance
     ~gelios_plain_batch() {
         if (stream) cudaStreamDestroy(stream);
     }
@@ -2688,7 +2683,8 @@ namespace {
 // instances; the contexts' streams are drained first so their earlier work
 // is ordered before the batch's.
 int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
-    std::vector<PlainInstance> host(B->ctxs.size());
+    std::vector<PlainInstance>& host = B->host;
+    host.resize(B->ctxs.size());
     for (size_t i = 0; i < B->ctxs.size(); i++) {
         gelios_ctx* c = B->ctxs[i];
         if (c->prm.precision != B->prec) {
@@ -2742,6 +2738,24 @@ int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
     GELIOS_CUDA_TRY(cudaGetLastError());
     return GELIOS_OK;
 }
+// `nsteps` steps of the listed instances: a cluster of at most 16 SMs each,
+// all at once, or, of a few instances of a large mesh, one instance after the
+// other on the whole chip (plain_batch_serial).
+cudaError_t plain_batch_steps(gelios_plain_batch* B, const std::vector<int>& list, int nsteps) {
+    const DevMesh& d = B->ctxs[0]->d;
+    const int n = static_cast<int>(list.size());
+    if (nsteps > 0 && B->prec != GELIOS_PREC_FP32_FLUX && plain_batch_serial(d.n_cells, n)) {
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < n && e == cudaSuccess; k++) {
+            const PlainInstance& I = B->host[list[k]];
+            e = launch_stationary_persistent(d, I.P, I.b[0], I.b[1], I.fl, nsteps, B->stream);
+            if (e != cudaSuccess && k > 0) return e;
+        }
+        if (e == cudaSuccess) return e;
+        cudaGetLastError();  // no cooperative launch: the clusters
+    }
+    return launch_stationary_batch(d, B->inst.as<PlainInstance>(), B->active.as<int>(), n, nsteps, B->prec, B->stream);
+}
 }  // namespace
 
 extern "C" int gelios_plain_batch_step(gelios_plain_batch* B, int nsteps, gelios_status* statuses) {
@@ -2752,8 +2766,7 @@ extern "C" int gelios_plain_batch_step(gelios_plain_batch* B, int nsteps, gelios
     for (int i = 0; i < n; i++) list[i] = i;
     int rc = plain_batch_prepare(B, list);
     if (rc) return rc;
-    GELIOS_CUDA_TRY(launch_stationary_batch(B->ctxs[0]->d, B->inst.as<PlainInstance>(), B->active.as<int>(), n, nsteps,
-                                            B->prec, B->stream));
+    GELIOS_CUDA_TRY(plain_batch_steps(B, list, nsteps));
     GELIOS_CUDA_TRY(cudaStreamSynchronize(B->stream));
     for (int i = 0; i < n; i++) {
         gelios_ctx* c = B->ctxs[i];
@@ -2795,8 +2808,7 @@ extern "C" int gelios_plain_batch_run_to_residual(gelios_plain_batch* B, double 
         if (chunk <= 0) break;
         int rc = plain_batch_prepare(B, list);
         if (rc) return rc;
-        GELIOS_CUDA_TRY(launch_stationary_batch(B->ctxs[0]->d, B->inst.as<PlainInstance>(), B->active.as<int>(),
-                                                static_cast<int>(list.size()), chunk, B->prec, B->stream));
+        GELIOS_CUDA_TRY(plain_batch_steps(B, list, chunk));
         double* sums = B->resid.as<double>() + static_cast<size_t>(kResidualScratch) * n;
         launch_residual_batch(B->inst.as<PlainInstance>(), B->active.as<int>(), static_cast<int>(list.size()),
                               B->ctxs[0]->d.n_cells, B->resid.as<double>(), sums, B->stream);

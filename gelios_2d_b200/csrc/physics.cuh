@@ -45,8 +45,6 @@ struct St5 {
 
 __device__ __forceinline__ double dmin_ref(double a, double b) { return (b < a) ? b : a; }  // std::min
 __device__ __forceinline__ double dmax_ref(double a, double b) { return (a < b) ? b : a; }  // std::max
-__device__ __forceinline__ float fmin_ref(float a, float b) { return (b < a) ? b : a; }
-__device__ __forceinline__ float fmax_ref(float a, float b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double sq(double x) { return x * x; }
 
 // sign / minmod / linear: Help.cpp:67-120
@@ -66,10 +64,6 @@ __device__ __forceinline__ double linear3(double x1, double t1, double x2, doubl
 __device__ __forceinline__ double linear3r(double t1, double t2, double t3, double r12, double r23, double x2) {
     const double d = minmod((t1 - t2) * r12, (t2 - t3) * r23);
     return d * (0.0 - x2) + t2;
-}
-__device__ __forceinline__ double linear2(double x1, double t1, double x2, double t2, double y) {
-    const double d = (t1 - t2) / (x1 - x2);
-    return (d * (y - x2) + t2);
 }
 
 // cos/sin of polar_angle(x, y) (Help.cpp:37-65).  The reference takes atan of

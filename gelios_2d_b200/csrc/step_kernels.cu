@@ -1,7 +1,7 @@
 // sm_100a kernels of the Gelios_2D plasma time step.
 //
 // One time step of Setka::Go_5_komponent__MK2 (Setka.cpp:10121-10482) is,
-// on two streams:
+// on several streams:
 //   mk2_recon_tracked_kernel  TVD states of the tracked face units (pre-motion)
 //   mk2_tracked_solve_kernel  star pressures of the tracked faces' exact
 //                             Riemann problems (warp per face)
@@ -17,20 +17,26 @@
 //                             one CTA per rail
 //   mk2_flux_tracked_kernel   tracked faces: HLL + the Riemann solution
 //                             sampled at the moved face speed
-//   mk2_tile_kernel           one tile of cells per block: reconstruction and
-//                             HLL flux of every other face unit touching the
-//                             tile (face speed from the moved points), slot
-//                             fluxes in shared memory, then the per-cell sums
-//                             in Grans order, the conservative ALE update,
-//                             the next step's geometry cache, CFL block-min
-//   commit_kernel             x = x2; dt of the next step
-// Go_stationary (Setka.cpp:5205-5343) and
-// Go_stationary_5_komponent_inner_MK2 (Setka.cpp:6999-7212) are
-// stationary_cell_kernel / inner_cell_kernel + dt_finalize_kernel.
+//   mk2_face_kernel           reconstruction and HLL flux of the plain interior
+//                             face units (face speed from the moved points),
+//                             F.S once per unit; CFL block-min
+//   mk2_face_rest_kernel      the C_1 interior and the one-sided units
+//   mk2_update_kernel         a cell's fluxes summed in Grans order, the
+//                             conservative ALE update, the next step's
+//                             geometry cache
+//   commit_kernel             x = x2; dt of the next step (the last step of a
+//                             call; within one the surface kernel finalises dt)
+// (mk2_tile_kernel, one tile of cells per block with the fluxes in shared
+// memory, is the other arrangement of the last four.)
+// Go_stationary (Setka.cpp:5205-5343) is stationary_lanes_kernel (four lanes
+// per cell, every step of a call) or, where that does not take the grid,
+// stationary_persistent_kernel; Go_stationary_5_komponent_inner_MK2
+// (Setka.cpp:6999-7212) is inner_table_kernel + inner_lanes_kernel, or
+// inner_cell_kernel + dt_finalize_kernel.
 //
-// Owner-computes: a thread owns a cell and sums its faces in the reference's
-// Grans order, so no floating-point atomics are needed and results are
-// deterministic run to run.  The CFL minimum is exact under any order
+// A cell's faces are summed by one thread or one group of lanes in the
+// reference's Grans order, so no floating-point atomics are needed and results
+// are deterministic run to run.  The CFL minimum is exact under any order
 // (atomicMin on the bit pattern of non-negative doubles).
 #include <cuda_runtime.h>
 
@@ -691,8 +697,9 @@ __global__ void centroid_kernel(DevMesh d, const double* __restrict__ X, const d
 // evaluated once for both sides: the reference evaluates it from each side
 // and the two results are the negatives of each other up to rounding,
 // Setka.cpp:10195-10380) or a one-sided face (boundary types, evaluated for
-// its owner only).  Each unit writes F*S into the per-slot flux buffer of the
-// owner slot (and -F*S into the twin's slot of the neighbour), and folds the
+// its owner only).  Each unit writes F*S once, into its own flux row, as the
+// owner sees it (the neighbour's sum subtracts it; the plain form's FP32-flux
+// kernels keep a row per slot and write -F*S into the twin's), and folds the
 // CFL candidates of the sides whose cell is updated this step into the dt
 // word.  The cell kernels then sum their slots in Grans order.
 
@@ -1857,30 +1864,26 @@ __global__ void __launch_bounds__(32) mk2_flux_tracked_kernel(DevMesh d, gelios_
     block_reduce_commit(tmin_u, 0, 0, status, b.dt_acc, b.counters, b.status);
 }
 
-// Every other face unit after the motion, reconstruction and flux in one
-// pass: the reconstructed states stay in registers (no per-unit scratch);
-// F.S to the owner's flux slot and -F.S to the twin's.  Index i is remapped
-// around the tracked range [u_tr0, u_tr1).
-// One launch per unit group (compiled without the branches the group cannot
-// take): kPlainGroup [0, u_c1), kC1Group [u_c1, u_tr0), kAnyGroup the
-// one-sided units [u_tr1, n_units).
+// The plain interior face units [0, u_c1) after the motion, reconstruction and
+// flux in one pass: the reconstructed states stay in registers (no per-unit
+// scratch); F.S once per unit, as its owner sees it.  Compiled without the
+// branches that the C_1 and the one-sided units take (mk2_face_rest_kernel).
 // PF: every gathered address of the unit is prefetched into L1 as soon as
 // the unit's indices are in (mk2_prefetch_unit), so that the loads of the
 // reconstruction's later levels hit L1 instead of waiting for L2 / DRAM one
 // level at a time; the arithmetic is the same code.
-template <typename TF, int MINB, int GROUP, bool PF = false>
+template <typename TF, int MINB, bool PF>
 __global__ void __launch_bounds__(128, MINB) mk2_face_kernel(DevMesh d, gelios_params P, StepBuffers b,
                                                            double* __restrict__ fl, int n_launch) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
     double tmin_u = __longlong_as_double(0x7ff0000000000000LL);
     int status = 0;
-    if (i < n_launch) {
-        const int u = GROUP == kPlainGroup ? i : GROUP == kC1Group ? d.u_c1 + i : d.u_tr1 + i;
-        if (PF) mk2_prefetch_unit<GROUP != kPlainGroup>(d, b, u);
+    if (u < n_launch) {
+        if (PF) mk2_prefetch_unit<false>(d, b, u);
         RecUnit r;
         r.a = St5{};
         r.o = St5{};
-        mk2_recon_unit<GROUP>(d, P, b, u, r, &status);
+        mk2_recon_unit<kPlainGroup>(d, P, b, u, r, &status);
         mk2_flux_unit<TF, false>(d, P, b, u, r, fl, nullptr, tmin_u, &status);
     }
     block_reduce_commit(tmin_u, 0, 0, status, b.dt_acc, b.counters, b.status);
@@ -2253,12 +2256,12 @@ __global__ void __launch_bounds__(NT, MINB) mk2_tile_kernel(DevMesh d, gelios_pa
     block_reduce_commit(tmin, nro, npc, status, b.dt_acc, b.counters, b.status);
 }
 
-// The cell update alone, from the flux slots in global memory (the update
+// The cell update alone, from the units' flux rows in global memory (the update
 // phase of the tile kernel for the face-kernel arrangement).
 // MODE kUpdAll: every cell, the 1e7 start of the CFL minimum folded into the
 // accumulator (the reference's `time`, Setka.cpp:10141) when a cell takes
 // part.  The pipelined step leaves that to its dt finalisation
-// (dt_finalize_cap_kernel, commit with cap) and updates in two parts:
+// (in the surface kernel, commit with cap) and updates in two parts:
 // kUpdEarly the listed cells (CF_EARLY), kUpdRest every other cell;
 // kUpdAllNoMark every cell (its last step).
 enum : int { kUpdAll = 0, kUpdEarly = 1, kUpdRest = 2, kUpdAllNoMark = 3 };
@@ -2723,7 +2726,6 @@ __device__ __forceinline__ void dt_finalize_cap(const StepBuffers& b) {
     *b.dt_next = t;
     *b.dt_acc = 0x7ff0000000000000ULL;
 }
-__global__ void dt_finalize_cap_kernel(StepBuffers b) { dt_finalize_cap(b); }
 
 // x = x2, y = y2 (Setka.cpp:10473-10480; the zeroed V and count are never
 // stored, see point_velocity) + dt finalisation (CAP: dt_finalize_cap).
@@ -3980,7 +3982,7 @@ __global__ void __launch_bounds__(128, 6) k5_update_kernel(DevMesh d, gelios_par
 // surface tracking and the rails run on them unchanged; the extra rows hold
 // the ion's w (u_phi) and B (x, y, phi) and the pickup protons' ro, p, u, v.
 enum : int { kXw = 0, kXbx, kXby, kXbz, kXro, kXp, kXu, kXv, kMhdExtra };
-constexpr int kMhdFlux = 13;  // per slot: ion mass, mom x, y, phi, energy, Bx, By, Bphi, Q; pickup mass, mom x, y, energy
+constexpr int kMhdFlux = 13;  // per unit: ion mass, mom x, y, phi, energy, Bx, By, Bphi, Q; pickup mass, mom x, y, energy
 
 struct Ext8 {
     double f[kMhdExtra];
@@ -4873,7 +4875,7 @@ __global__ void plain_batch_words_init_kernel(const PlainInstance* inst, const i
     double* T = const_cast<double*>(I.b[0].dt_cur);  // T[0]; b[1].dt_cur is T[1]
     T[0] = I.P.dt0;
     T[1] = I.P.dt0;
-    *I.b[0].dt_acc = 0x7ff0000000000000ULL;
+    for (int a = 0; a < 3; a++) *plain_acc(I.b[0].dt_acc, a) = 0x7ff0000000000000ULL;
     I.b[0].counters[0] = 0;
     I.b[0].counters[1] = 0;
     *I.b[0].status = 0;
@@ -4908,14 +4910,14 @@ static void launch_faces_v(const DevMesh& d, const gelios_params& P, const StepB
                            cudaStream_t s) {
     // the plain interior group in the variant's shape
     const int n0 = d.u_c1;
-    if (n0 > 0) mk2_face_kernel<TF, MINB, kPlainGroup><<<blocks_for(n0, 128), 128, 0, s>>>(d, P, b, fl, n0);
+    if (n0 > 0) mk2_face_kernel<TF, MINB, false><<<blocks_for(n0, 128), 128, 0, s>>>(d, P, b, fl, n0);
 }
 // the plain interior group with the unit's gathers prefetched into L1
 template <typename TF, int MINB>
 static void launch_faces_pf(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* fl,
                             cudaStream_t s) {
     const int n0 = d.u_c1;
-    if (n0 > 0) mk2_face_kernel<TF, MINB, kPlainGroup, true><<<blocks_for(n0, 128), 128, 0, s>>>(d, P, b, fl, n0);
+    if (n0 > 0) mk2_face_kernel<TF, MINB, true><<<blocks_for(n0, 128), 128, 0, s>>>(d, P, b, fl, n0);
 }
 // the C_1 interior and one-sided groups, each in an instance compiled for it
 template <typename TF, bool PF>
@@ -5038,7 +5040,6 @@ void launch_commit(const DevMesh& d, const StepBuffers& b, cudaStream_t s, bool 
     else
         commit_kernel<false><<<blocks_for(d.n_points > 0 ? d.n_points : 1, 256), 256, 0, s>>>(d, b);
 }
-void launch_dt_finalize_cap(const StepBuffers& b, cudaStream_t s) { dt_finalize_cap_kernel<<<1, 1, 0, s>>>(b); }
 void launch_mk2_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
                        const double* aux, cudaStream_t s, int mode, const int32_t* list, int n_list) {
     if (mode == kUpdEarly) {
@@ -5207,7 +5208,11 @@ void launch_residual_batch(const PlainInstance* inst, const int* active, int n_a
     int nb = blocks_for(n_cells, 256);
     if (nb > 296) nb = 296;
     if (nb < 1) nb = 1;
-    residual_batch_partial_kernel<<<dim3(nb, n_active), 256, 0, s>>>(inst, active, n_cells, part);
+    for (int i = 0; i < n_active; i += 65535) {  // a grid's y extent
+        const int k = n_active - i < 65535 ? n_active - i : 65535;
+        residual_batch_partial_kernel<<<dim3(nb, k), 256, 0, s>>>(inst, active + i, n_cells,
+                                                                  part + static_cast<size_t>(kResidualScratch) * i);
+    }
     residual_batch_final_kernel<<<n_active, 1, 0, s>>>(inst, active, nb, part, out);
 }
 void launch_words_init(void* words, double dt0, cudaStream_t s) {

@@ -56,7 +56,6 @@ struct DevMesh {
                   *rkeys = nullptr;
     const double* rs = nullptr;
     int n_rail_a = 0, n_rail_b = 0, n_rail_c = 0, n_rail_d = 0;
-    const int32_t *lc = nullptr, *li = nullptr, *lo = nullptr;
     int n_lc = 0, n_li = 0, n_lo = 0;
     // surface-tracking nodes (points of the three tracked lines): point id,
     // line (0 contact, 1 inner, 2 outer), up to 4 face incidences (j << 1 |
@@ -151,14 +150,23 @@ void launch_stationary_update(const DevMesh& d, const gelios_params& P, const St
 cudaError_t launch_stationary_persistent(const DevMesh& d, const gelios_params& P, const StepBuffers& b0,
                                          const StepBuffers& b1, double* fl, int nsteps, cudaStream_t s);
 // Instances of the plain form that share one mesh: parameters, the buffers
-// of even / odd steps (dt words included) and the flux slots of each.
+// of even / odd steps (dt words included) and the flux rows of each.
 struct PlainInstance {
     gelios_params P;
     StepBuffers b[2];
     double* fl;
 };
+// A batch of n instances takes them one after the other, each on the whole
+// chip (launch_stationary_persistent), instead of a cluster per instance:
+// a cluster is at most 16 SMs.  us of 40 / 100 / 20 steps, one after the other
+// against clusters: 180x120 cells, 1, 2, 8 instances 279 / 1670, 487 / 1681,
+// 1725 / 2301; 120x90, 4: 1650 / 2342; 90x60, 1, 2: 422 / 1468, 776 / 1488;
+// 360x240, 1, 4, 20: 537 / 2840, 1887 / 3817, 9052 / 9063.  A step of a mesh
+// that the lanes hold takes 4-5 us on the whole chip, a cluster's about
+// 5.5 us + 1.7 ns per cell: the line lies where n of the one make the other.
+inline bool plain_batch_serial(int n_cells, int n) { return 3000 * static_cast<int64_t>(n) <= n_cells + 3000LL; }
 // `nsteps` steps of the instances listed in `active` (device arrays) in one
-// cooperative launch; returns the launch's error code.
+// launch; returns the launch's error code.
 cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst, const int* active, int n_active,
                                     int nsteps, int prec, cudaStream_t s);
 void launch_plain_batch_words_init(const PlainInstance* inst, const int* active, int n, cudaStream_t s);
@@ -183,10 +191,10 @@ struct TileView {
 // (rec: kRecRows x n_tracked); after it, every other face unit and the cell
 // update in one of two arrangements, kMk2Variants launch shapes in all:
 //   variants 0-3  mk2_face_kernel (reconstruction and flux in registers, F.S
-//                 to the flux slots in global memory; 128 threads x 8, 5, 6,
-//                 4 resident blocks; the plain interior group in its own
-//                 launch of a lean instance) + mk2_update_kernel (slot sums,
-//                 update);
+//                 to the units' flux rows in global memory; 128 threads x 8,
+//                 5, 6, 4 resident blocks; the C_1 interior and the one-sided
+//                 units in mk2_face_rest_kernel) + mk2_update_kernel (a cell's
+//                 sums, update);
 //   variants 4-7  mk2_tile_kernel, one tile of cells per block, slot fluxes
 //                 in shared memory (256 x 3, 256 x 2, 128 x 5, 128 x 4);
 //   variants 8-10 as 0-3 with every gather of a face unit prefetched into
@@ -236,9 +244,6 @@ cudaError_t launch_inner_lanes(const DevMesh& d, const gelios_params& P, const S
                                const int32_t* list, int n, double* tab, int nsteps, cudaStream_t s);
 void launch_dt_finalize(const StepBuffers& b, cudaStream_t s);
 void launch_commit(const DevMesh& d, const StepBuffers& b, cudaStream_t s, bool cap = false);
-// dt of the next step from the CFL accumulator when the update did not fold
-// the 1e7 start in (the pipelined moving-grid step); re-arms the accumulator
-void launch_dt_finalize_cap(const StepBuffers& b, cudaStream_t s);
 // the moving-grid cell update: mode 0 every cell (1e7 start of the CFL
 // minimum folded in), 1 the listed cells, 2 every cell not flagged CF_EARLY,
 // 3 every cell (modes 1-3 fold nothing into the CFL accumulator)
@@ -263,7 +268,7 @@ int launch_k5_faces(const DevMesh& d, const gelios_params& P, const StepBuffers&
 void launch_k5_update(const DevMesh& d, const gelios_params& P, const StepBuffers& b, const double* fl,
                       const double* hcur, double* hnxt, cudaStream_t s);
 // MHD + pickup-proton form: extra rows (8 x n_cells: w, Bx, By, Bz, pickup
-// ro, p, u, v), 13 flux rows per slot, fixed sources (3 x n_cells).
+// ro, p, u, v), 13 flux rows per unit, fixed sources (3 x n_cells).
 constexpr int kMhdFluxRows = 13;
 // The face kernel has kMhdFaceVariants launch shapes (threads per block x
 // minimum blocks per SM); kMhdFaceDefault is the default, gelios_autotune picks
@@ -289,7 +294,7 @@ struct alignas(16) BatchInstance {
     StepBuffers b[2];          // buffers of the even / odd steps of a call
     const double* hs[2];       // extra rows read by the even / odd steps
     double* hn[2];             // extra rows written by them
-    double* fl;                // 13 flux rows per face slot
+    double* fl;                // 13 flux rows per face unit
     const double* src;         // fixed charge-exchange sources
     double* surface;           // Move_surface scratch
 };

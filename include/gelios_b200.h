@@ -401,7 +401,7 @@ int gelios_mlp_time_layer(int M, int N, int K, int reps, int tma, double *ms);
  * gelios_variant_count(form) launch shapes (threads per block x resident
  * blocks per SM, i.e. a register cap); the moving-grid form
  * (GELIOS_FORM_MK2) has as many variants of its face units + cell update:
- * a face kernel writing flux slots in global memory followed by an update
+ * a face kernel writing flux rows in global memory followed by an update
  * kernel (variants 0-3; 8-10 the same with every gather of a face unit
  * prefetched into L1), or one kernel per tile of cells with the slots in
  * shared memory (4-7, slower in the whole step; gelios_autotune for this
@@ -411,8 +411,9 @@ int gelios_mlp_time_layer(int M, int N, int K, int reps, int tma, double *ms);
  * buffers are written, the state and the points are not touched), keeps the
  * fastest for the steps that follow and returns its index and mean time in
  * ms (either pointer may be NULL).  gelios_set_variant picks a shape by
- * hand (GELIOS_E_ARG outside [0, count)).  Forms without variants: count 1,
- * autotune returns variant 0. */
+ * hand (GELIOS_E_ARG outside [0, count)).  A new context uses variant 0 of the
+ * moving-grid form and variant 2 (128 threads x 4 blocks) of the MHD form.
+ * Forms without variants: count 1, autotune returns variant 0. */
 int gelios_variant_count(int form);
 int gelios_autotune(gelios_ctx *ctx, int form, int reps, int32_t *variant, double *ms);
 int gelios_set_variant(gelios_ctx *ctx, int form, int32_t variant);

@@ -76,3 +76,43 @@ def test_batch_clusters_equal_single_contexts(n):
     finally:
         for S in ss:
             S.close()
+
+
+@pytest.mark.parametrize("dims,n", [((60, 50), 2), ((60, 50), 3), ((186, 128), 2)])
+def test_few_instances_of_a_large_mesh(dims, n):
+    """One instance after the other up to 2 instances of 3000 cells (lanes) and
+    of 23808 (two phases), clusters from 3 instances on: the same bits as
+    single contexts where the kernel is the same, else 1e-13 (as above)."""
+    import gelios_2d_b200 as g
+
+    mesh = Mesh.polar(*dims, 1.0, 600.0)
+    th = W.sample_inflows(n, 9)
+    sts = [W.cold_state(mesh, W.inflow_params(t)) for t in th]
+    ss = [g.Setka(mesh, W.inflow_params(t)) for t in th]
+    try:
+        for S, st in zip(ss, sts):
+            S.set_par(0, st)
+            S.set_par(1, st)
+        b = C.c_void_p()
+        hs = (C.c_void_p * n)(*[S._h for S in ss])
+        N.check(N.lib().gelios_plain_batch_create(C.byref(b), hs, n), "gelios_plain_batch_create")
+        got = (N.GeliosStatus * n)()
+        try:
+            for _ in range(2):  # the second call arms the accumulators again
+                N.check(N.lib().gelios_plain_batch_step(b, 6, got), "gelios_plain_batch_step")
+        finally:
+            N.lib().gelios_plain_batch_destroy(b)
+        for i in range(n):
+            S = g.Setka(mesh, W.inflow_params(th[i]))
+            S.set_par(0, sts[i])
+            S.set_par(1, sts[i])
+            S.Go_stationary(6)
+            r = S.Go_stationary(6)
+            for x, y in ((ss[i].par(0), S.par(0)), (ss[i].par(1), S.par(1))):
+                scale = np.abs(y).max(axis=1, keepdims=True)
+                assert np.max(np.abs(x - y) / np.maximum(np.abs(y), 1e-6 * scale)) <= 1e-13
+            assert abs(got[i].dt - r.dt) <= 1e-13 * r.dt
+            S.close()
+    finally:
+        for S in ss:
+            S.close()
