@@ -56,10 +56,12 @@
 #include <vector>
 
 #include "../../include/gelios_b200.h"
+#include "mlp_plan.cuh"
 
 namespace gelios {
 void set_error(const std::string& msg);
 }  // namespace gelios
+using namespace gelios;
 
 namespace {
 
@@ -88,7 +90,7 @@ __device__ __forceinline__ void cp_async_wait_ring() { asm volatile("cp.async.wa
 // which frees the stage for the load of the tile four steps on; the epilogue
 // reads the accumulator with tcgen05.ld (warp w: rows 32w..32w+31).  Every
 // mbarrier wait is bounded: on expiry the CTA raises `status` and goes on.
-constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64, TC_THREADS = 128;
+constexpr int TC_BM = 128, TC_BN = 128, TC_BK = kGemmBK, TC_THREADS = 128;
 constexpr int TC_TILE = TC_BM * TC_BK * 2;  // bytes of one operand tile
 constexpr int TC_STAGES = 4;
 constexpr int TC_SMEM = 2 * TC_STAGES * TC_TILE;  // A and B per stage
@@ -939,9 +941,6 @@ struct Buf {
     }
 };
 
-// number of K slices of length kc
-inline int split_count(int K, int kc) { return K > 0 ? (K + kc - 1) / kc : 1; }
-
 inline bool vec_ok(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 8 == 0; }
 
 // status word of the tensor-core GEMM (bit 0: an mbarrier wait expired)
@@ -1054,12 +1053,6 @@ bool launch_tma(dim3 grid, int M, int N, int K, int kc, const __nv_bfloat16* A, 
     return true;
 }
 
-// K slice of a GEMM split `splits` ways (a multiple of the K stage)
-inline int tc_split_len(int K, int splits) {
-    int kc = (K + splits - 1) / splits;
-    return kc > 0 ? (kc + TC_BK - 1) / TC_BK * TC_BK : TC_BK;
-}
-
 // C = A . B^T with A [M][lda], B [N][ldb] (k contiguous); see gemm_tc_kernel
 void gemm(int M, int N, int K, const __nv_bfloat16* A, int64_t lda, const __nv_bfloat16* B, int64_t ldb, float* C,
           int64_t ldc, cudaStream_t s, int splits = 1, int64_t c_split = 0) {
@@ -1101,8 +1094,6 @@ void transpose(int R, int Cc, const __nv_bfloat16* in, int64_t ldin, __nv_bfloat
     if (R <= 0 || Cc <= 0) return;
     transpose_bf16_kernel<<<dim3(blocks(Cc, 32), blocks(R, 32)), dim3(32, 8), 0, s>>>(R, Cc, in, ldin, out, ldout);
 }
-
-constexpr int kMaxSplit = 32;
 
 }  // namespace
 
@@ -1159,12 +1150,6 @@ struct gelios_mlp {
             if (ev_chunk[k]) cudaEventDestroy(ev_chunk[k]);
     }
     int layers() const { return depth + 1; }
-    // splits of a weight GEMM over the rows of the batch
-    static int split_target(int M) {
-        const int s = (M + 255) / 256;
-        return s > kMaxSplit ? kMaxSplit : s < 1 ? 1 : s;
-    }
-    static int splits_of(int M) { return split_count(M, tc_split_len(M, split_target(M))); }
     // H_l^T (din[l] rows) and dZ_l^T (dout[l] rows), max_batch rounded up to 8 apart
     __nv_bfloat16* ht_of(int l) const {
         return f_ht.as<__nv_bfloat16>() + (l == 0 ? 0 : pad8(max_batch) * (in_w + static_cast<int64_t>(l - 1) * width));
@@ -1232,7 +1217,7 @@ bool backward_fused(gelios_mlp* n, int M, float* loss, int* at) {
     cudaStream_t s = n->stream, s2 = n->side;
     const int L = n->layers();
     const int64_t Mp = pad8(M);
-    const int S = n->splits_of(M), kc = tc_split_len(M, n->split_target(M)), chunks = (M + kColRows - 1) / kColRows;
+    const int S = splits_of(M), kc = tc_split_len(M, split_target(M)), chunks = (M + kColRows - 1) / kColRows;
     const int ldo = static_cast<int>(pad8(n->n_out));
     __nv_bfloat16* dz[2] = {n->dzb.as<__nv_bfloat16>(), n->f_dzb2.as<__nv_bfloat16>()};
     float* col = n->f_col.as<float>();
@@ -1272,7 +1257,7 @@ void reduce_fused(gelios_mlp* n, int M, const StepArgs* args, const int* at) {
     for (int l = 0; l < n->layers(); l++)
         most = std::max(most, static_cast<int64_t>(n->din[l] + 1) * n->dout[l]);
     grad_adam_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(
-        n->f_layers.as<LayerGrad>(), n->splits_of(M), (M + kColRows - 1) / kColRows, n->f_part.as<float>(),
+        n->f_layers.as<LayerGrad>(), splits_of(M), (M + kColRows - 1) / kColRows, n->f_part.as<float>(),
         n->f_col.as<float>(), n->g32.as<float>(), args, at, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(),
         kAdamB1, kAdamB2, kAdamEps, n->wb.as<__nv_bfloat16>());
 }
@@ -1321,7 +1306,7 @@ void backward(gelios_mlp* n, int M, float* loss, int* at) {
                                                    n->dzb.as<__nv_bfloat16>(), 0);
     const __nv_bfloat16* wb = n->wb.as<__nv_bfloat16>();
     float* g = n->g32.as<float>();
-    const int splits = n->split_target(M), S = n->splits_of(M);
+    const int splits = split_target(M), S = splits_of(M);
     const int64_t Mp = pad8(M);
     __nv_bfloat16* dzt = n->dzt.as<__nv_bfloat16>();
     __nv_bfloat16* ht = n->ht.as<__nv_bfloat16>();
@@ -1372,7 +1357,7 @@ int ensure_fused(gelios_mlp* n) {
         LayerGrad& g = n->layers_host[l];
         g.part_off = part;
         g.col_off = col;
-        part += static_cast<int64_t>(gelios_mlp::splits_of(n->max_batch)) * g.din * g.dout;
+        part += static_cast<int64_t>(reserved_splits(n->max_batch)) * g.din * g.dout;
         col += chunks * g.dout;
         if (l > 0) wt += static_cast<int64_t>(g.din) * g.ld_t;
     }
