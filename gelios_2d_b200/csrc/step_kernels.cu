@@ -3594,7 +3594,9 @@ template <int GROUP, bool COOP>
 __device__ __forceinline__ double k5_face_body(const DevMesh& d, const gelios_params& P, const StepBuffers& b,
                                                const double* __restrict__ hcur, double* __restrict__ fl, int u,
                                                int& status) {
-    constexpr bool USUALY = GROUP != kAnyGroup || COOP;
+    // a face whose two end points lie on one surface counts as tracked even on
+    // the grid's boundary, so the tracked units are not all interior ones
+    constexpr bool USUALY = GROUP != kAnyGroup;
     const double inf = __longlong_as_double(0x7ff0000000000000LL);
     const size_t nu = d.n_units;
     const int K = d.u_cell[u], nb = d.u_nb[u];
