@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/gelios_b200.h"
+#include "graph_capture.cuh"
 #include "physics.cuh"
 #include "step_kernels.cuh"
 
@@ -1308,22 +1309,12 @@ int graph_or_direct(gelios_ctx* ctx, int form, int kind, bool first, int parity,
             return g.launches;
         }
     cudaStream_t s = ctx->stream;
-    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        cudaGetLastError();
-        ctx->graphs_off = true;
-        return enqueue();
-    }
-    const int n = enqueue();
-    cudaGraph_t graph = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(s, &graph);
+    int n = 0;
     cudaGraphExec_t exec = nullptr;
-    if (n < 0 || e != cudaSuccess || !graph || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
+    if (!capture_graph(s, &exec, [&]() { return (n = enqueue()) >= 0; })) {
         ctx->graphs_off = true;
         return enqueue();
     }
-    cudaGraphDestroy(graph);
     gelios_ctx::StepGraph* slot = &ctx->graphs[0];
     for (auto& g : ctx->graphs)
         if (!g.exec) {
@@ -2395,19 +2386,9 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
     for (int st = 0; st < (B->schedule > 0 ? 0 : nsteps); st++) {
         const int par = st & 1;
         if (!B->graphs_off && !B->graph[par]) {
-            cudaGraph_t g = nullptr;
-            if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-                const cudaError_t le = launch_batch_mhd_step(B->tab, par, s, c0->side, c0->ev_fork, c0->ev_tracked);
-                if (le != cudaSuccess || cudaStreamEndCapture(s, &g) != cudaSuccess || !g ||
-                    cudaGraphInstantiate(&B->graph[par], g, 0) != cudaSuccess) {
-                    B->graph[par] = nullptr;
-                    B->graphs_off = true;
-                }
-                if (g) cudaGraphDestroy(g);
-            } else {
-                B->graphs_off = true;
-            }
-            cudaGetLastError();
+            B->graphs_off = !capture_graph(s, &B->graph[par], [&]() {
+                return launch_batch_mhd_step(B->tab, par, s, c0->side, c0->ev_fork, c0->ev_tracked) == cudaSuccess;
+            });
         }
         if (B->graph[par]) {
             GELIOS_CUDA_TRY(cudaGraphLaunch(B->graph[par], s));

@@ -56,6 +56,7 @@
 #include <vector>
 
 #include "../../include/gelios_b200.h"
+#include "graph_capture.cuh"
 #include "mlp_plan.cuh"
 
 namespace gelios {
@@ -1280,16 +1281,7 @@ bool enqueue_train_step(gelios_mlp* n, int batch) {
 cudaGraphExec_t train_graph(gelios_mlp* n, int batch) {
     if (n->graph && n->graph_batch == batch) return n->graph;
     n->drop_graph();
-    if (cudaStreamBeginCapture(n->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    const bool ok = enqueue_train_step(n, batch);
-    cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(n->stream, &g);
-    if (!ok || e != cudaSuccess || !g || cudaGraphInstantiate(&n->graph, g, 0) != cudaSuccess) n->graph = nullptr;
-    if (g) cudaGraphDestroy(g);
-    cudaGetLastError();
+    capture_graph(n->stream, &n->graph, [&]() { return enqueue_train_step(n, batch); });
     n->graph_batch = batch;
     return n->graph;
 }
