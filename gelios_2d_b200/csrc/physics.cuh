@@ -263,10 +263,11 @@ __device__ __forceinline__ double fma_rn(double a, double b, double c) { return 
 // sqrt(gp / ro) (a sound speed, gp = gamma p) as gp rsqrt(gp ro): one
 // reciprocal square root instead of a quotient and a square root in a row
 // (within 2 ulp of them); the quotient's own form where the product is not a
-// positive normal number.
+// positive normal number, and where both are negative (a caller's state before
+// the first step), whose root is positive too.
 __device__ __forceinline__ double sound_speed(double gp, double ro) {
     const double x = __dmul_rn(gp, ro);
-    if (x > 1e-290 && x < 1e290) return __dmul_rn(gp, rsqrt(x));
+    if (gp > 0.0 && x > 1e-290 && x < 1e290) return __dmul_rn(gp, rsqrt(x));
     return sqrt(gp / ro);
 }
 
