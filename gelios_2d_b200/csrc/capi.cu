@@ -159,10 +159,30 @@ struct gelios_ctx {
         int first = 0;  // the first step of a call: the graph starts with the words' initialisation
         int parity = -1;
         const void* cen = nullptr;
+        int uses = 0;  // how often it was asked for while there was none
         cudaGraphExec_t exec = nullptr;
         int launches = 0;
     };
     StepGraph graphs[48];
+    // the entry of these keys, a new one (no graph yet) if there is none
+    StepGraph& step_graph(int form, int kind, int first, int parity, const void* cen) {
+        StepGraph* at = nullptr;
+        for (auto& g : graphs) {
+            if (g.form == form && g.kind == kind && g.first == first && g.parity == parity && g.cen == cen) return g;
+            if (!at && g.form < 0) at = &g;
+        }
+        if (!at) {  // full: the oldest one goes
+            at = &graphs[0];
+            if (at->exec) cudaGraphExecDestroy(at->exec);
+            *at = StepGraph{};
+        }
+        at->form = form;
+        at->kind = kind;
+        at->first = first;
+        at->parity = parity;
+        at->cen = cen;
+        return *at;
+    }
     bool graphs_off = false;  // capture failed once: launch directly
     bool coop_off = false;    // the cooperative plain step could not launch once: three kernels per step
     void drop_graphs() {
@@ -1298,45 +1318,40 @@ int enqueue_form(gelios_ctx* ctx, const StepBuffers& b, int form) {
 // centroid buffer), or captures `enqueue` (which enqueues on ctx->stream,
 // may fork to the other streams and join them back, and returns its kernel
 // count or a negative error code) into a new one and launches it.  Launches
-// directly while phase timing is on or once a capture has failed.
+// directly while phase timing is on or once a capture has failed, and the
+// first worth - 1 times.
 template <class F>
-int graph_or_direct(gelios_ctx* ctx, int form, int kind, bool first, int parity, const void* cen, F&& enqueue) {
+int graph_or_direct(gelios_ctx* ctx, int form, int kind, bool first, int parity, const void* cen, F&& enqueue,
+                    int worth = 1) {
     if (ctx->timing || ctx->graphs_off) return enqueue();
-    for (auto& g : ctx->graphs)
-        if (g.exec && g.form == form && g.kind == kind && g.first == static_cast<int>(first) && g.parity == parity &&
-            g.cen == cen) {
-            GELIOS_CUDA_TRY(cudaGraphLaunch(g.exec, ctx->stream));
-            return g.launches;
+    gelios_ctx::StepGraph& g = ctx->step_graph(form, kind, first, parity, cen);
+    if (!g.exec) {
+        if (++g.uses < worth) return enqueue();
+        int n = 0;
+        if (!capture_graph(ctx->stream, &g.exec, [&]() { return (n = enqueue()) >= 0; })) {
+            ctx->graphs_off = true;
+            return enqueue();
         }
-    cudaStream_t s = ctx->stream;
-    int n = 0;
-    cudaGraphExec_t exec = nullptr;
-    if (!capture_graph(s, &exec, [&]() { return (n = enqueue()) >= 0; })) {
-        ctx->graphs_off = true;
-        return enqueue();
+        g.launches = n;
     }
-    gelios_ctx::StepGraph* slot = &ctx->graphs[0];
-    for (auto& g : ctx->graphs)
-        if (!g.exec) {
-            slot = &g;
-            break;
-        }
-    if (slot->exec) cudaGraphExecDestroy(slot->exec);
-    slot->form = form;
-    slot->kind = kind;
-    slot->first = first;
-    slot->parity = parity;
-    slot->cen = cen;
-    slot->exec = exec;
-    slot->launches = n;
-    GELIOS_CUDA_TRY(cudaGraphLaunch(exec, s));
-    return n;
+    GELIOS_CUDA_TRY(cudaGraphLaunch(g.exec, ctx->stream));
+    return g.launches;
 }
 
-// One moving-grid step (MK2 or MHD form) as one graph: the instantiated graph
-// of this form and these buffers (captured on first use), or direct launches
-// while phase timing is on or if capture is unavailable.  Returns the kernel
-// count or a negative error code.
+// Whether the call runs its next two steps as one graph (kind 4; see
+// pair_graph_worth), `ahead` of which it has left.
+bool pair_graph(gelios_ctx* ctx, int form, int parity, const void* cen, int ahead) {
+    if (ctx->timing || ctx->graphs_off) return false;
+    gelios_ctx::StepGraph& g = ctx->step_graph(form, 4, 0, parity, cen);
+    if (g.exec || pair_graph_worth(form == GELIOS_FORM_5_KOMPONENT, ahead, g.uses)) return true;
+    g.uses++;
+    return false;
+}
+
+// One moving-grid step as one graph: the instantiated graph of this form and
+// these buffers (captured on first use, the five-fluid form's later: see
+// kStepGraphUses), or direct launches while phase timing is on or if capture
+// is unavailable.  Returns the kernel count or a negative error code.
 // first: the first step of a call, whose graph begins with the initialisation
 // of the dt / status words (one launch per step, not two).
 int step_graph(gelios_ctx* ctx, const StepBuffers& b, int form, bool first) {
@@ -1345,7 +1360,7 @@ int step_graph(gelios_ctx* ctx, const StepBuffers& b, int form, bool first) {
         if (first) launch_words_init(ctx->words.p, ctx->prm.dt0, ctx->stream);
         const int m = enqueue_form(ctx, b, form);
         return m < 0 ? m : m + (first ? 1 : 0);
-    });
+    }, form == GELIOS_FORM_5_KOMPONENT ? kStepGraphUses : 1);
 }
 
 // ---- the pipelined moving-grid call
@@ -1540,8 +1555,9 @@ int mk2_pipelined(gelios_ctx* ctx, int nsteps, double* cen0, double* cen1) {
                             [&]() { return enqueue_pipe_head(ctx, 0, b, true); });
     if (n < 0) return n;
     launches += n;
-    // two bodies (an even and an odd step) are one graph: a graph launch costs
-    // the chain of a small grid about as much as a kernel of it
+    // two bodies (an even and an odd step) are one graph where that is worth it
+    // (pair_graph): a graph launch costs the chain of a small grid about as
+    // much as a kernel of it
     for (int st = 0; st < nsteps;) {
         const int left = nsteps - st;
         const StepBuffers b1 = mk2_buffers(ctx, st + 1, cen0, cen1);
@@ -1549,7 +1565,7 @@ int mk2_pipelined(gelios_ctx* ctx, int nsteps, double* cen0, double* cen1) {
             n = graph_or_direct(ctx, GELIOS_FORM_MK2, 3, false, st & 1, b.cx,
                                 [&]() { return enqueue_pipe_step(ctx, st, b, nullptr); });
             st += 1;
-        } else if (left >= 3 && !(st & 1)) {
+        } else if (left >= 3 && !(st & 1) && pair_graph(ctx, GELIOS_FORM_MK2, 0, b.cx, (left - 1) / 2)) {
             const StepBuffers b2 = mk2_buffers(ctx, st + 2, cen0, cen1);
             n = graph_or_direct(ctx, GELIOS_FORM_MK2, 4, false, 0, b.cx, [&]() {
                 const int n0 = enqueue_pipe_step(ctx, st, b, &b1);
@@ -1709,11 +1725,11 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
     for (int st = first; st < nsteps; st++) {
         const int cur = st & 1, nxt = cur ^ 1;
         if (moving) {
-            // a step of a moving-grid form in one graph, two steps after the
-            // first in one (as in mk2_pipelined)
+            // a step of a moving-grid form in one graph; after the first, two
+            // in one where that is worth it (as in mk2_pipelined)
             const StepBuffers b = mk2_buffers(ctx, st, cen0, cen1);
             int n;
-            if (st > 0 && st + 1 < nsteps) {
+            if ((st & 1) && st + 1 < nsteps && pair_graph(ctx, form, cur, b.cx, (nsteps - st) / 2)) {
                 const StepBuffers b1 = mk2_buffers(ctx, st + 1, cen0, cen1);
                 n = graph_or_direct(ctx, form, 4, false, cur, b.cx, [&]() {
                     const int n0 = enqueue_form(ctx, b, form);
