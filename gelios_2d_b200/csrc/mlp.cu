@@ -1072,10 +1072,10 @@ void gemm(int M, int N, int K, const __nv_bfloat16* A, int64_t lda, const __nv_b
         launch_tc<false, false>(grid, M, N, K, kc, A, lda, B, ldb, C, ldc, c_split, s);
 }
 
-// enqueues the read of the GEMM status word into pinned memory, before the
-// call's own synchronisation
-void gemm_status_fetch(int* pinned, cudaStream_t s) {
-    cudaMemcpyAsync(pinned, gemm_status_ptr(), sizeof(int), cudaMemcpyDeviceToHost, s);
+// enqueues the read of the GEMM status word before the call's own
+// synchronisation
+void gemm_status_fetch(int* to, cudaStream_t s) {
+    cudaMemcpyAsync(to, gemm_status_ptr(), sizeof(int), cudaMemcpyDeviceToHost, s);
 }
 // reads and clears the GEMM status word (after a synchronisation)
 bool gemm_status_ok() {
@@ -1110,20 +1110,22 @@ struct gelios_mlp {
     Buf w32, g32, m, v, wb;
     std::vector<Buf> h;  // bf16 inputs of every layer [max_batch][din]
     std::vector<Buf> z;  // fp32 pre-activations of every hidden layer
-    Buf c, y, dh, dz, dzb, tb, rowerr, part, colpart, loss, xin;
-    Buf wt, dzt, ht;  // transposes for the backward GEMMs: W_l^T, dZ^T, H_l^T
+    Buf c, y, dzb, tb, rowerr, loss, xin;
     int ld0 = 0;      // row stride of the first layer's input and of wpad (in_w rounded up to 8: TMA rows)
     Buf wpad;         // bf16 W of the first layer, rows of ld0
-    // the fused training step (ensure_fused): per layer H^T and dZ^T, W^T,
-    // gradient partials
-    bool fused = false, fused_known = false;
-    Buf f_ht, f_dzt, f_wt, f_part, f_col, f_dzb2, f_layers;
+    // what a gradient needs, one allocation at its first use (ensure_training)
+    bool fused = false, training_known = false;
+    Buf train_mem;
+    // fused: per layer H^T and dZ^T, W^T, gradient partials
+    __nv_bfloat16 *f_ht = nullptr, *f_dzt = nullptr, *f_dzb2 = nullptr;
+    float *f_part = nullptr, *f_col = nullptr;
+    // separate kernels: dH and dZ of a layer, partials, transposes W_l^T, dZ^T, H_l^T
+    float *dh = nullptr, *dz = nullptr, *part = nullptr, *colpart = nullptr;
+    __nv_bfloat16 *wt = nullptr, *dzt = nullptr, *ht = nullptr;
+    Buf f_layers;
     std::vector<LayerGrad> layers_host;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_dz = nullptr, ev_side = nullptr;
-    // one pinned allocation: a copy of the GEMM status word, then the staging
-    // of gelios_mlp_predict (px, py)
-    int* status_host = nullptr;
     // steps of a training call: their StepArgs, losses and the step counter,
     // kept from call to call (they grow with the longest call)
     Buf args, hist, at;
@@ -1134,8 +1136,12 @@ struct gelios_mlp {
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
     }
-    // gelios_mlp_predict: pinned staging of two chunks' inputs and outputs
-    int64_t stage_rows = 0;
+    // gelios_mlp_predict: rows of a chunk; once it is worth it (staging_worth)
+    // one pinned allocation: a copy of the GEMM status word, then two chunks'
+    // inputs and outputs
+    int64_t chunk_rows = 0, io_bytes = 0;
+    int* stage = nullptr;
+    bool stage_failed = false;
     float *px[2] = {nullptr, nullptr}, *py[2] = {nullptr, nullptr};
     cudaEvent_t ev_chunk[2] = {nullptr, nullptr};
     Buf X, T;  // training set (fp32 rows)
@@ -1145,7 +1151,7 @@ struct gelios_mlp {
         if (stream) cudaStreamDestroy(stream);
         if (ev_dz) cudaEventDestroy(ev_dz);
         if (ev_side) cudaEventDestroy(ev_side);
-        if (status_host) cudaFreeHost(status_host);
+        if (stage) cudaFreeHost(stage);
         drop_graph();
         for (int k = 0; k < 2; k++)
             if (ev_chunk[k]) cudaEventDestroy(ev_chunk[k]);
@@ -1153,9 +1159,9 @@ struct gelios_mlp {
     int layers() const { return depth + 1; }
     // H_l^T (din[l] rows) and dZ_l^T (dout[l] rows), max_batch rounded up to 8 apart
     __nv_bfloat16* ht_of(int l) const {
-        return f_ht.as<__nv_bfloat16>() + (l == 0 ? 0 : pad8(max_batch) * (in_w + static_cast<int64_t>(l - 1) * width));
+        return f_ht + (l == 0 ? 0 : pad8(max_batch) * (in_w + static_cast<int64_t>(l - 1) * width));
     }
-    __nv_bfloat16* dzt_of(int l) const { return f_dzt.as<__nv_bfloat16>() + pad8(max_batch) * width * l; }
+    __nv_bfloat16* dzt_of(int l) const { return f_dzt + pad8(max_batch) * width * l; }
 };
 
 namespace {
@@ -1220,8 +1226,8 @@ bool backward_fused(gelios_mlp* n, int M, float* loss, int* at) {
     const int64_t Mp = pad8(M);
     const int S = splits_of(M), kc = tc_split_len(M, split_target(M)), chunks = (M + kColRows - 1) / kColRows;
     const int ldo = static_cast<int>(pad8(n->n_out));
-    __nv_bfloat16* dz[2] = {n->dzb.as<__nv_bfloat16>(), n->f_dzb2.as<__nv_bfloat16>()};
-    float* col = n->f_col.as<float>();
+    __nv_bfloat16* dz[2] = {n->dzb.as<__nv_bfloat16>(), n->f_dzb2};
+    float* col = n->f_col;
     mse_grad_kernel<<<chunks, kColRows, 0, s>>>(M, n->n_out, ldo, n->y.as<float>(), n->tb.as<float>(), dz[0],
                                                 n->dzt_of(L - 1), Mp, col + n->layers_host[L - 1].col_off,
                                                 n->rowerr.as<float>());
@@ -1232,7 +1238,7 @@ bool backward_fused(gelios_mlp* n, int M, float* loss, int* at) {
         if (l == L - 1) loss_kernel<<<1, 256, 0, s2>>>(M, n->n_out, n->rowerr.as<float>(), loss, at);
         // dW[dO][di] = dZ^T . H_l, split over the rows of the batch
         bool ok = launch_tma<0>(dim3(1, blocks(dO, TC_BM), S), dO, di, M, kc, n->dzt_of(l), Mp, n->ht_of(l), Mp,
-                                n->f_part.as<float>() + n->layers_host[l].part_off, di, static_cast<int64_t>(dO) * di,
+                                n->f_part + n->layers_host[l].part_off, di, static_cast<int64_t>(dO) * di,
                                 GemmEpilogue{}, s2);
         if (!ok) return false;  // an operand without a tensor map (not with the strides gelios_mlp_create chose)
         if (l == 0) break;
@@ -1258,8 +1264,8 @@ void reduce_fused(gelios_mlp* n, int M, const StepArgs* args, const int* at) {
     for (int l = 0; l < n->layers(); l++)
         most = std::max(most, static_cast<int64_t>(n->din[l] + 1) * n->dout[l]);
     grad_adam_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(
-        n->f_layers.as<LayerGrad>(), splits_of(M), (M + kColRows - 1) / kColRows, n->f_part.as<float>(),
-        n->f_col.as<float>(), n->g32.as<float>(), args, at, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(),
+        n->f_layers.as<LayerGrad>(), splits_of(M), (M + kColRows - 1) / kColRows, n->f_part,
+        n->f_col, n->g32.as<float>(), args, at, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(),
         kAdamB1, kAdamB2, kAdamEps, n->wb.as<__nv_bfloat16>());
 }
 void draw_batch(gelios_mlp* n, int batch) {
@@ -1291,17 +1297,17 @@ void backward(gelios_mlp* n, int M, float* loss, int* at) {
     cudaStream_t s = n->stream;
     const int L = n->layers();
     const int64_t eo = static_cast<int64_t>(M) * n->n_out;
-    mse_kernel<<<blocks(M, 256), 256, 0, s>>>(M, n->n_out, n->y.as<float>(), n->tb.as<float>(), n->dh.as<float>(),
+    mse_kernel<<<blocks(M, 256), 256, 0, s>>>(M, n->n_out, n->y.as<float>(), n->tb.as<float>(), n->dh,
                                               n->rowerr.as<float>());
     loss_kernel<<<1, 256, 0, s>>>(M, n->n_out, n->rowerr.as<float>(), loss, at);
-    act_bwd_kernel<<<blocks(eo, 256), 256, 0, s>>>(eo, n->dh.as<float>(), nullptr, n->dz.as<float>(),
+    act_bwd_kernel<<<blocks(eo, 256), 256, 0, s>>>(eo, n->dh, nullptr, n->dz,
                                                    n->dzb.as<__nv_bfloat16>(), 0);
     const __nv_bfloat16* wb = n->wb.as<__nv_bfloat16>();
     float* g = n->g32.as<float>();
     const int splits = split_target(M), S = splits_of(M);
     const int64_t Mp = pad8(M);
-    __nv_bfloat16* dzt = n->dzt.as<__nv_bfloat16>();
-    __nv_bfloat16* ht = n->ht.as<__nv_bfloat16>();
+    __nv_bfloat16* dzt = n->dzt;
+    __nv_bfloat16* ht = n->ht;
     for (int l = L - 1; l >= 0; l--) {
         const int di = n->din[l], dO = n->dout[l];
         // dW[dO][di] = dZ^T . H_l (both transposed so k = batch row is
@@ -1309,21 +1315,21 @@ void backward(gelios_mlp* n, int M, float* loss, int* at) {
         const int64_t wn = static_cast<int64_t>(dO) * di;
         transpose(M, dO, n->dzb.as<__nv_bfloat16>(), dO, dzt, Mp, s);
         transpose(M, di, n->h[l].as<__nv_bfloat16>(), l == 0 ? n->ld0 : di, ht, Mp, s);
-        gemm(dO, di, M, dzt, Mp, ht, Mp, n->part.as<float>(), di, s, splits, wn);
-        splitk_reduce_kernel<<<blocks(wn, 256), 256, 0, s>>>(wn, S, n->part.as<float>(), g + n->w_off[l]);
+        gemm(dO, di, M, dzt, Mp, ht, Mp, n->part, di, s, splits, wn);
+        splitk_reduce_kernel<<<blocks(wn, 256), 256, 0, s>>>(wn, S, n->part, g + n->w_off[l]);
         // db = column sums of dZ
         const int chunks = (M + kColRows - 1) / kColRows;
-        col_sum_partial_kernel<<<dim3(blocks(dO, 128), chunks), 128, 0, s>>>(M, dO, n->dz.as<float>(),
-                                                                             n->colpart.as<float>());
-        col_sum_final_kernel<<<blocks(dO, 128), 128, 0, s>>>(chunks, dO, n->colpart.as<float>(), g + n->b_off[l]);
+        col_sum_partial_kernel<<<dim3(blocks(dO, 128), chunks), 128, 0, s>>>(M, dO, n->dz,
+                                                                             n->colpart);
+        col_sum_final_kernel<<<blocks(dO, 128), 128, 0, s>>>(chunks, dO, n->colpart, g + n->b_off[l]);
         if (l == 0) break;
         // dH_l[M][di] = dZ . W_l, then dZ_{l-1} = dH_l * GELU'(Z_{l-1})
-        transpose(dO, di, wb + n->w_off[l], di, n->wt.as<__nv_bfloat16>(), pad8(dO), s);
-        gemm(M, di, dO, n->dzb.as<__nv_bfloat16>(), dO, n->wt.as<__nv_bfloat16>(), pad8(dO), n->dh.as<float>(), di,
+        transpose(dO, di, wb + n->w_off[l], di, n->wt, pad8(dO), s);
+        gemm(M, di, dO, n->dzb.as<__nv_bfloat16>(), dO, n->wt, pad8(dO), n->dh, di,
              s);
         const int64_t e = static_cast<int64_t>(M) * di;
-        act_bwd_kernel<<<blocks(e, 256), 256, 0, s>>>(e, n->dh.as<float>(), n->z[l - 1].as<float>(),
-                                                      n->dz.as<float>(), n->dzb.as<__nv_bfloat16>(), 1);
+        act_bwd_kernel<<<blocks(e, 256), 256, 0, s>>>(e, n->dh, n->z[l - 1].as<float>(),
+                                                      n->dz, n->dzb.as<__nv_bfloat16>(), 1);
     }
 }
 
@@ -1339,10 +1345,13 @@ void copy_weights(gelios_mlp* n) {
 // takes the network (16-byte rows for the TMA: a width that is a multiple of
 // 8; the output columns in mse_grad_kernel's tile; partial sums of at most
 // 256 MB) and allocates what it needs: per layer H^T, dZ^T, W^T, the partial
-// and column sums.  Without room for them the separate kernels run.
-int ensure_fused(gelios_mlp* n) {
-    if (n->fused_known) return GELIOS_OK;
+// and column sums.  Otherwise, and without room for them, the separate
+// kernels run, with their own workspaces.
+int ensure_training(gelios_mlp* n) {
+    if (n->training_known) return GELIOS_OK;
     const int depth = n->depth, width = n->width;
+    const size_t MB = static_cast<size_t>(n->max_batch), Mp = static_cast<size_t>(pad8(n->max_batch));
+    const size_t widest = static_cast<size_t>(std::max({n->in_w, width, n->n_out}));
     const int64_t chunks = (n->max_batch + kColRows - 1) / kColRows;
     int64_t part = 0, col = 0, wt = 0;
     for (int l = 0; l <= depth; l++) {
@@ -1354,40 +1363,78 @@ int ensure_fused(gelios_mlp* n) {
         if (l > 0) wt += static_cast<int64_t>(g.din) * g.ld_t;
     }
     CUtensorMap tz, th;
-    bool ok = width % 8 == 0 && n->n_out <= kMseCols && part <= (int64_t(64) << 20) &&
-              output_map(&tz, n->z[0].p, true, n->max_batch, width) &&
-              output_map(&th, n->h[1].p, false, n->max_batch, width);
-    if (ok) {
-        const size_t Mp = static_cast<size_t>(pad8(n->max_batch));
-        const int64_t widest = std::max({n->in_w, width, n->n_out});
-        ok = n->f_ht.alloc(Mp * (n->in_w + static_cast<size_t>(depth) * width) * 2) &&
-             n->f_dzt.alloc(Mp * width * (static_cast<size_t>(depth) + 1) * 2 + Mp * kMseCols * 2) &&
-             n->f_wt.alloc(static_cast<size_t>(wt) * 2) && n->f_part.alloc(static_cast<size_t>(part) * 4) &&
-             n->f_col.alloc(static_cast<size_t>(col) * 4) &&
-             n->f_dzb2.alloc(static_cast<size_t>(n->max_batch) * pad8(widest) * 2);
-        if (!ok) {
-            cudaGetLastError();
-            for (Buf* b : {&n->f_ht, &n->f_dzt, &n->f_wt, &n->f_part, &n->f_col, &n->f_dzb2}) b->release();
+    if (width % 8 == 0 && n->n_out <= kMseCols && part <= (int64_t(64) << 20) &&
+        output_map(&tz, n->z[0].p, true, n->max_batch, width) &&
+        output_map(&th, n->h[1].p, false, n->max_batch, width)) {
+        Carve c;
+        const size_t o_ht = c.take(Mp * (n->in_w + static_cast<size_t>(depth) * width) * 2);
+        const size_t o_dzt = c.take(Mp * width * (static_cast<size_t>(depth) + 1) * 2 + Mp * kMseCols * 2);
+        const size_t o_wt = c.take(static_cast<size_t>(wt) * 2), o_part = c.take(static_cast<size_t>(part) * 4);
+        const size_t o_col = c.take(static_cast<size_t>(col) * 4), o_dz = c.take(MB * pad8(widest) * 2);
+        if (n->train_mem.alloc(c.bytes)) {
+            char* p = n->train_mem.as<char>();
+            n->f_ht = reinterpret_cast<__nv_bfloat16*>(p + o_ht);
+            n->f_dzt = reinterpret_cast<__nv_bfloat16*>(p + o_dzt);
+            n->f_dzb2 = reinterpret_cast<__nv_bfloat16*>(p + o_dz);
+            n->f_part = reinterpret_cast<float*>(p + o_part);
+            n->f_col = reinterpret_cast<float*>(p + o_col);
+            __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(p + o_wt);
+            for (int l = 1; l <= depth; l++) {
+                LayerGrad& g = n->layers_host[l];
+                g.wt = w;
+                w += static_cast<int64_t>(g.din) * g.ld_t;
+            }
+            MLP_TRY(cudaStreamCreateWithFlags(&n->side, cudaStreamNonBlocking));
+            MLP_TRY(cudaEventCreateWithFlags(&n->ev_dz, cudaEventDisableTiming));
+            MLP_TRY(cudaEventCreateWithFlags(&n->ev_side, cudaEventDisableTiming));
+            MLP_TRY(cudaMemsetAsync(p + o_wt, 0, static_cast<size_t>(wt) * 2, n->stream));
+            MLP_TRY(cudaMemcpyAsync(n->f_layers.p, n->layers_host.data(), sizeof(LayerGrad) * n->layers_host.size(),
+                                    cudaMemcpyHostToDevice, n->stream));
+            copy_weights(n);
+            MLP_TRY(cudaGetLastError());
+            n->fused = n->training_known = true;
+            return GELIOS_OK;
         }
+        cudaGetLastError();
     }
-    n->fused_known = true;
-    if (!ok) return GELIOS_OK;
-    int64_t wo = 0;
-    for (int l = 1; l <= depth; l++) {
-        LayerGrad& g = n->layers_host[l];
-        g.wt = n->f_wt.as<__nv_bfloat16>() + wo;
-        wo += static_cast<int64_t>(g.din) * g.ld_t;
-    }
-    MLP_TRY(cudaStreamCreateWithFlags(&n->side, cudaStreamNonBlocking));
-    MLP_TRY(cudaEventCreateWithFlags(&n->ev_dz, cudaEventDisableTiming));
-    MLP_TRY(cudaEventCreateWithFlags(&n->ev_side, cudaEventDisableTiming));
-    MLP_TRY(cudaMemsetAsync(n->f_wt.p, 0, n->f_wt.bytes, n->stream));
-    MLP_TRY(cudaMemcpyAsync(n->f_layers.p, n->layers_host.data(), sizeof(LayerGrad) * n->layers_host.size(),
-                            cudaMemcpyHostToDevice, n->stream));
-    copy_weights(n);
-    MLP_TRY(cudaGetLastError());
-    n->fused = true;
+    Carve c;
+    const size_t o_dh = c.take(MB * widest * 4), o_dz = c.take(MB * widest * 4);
+    const size_t o_part = c.take(static_cast<size_t>(kMaxSplit) * widest * widest * 4);
+    const size_t o_col = c.take(static_cast<size_t>(chunks) * widest * 4), o_wt = c.take(widest * pad8(widest) * 2);
+    const size_t o_dzt = c.take(widest * Mp * 2), o_ht = c.take(widest * Mp * 2);
+    if (!n->train_mem.alloc(c.bytes)) return cuda_fail(cudaErrorMemoryAllocation);
+    char* p = n->train_mem.as<char>();
+    n->dh = reinterpret_cast<float*>(p + o_dh);
+    n->dz = reinterpret_cast<float*>(p + o_dz);
+    n->part = reinterpret_cast<float*>(p + o_part);
+    n->colpart = reinterpret_cast<float*>(p + o_col);
+    n->wt = reinterpret_cast<__nv_bfloat16*>(p + o_wt);
+    n->dzt = reinterpret_cast<__nv_bfloat16*>(p + o_dzt);
+    n->ht = reinterpret_cast<__nv_bfloat16*>(p + o_ht);
+    n->training_known = true;
     return GELIOS_OK;
+}
+
+// The pinned staging of gelios_mlp_predict; without it the copies go through
+// the driver's.
+void ensure_staging(gelios_mlp* n) {
+    const int64_t xf = pad8(n->chunk_rows * n->n_in), yf = pad8(n->chunk_rows * n->n_out);
+    const int64_t bytes = (16 + 2 * (xf + yf)) * 4;
+    if (n->stage || n->stage_failed || !staging_worth(n->io_bytes, bytes)) return;
+    void* p = nullptr;
+    n->stage_failed = cudaMallocHost(&p, static_cast<size_t>(bytes)) != cudaSuccess;
+    for (cudaEvent_t& e : n->ev_chunk)
+        n->stage_failed = n->stage_failed || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess;
+    if (n->stage_failed) {
+        cudaGetLastError();
+        if (p) cudaFreeHost(p);
+        return;
+    }
+    n->stage = static_cast<int*>(p);
+    for (int k = 0; k < 2; k++) {
+        n->px[k] = static_cast<float*>(p) + 16 + k * (xf + yf);
+        n->py[k] = n->px[k] + xf;
+    }
 }
 }  // namespace
 
@@ -1432,24 +1479,10 @@ extern "C" int gelios_mlp_create(gelios_mlp** out, int device, int n_in, int n_f
     for (int l = 0; l <= depth; l++) ok = ok && n->h[l].alloc(MB * (l == 0 ? n->ld0 : n->din[l]) * 2);
     ok = ok && n->wpad.alloc(static_cast<size_t>(n->dout[0]) * n->ld0 * 2);
     for (int l = 0; l < depth; l++) ok = ok && n->z[l].alloc(MB * width * 4);
-    ok = ok && n->c.alloc(MB * W * 4) && n->y.alloc(MB * n_out * 4) && n->dh.alloc(MB * W * 4) &&
-         n->dz.alloc(MB * W * 4) && n->dzb.alloc(MB * pad8(widest) * 2) && n->tb.alloc(MB * n_out * 4) &&
-         n->rowerr.alloc(MB * 4) && n->part.alloc(static_cast<size_t>(kMaxSplit) * W * W * 4) &&
-         n->colpart.alloc(((MB + kColRows - 1) / kColRows) * W * 4) && n->loss.alloc(16) &&
-         n->xin.alloc(MB * n_in * 4) && n->wt.alloc(W * pad8(widest) * 2) &&
-         n->dzt.alloc(W * pad8(max_batch) * 2) && n->ht.alloc(W * pad8(max_batch) * 2);
+    ok = ok && n->c.alloc(MB * W * 4) && n->y.alloc(MB * n_out * 4) && n->dzb.alloc(MB * pad8(widest) * 2) &&
+         n->tb.alloc(MB * n_out * 4) && n->rowerr.alloc(MB * 4) && n->loss.alloc(16) && n->xin.alloc(MB * n_in * 4);
     if (!ok) return cuda_fail(cudaErrorMemoryAllocation);
-    // at most 16 MB of staging per chunk
-    n->stage_rows = std::min<int64_t>(max_batch, std::max<int64_t>(1024, (int64_t(4) << 20) / (n_in + n_out)));
-    const int64_t xf = pad8(n->stage_rows * n_in), yf = pad8(n->stage_rows * n_out);
-    float* pin = nullptr;
-    MLP_TRY(cudaMallocHost(&pin, static_cast<size_t>(16 + 2 * (xf + yf)) * 4));
-    n->status_host = reinterpret_cast<int*>(pin);
-    for (int k = 0; k < 2; k++) {
-        n->px[k] = pin + 16 + k * (xf + yf);
-        n->py[k] = n->px[k] + xf;
-        MLP_TRY(cudaEventCreateWithFlags(&n->ev_chunk[k], cudaEventDisableTiming));
-    }
+    n->chunk_rows = stage_rows(max_batch, n_in, n_out);
     MLP_TRY(cudaMemsetAsync(n->wpad.p, 0, n->wpad.bytes, n->stream));
     for (int l = 0; l <= depth; l++) {
         LayerGrad g{};
@@ -1510,7 +1543,7 @@ extern "C" int gelios_mlp_get_params(const gelios_mlp* n, float* host, int64_t c
 extern "C" int gelios_mlp_loss_grad(gelios_mlp* n, const float* x, const float* t, int M, double* loss, float* grad) {
     if (!n || !x || !t || M < 1 || M > n->max_batch) return fail("gelios_mlp_loss_grad: bad arguments");
     MLP_TRY(cudaSetDevice(n->device));
-    if (const int rc = ensure_fused(n)) return rc;
+    if (const int rc = ensure_training(n)) return rc;
     cudaStream_t s = n->stream;
     MLP_TRY(cudaMemcpyAsync(n->xin.p, x, static_cast<size_t>(M) * n->n_in * 4, cudaMemcpyHostToDevice, s));
     MLP_TRY(cudaMemcpyAsync(n->tb.p, t, static_cast<size_t>(M) * n->n_out * 4, cudaMemcpyHostToDevice, s));
@@ -1529,9 +1562,10 @@ extern "C" int gelios_mlp_loss_grad(gelios_mlp* n, const float* x, const float* 
     MLP_TRY(cudaMemcpyAsync(&l, n->loss.p, 4, cudaMemcpyDeviceToHost, s));
     if (grad)
         MLP_TRY(cudaMemcpyAsync(grad, n->g32.p, static_cast<size_t>(n->n_params) * 4, cudaMemcpyDeviceToHost, s));
-    gemm_status_fetch(n->status_host, s);
+    int bad = 0;
+    gemm_status_fetch(&bad, s);
     MLP_TRY(cudaStreamSynchronize(s));
-    if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    if (bad && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     if (loss) *loss = l;
     return GELIOS_OK;
 }
@@ -1540,7 +1574,7 @@ extern "C" int gelios_mlp_set_data(gelios_mlp* n, const float* x, const float* t
     if (!n || !x || !t || n_rows < 1) return fail("gelios_mlp_set_data: bad arguments");
     MLP_TRY(cudaSetDevice(n->device));
     n->drop_graph();  // it holds the training set's addresses and size
-    if (const int rc = ensure_fused(n)) return rc;
+    if (const int rc = ensure_training(n)) return rc;
     n->n_rows = 0;
     if (!n->X.alloc(static_cast<size_t>(n_rows) * n->n_in * 4) ||
         !n->T.alloc(static_cast<size_t>(n_rows) * n->n_out * 4))
@@ -1609,9 +1643,10 @@ extern "C" int gelios_mlp_train(gelios_mlp* n, int iters, int batch, float lr_ma
     }
     if (loss_hist && iters > 0)
         MLP_TRY(cudaMemcpyAsync(loss_hist, n->hist.p, static_cast<size_t>(iters) * 4, cudaMemcpyDeviceToHost, s));
-    gemm_status_fetch(n->status_host, s);
+    int bad = 0;
+    gemm_status_fetch(&bad, s);
     MLP_TRY(cudaStreamSynchronize(s));
-    if (*n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    if (bad && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     return GELIOS_OK;
 }
 
@@ -1619,9 +1654,13 @@ extern "C" int gelios_mlp_predict(gelios_mlp* n, const float* x, int64_t M, floa
     if (!n || !x || !y || M < 0) return fail("gelios_mlp_predict: bad arguments");
     MLP_TRY(cudaSetDevice(n->device));
     cudaStream_t s = n->stream;
-    // the chunks pass through pinned staging, two at a time: a copy from or to
-    // pageable memory of this size goes through the driver's own, in turn
-    const int64_t mb = n->stage_rows;
+    // The chunks pass through pinned staging, two at a time, once that is worth
+    // it: a copy from or to pageable memory of this size goes through the
+    // driver's own, in turn.
+    n->io_bytes += M * (n->n_in + n->n_out) * 4;
+    ensure_staging(n);
+    const bool staged = n->stage != nullptr;
+    const int64_t mb = n->chunk_rows;
     auto rows = [&](int64_t k) { return std::min(mb, M - k * mb); };
     auto collect = [&](int64_t k) {
         const cudaError_t e = cudaEventSynchronize(n->ev_chunk[k & 1]);
@@ -1632,20 +1671,34 @@ extern "C" int gelios_mlp_predict(gelios_mlp* n, const float* x, int64_t M, floa
     const int64_t chunks = (M + mb - 1) / mb;
     for (int64_t k = 0; k < chunks; k++) {
         const int b = static_cast<int>(k & 1), m = static_cast<int>(rows(k));
-        if (k >= 2) MLP_TRY(collect(k - 2));
         const size_t xb = static_cast<size_t>(m) * n->n_in * 4;
-        std::memcpy(n->px[b], x + k * mb * n->n_in, xb);
-        MLP_TRY(cudaMemcpyAsync(n->xin.p, n->px[b], xb, cudaMemcpyHostToDevice, s));
+        const float* xs = x + k * mb * n->n_in;
+        if (staged) {
+            if (k >= 2) MLP_TRY(collect(k - 2));
+            std::memcpy(n->px[b], xs, xb);
+            xs = n->px[b];
+        }
+        MLP_TRY(cudaMemcpyAsync(n->xin.p, xs, xb, cudaMemcpyHostToDevice, s));
         features_kernel<<<blocks(static_cast<int64_t>(m) * kRowThreads, 128), 128, 0, s>>>(
             m, n->n_in, n->nf, n->ld0, n->xin.as<float>(), n->h[0].as<__nv_bfloat16>());
         forward(n, m);
         MLP_TRY(cudaGetLastError());
-        MLP_TRY(cudaMemcpyAsync(n->py[b], n->y.p, static_cast<size_t>(m) * n->n_out * 4, cudaMemcpyDeviceToHost, s));
-        if (k + 1 == chunks) gemm_status_fetch(n->status_host, s);
-        MLP_TRY(cudaEventRecord(n->ev_chunk[b], s));
+        MLP_TRY(cudaMemcpyAsync(staged ? n->py[b] : y + k * mb * n->n_out, n->y.p,
+                                static_cast<size_t>(m) * n->n_out * 4, cudaMemcpyDeviceToHost, s));
+        if (staged) {
+            if (k + 1 == chunks) gemm_status_fetch(n->stage, s);
+            MLP_TRY(cudaEventRecord(n->ev_chunk[b], s));
+        }
     }
-    for (int64_t k = std::max<int64_t>(0, chunks - 2); k < chunks; k++) MLP_TRY(collect(k));
-    if (chunks > 0 && *n->status_host && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    int bad = 0;
+    if (staged) {
+        for (int64_t k = std::max<int64_t>(0, chunks - 2); k < chunks; k++) MLP_TRY(collect(k));
+        bad = chunks > 0 ? *n->stage : 0;
+    } else {
+        gemm_status_fetch(&bad, s);
+        MLP_TRY(cudaStreamSynchronize(s));
+    }
+    if (bad && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     return GELIOS_OK;
 }
 
