@@ -56,6 +56,11 @@ struct DBuf {
         }
         return GELIOS_OK;
     }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        bytes = 0;
+    }
     template <typename T>
     T* as() const {
         return static_cast<T*>(p);
@@ -137,7 +142,8 @@ struct gelios_ctx {
     DBuf surface;  // Move_surface per-face speeds
     DBuf inner;
     int n_inner = 0;
-    DBuf inner_tab;  // constants of an inner call (launch_inner_lanes); empty: one thread per cell
+    DBuf inner_tab;  // constants of an inner call with a long list (inner_table)
+    bool inner_tab_failed = false;
     int n_sp = 0;
     // cen[0] holds the centroids of the current points (rows cx, cy,
     // |c|^(2 gamma), area, rotated volume); after a moving-grid call row 2
@@ -146,7 +152,8 @@ struct gelios_ctx {
     bool cen_rp_partial = false;
     // the face units' geometry of the plain form (UnitGeo rows); stale once
     // the points move, the topology or the parameters change
-    DBuf ugeo;
+    // (kUnitGeoRows + 1 rows, behind the flux rows in one allocation)
+    double* ugeo() const { return flux.as<double>() + 5 * static_cast<size_t>(d.n_slots); }
     bool ugeo_valid = false;
     // Instantiated graphs of one moving-grid step, keyed by the buffers the
     // step reads (state parity and centroid buffer); dropped whenever the
@@ -184,7 +191,8 @@ struct gelios_ctx {
         return *at;
     }
     bool graphs_off = false;  // capture failed once: launch directly
-    bool coop_off = false;    // the cooperative plain step could not launch once: three kernels per step
+    // the cooperative launch of the plain / inner form failed once: kernels per step
+    bool coop_off = false, inner_coop_off = false;
     void drop_graphs() {
         for (auto& g : graphs) {
             if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -861,8 +869,7 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     rc |= upload(ctx->t_lbase, tb.lbase.data(), tb.lbase.size(), s);
     rc |= upload(ctx->t_fstart, tb.fstart.data(), tb.fstart.size(), s);
     rc |= upload(ctx->t_faces, tb.faces.data(), tb.faces.size(), s);
-    rc |= upload<double>(ctx->flux, nullptr, 5 * static_cast<size_t>(ng), s);
-    rc |= upload<double>(ctx->ugeo, nullptr, static_cast<size_t>(kUnitGeoRows + 1) * u_slot.size(), s);
+    rc |= upload<double>(ctx->flux, nullptr, 5 * static_cast<size_t>(ng) + (kUnitGeoRows + 1) * u_slot.size(), s);
     int max_faces = 0;
     for (int c = 0; c < nc; c++)
         if (v->cell_type[c] != C_CENTR) max_faces = std::max(max_faces, v->gran_start[c + 1] - v->gran_start[c]);
@@ -1057,6 +1064,7 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     ctx->tiles.faces = ctx->t_faces.as<int2>();
     ctx->have_mesh = true;
     ctx->n_inner = 0;
+    ctx->inner_tab.release();
     ctx->cen_valid = false;
     ctx->ugeo_valid = false;
     ctx->drop_graphs();
@@ -1186,12 +1194,8 @@ extern "C" int gelios_set_inner_cells(gelios_ctx* ctx, const int32_t* cells, int
     if (upload(ctx->inner, cells, n, ctx->stream)) return GELIOS_E_CUDA;
     GELIOS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     ctx->n_inner = n;
-    const size_t tb = inner_lanes_ok(ctx->d, ctx->prm, n) ? inner_table_bytes(n) : 0;
-    if (ctx->inner_tab.bytes != tb && ctx->inner_tab.alloc(tb)) {
-        // no room for the table: the steps run without it
-        cudaGetLastError();
-        ctx->inner_tab.bytes = 0;
-    }
+    ctx->inner_tab.release();  // of the list before; the next step that needs one allocates its own
+    ctx->inner_tab_failed = false;
     return GELIOS_OK;
 }
 
@@ -1525,10 +1529,10 @@ int enqueue_pipe_step(gelios_ctx* ctx, int st, const StepBuffers& b, const StepB
 // the cached unit geometry in the layout the context's flux precision reads
 void set_unit_geometry(const gelios_ctx* ctx, StepBuffers& b) {
     if (ctx->prm.precision == GELIOS_PREC_FP32_FLUX) {
-        b.upf = ctx->ugeo.as<double>();
+        b.upf = ctx->ugeo();
         b.fgeo = b.upf + ctx->d.n_units;
     } else {
-        b.ugeo = ctx->ugeo.as<double>();
+        b.ugeo = ctx->ugeo();
     }
 }
 
@@ -1539,6 +1543,27 @@ void ensure_rail_table(gelios_ctx* ctx, cudaStream_t s) {
     launch_rail_table(d, ctx->prm.n_inner, const_cast<double*>(d.rcs), const_cast<double*>(d.rsn),
                       const_cast<double*>(d.rfrac), s);
     ctx->rail_tab_valid = true;
+}
+
+// Room for the constants of an inner call (launch_inner_lanes), null if the
+// list takes one thread per cell.  Every call computes them anew, and the
+// inner form uses neither flux rows nor the plain form's unit geometry, so
+// those hold them where they are long enough: lists of up to 0.4 of the cells
+// (the inner region has 0.15 to 0.32).  An allocation of its own takes 340 us
+// on the first step, as long as eleven steps gain on the 8k grid.
+double* inner_table(gelios_ctx* ctx) {
+    if (!inner_lanes_ok(ctx->d, ctx->prm, ctx->n_inner)) return nullptr;
+    const size_t need = inner_table_bytes(ctx->n_inner);
+    if (need <= ctx->flux.bytes) {
+        if (need > 5 * static_cast<size_t>(ctx->d.n_slots) * sizeof(double)) ctx->ugeo_valid = false;
+        return ctx->flux.as<double>();
+    }
+    if (ctx->inner_tab.bytes < need && !ctx->inner_tab_failed && ctx->inner_tab.alloc(need)) {
+        cudaGetLastError();
+        ctx->inner_tab.release();
+        ctx->inner_tab_failed = true;
+    }
+    return ctx->inner_tab.as<double>();
 }
 
 bool pipe_ok(const gelios_ctx* ctx) {
@@ -1653,7 +1678,7 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
         ctx->cen_rp_partial = false;
     }
     if (form == GELIOS_FORM_STATIONARY && !ctx->ugeo_valid && nsteps > 0) {
-        launch_unit_geometry(d, P, cen0, cen0 + ncz, cen0 + 2 * ncz, ctx->ugeo.as<double>(), s);
+        launch_unit_geometry(d, P, cen0, cen0 + ncz, cen0 + 2 * ncz, ctx->ugeo(), s);
         launches++;
         ctx->ugeo_valid = true;
     }
@@ -1686,8 +1711,9 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             ctx->coop_off = true;
         }
     }
-    if (form == GELIOS_FORM_INNER_MK2 && nsteps > 0 && !ctx->timing && !ctx->coop_off && ctx->n_inner > 0 &&
-        inner_lanes_ok(d, P, ctx->n_inner) && ctx->inner_tab.bytes >= inner_table_bytes(ctx->n_inner)) {
+    double* itab = nullptr;
+    if (form == GELIOS_FORM_INNER_MK2 && nsteps > 0 && !ctx->timing && !ctx->inner_coop_off &&
+        (itab = inner_table(ctx))) {
         // all steps of the inner form in one cooperative launch
         StepBuffers bb[2];
         for (int par = 0; par < 2; par++) {
@@ -1705,13 +1731,13 @@ extern "C" int gelios_step(gelios_ctx* ctx, int form, int nsteps, gelios_status*
             b.cy = cen0 + ncz;
             b.rp = cen0 + 2 * ncz;
         }
-        if (launch_inner_lanes(d, P, bb[0], bb[1], ctx->inner.as<int32_t>(), ctx->n_inner,
-                               ctx->inner_tab.as<double>(), nsteps, s) == cudaSuccess) {
+        if (launch_inner_lanes(d, P, bb[0], bb[1], ctx->inner.as<int32_t>(), ctx->n_inner, itab, nsteps, s) ==
+            cudaSuccess) {
             launches += 2;
             first = nsteps;
         } else {
             cudaGetLastError();
-            ctx->coop_off = true;
+            ctx->inner_coop_off = true;
         }
     }
     if (moving) ensure_rail_table(ctx, s);
@@ -2700,7 +2726,7 @@ int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
         if (!c->ugeo_valid) {
             const double* cen = c->cen[0].as<double>();
             const size_t n = c->d.n_cells;
-            launch_unit_geometry(c->d, c->prm, cen, cen + n, cen + 2 * n, c->ugeo.as<double>(), B->stream);
+            launch_unit_geometry(c->d, c->prm, cen, cen + n, cen + 2 * n, c->ugeo(), B->stream);
             c->ugeo_valid = true;
         }
         PlainInstance& I = host[i];
