@@ -110,11 +110,10 @@ struct gelios_ctx {
     bool have_mesh = false;
     DevMesh d;
     // topology / geometry
-    DBuf X, Y, X2, Y2, ptype, cstart, contour, gstart, cflags, ctype, sA, sB, snb, ssd, ssd2, sinfo, qcorner;
-    DBuf fA, fB, ftype, fmaster, fsosed, fcopy, fsdown;
+    DBuf X, Y, X2, Y2, cstart, contour, gstart, cflags, ctype, sA, sB, snb, ssd, ssd2, sinfo, qcorner;
     DBuf rtype, rM, rpstart, rpts, rkstart, rkeys, rs;
     DBuf sp_point, sp_line, sp_inc, sp_ainc, sp_fix, sp_of_point, rk_point, rk_node, sf_rec, rail_tab;
-    bool rail_tab_valid = false;  // launch_rail_table; stale once the topology or the parameters change
+    bool rail_tab_valid = false;  // launch_rail_table; stale once n_inner changes
     DBuf u_slot, u_cell, u_twin, u_A, u_B, u_info, u_nb, u_sd, u_sd2, s_unit, flux, aux, rec, pstar, src_lo;
     DBuf Hn, Hu, Hv, HT, ku, kv, kT, r_istoch, cback, cnext;
     // state par[2] x 5 fields, centroids [2], scratch
@@ -334,11 +333,11 @@ double sqrt_threshold(double R);
 
 extern "C" int gelios_set_params(gelios_ctx* ctx, const gelios_params* prm) {
     if (!ctx || !prm) return GELIOS_E_ARG;
+    ctx->rail_tab_valid = ctx->rail_tab_valid && prm->n_inner == ctx->prm.n_inner;
     ctx->prm = *prm;
     ctx->d.r11_sq = sqrt_threshold(prm->R11);
     ctx->cen_valid = false;  // the cached |centroid|^(2 gamma) depends on gamma
     ctx->ugeo_valid = false;
-    ctx->rail_tab_valid = false;
     ctx->drop_graphs();      // the parameters are kernel arguments
     return GELIOS_OK;
 }
@@ -790,7 +789,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     rc |= upload(ctx->Y, v->y, np, s);
     rc |= upload(ctx->X2, v->x, np, s);
     rc |= upload(ctx->Y2, v->y, np, s);
-    rc |= upload(ctx->ptype, v->point_type, np, s);
     rc |= upload(ctx->cstart, v->contour_start, nc + 1, s);
     rc |= upload(ctx->contour, v->contour, v->contour_start[nc], s);
     {
@@ -815,13 +813,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     rc |= upload(ctx->ssd, ssd.data(), ng, s);
     rc |= upload(ctx->ssd2, ssd2.data(), ng, s);
     rc |= upload(ctx->sinfo, sinfo.data(), ng, s);
-    rc |= upload(ctx->fA, v->face_A, nf, s);
-    rc |= upload(ctx->fB, v->face_B, nf, s);
-    rc |= upload(ctx->ftype, v->face_type, nf, s);
-    rc |= upload(ctx->fmaster, v->face_master, nf, s);
-    rc |= upload(ctx->fsosed, v->face_sosed, nf, s);
-    rc |= upload(ctx->fcopy, v->face_copy, nf, s);
-    rc |= upload(ctx->fsdown, fsdown, nf, s);
     const int nr = v->n_rails;
     if (nr > 0) {
         rc |= upload(ctx->rtype, v->rail_type, nr, s);
@@ -935,7 +926,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     }
     rc |= upload<double>(ctx->rail_tab, nullptr,
                          2 * static_cast<size_t>(nr) + (nr > 0 ? v->rail_pstart[nr] : 0) + 1, s);
-    ctx->rail_tab_valid = false;
     rc |= upload<double>(ctx->Hn, nullptr, 4 * static_cast<size_t>(nc), s);
     rc |= upload<double>(ctx->Hu, nullptr, 4 * static_cast<size_t>(nc), s);
     rc |= upload<double>(ctx->Hv, nullptr, 4 * static_cast<size_t>(nc), s);
@@ -978,7 +968,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     d.Y = ctx->Y.as<double>();
     d.X2 = ctx->X2.as<double>();
     d.Y2 = ctx->Y2.as<double>();
-    d.ptype = ctx->ptype.as<int32_t>();
     d.r11_sq = sqrt_threshold(ctx->prm.R11);
     d.cstart = ctx->cstart.as<int32_t>();
     d.qcorner = reinterpret_cast<const int4*>(ctx->qcorner.as<int32_t>());
@@ -1008,13 +997,6 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     d.u_c1 = u_c1;
     d.u_tr0 = u_tr0;
     d.u_tr1 = u_tr1;
-    d.fA = ctx->fA.as<int32_t>();
-    d.fB = ctx->fB.as<int32_t>();
-    d.ftype = ctx->ftype.as<int32_t>();
-    d.fmaster = ctx->fmaster.as<int32_t>();
-    d.fsosed = ctx->fsosed.as<int32_t>();
-    d.fcopy = ctx->fcopy.as<int32_t>();
-    d.fsdown = ctx->fsdown.as<int32_t>();
     d.rtype = ctx->rtype.as<int32_t>();
     d.rM = ctx->rM.as<int32_t>();
     d.rpstart = ctx->rpstart.as<int32_t>();
@@ -1062,6 +1044,9 @@ extern "C" int gelios_upload_topology(gelios_ctx* ctx, const gelios_mesh_view* v
     ctx->tiles.lbase = ctx->t_lbase.as<int32_t>();
     ctx->tiles.fstart = ctx->t_fstart.as<int32_t>();
     ctx->tiles.faces = ctx->t_faces.as<int2>();
+    launch_rail_table(d, ctx->prm.n_inner, s);
+    GELIOS_CUDA_TRY(cudaGetLastError());
+    ctx->rail_tab_valid = true;
     ctx->have_mesh = true;
     ctx->n_inner = 0;
     ctx->inner_tab.release();
@@ -1539,9 +1524,7 @@ void set_unit_geometry(const gelios_ctx* ctx, StepBuffers& b) {
 // the rails' constant tables, before the motion kernels read them
 void ensure_rail_table(gelios_ctx* ctx, cudaStream_t s) {
     if (ctx->rail_tab_valid) return;
-    const DevMesh& d = ctx->d;
-    launch_rail_table(d, ctx->prm.n_inner, const_cast<double*>(d.rcs), const_cast<double*>(d.rsn),
-                      const_cast<double*>(d.rfrac), s);
+    launch_rail_table(ctx->d, ctx->prm.n_inner, s);
     ctx->rail_tab_valid = true;
 }
 
@@ -2241,6 +2224,7 @@ struct gelios_batch {
     cudaEvent_t ev = nullptr, ev_table = nullptr;
     bool table_pending = false;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    int uses[2] = {0, 0};  // how often each was asked for while there was none
     bool graphs_off = false;
     // 0: one launch per phase, a captured graph per step; k > 0: all steps
     // of a call in one cooperative launch of k blocks per SM
@@ -2427,7 +2411,7 @@ extern "C" int gelios_batch_step(gelios_batch* B, int form, int nsteps, gelios_s
     }
     for (int st = 0; st < (B->schedule > 0 ? 0 : nsteps); st++) {
         const int par = st & 1;
-        if (!B->graphs_off && !B->graph[par]) {
+        if (!B->graphs_off && !B->graph[par] && ++B->uses[par] >= kStepGraphUses) {
             B->graphs_off = !capture_graph(s, &B->graph[par], [&]() {
                 return launch_batch_mhd_step(B->tab, par, s, c0->side, c0->ev_fork, c0->ev_tracked) == cudaSuccess;
             });

@@ -40,10 +40,10 @@ constexpr int kPairAhead = 4, kPairAheadDirect = 8, kPairUses = 64;
 inline bool pair_graph_worth(bool direct_otherwise, int ahead, int uses) {
     return ahead >= (direct_otherwise ? kPairAheadDirect : kPairAhead) || uses >= kPairUses;
 }
-// The five-fluid form launches a step's ten kernels directly until a step
-// graph has been asked for this often: capturing it costs 165 us and saves 15.
-// (MK2 and MHD steps are longer chains on more streams: their graphs are
-// captured at once.)
+// The five-fluid form and the batched sweep launch a step's ten (six) kernels
+// directly until a step graph has been asked for this often: capturing it costs
+// 165 us (200 for the sweep's two branches) and saves 15.  (MK2 and MHD steps
+// are longer chains on more streams: their graphs are captured at once.)
 constexpr int kStepGraphUses = 16;
 
 }  // namespace gelios

@@ -3395,8 +3395,6 @@ __global__ void hlld_batch_kernel(gelios_params P, int n, const double* __restri
 // Move_surface + Move_Setka_Calculate.  The 21-field state follows the
 // member order of Parametr's aggregate initialisers (Gran.cpp:262-265):
 // ro, p, u, v, Q, then ro, p, u, v of H1..H4.
-constexpr int kRo = 0, kP = 1, kU = 2, kV = 3, kQ = 4;
-constexpr double kHPow = 0.5;              // H_pow, Help.h:90
 constexpr double kNHOverKn = 1.0 / 6.0;   // n_H_LISM_ / Kn_, Help.h:60, 65
 
 // The state rows of the five fluids: fluid 0 the plasma (with Q), 1..4 the
@@ -5057,9 +5055,11 @@ void launch_mk2_update(const DevMesh& d, const gelios_params& P, const StepBuffe
     else
         mk2_update_kernel<kUpdAll><<<nb, 128, 0, s>>>(d, P, b, fl, aux, list, n_list);
 }
-void launch_rail_table(const DevMesh& d, int n_inner, double* rcs, double* rsn, double* rfrac, cudaStream_t s) {
+void launch_rail_table(const DevMesh& d, int n_inner, cudaStream_t s) {
     const int nr = d.n_rail_a + d.n_rail_b + d.n_rail_c + d.n_rail_d;
-    if (nr > 0) rail_table_kernel<<<nr, 128, 0, s>>>(d, n_inner, rcs, rsn, rfrac);
+    if (nr > 0)
+        rail_table_kernel<<<nr, 128, 0, s>>>(d, n_inner, const_cast<double*>(d.rcs), const_cast<double*>(d.rsn),
+                                             const_cast<double*>(d.rfrac));
 }
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
                   bool copy_outer_shock, const StepBuffers* fin) {

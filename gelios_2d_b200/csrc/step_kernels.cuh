@@ -26,7 +26,6 @@ struct DevMesh {
     double r11_sq = 0.0;
     int dims[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     double *X = nullptr, *Y = nullptr, *X2 = nullptr, *Y2 = nullptr;
-    const int32_t* ptype = nullptr;
     const int32_t *cstart = nullptr, *contour = nullptr, *gstart = nullptr;
     // contour of every quadrilateral cell as one int4 ({-1, -1, -1, -1} for
     // other cells); may be null (the contour arrays are read instead)
@@ -50,8 +49,6 @@ struct DevMesh {
     // the unit of every slot << 1 | 1 where the slot is its twin side
     const int32_t* s_unit = nullptr;
     int max_faces = 0;  // most faces of a cell that is not C_centr
-    const int32_t *fA = nullptr, *fB = nullptr, *ftype = nullptr, *fmaster = nullptr, *fsosed = nullptr,
-                  *fcopy = nullptr, *fsdown = nullptr;
     const int32_t *rtype = nullptr, *rM = nullptr, *rpstart = nullptr, *rpts = nullptr, *rkstart = nullptr,
                   *rkeys = nullptr;
     const double* rs = nullptr;
@@ -252,8 +249,8 @@ void launch_mk2_update(const DevMesh& d, const gelios_params& P, const StepBuffe
 // flags of a tracked face record: types of the face and of its copy, whether
 // their masters have an Axis face, both end points on one tracked surface
 enum : int { SF_TYPE2 = 3, SF_AXIS1 = 1 << 6, SF_AXIS2 = 1 << 7, SF_TRACKED = 1 << 8 };
-// rcs, rsn (n_rails each) and rfrac (one per rail point) of d
-void launch_rail_table(const DevMesh& d, int n_inner, double* rcs, double* rsn, double* rfrac, cudaStream_t s);
+// fills rcs, rsn (n_rails each) and rfrac (one per rail point) of d
+void launch_rail_table(const DevMesh& d, int n_inner, cudaStream_t s);
 int launch_motion(const DevMesh& d, const gelios_params& P, const StepBuffers& b, double* scratch, cudaStream_t s,
                   bool copy_outer_shock = true, const StepBuffers* fin = nullptr);
 // Go_5_komponent: face units, then the cell update.  Hydrogen state rows

@@ -129,3 +129,28 @@ def test_rail_table_follows_the_parameters():
         assert np.array_equal(a, b)
     ref.close()
     S.close()
+
+
+@pytest.mark.gpu
+def test_batch_before_and_after_its_graphs():
+    """Calls of one to three steps of a batch, 46 in all: directly launched
+    steps and the graphs formed at the sixteenth of each parity give the bits of
+    single contexts that make the same calls."""
+    from gelios_2d_b200.sweep import Sweep
+
+    meshes = [g.Mesh.setka(9, 5, 3, 17, 25, 7, 11, 6), g.Mesh.setka(5, 3, 4, 9, 23, 6, 7, 9)]
+    mp = W.mhd_params()
+    inst = []
+    for k, m in enumerate(meshes):
+        st = W.init_conditions_reference(m)
+        inst.append((m, N.reference_params(), st, (mp, W.mhd_initial(m, st, mp), W.mhd_sources(m, seed=k))))
+    B = Sweep(inst, form=N.FORM_MHD_PUI, batched=True)
+    ref = Sweep(inst, form=N.FORM_MHD_PUI, batched=False)
+    for n in (1, 2, 3) * 7 + (1, 3):
+        got = B.batch_step(n, statuses=True)
+        for i, S in enumerate(ref.items):
+            assert S.Go_MHD_pickup(n).dt == got[i].dt
+    for i, S in enumerate(ref.items):
+        for b in (0, 1):
+            assert np.array_equal(B.par(i, b), S.par(b))
+        assert np.array_equal(B.items[i].points()[0], S.points()[0])
