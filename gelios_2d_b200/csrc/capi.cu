@@ -2751,7 +2751,7 @@ int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
 cudaError_t plain_batch_steps(gelios_plain_batch* B, const std::vector<int>& list, int nsteps) {
     const DevMesh& d = B->ctxs[0]->d;
     const int n = static_cast<int>(list.size());
-    if (nsteps > 0 && B->prec != GELIOS_PREC_FP32_FLUX && plain_batch_serial(d.n_cells, n)) {
+    if (nsteps > 0 && plain_batch_serial(d, n, B->prec)) {
         cudaError_t e = cudaSuccess;
         for (int k = 0; k < n && e == cudaSuccess; k++) {
             const PlainInstance& I = B->host[list[k]];

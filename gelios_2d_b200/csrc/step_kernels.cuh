@@ -153,15 +153,9 @@ struct PlainInstance {
     StepBuffers b[2];
     double* fl;
 };
-// A batch of n instances takes them one after the other, each on the whole
-// chip (launch_stationary_persistent), instead of a cluster per instance:
-// a cluster is at most 16 SMs.  us of 40 / 100 / 20 steps, one after the other
-// against clusters: 180x120 cells, 1, 2, 8 instances 279 / 1670, 487 / 1681,
-// 1725 / 2301; 120x90, 4: 1650 / 2342; 90x60, 1, 2: 422 / 1468, 776 / 1488;
-// 360x240, 1, 4, 20: 537 / 2840, 1887 / 3817, 9052 / 9063.  A step of a mesh
-// that the lanes hold takes 4-5 us on the whole chip, a cluster's about
-// 5.5 us + 1.7 ns per cell: the line lies where n of the one make the other.
-inline bool plain_batch_serial(int n_cells, int n) { return 3000 * static_cast<int64_t>(n) <= n_cells + 3000LL; }
+// Whether `n` instances of the mesh run one after the other on the whole chip
+// instead of a cluster each (plain_plan.cuh); not with FP32 fluxes.
+bool plain_batch_serial(const DevMesh& d, int n, int prec);
 // `nsteps` steps of the instances listed in `active` (device arrays) in one
 // launch; returns the launch's error code.
 cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst, const int* active, int n_active,
