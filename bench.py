@@ -82,11 +82,13 @@ STEP_KERNELS = {
            "autotuned arrangement), update of the cells the next motion reads, then the next step's dt, "
            "surface_faces, rails, tracked recon + solve beside the update of the other cells "
            "(CUDA graphs, 4 streams; one commit per call)",
-    "plain": "whole plain step: stationary_persistent_kernel (face units, cell update, dt; all steps of a call "
-             "in one cooperative launch)",
-    "k5": "whole four-fluid step: centroid, surface_faces, rails, k5_cell, commit",
+    "plain": "whole plain step: stationary_lanes_kernel (four lanes per cell: face fluxes, cell update, dt; all "
+             "steps of a call in one cooperative launch)",
+    "k5": "whole four-fluid step: surface_faces, rails, k5_tracked + k5_face (plain, C_1, one-sided units), "
+          "k5_update, commit",
     "mhd": "whole MHD + pickup step: surface_faces, rails, mhd_face, mhd_update, commit",
-    "inner": "whole inner-region step: inner_cell + dt_finalize",
+    "inner": "whole inner-region step: inner_lanes_kernel (all steps of a call in one cooperative launch, after "
+             "inner_table_kernel)",
 }
 
 

@@ -1457,8 +1457,10 @@ int enqueue_pipe_step(gelios_ctx* ctx, int st, const StepBuffers& b, const StepB
     // (side stream) overwrite the rows the tracked fluxes read: they wait
     // for the early update, which waits for the motion stream.
     // On a small grid (kMk2SmallCells) every one of these kernels is a few
-    // blocks bound by latency: the source terms and the one-sided group then
-    // run on the side and extra streams, beside instead of behind the others.
+    // blocks bound by latency: the source terms then run on the side stream,
+    // beside the tracked fluxes and the C_1 / one-sided groups instead of
+    // behind the tracked fluxes.  The main stream waits for them here, so the
+    // plain units start after them.
     const bool small = d.n_cells <= kMk2SmallCells;
     GELIOS_CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
     GELIOS_CUDA_TRY(cudaStreamWaitEvent(sm, ctx->ev_fork, 0));

@@ -925,11 +925,6 @@ struct Buf {
     ~Buf() {
         if (p) cudaFree(p);
     }
-    void release() {
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-    }
     bool alloc(size_t n) {
         if (p) cudaFree(p);
         p = nullptr;
@@ -1219,7 +1214,8 @@ void forward(gelios_mlp* n, int M, bool train = false) {
 // stream.  Per 8192-row step of the 31 -> 5 x 256 -> 5 network, as ~45
 // launches of separate transposes, activations, sums and reductions the
 // whole step took 480 us, 189 here;
-// as a captured graph (train_graph) 156 (115 of 4096 rows, 97 of 128).
+// as a captured graph (train_graph) 156 (117 of 4096 rows, 100 of 128; the
+// slope between calls of 200 and 600 steps).
 bool backward_fused(gelios_mlp* n, int M, float* loss, int* at) {
     cudaStream_t s = n->stream, s2 = n->side;
     const int L = n->layers();

@@ -428,7 +428,7 @@ __device__ __forceinline__ double lev_dev(double ga, double enI, double pI, doub
 // must hold.  A window that misses is followed by a plain D = 5 round.  The
 // midpoints, the values that decide and the order of the decisions are the
 // sequential loop's, so the result and the iteration count are too.  About 30
-// levels take three rounds instead of six (one lev costs ~2400 cycles).
+// levels take three rounds instead of six or seven (one lev costs ~2400 cycles).
 template <bool COOP>
 __device__ __forceinline__ double godunov_devtwo(double ga, double enI, double pI, double rI, double enII, double pII,
                                                  double rII, int max_iter, int* status) {

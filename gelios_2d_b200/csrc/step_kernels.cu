@@ -699,7 +699,7 @@ __global__ void centroid_kernel(DevMesh d, const double* __restrict__ X, const d
 // and the two results are the negatives of each other up to rounding,
 // Setka.cpp:10195-10380) or a one-sided face (boundary types, evaluated for
 // its owner only).  Each unit writes F*S once, into its own flux row, as the
-// owner sees it (the neighbour's sum subtracts it; the plain form's FP32-flux
+// owner sees it (the neighbour's sum subtracts it; the plain form's two-phase
 // kernels keep a row per slot and write -F*S into the twin's), and folds the
 // CFL candidates of the sides whose cell is updated this step into the dt
 // word.  The cell kernels then sum their slots in Grans order.
@@ -717,7 +717,6 @@ __global__ void centroid_kernel(DevMesh d, const double* __restrict__ X, const d
 struct FaceGeo {
     double x2, y2, n1, n2, f2, S, dist, distn;
 };
-constexpr int kFaceGeoRows = 8;
 __device__ __forceinline__ FaceGeo face_geo(double xa, double ya, double xb, double yb, double x, double y,
                                             bool has_nb, double x3, double y3) {
     FaceGeo f;
