@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
                                                             const __grid_constant__ CUtensorMap tmZ,
                                                             const __grid_constant__ CUtensorMap tmH, int tstore) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
-    __shared__ uint64_t full[TC_STAGES], empty[TC_STAGES];
+    __shared__ uint64_t full[TC_STAGES], empty[TC_STAGES], done;
     __shared__ uint32_t tmem_slot;
     static_assert(3 * (TC_BM * 128) + TM_BN * TM_TPITCH * 2 <= TC_STAGES * (TC_TILE + TM_TILE_B) &&
                       TC_BM * (TM_BN + 1) * 4 <= 3 * (TC_BM * 128),
@@ -411,6 +411,7 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
+        mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     tc_fence_before();
@@ -446,8 +447,12 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
                     "l"(ad), "l"(bd), "r"(TM_IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
                     : "memory");
             }
+            // The last commit goes to a barrier of its own.  The warps that wait
+            // for the accumulator have not followed the stage's phases: on
+            // empty[st] a second use (K > 256) is the parity that an unused
+            // barrier already passes.
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             smem_u32(&empty[st]))
+                             smem_u32(it + 1 < nk ? &empty[st] : &done))
                          : "memory");
             if (it + TC_STAGES < nk) {
                 // the stage is free once its MMAs have read it
@@ -457,7 +462,7 @@ __global__ void __launch_bounds__(TM_THREADS, 2) gemm_tma_kernel(const __grid_co
         }
     }
     __syncwarp();
-    if (nk > 0 && !mbar_wait(&empty[(nk - 1) % TC_STAGES], ((nk - 1) / TC_STAGES) & 1)) ok = false;
+    if (nk > 0 && !mbar_wait(&done, 0)) ok = false;
     tc_fence_after();
     const int wl = warp & 3, wc = warp >> 2;
     const int64_t row = m0 + wl * 32 + lane;
