@@ -796,9 +796,18 @@ __global__ void loss_kernel(int M, int N, const float* __restrict__ row_err, flo
     }
 }
 
+// One layer as grad_adam_kernel reads it.
+struct LayerGrad {
+    int64_t w_off, b_off, part_off;  // part_off: its S x (dout * din) weight partials
+    int din, dout, ld_in, ld_t;      // row strides of the padded W (layer 0) and of W^T
+    int64_t col_off;                 // its chunks x dout column sums
+    __nv_bfloat16* wpad;             // layer 0: W with rows of ld_in (or null)
+    __nv_bfloat16* wt;               // W^T, din rows of ld_t (null for layer 0)
+};
+
 __global__ void adam_kernel(int64_t n, float* __restrict__ w, const float* __restrict__ gr, float* __restrict__ m,
                             float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
-                            __nv_bfloat16* __restrict__ wb) {
+                            __nv_bfloat16* __restrict__ wb, LayerGrad first) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float g = gr[i];
@@ -808,7 +817,13 @@ __global__ void adam_kernel(int64_t n, float* __restrict__ w, const float* __res
     v[i] = vi;
     const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
-    wb[i] = __float2bfloat16(wi);
+    const __nv_bfloat16 h = __float2bfloat16(wi);
+    wb[i] = h;
+    // the first layer's padded copy (its weights come first)
+    if (i < static_cast<int64_t>(first.din) * first.dout) {
+        const int k = static_cast<int>(i), o = k / first.din;
+        first.wpad[static_cast<int64_t>(o) * first.ld_in + (k - o * first.din)] = h;
+    }
 }
 
 // The last layer's dZ = dY of kColRows rows per block: bf16 rows of ld (zeros
@@ -847,14 +862,6 @@ __global__ void __launch_bounds__(kColRows) mse_grad_kernel(int M, int N, int ld
     }
 }
 
-// One layer as grad_adam_kernel reads it.
-struct LayerGrad {
-    int64_t w_off, b_off, part_off;  // part_off: its S x (dout * din) weight partials
-    int din, dout, ld_in, ld_t;      // row strides of the padded W (layer 0) and of W^T
-    int64_t col_off;                 // its chunks x dout column sums
-    __nv_bfloat16* wpad;             // layer 0: W with rows of ld_in (or null)
-    __nv_bfloat16* wt;               // W^T, din rows of ld_t (null for layer 0)
-};
 // The gradients of layer blockIdx.y (weights: the S split partial sums in
 // order; bias: the chunks' column sums in order) into g, then, given args, the
 // Adam step and the bf16 copies.
@@ -864,10 +871,14 @@ __global__ void __launch_bounds__(256) grad_adam_kernel(const LayerGrad* __restr
                                                         const StepArgs* __restrict__ args,
                                                         const int* __restrict__ at, float* __restrict__ w,
                                                         float* __restrict__ m, float* __restrict__ v, float b1, float b2,
-                                                        float eps, __nv_bfloat16* __restrict__ wb) {
+                                                        float eps, __nv_bfloat16* __restrict__ wb,
+                                                        const int* __restrict__ status, float* __restrict__ loss) {
     const LayerGrad L = layers[blockIdx.y];
     const int64_t wn = static_cast<int64_t>(L.din) * L.dout;
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    // the GEMM status word behind the loss just written, so that one copy
+    // brings both (every GEMM of the step is done by now)
+    if (i == 0 && blockIdx.y == 0) reinterpret_cast<int*>(loss)[at ? *at : 1] = *status;
     if (i >= wn + L.dout) return;
     const bool weight = i < wn;
     const float* p = weight ? part + L.part_off + i : colpart + L.col_off + (i - wn);
@@ -1139,7 +1150,7 @@ struct gelios_mlp {
     // gelios_mlp_predict: rows of a chunk; once it is worth it (staging_worth)
     // one pinned allocation: a copy of the GEMM status word, then two chunks'
     // inputs and outputs
-    int64_t chunk_rows = 0, io_bytes = 0;
+    int64_t chunk_rows = 0, predictions = 0, io_bytes = 0;
     int* stage = nullptr;
     bool stage_failed = false;
     float *px[2] = {nullptr, nullptr}, *py[2] = {nullptr, nullptr};
@@ -1203,7 +1214,9 @@ void forward(gelios_mlp* n, int M, bool train = false) {
         const __nv_bfloat16* W = l == 0 ? n->wpad.as<__nv_bfloat16>() : wb + n->w_off[l];
         const int ld = l == 0 ? n->ld0 : di;
         dim3 grid(blocks(dO, TC_BN), blocks(M, TC_BM), 1);
-        if (M > 0 &&
+        // (a hidden layer whose rows the TMA cannot store: gemm_tc_kernel and the
+        // coalesced bias_act_kernel: a training step of 8192 rows of 100 304 us, 294 so)
+        if (M > 0 && (last || dO % 8 == 0) &&
             launch_tma<1>(grid, M, dO, di, tc_split_len(di, 1), A, ld, W, ld, nullptr, 0, 0, ep, s))
             continue;
         gemm(M, dO, di, A, ld, W, ld, n->c.as<float>(), dO, s);
@@ -1260,14 +1273,14 @@ bool backward_fused(gelios_mlp* n, int M, float* loss, int* at) {
 }
 // the gradients into g32 and, given args, the Adam step (see grad_adam_kernel)
 constexpr float kAdamB1 = 0.9f, kAdamB2 = 0.999f, kAdamEps = 1e-8f;
-void reduce_fused(gelios_mlp* n, int M, const StepArgs* args, const int* at) {
+void reduce_fused(gelios_mlp* n, int M, const StepArgs* args, const int* at, float* loss) {
     int64_t most = 0;
     for (int l = 0; l < n->layers(); l++)
         most = std::max(most, static_cast<int64_t>(n->din[l] + 1) * n->dout[l]);
     grad_adam_kernel<<<dim3(blocks(most, 256), n->layers()), 256, 0, n->stream>>>(
         n->f_layers.as<LayerGrad>(), splits_of(M), (M + kColRows - 1) / kColRows, n->f_part,
         n->f_col, n->g32.as<float>(), args, at, n->w32.as<float>(), n->m.as<float>(), n->v.as<float>(),
-        kAdamB1, kAdamB2, kAdamEps, n->wb.as<__nv_bfloat16>());
+        kAdamB1, kAdamB2, kAdamEps, n->wb.as<__nv_bfloat16>(), gemm_status_ptr(), loss);
 }
 void draw_batch(gelios_mlp* n, int batch) {
     gather_kernel<<<blocks(static_cast<int64_t>(batch) * kRowThreads, 128), 128, 0, n->stream>>>(
@@ -1280,7 +1293,7 @@ bool enqueue_train_step(gelios_mlp* n, int batch) {
     draw_batch(n, batch);
     forward(n, batch, true);
     if (!backward_fused(n, batch, n->hist.as<float>(), n->at.as<int>())) return false;
-    reduce_fused(n, batch, n->args.as<StepArgs>(), n->at.as<int>());
+    reduce_fused(n, batch, n->args.as<StepArgs>(), n->at.as<int>(), n->hist.as<float>());
     return cudaGetLastError() == cudaSuccess;
 }
 // The same as a graph, captured once per batch size and training set; null
@@ -1421,7 +1434,7 @@ int ensure_training(gelios_mlp* n) {
 void ensure_staging(gelios_mlp* n) {
     const int64_t xf = pad8(n->chunk_rows * n->n_in), yf = pad8(n->chunk_rows * n->n_out);
     const int64_t bytes = (16 + 2 * (xf + yf)) * 4;
-    if (n->stage || n->stage_failed || !staging_worth(n->io_bytes, bytes)) return;
+    if (n->stage || n->stage_failed || !staging_worth(n->predictions, n->io_bytes, bytes)) return;
     void* p = nullptr;
     n->stage_failed = cudaMallocHost(&p, static_cast<size_t>(bytes)) != cudaSuccess;
     for (cudaEvent_t& e : n->ev_chunk)
@@ -1554,20 +1567,22 @@ extern "C" int gelios_mlp_loss_grad(gelios_mlp* n, const float* x, const float* 
     if (n->fused) {
         transpose(M, n->in_w, n->h[0].as<__nv_bfloat16>(), n->ld0, n->ht_of(0), pad8(M), s);
         if (!backward_fused(n, M, n->loss.as<float>(), nullptr)) return cuda_fail(cudaErrorInvalidValue);
-        reduce_fused(n, M, nullptr, nullptr);
+        reduce_fused(n, M, nullptr, nullptr, n->loss.as<float>());
     } else {
         backward(n, M, n->loss.as<float>(), nullptr);
     }
     MLP_TRY(cudaGetLastError());
-    float l = 0.f;
-    MLP_TRY(cudaMemcpyAsync(&l, n->loss.p, 4, cudaMemcpyDeviceToHost, s));
+    struct {
+        float loss;
+        int bad;
+    } got{};
+    MLP_TRY(cudaMemcpyAsync(&got, n->loss.p, n->fused ? 8 : 4, cudaMemcpyDeviceToHost, s));
     if (grad)
         MLP_TRY(cudaMemcpyAsync(grad, n->g32.p, static_cast<size_t>(n->n_params) * 4, cudaMemcpyDeviceToHost, s));
-    int bad = 0;
-    gemm_status_fetch(&bad, s);
+    if (!n->fused) gemm_status_fetch(&got.bad, s);
     MLP_TRY(cudaStreamSynchronize(s));
-    if (bad && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
-    if (loss) *loss = l;
+    if (got.bad && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
+    if (loss) *loss = got.loss;
     return GELIOS_OK;
 }
 
@@ -1599,7 +1614,7 @@ extern "C" int gelios_mlp_train(gelios_mlp* n, int iters, int batch, float lr_ma
         n->drop_graph();
         n->steps_cap = 0;
         if (!n->args.alloc(static_cast<size_t>(cap) * sizeof(StepArgs)) ||
-            !n->hist.alloc(static_cast<size_t>(cap) * 4) || (!n->at.p && !n->at.alloc(sizeof(int))))
+            !n->hist.alloc(static_cast<size_t>(cap + 1) * 4) || (!n->at.p && !n->at.alloc(sizeof(int))))
             return cuda_fail(cudaErrorMemoryAllocation);
         n->steps_cap = cap;
     }
@@ -1636,17 +1651,25 @@ extern "C" int gelios_mlp_train(gelios_mlp* n, int iters, int batch, float lr_ma
             const StepArgs& a = args[it];
             adam_kernel<<<blocks(n->n_params, 256), 256, 0, s>>>(n->n_params, n->w32.as<float>(), n->g32.as<float>(),
                                                                  n->m.as<float>(), n->v.as<float>(), a.lr, b1, b2,
-                                                                 kAdamEps, a.c1, a.c2, n->wb.as<__nv_bfloat16>());
-            weight_copies_kernel<<<dim3(blocks(static_cast<int64_t>(n->din[0]) * n->dout[0], 256), 1), 256, 0, s>>>(
-                n->f_layers.as<LayerGrad>(), n->wb.as<__nv_bfloat16>());
+                                                                 kAdamEps, a.c1, a.c2, n->wb.as<__nv_bfloat16>(),
+                                                                 n->layers_host[0]);
         }
         MLP_TRY(cudaGetLastError());
     }
-    if (loss_hist && iters > 0)
-        MLP_TRY(cudaMemcpyAsync(loss_hist, n->hist.p, static_cast<size_t>(iters) * 4, cudaMemcpyDeviceToHost, s));
+    // the losses, and behind them the GEMM status word (grad_adam_kernel)
     int bad = 0;
-    gemm_status_fetch(&bad, s);
-    MLP_TRY(cudaStreamSynchronize(s));
+    if (n->fused && iters > 0) {
+        std::vector<float> got(static_cast<size_t>(iters) + 1);
+        MLP_TRY(cudaMemcpyAsync(got.data(), n->hist.p, got.size() * 4, cudaMemcpyDeviceToHost, s));
+        MLP_TRY(cudaStreamSynchronize(s));
+        if (loss_hist) std::memcpy(loss_hist, got.data(), static_cast<size_t>(iters) * 4);
+        std::memcpy(&bad, &got[iters], 4);
+    } else {
+        if (loss_hist && iters > 0)
+            MLP_TRY(cudaMemcpyAsync(loss_hist, n->hist.p, static_cast<size_t>(iters) * 4, cudaMemcpyDeviceToHost, s));
+        gemm_status_fetch(&bad, s);
+        MLP_TRY(cudaStreamSynchronize(s));
+    }
     if (bad && !gemm_status_ok()) return cuda_fail(cudaErrorLaunchTimeout);
     return GELIOS_OK;
 }
@@ -1658,6 +1681,7 @@ extern "C" int gelios_mlp_predict(gelios_mlp* n, const float* x, int64_t M, floa
     // The chunks pass through pinned staging, two at a time, once that is worth
     // it: a copy from or to pageable memory of this size goes through the
     // driver's own, in turn.
+    n->predictions++;
     n->io_bytes += M * (n->n_in + n->n_out) * 4;
     ensure_staging(n);
     const bool staged = n->stage != nullptr;

@@ -52,12 +52,14 @@ inline int64_t stage_rows(int max_batch, int n_in, int n_out) {
     if (r < 1024) r = 1024;
     return r < max_batch ? r : max_batch;
 }
-// Whether it is worth its cost once io_bytes of inputs and outputs have been
-// asked for over the life of the network.  Pinning 0.8 MB (8192 rows, 7 in, 5
-// out) takes 1.0-2.7 ms and 32 MB 18 ms; a call of 5400 rows (260 KB) then
-// takes 118 us instead of 155 through the driver's own staging, one of 86400
-// rows (4.1 MB) 1.13 ms instead of 1.6: 110-170 us a megabyte, so 20 times its
-// size pays for it.  A network that is asked to predict once never pins.
-inline bool staging_worth(int64_t io_bytes, int64_t staging_bytes) { return io_bytes >= 20 * staging_bytes; }
+// Whether it is worth its cost: `calls` predictions of io_bytes of inputs and
+// outputs in all over the life of the network.  Pinning 0.8 MB (8192 rows, 7
+// in, 5 out) takes 1.0-2.7 ms and 32 MB 18 ms.  A call of one row then takes 62
+// us instead of 71 through the driver's own staging, one of 5400 rows (260 KB)
+// 118 instead of 155, one of 86400 rows (4.1 MB) 1.13 ms instead of 1.6: 9 us a
+// call and 115 a megabyte.  A network that is asked to predict once never pins.
+inline bool staging_worth(int64_t calls, int64_t io_bytes, int64_t staging_bytes) {
+    return 9.0 * calls + 115e-6 * io_bytes >= 1500.0 + 550e-6 * staging_bytes;
+}
 
 }  // namespace gelios

@@ -368,8 +368,8 @@ void gelios_plain_batch_destroy(gelios_plain_batch *batch);
  * from 0 over `warmup` steps, then cosine from lr_max down to lr_min; the
  * batch loss of every step into loss_hist (iters floats, may be NULL).
  * gelios_mlp_predict: outputs of M host rows (in chunks of at most max_batch;
- * through pinned staging of the network's own once its calls have moved 20
- * times the staging's size).
+ * through pinned staging of the network's own once its calls have saved that
+ * allocation's cost).
  * gelios_mlp_gemm_bf16: the GEMM alone (device pointers; C = A . B^T with
  * A[m][k] at A[m lda + k], B[n][k] at B[n ldb + k], C fp32 rows of ldc;
  * stream may be NULL), for checks. */

@@ -19,9 +19,10 @@ int main() {
     int bad = 0;
     const int64_t staging = 2 * stage_rows(8192, 7, 5) * 12 * 4;
     // one prediction of any grid of the warm start does not pin
-    for (int64_t rows : {1LL, 5400LL, 86400LL, 200000LL}) bad += staging_worth(rows * 48, staging);
-    // a program that predicts a 5400-row grid again and again does
-    bad += staging_worth(40 * 5400LL * 48, staging) || !staging_worth(100 * 5400LL * 48, staging);
+    for (int64_t rows : {1LL, 5400LL, 86400LL, 200000LL}) bad += staging_worth(1, rows * 48, staging);
+    // a program that predicts again and again does
+    bad += staging_worth(30, 30 * 5400LL * 48, staging) || !staging_worth(100, 100 * 5400LL * 48, staging);
+    bad += staging_worth(100, 100 * 48, staging) || !staging_worth(300, 300 * 48, staging);
     // chunks: at most the largest batch and 16 MB, at least 1024 rows of wide networks
     bad += stage_rows(8192, 7, 5) != 8192 || stage_rows(1 << 20, 7, 5) * 12 > (4 << 20) || stage_rows(100, 4096, 4096) != 100 ||
            stage_rows(1 << 20, 4096, 4096) != 1024;
@@ -45,17 +46,17 @@ def test_rules(tmp_path):
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [1, 512, 513, 1500, 1537])
 def test_predictions_before_and_after_staging(rows):
-    """A network of 512-row chunks pins after 1 MB: one to three chunks through
-    the driver's staging, then through its own; the same bits."""
+    """One to three chunks of 512 rows through the driver's staging, then (a
+    prediction of 16 MB later) through its own; the same bits."""
     net = W.Mlp(7, 6, 64, 2, 5, 512)
     try:
         net.init_params(2)
         x = np.random.default_rng(rows).uniform(-1, 1, (rows, 7)).astype(np.float32)
         first = net.predict(x)
-        for _ in range(30 if rows > 1 else 3):
-            assert np.array_equal(net.predict(x), first)
-        net.predict(np.zeros((30000, 7), np.float32))
         assert np.array_equal(net.predict(x), first)
+        net.predict(np.zeros((350000, 7), np.float32))
+        for _ in range(3):
+            assert np.array_equal(net.predict(x), first)
         assert net.predict(x[:0]).shape == (0, 5)
     finally:
         net.close()
