@@ -2631,6 +2631,7 @@ struct gelios_plain_batch {
     DBuf inst, active, resid;
     std::vector<PlainInstance> host;  // what inst holds, rebuilt per call
     int prec = GELIOS_PREC_FP64;      // flux precision of every instance
+    int cluster_n = 0, cluster_size = 0;  // plain_cluster_size of the last number of active instances
     ~gelios_plain_batch() {
         if (stream) cudaStreamDestroy(stream);
     }
@@ -2753,7 +2754,11 @@ int plain_batch_prepare(gelios_plain_batch* B, const std::vector<int>& list) {
 cudaError_t plain_batch_steps(gelios_plain_batch* B, const std::vector<int>& list, int nsteps) {
     const DevMesh& d = B->ctxs[0]->d;
     const int n = static_cast<int>(list.size());
-    if (nsteps > 0 && plain_batch_serial(d, n, B->prec)) {
+    if (B->cluster_n != n) {  // three occupancy queries, 15 us each
+        B->cluster_size = plain_cluster_size(n, B->prec);
+        B->cluster_n = n;
+    }
+    if (nsteps > 0 && plain_batch_serial(d, n, B->cluster_size)) {
         cudaError_t e = cudaSuccess;
         for (int k = 0; k < n && e == cudaSuccess; k++) {
             const PlainInstance& I = B->host[list[k]];
@@ -2763,7 +2768,8 @@ cudaError_t plain_batch_steps(gelios_plain_batch* B, const std::vector<int>& lis
         if (e == cudaSuccess) return e;
         cudaGetLastError();  // no cooperative launch: the clusters
     }
-    return launch_stationary_batch(d, B->inst.as<PlainInstance>(), B->active.as<int>(), n, nsteps, B->prec, B->stream);
+    return launch_stationary_batch(d, B->inst.as<PlainInstance>(), B->active.as<int>(), n, nsteps, B->prec,
+                                   B->cluster_size, B->stream);
 }
 }  // namespace
 

@@ -4830,46 +4830,45 @@ static cudaError_t launch_stationary32_batch(const DevMesh& d, const PlainInstan
     void* args[] = {&dd, &ip, &ap, &na, &n};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(128), args, 0, s);
 }
-static const void* plain_cluster_fn(int prec) {
-    return prec == GELIOS_PREC_FP32_WAVES ? reinterpret_cast<const void*>(&stationary_cluster_kernel<WaveF32>)
-                                          : reinterpret_cast<const void*>(&stationary_cluster_kernel<double>);
-}
-// The launch of one cluster per instance, of the largest size at which every
-// instance is resident; more instances than that run in waves (they are
-// independent).  16 blocks need the non-portable size.
+// The launch of one cluster of `size` blocks per instance.  16 blocks need the
+// non-portable size.
 struct PlainClusters {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     const void* fn;
-    cudaError_t plan(int n, int prec) {
-        fn = plain_cluster_fn(prec);
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
+    PlainClusters(int n, int prec, int size) {
+        fn = prec == GELIOS_PREC_FP32_WAVES ? reinterpret_cast<const void*>(&stationary_cluster_kernel<WaveF32>)
+                                            : reinterpret_cast<const void*>(&stationary_cluster_kernel<double>);
+        cfg.gridDim = dim3(static_cast<unsigned>(n) * size);
         cfg.blockDim = dim3(kClusterThreads);
         at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = size;
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        for (int size = 16;; size /= 2) {
-            at.val.clusterDim.x = size;
-            cfg.gridDim = dim3(static_cast<unsigned>(n) * size);
-            int fit = 0;
-            e = cudaOccupancyMaxActiveClusters(&fit, fn, &cfg);
-            if (e != cudaSuccess) {  // a size the device does not offer
-                cudaGetLastError();
-                fit = 0;
-            }
-            if (fit >= n || size == 1) return cudaSuccess;
-        }
     }
+    PlainClusters(const PlainClusters&) = delete;
 };
+// More instances than are resident at size 1 run in waves (they are
+// independent).
+int plain_cluster_size(int n, int prec) {
+    if (n <= 0 || prec == GELIOS_PREC_FP32_FLUX) return 0;
+    for (int size = 16;; size /= 2) {
+        PlainClusters c(n, prec, size);
+        int fit = 0;
+        if (cudaFuncSetAttribute(c.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&fit, c.fn, &c.cfg) != cudaSuccess) {  // a size the device does not offer
+            cudaGetLastError();
+            fit = 0;
+        }
+        if (fit >= n || size == 1) return size;
+    }
+}
 cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst, const int* active, int n_active,
-                                    int nsteps, int prec, cudaStream_t s) {
+                                    int nsteps, int prec, int cluster_size, cudaStream_t s) {
     if (n_active <= 0 || nsteps <= 0) return cudaSuccess;
     if (prec == GELIOS_PREC_FP32_FLUX) return launch_stationary32_batch(d, inst, active, n_active, nsteps, s);
-    PlainClusters c;
-    const cudaError_t e = c.plan(n_active, prec);
-    if (e != cudaSuccess) return e;
+    PlainClusters c(n_active, prec, cluster_size);
     DevMesh dd = d;
     const PlainInstance* ip = inst;
     const int* ap = active;
@@ -4878,17 +4877,14 @@ cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst,
     c.cfg.stream = s;
     return cudaLaunchKernelExC(&c.cfg, c.fn, args);
 }
-bool plain_batch_serial(const DevMesh& d, int n, int prec) {
+bool plain_batch_serial(const DevMesh& d, int n, int cluster_size) {
     int dev = 0, sms = 0;
-    PlainClusters c;
-    if (n <= 0 || prec == GELIOS_PREC_FP32_FLUX || cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        c.plan(n, prec) != cudaSuccess) {
+    if (cluster_size <= 0 || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return plain_serial_faster(d.n_cells, n, plain_lane_threads(d, sms) > 0,
-                               static_cast<int>(c.at.val.clusterDim.x));
+    return plain_serial_faster(d.n_cells, n, plain_lane_threads(d, sms) > 0, cluster_size);
 }
 __global__ void plain_batch_words_init_kernel(const PlainInstance* inst, const int* active, int n) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

@@ -153,13 +153,16 @@ struct PlainInstance {
     StepBuffers b[2];
     double* fl;
 };
+// Blocks per cluster of a batch of n instances: the largest size at which
+// every instance is resident; 0 with FP32 fluxes (no clusters).
+int plain_cluster_size(int n, int prec);
 // Whether `n` instances of the mesh run one after the other on the whole chip
-// instead of a cluster each (plain_plan.cuh); not with FP32 fluxes.
-bool plain_batch_serial(const DevMesh& d, int n, int prec);
+// instead of a cluster each (plain_plan.cuh).
+bool plain_batch_serial(const DevMesh& d, int n, int cluster_size);
 // `nsteps` steps of the instances listed in `active` (device arrays) in one
 // launch; returns the launch's error code.
 cudaError_t launch_stationary_batch(const DevMesh& d, const PlainInstance* inst, const int* active, int n_active,
-                                    int nsteps, int prec, cudaStream_t s);
+                                    int nsteps, int prec, int cluster_size, cudaStream_t s);
 void launch_plain_batch_words_init(const PlainInstance* inst, const int* active, int n, cudaStream_t s);
 // Tiles of the moving-grid step, built at topology upload: spatially compact
 // groups of at most kTileCells cells.  Cells of tile t are
